@@ -671,95 +671,263 @@ __global__ void k_l_invert(const int* orig, int R, int* newpos) {
 
 // ---------------------------------------------------------------------------
 // Training kernels (FP32 accumulation; operands rounded to BF16 exactly where
-// the tensor-core inference rounds them: the layer inputs and the weights)
+// the tensor-core inference rounds them: the layer inputs and the weights).
+// An Adam step is two kernels:
+//   k_t_rows   everything that belongs to one batch row: both layers, the
+//              output and its error, and the errors of the hidden layers;
+//   k_t_wgrad  the sums over the batch, and Adam on the sums it made.
+// Every sum runs over its index in ascending order in one FP32 chain, so the
+// results do not depend on the tiling.
 // ---------------------------------------------------------------------------
 namespace vnm {
 
 __device__ __forceinline__ float bf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-// Y[b][o] = act(sum_i bf(X[b][i]) * bf(W[o][i]) + bias[o])
-__global__ void k_t_fwd(const float* X, const float* W, const float* bias, int B, int I, int O, int relu, float* Y) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)B * O;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(e / O), o = (int)(e % O);
-    float s = 0.f;
-    for (int i = 0; i < I; ++i) s += bf(X[(size_t)b * I + i]) * bf(W[(size_t)o * I + i]);
-    s += bias[o];
-    Y[e] = relu ? fmaxf(s, 0.f) : s;
-  }
+// What a step's rows leave for the sums over the batch, transposed so that a
+// unit's values of consecutive rows are contiguous; ld = the batch rounded up
+// to 8 rows, the rows past the batch zero.
+struct TrainActs {
+  __nv_bfloat16* X;   // [LF][ld] inputs
+  __nv_bfloat16* H1;  // [LH][ld] first hidden layer
+  __nv_bfloat16* H2;  // [LH][ld] second
+  float* dZ1;         // [LH][ld] dL / d(first layer before the ReLU)
+  float* dZ2;         // [LH][ld]
+  float* dy;          // [ld]
+  int ld;
+};
+
+// 8 rows a block, and per thread one unit of both hidden layers for 4 of the
+// rows.  Bound by shared-memory loads (a weight and a broadcast 16-byte
+// quadruple of activations for 4 FMAs) and by staging 80 KB of weights per
+// block; 8 rows put a 1024-row batch on 128 of the 152 SMs.  The weights'
+// rows are padded by one word: a warp reads them along units (forward) and
+// along inputs (backward) without bank conflicts.  One thread per output
+// over global memory, a launch per layer, took 0.26 ms at 1024 rows.
+constexpr int T_ROWS = 8;
+constexpr int T_THREADS = 2 * LH;
+struct TrainRowsSmem {
+  float W1[LH][LF + 1];
+  float W2[LH][LH + 1];
+  alignas(16) float x[LF][T_ROWS];
+  alignas(16) float h1[LH][T_ROWS];
+  alignas(16) float h2[LH][T_ROWS];
+  alignas(16) float d2[LH][T_ROWS];
+  float w3[LH];
+  float dy[T_ROWS];
+};
+
+__device__ __forceinline__ uint2 bf16x4(const float (&v)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// last layer (fp32 dot, as the inference epilogue does) and dL/dy of
-// L = mean((y - t)^2) / 2
-__global__ void k_t_out(const float* H2, const float* w3, const float* b3, const float* t, int B, float* y,
-                        float* dy, float* loss) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) {
-    float s = b3[0];
-    for (int o = 0; o < LH; ++o) s += bf(H2[(size_t)b * LH + o]) * w3[o];
-    y[b] = s;
-    const float d = s - t[b];
-    dy[b] = d / B;
-    atomicAdd(loss, 0.5f * d * d / B);
+__global__ void __launch_bounds__(T_THREADS) k_t_rows(const float* __restrict__ X, const float* __restrict__ t, int B,
+                                                      MlpW W, TrainActs A, float* loss) {
+  extern __shared__ __align__(16) unsigned char t_raw[];
+  TrainRowsSmem& sm = *reinterpret_cast<TrainRowsSmem*>(t_raw);
+  const int tid = threadIdx.x, u = tid % LH, r0 = (tid / LH) * 4;  // this thread's unit and first row
+  const int b0 = blockIdx.x * T_ROWS, live = min(T_ROWS, B - b0);
+  for (int e = tid; e < LH * LF; e += T_THREADS) sm.W1[e / LF][e % LF] = bf(W.W1[e]);
+#pragma unroll 16
+  for (int e = tid; e < LH * LH; e += T_THREADS) sm.W2[e / LH][e % LH] = bf(W.W2[e]);
+  if (tid < LH) sm.w3[tid] = W.w3[tid];
+  {
+    static_assert(LF * T_ROWS == T_THREADS, "one input value a thread");
+    const int r = tid / LF, k = tid % LF;
+    sm.x[k][r] = r < live ? bf(X[(size_t)(b0 + r) * LF + k]) : 0.f;
   }
+  const float b1 = W.b1[u], b2 = W.b2[u];
+  __syncthreads();
+  // sums of 4 rows over n inputs: s[r] = sum_k a[k][r0 + r] * w[k * step]
+  auto dot4 = [&](const float (*a)[T_ROWS], const float* w, int step, int n, float (&s)[4]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r] = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) {
+      const float wk = w[k * step];
+      const float4 v = *reinterpret_cast<const float4*>(&a[k][r0]);
+      s[0] = fmaf(v.x, wk, s[0]);
+      s[1] = fmaf(v.y, wk, s[1]);
+      s[2] = fmaf(v.z, wk, s[2]);
+      s[3] = fmaf(v.w, wk, s[3]);
+    }
+  };
+  const size_t at = (size_t)u * A.ld + b0 + r0;
+  auto layer = [&](const float (*a)[T_ROWS], const float* w, int n, float bias, float (*h)[T_ROWS],
+                   __nv_bfloat16* out, float (&z)[4]) {
+    dot4(a, w, 1, n, z);
+    float v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      z[r] = fmaxf(z[r] + bias, 0.f);
+      v[r] = bf(z[r]);
+      h[u][r0 + r] = v[r];
+      if (r0 + r >= live) v[r] = 0.f;
+    }
+    *reinterpret_cast<uint2*>(out + at) = bf16x4(v);
+  };
+  float z1[4], z2[4];
+  layer(sm.x, sm.W1[u], LF, b1, sm.h1, A.H1, z1);
+  __syncthreads();
+  layer(sm.h1, sm.W2[u], LH, b2, sm.h2, A.H2, z2);
+  if (tid < LF) {
+    float v[4], w[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      v[r] = sm.x[tid][r];
+      w[r] = sm.x[tid][4 + r];
+    }
+    const uint2 lo = bf16x4(v), hi = bf16x4(w);
+    *reinterpret_cast<uint4*>(A.X + (size_t)tid * A.ld + b0) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+  }
+  __syncthreads();
+  if (tid < T_ROWS) {  // the output, its error and the row's part of mean((y - t)^2) / 2
+    float s = W.b3[0];
+#pragma unroll 16
+    for (int o = 0; o < LH; ++o) s = fmaf(sm.h2[o][tid], sm.w3[o], s);
+    float dy = 0.f, l = 0.f;
+    if (tid < live) {
+      const float d = s - t[b0 + tid];
+      dy = d / B;
+      l = 0.5f * d * d / B;
+    }
+    sm.dy[tid] = dy;
+    A.dy[b0 + tid] = dy;
+#pragma unroll
+    for (int o = T_ROWS / 2; o > 0; o >>= 1) l += __shfl_xor_sync((1u << T_ROWS) - 1u, l, o);
+    if (tid == 0) atomicAdd(loss, l);
+  }
+  __syncthreads();
+  float d[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) d[r] = z2[r] > 0.f ? sm.dy[r0 + r] * sm.w3[u] : 0.f;
+  *reinterpret_cast<float4*>(&sm.d2[u][r0]) = make_float4(d[0], d[1], d[2], d[3]);
+  *reinterpret_cast<float4*>(A.dZ2 + at) = make_float4(d[0], d[1], d[2], d[3]);
+  __syncthreads();
+  dot4(sm.d2, &sm.W2[0][u], LH + 1, LH, d);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) d[r] = z1[r] > 0.f ? d[r] : 0.f;
+  *reinterpret_cast<float4*>(A.dZ1 + at) = make_float4(d[0], d[1], d[2], d[3]);
 }
 
-// dW[o][i] = sum_b dZ[b][o] * bf(A[b][i]);  db[o] = sum_b dZ[b][o]
-__global__ void k_t_wgrad(const float* dZ, const float* A, int B, int I, int O, float* dW, float* db) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)O * (I + 1);
-       e += (long long)gridDim.x * blockDim.x) {
-    const int o = (int)(e / (I + 1)), i = (int)(e % (I + 1));
-    float s = 0.f;
-    if (i < I) {
-      for (int b = 0; b < B; ++b) s += dZ[(size_t)b * O + o] * bf(A[(size_t)b * I + i]);
-      dW[(size_t)o * I + i] = s;
+struct AdamArgs {
+  float *p, *m, *v;  // parameters and moments
+  float lr, b1, b2, eps, c1, c2;
+};
+
+// dW[o][i] = sum_b dZ[o][b] * bf(A[i][b]), db[o] = sum_b dZ[o][b]: one sum a
+// thread, 16 x 8 of a layer's a block (the last layer: one row of 8), and one
+// warp for the biases beside the first 8 inputs.  kAdam: the step of Adam on
+// each sum instead of writing it to g.
+// Bound by the chain of B dependent FMAs (4 cycles each: 2 us at B = 1024),
+// so the tiles are as small as puts all 20865 sums on the chip at once (176
+// blocks), the rows come 8 to a 16-byte (activations) or two 16-byte loads,
+// and the copies of T_STAGES chunks of T_CB rows are in flight together.
+constexpr int T_TO = 16, T_TI = 8;    // units x inputs a block
+constexpr int T_CB = 256;             // rows of the batch a chunk
+constexpr int T_STAGES = 4;
+constexpr int T_W_THREADS = T_TO * T_TI + 32;
+struct TrainWgradSmem {  // rows padded by 16 bytes: 8 rows' 16-byte pieces in different banks
+  float dz[T_STAGES][T_TO][T_CB + 4];
+  __nv_bfloat16 a[T_STAGES][T_TI][T_CB + 8];
+};
+constexpr int T_W2_TILES = (LH / T_TO) * (LH / T_TI), T_W1_TILES = (LH / T_TO) * (LF / T_TI), T_W3_TILES = LH / T_TI;
+constexpr int T_WGRAD_GRID = T_W2_TILES + T_W1_TILES + T_W3_TILES;
+
+constexpr int L_OFF_W1 = 0;  // the parameter vector: W1 [LH][LF], b1 [LH], W2 [LH][LH], b2 [LH], w3 [LH], b3 [1]
+constexpr int L_OFF_B1 = L_OFF_W1 + LH * LF;
+constexpr int L_OFF_W2 = L_OFF_B1 + LH;
+constexpr int L_OFF_B2 = L_OFF_W2 + LH * LH;
+constexpr int L_OFF_W3 = L_OFF_B2 + LH;
+constexpr int L_OFF_B3 = L_OFF_W3 + LH;
+constexpr int L_NPARAM = L_OFF_B3 + 1;
+
+template <bool kAdam>
+__global__ void __launch_bounds__(T_W_THREADS) k_t_wgrad(TrainActs A, float* g, AdamArgs ad) {
+  extern __shared__ __align__(16) unsigned char t_raw[];
+  TrainWgradSmem& sm = *reinterpret_cast<TrainWgradSmem*>(t_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // this block's tile: units o0 .. o0 + no - 1 of dz, inputs i0 .. i0 + 7 of a
+  int tile = blockIdx.x, I, offw, offb, no = T_TO;
+  const float* dz;
+  const __nv_bfloat16* a;
+  if (tile < T_W2_TILES) {
+    I = LH, offw = L_OFF_W2, offb = L_OFF_B2, dz = A.dZ2, a = A.H1;
+  } else if (tile < T_W2_TILES + T_W1_TILES) {
+    tile -= T_W2_TILES;
+    I = LF, offw = L_OFF_W1, offb = L_OFF_B1, dz = A.dZ1, a = A.X;
+  } else {
+    tile -= T_W2_TILES + T_W1_TILES;
+    I = LH, offw = L_OFF_W3, offb = L_OFF_B3, dz = A.dy, a = A.H2, no = 1;
+  }
+  const int i0 = tile % (I / T_TI) * T_TI, o0 = tile / (I / T_TI) * T_TO;
+  const int nchunk = (A.ld + T_CB - 1) / T_CB;
+  auto load = [&](int c) {  // chunk c's rows, zeros past ld
+    if (c < nchunk) {
+      const int s = c % T_STAGES, b0 = c * T_CB;
+      for (int e = tid; e < no * (T_CB / 4); e += T_W_THREADS) {
+        const int o = e / (T_CB / 4), b = e % (T_CB / 4) * 4;
+        const bool in = b0 + b < A.ld;
+        ptx::cp_async16_zfill(&sm.dz[s][o][b], dz + (in ? (size_t)(o0 + o) * A.ld + b0 + b : 0), in ? 16u : 0u);
+      }
+      for (int e = tid; e < T_TI * (T_CB / 8); e += T_W_THREADS) {
+        const int i = e / (T_CB / 8), b = e % (T_CB / 8) * 8;
+        const bool in = b0 + b < A.ld;
+        ptx::cp_async16_zfill(&sm.a[s][i][b], a + (in ? (size_t)(i0 + i) * A.ld + b0 + b : 0), in ? 16u : 0u);
+      }
+    }
+    ptx::cp_async_commit();
+  };
+  for (int c = 0; c < T_STAGES - 1; ++c) load(c);
+  // threads 0 .. 127: unit 4 warp + lane / 8, input lane % 8; the last warp: the bias of unit `lane`
+  const bool bias = warp == T_TO * T_TI / 32;
+  const int o = bias ? lane : 4 * warp + (lane >> 3), i = lane & 7;
+  const bool on = o < no && (!bias || i0 == 0);
+  float s = 0.f;
+  for (int c = 0; c < nchunk; ++c) {
+    ptx::cp_async_wait<T_STAGES - 2>();
+    __syncthreads();  // chunk c has landed, and nobody reads the stage that the next copy overwrites
+    load(c + T_STAGES - 1);
+    if (!on) continue;
+    const int n = min(T_CB, A.ld - c * T_CB);  // a multiple of 8
+    const float4* zr = reinterpret_cast<const float4*>(sm.dz[c % T_STAGES][o]);
+    const uint4* ar = reinterpret_cast<const uint4*>(sm.a[c % T_STAGES][i]);
+    if (bias) {
+#pragma unroll 4
+      for (int b = 0; b < n / 4; ++b) {
+        const float4 z = zr[b];
+        s += z.x;
+        s += z.y;
+        s += z.z;
+        s += z.w;
+      }
     } else {
-      for (int b = 0; b < B; ++b) s += dZ[(size_t)b * O + o];
-      db[o] = s;
+#pragma unroll 4
+      for (int b = 0; b < n / 8; ++b) {
+        const float4 z0 = zr[2 * b], z1 = zr[2 * b + 1];
+        const uint4 v = ar[b];
+        s = fmaf(z0.x, __uint_as_float(v.x << 16), s);
+        s = fmaf(z0.y, __uint_as_float(v.x & 0xffff0000u), s);
+        s = fmaf(z0.z, __uint_as_float(v.y << 16), s);
+        s = fmaf(z0.w, __uint_as_float(v.y & 0xffff0000u), s);
+        s = fmaf(z1.x, __uint_as_float(v.z << 16), s);
+        s = fmaf(z1.y, __uint_as_float(v.z & 0xffff0000u), s);
+        s = fmaf(z1.z, __uint_as_float(v.w << 16), s);
+        s = fmaf(z1.w, __uint_as_float(v.w & 0xffff0000u), s);
+      }
     }
   }
-}
-
-// dA[b][i] = (sum_o dZ[b][o] * bf(W[o][i])) * [A[b][i] > 0]
-__global__ void k_t_dgrad(const float* dZ, const float* W, const float* A, int B, int I, int O, float* dA) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)B * I;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(e / I), i = (int)(e % I);
-    float s = 0.f;
-    for (int o = 0; o < O; ++o) s += dZ[(size_t)b * O + o] * bf(W[(size_t)o * I + i]);
-    dA[e] = A[e] > 0.f ? s : 0.f;
+  if (!on) return;
+  const int e = bias ? offb + o0 + o : offw + (o0 + o) * I + i0 + i;
+  if (!kAdam) {
+    g[e] = s;
+    return;
   }
-}
-
-// gradient of the last layer: dw3[o] = sum_b dy[b] * bf(H2[b][o]), db3;
-// dH2[b][o] = dy[b] * w3[o] * [H2 > 0]
-__global__ void k_t_out_grad(const float* dy, const float* H2, const float* w3, int B, float* dw3, float* db3,
-                             float* dH2) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)B * LH + LH + 1;
-       e += (long long)gridDim.x * blockDim.x) {
-    if (e < (long long)B * LH) {
-      const int b = (int)(e / LH), o = (int)(e % LH);
-      dH2[e] = H2[e] > 0.f ? dy[b] * w3[o] : 0.f;
-    } else if (e < (long long)B * LH + LH) {
-      const int o = (int)(e - (long long)B * LH);
-      float s = 0.f;
-      for (int b = 0; b < B; ++b) s += dy[b] * bf(H2[(size_t)b * LH + o]);
-      dw3[o] = s;
-    } else {
-      float s = 0.f;
-      for (int b = 0; b < B; ++b) s += dy[b];
-      db3[0] = s;
-    }
-  }
-}
-
-__global__ void k_t_adam(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
-                         float c1, float c2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    m[i] = b1 * m[i] + (1.f - b1) * gi;
-    v[i] = b2 * v[i] + (1.f - b2) * gi * gi;
-    p[i] -= lr * (m[i] / c1) / (sqrtf(v[i] / c2) + eps);
-  }
+  const float m = ad.b1 * ad.m[e] + (1.f - ad.b1) * s;
+  const float v = ad.b2 * ad.v[e] + (1.f - ad.b2) * s * s;
+  ad.m[e] = m;
+  ad.v[e] = v;
+  ad.p[e] -= ad.lr * (m / ad.c1) / (sqrtf(v / ad.c2) + ad.eps);
 }
 
 }  // namespace vnm
@@ -767,14 +935,7 @@ __global__ void k_t_adam(float* p, const float* g, float* m, float* v, int n, fl
 // ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
-// parameter vector layout: W1 [LH][LF], b1 [LH], W2 [LH][LH], b2 [LH], w3 [LH], b3 [1]
-constexpr int L_OFF_W1 = 0;
-constexpr int L_OFF_B1 = L_OFF_W1 + vnm::LH * vnm::LF;
-constexpr int L_OFF_W2 = L_OFF_B1 + vnm::LH;
-constexpr int L_OFF_B2 = L_OFF_W2 + vnm::LH * vnm::LH;
-constexpr int L_OFF_W3 = L_OFF_B2 + vnm::LH;
-constexpr int L_OFF_B3 = L_OFF_W3 + vnm::LH;
-constexpr int L_NPARAM = L_OFF_B3 + 1;
+using namespace vnm;
 
 struct vnm_mlp {
   int device = 0;
@@ -800,26 +961,41 @@ static MlpW mlp_view(const vnm_mlp* n) {
 
 static size_t mlp_smem() { return sizeof(MlpSmem) + 1024; }
 
-// forward + backward of one batch (device X [B][LF], t [B]); gradients land in n->g
-static vnm_status mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t, int B, float* d_loss) {
-  float* H1 = arena_take<float>(ctx, (size_t)B * LH);
-  float* H2 = arena_take<float>(ctx, (size_t)B * LH);
-  float* y = arena_take<float>(ctx, B);
-  float* dy = arena_take<float>(ctx, B);
-  float* dH2 = arena_take<float>(ctx, (size_t)B * LH);
-  float* dH1 = arena_take<float>(ctx, (size_t)B * LH);
-  if (!H1 || !H2 || !y || !dy || !dH2 || !dH1) return VNM_ERR_NOMEM;
-  const int G = ctx->num_sms * 8;
-  float* p = n->p;
-  float* g = n->g;
-  VNM_LAUNCH(ctx, k_t_fwd, G, 256, 0, X, p + L_OFF_W1, p + L_OFF_B1, B, LF, LH, 1, H1);
-  VNM_LAUNCH(ctx, k_t_fwd, G, 256, 0, H1, p + L_OFF_W2, p + L_OFF_B2, B, LH, LH, 1, H2);
-  VNM_CUDA_TRY(cudaMemsetAsync(d_loss, 0, sizeof(float), ctx->stream));
-  VNM_LAUNCH(ctx, k_t_out, G, 256, 0, H2, p + L_OFF_W3, p + L_OFF_B3, t, B, y, dy, d_loss);
-  VNM_LAUNCH(ctx, k_t_out_grad, G, 256, 0, dy, H2, p + L_OFF_W3, B, g + L_OFF_W3, g + L_OFF_B3, dH2);
-  VNM_LAUNCH(ctx, k_t_wgrad, G, 256, 0, dH2, H1, B, LH, LH, g + L_OFF_W2, g + L_OFF_B2);
-  VNM_LAUNCH(ctx, k_t_dgrad, G, 256, 0, dH2, p + L_OFF_W2, H1, B, LH, LH, dH1);
-  VNM_LAUNCH(ctx, k_t_wgrad, G, 256, 0, dH1, X, B, LF, LH, g + L_OFF_W1, g + L_OFF_B1);
+// Arena bytes and storage of a step's activations (batches of B rows).
+static int train_ld(int B) { return (B + T_ROWS - 1) / T_ROWS * T_ROWS; }
+static size_t train_bytes(int B) {
+  const size_t ld = (size_t)train_ld(B);
+  return arena_bytes(ld * LF, 2) + 2 * arena_bytes(ld * LH, 2) + 2 * arena_bytes(ld * LH, 4) + arena_bytes(ld, 4);
+}
+static vnm_status train_acts(vnm_ctx* ctx, int B, TrainActs& A) {
+  A.ld = train_ld(B);
+  const size_t ld = (size_t)A.ld;
+  A.X = arena_take<__nv_bfloat16>(ctx, ld * LF);
+  A.H1 = arena_take<__nv_bfloat16>(ctx, ld * LH);
+  A.H2 = arena_take<__nv_bfloat16>(ctx, ld * LH);
+  A.dZ1 = arena_take<float>(ctx, ld * LH);
+  A.dZ2 = arena_take<float>(ctx, ld * LH);
+  A.dy = arena_take<float>(ctx, ld);
+  if (!A.X || !A.H1 || !A.H2 || !A.dZ1 || !A.dZ2 || !A.dy) return VNM_ERR_NOMEM;
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(TrainRowsSmem)));
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_wgrad<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(TrainWgradSmem)));
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_wgrad<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(TrainWgradSmem)));
+  return VNM_OK;
+}
+
+// Forward and backward of one batch (device X [B][LF], t [B]): the batch's
+// loss is added to *d_loss (zeroed by the caller), and the gradient goes to
+// n->g or, with `adam`, straight into a step of Adam.
+static vnm_status mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t, int B, const TrainActs& A,
+                           float* d_loss, const AdamArgs* adam) {
+  VNM_LAUNCH(ctx, k_t_rows, A.ld / T_ROWS, T_THREADS, sizeof(TrainRowsSmem), X, t, B, mlp_view(n), A, d_loss);
+  if (adam)
+    VNM_LAUNCH(ctx, k_t_wgrad<true>, T_WGRAD_GRID, T_W_THREADS, sizeof(TrainWgradSmem), A, n->g, *adam);
+  else
+    VNM_LAUNCH(ctx, k_t_wgrad<false>, T_WGRAD_GRID, T_W_THREADS, sizeof(TrainWgradSmem), A, n->g, AdamArgs{});
   return VNM_OK;
 }
 
@@ -889,8 +1065,7 @@ vnm_status vnm_mlp_set(vnm_mlp* n, const float* params) {
 vnm_status vnm_mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t, int B, float* grads,
                         float* loss) {
   if (!ctx || !n || !X || !t || B <= 0 || !grads || !loss) return VNM_ERR_ARG;
-  VNM_TRY(arena_reserve(ctx, arena_bytes((size_t)B * LF, 4) + arena_bytes(B, 4) * 3 +
-                                 4 * arena_bytes((size_t)B * LH, 4) + 4096));
+  VNM_TRY(arena_reserve(ctx, arena_bytes((size_t)B * LF, 4) + arena_bytes(B, 4) + train_bytes(B) + 4096));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
   const float *dX, *dt;
@@ -898,7 +1073,10 @@ vnm_status vnm_mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t
   VNM_TRY(stage_in(ctx, t, (size_t)B, VNM_MEM_HOST, &dt));
   float* dl = arena_take<float>(ctx, 1);
   if (!dl) return VNM_ERR_NOMEM;
-  VNM_TRY(mlp_grad(ctx, n, dX, dt, B, dl));
+  TrainActs A;
+  VNM_TRY(train_acts(ctx, B, A));
+  VNM_CUDA_TRY(cudaMemsetAsync(dl, 0, sizeof(float), ctx->stream));
+  VNM_TRY(mlp_grad(ctx, n, dX, dt, B, A, dl, nullptr));
   VNM_CUDA_TRY(cudaMemcpyAsync(grads, n->g, sizeof(float) * L_NPARAM, cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(loss, dl, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   return end_call(ctx);
@@ -911,8 +1089,8 @@ vnm_status vnm_mlp_train(vnm_ctx* ctx, vnm_mlp* net, const float* X, const float
   if (!ctx || !net || !X || !t || n <= 0 || B <= 0 || epochs <= 0) return VNM_ERR_ARG;
   const int nb = n / B;
   if (nb == 0) return VNM_ERR_ARG;
-  VNM_TRY(arena_reserve(ctx, arena_bytes((size_t)n * LF, 4) + arena_bytes(n, 4) + arena_bytes(B, 4) * 3 +
-                                 4 * arena_bytes((size_t)B * LH, 4) + arena_bytes(nb + 1, 4) + 8192));
+  VNM_TRY(arena_reserve(ctx, arena_bytes((size_t)n * LF, 4) + arena_bytes(n, 4) + train_bytes(B) +
+                                 arena_bytes(nb + 1, 4) + 8192));
   VNM_TRY(pinned_reserve(ctx, 64 + nb));
   VNM_TRY(begin_call(ctx));
   const float *dX, *dt;
@@ -920,15 +1098,16 @@ vnm_status vnm_mlp_train(vnm_ctx* ctx, vnm_mlp* net, const float* X, const float
   VNM_TRY(stage_in(ctx, t, (size_t)n, VNM_MEM_HOST, &dt));
   float* losses = arena_take<float>(ctx, nb + 1);
   if (!losses) return VNM_ERR_NOMEM;
-  const size_t mark = ctx->arena.used;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  TrainActs A;
+  VNM_TRY(train_acts(ctx, B, A));
+  AdamArgs ad{net->p, net->m, net->v, lr, 0.9f, 0.999f, 1e-8f, 0.f, 0.f};
   for (int e = 0; e < epochs; ++e) {
+    VNM_CUDA_TRY(cudaMemsetAsync(losses, 0, sizeof(float) * nb, ctx->stream));
     for (int k = 0; k < nb; ++k) {
-      ctx->arena.used = mark;
-      VNM_TRY(mlp_grad(ctx, net, dX + (size_t)k * B * LF, dt + (size_t)k * B, B, losses + k));
       net->steps++;
-      const float c1 = 1.f - powf(b1, (float)net->steps), c2 = 1.f - powf(b2, (float)net->steps);
-      VNM_LAUNCH(ctx, k_t_adam, 64, 256, 0, net->p, net->g, net->m, net->v, L_NPARAM, lr, b1, b2, eps, c1, c2);
+      ad.c1 = 1.f - powf(ad.b1, (float)net->steps);
+      ad.c2 = 1.f - powf(ad.b2, (float)net->steps);
+      VNM_TRY(mlp_grad(ctx, net, dX + (size_t)k * B * LF, dt + (size_t)k * B, B, A, losses + k, &ad));
     }
   }
   VNM_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, losses, sizeof(float) * nb, cudaMemcpyDeviceToHost, ctx->stream));

@@ -100,6 +100,18 @@ __device__ __forceinline__ void cp_async16_zfill_hint(void* dst, const void* src
                : "memory");
 }
 
+// The same without a policy, and the thread's groups of copies: commit ends
+// a group, wait<N> waits until at most the N newest groups are in flight.
+__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, uint32_t src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(src_bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Arrive on `bar` once this thread's earlier cp.async copies have landed;
 // the arrival counts toward the barrier's expected count (.noinc).
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
