@@ -29,6 +29,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -677,119 +678,195 @@ __global__ void k_l_invert(const int* orig, int R, int* newpos) {
 //              output and its error, and the errors of the hidden layers;
 //   k_t_wgrad  the sums over the batch, and Adam on the sums it made.
 // Every sum runs over its index in ascending order in one FP32 chain, so the
-// results do not depend on the tiling.
+// results do not depend on the tiling.  At 1024 rows a step takes 18 us (one
+// thread per output over global memory, nine launches: 0.5 ms).
 // ---------------------------------------------------------------------------
 namespace vnm {
 
 __device__ __forceinline__ float bf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// The hidden layers' weights rounded to BF16, rows padded by 16 bytes: a warp
+// reads 8 rows' 16-byte pieces, or 32 consecutive words, without bank
+// conflicts.  Kept in global memory in the form that k_t_rows copies to
+// shared memory (made by k_t_round, kept up by Adam).
+struct TrainW {
+  float W1[LH][LF + 4];
+  float W2[LH][LH + 4];
+};
+
 // What a step's rows leave for the sums over the batch, transposed so that a
 // unit's values of consecutive rows are contiguous; ld = the batch rounded up
-// to 8 rows, the rows past the batch zero.
+// to 16 rows, the rows past the batch zero.
 struct TrainActs {
-  __nv_bfloat16* X;   // [LF][ld] inputs
-  __nv_bfloat16* H1;  // [LH][ld] first hidden layer
-  __nv_bfloat16* H2;  // [LH][ld] second
-  float* dZ1;         // [LH][ld] dL / d(first layer before the ReLU)
-  float* dZ2;         // [LH][ld]
-  float* dy;          // [ld]
+  float* X;    // [LF][ld] inputs, rounded to BF16 like the layers
+  float* H1;   // [LH][ld] first hidden layer
+  float* H2;   // [LH][ld] second
+  float* dZ1;  // [LH][ld] dL / d(first layer before the ReLU)
+  float* dZ2;  // [LH][ld]
+  float* dy;   // [ld]
+  TrainW* W;
   int ld;
 };
 
-// 8 rows a block, and per thread one unit of both hidden layers for 4 of the
-// rows.  Bound by shared-memory loads (a weight and a broadcast 16-byte
-// quadruple of activations for 4 FMAs) and by staging 80 KB of weights per
-// block; 8 rows put a 1024-row batch on 128 of the 152 SMs.  The weights'
-// rows are padded by one word: a warp reads them along units (forward) and
-// along inputs (backward) without bank conflicts.  One thread per output
-// over global memory, a launch per layer, took 0.26 ms at 1024 rows.
-constexpr int T_ROWS = 8;
-constexpr int T_THREADS = 2 * LH;
+__global__ void k_t_round(const float* W1, const float* W2, TrainW* W) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < LH * (LF + 4 + LH + 4); e += gridDim.x * blockDim.x) {
+    if (e < LH * (LF + 4)) {
+      const int o = e / (LF + 4), i = e % (LF + 4);
+      W->W1[o][i] = i < LF ? bf(W1[o * LF + i]) : 0.f;
+    } else {
+      const int o = (e - LH * (LF + 4)) / (LH + 4), i = (e - LH * (LF + 4)) % (LH + 4);
+      W->W2[o][i] = i < LH ? bf(W2[o * LH + i]) : 0.f;
+    }
+  }
+}
+
+// 8 rows a block (a 1024-row batch on 128 of the 152 SMs); a thread has 2
+// units of both hidden layers for 4 of the rows.  Bound by the words read
+// from shared memory, a 4-byte word a lane costing the SM a cycle whether or
+// not lanes share it: 6 words for 8 FMAs on each of 4 warps.  The 128-deep layer forward
+// takes 3.5 K cycles; one unit a thread on 8 warps (5 words for 4 FMAs) took
+// 7.5 K, 4 units on 2 warps, bound by their issue rate, 4.4 K.
+constexpr int T_ROWS = 8, T_U = 2, T_US = LH / T_U;  // a thread's units are T_US apart
+constexpr int T_THREADS = T_US * (T_ROWS / 4);
 struct TrainRowsSmem {
-  float W1[LH][LF + 1];
-  float W2[LH][LH + 1];
+  TrainW W;
   alignas(16) float x[LF][T_ROWS];
   alignas(16) float h1[LH][T_ROWS];
   alignas(16) float h2[LH][T_ROWS];
   alignas(16) float d2[LH][T_ROWS];
-  float w3[LH];
+  alignas(16) float w3[LH];
   float dy[T_ROWS];
 };
 
-__device__ __forceinline__ uint2 bf16x4(const float (&v)[4]) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+// s[j][r] = sum_k a[k][r] * w_j[k] for T_U units j and 4 rows r, k ascending in
+// one chain each, two rows to a packed FMA (two round-to-nearest FMAs).
+// kByRow: unit j's weights are a row of W (w[j * T_US * pitch + k]), else a
+// column (w[k * pitch + j * T_US]).  Four k's operands are loaded while the
+// four before them are summed.
+template <int N, int PITCH, bool kByRow>
+__device__ __forceinline__ void dot_rows(const float* a, const float* w, float (&s)[T_U][4]) {
+  unsigned long long s01[T_U], s23[T_U];
+#pragma unroll
+  for (int j = 0; j < T_U; ++j) s01[j] = s23[j] = 0ull;
+  float wk[2][T_U][4];
+  ulonglong2 v[2][4];
+  auto fetch = [&](int k0, int h) {
+#pragma unroll
+    for (int j = 0; j < T_U; ++j) {
+      if (kByRow) {
+        const float4 q = *reinterpret_cast<const float4*>(w + j * T_US * PITCH + k0);
+        wk[h][j][0] = q.x;
+        wk[h][j][1] = q.y;
+        wk[h][j][2] = q.z;
+        wk[h][j][3] = q.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) wk[h][j][k] = w[(k0 + k) * PITCH + j * T_US];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[h][k] = *reinterpret_cast<const ulonglong2*>(a + (k0 + k) * T_ROWS);
+  };
+  auto add = [&](int h) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int j = 0; j < T_U; ++j) {
+        unsigned long long ww;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "r"(__float_as_uint(wk[h][j][k])));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s01[j]) : "l"(v[h][k].x), "l"(ww));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s23[j]) : "l"(v[h][k].y), "l"(ww));
+      }
+  };
+  fetch(0, 0);
+#pragma unroll 1
+  for (int k0 = 0; k0 < N; k0 += 8) {
+    fetch(k0 + 4, 1);
+    add(0);
+    if (k0 + 8 < N) fetch(k0 + 8, 0);
+    add(1);
+  }
+#pragma unroll
+  for (int j = 0; j < T_U; ++j) {
+    s[j][0] = __uint_as_float((uint32_t)s01[j]);
+    s[j][1] = __uint_as_float((uint32_t)(s01[j] >> 32));
+    s[j][2] = __uint_as_float((uint32_t)s23[j]);
+    s[j][3] = __uint_as_float((uint32_t)(s23[j] >> 32));
+  }
 }
 
 __global__ void __launch_bounds__(T_THREADS) k_t_rows(const float* __restrict__ X, const float* __restrict__ t, int B,
                                                       MlpW W, TrainActs A, float* loss) {
   extern __shared__ __align__(16) unsigned char t_raw[];
   TrainRowsSmem& sm = *reinterpret_cast<TrainRowsSmem*>(t_raw);
-  const int tid = threadIdx.x, u = tid % LH, r0 = (tid / LH) * 4;  // this thread's unit and first row
+  const int tid = threadIdx.x, u0 = tid % T_US, r0 = (tid / T_US) * 4;  // this thread's first unit and first row
   const int b0 = blockIdx.x * T_ROWS, live = min(T_ROWS, B - b0);
-  for (int e = tid; e < LH * LF; e += T_THREADS) sm.W1[e / LF][e % LF] = bf(W.W1[e]);
-#pragma unroll 16
-  for (int e = tid; e < LH * LH; e += T_THREADS) sm.W2[e / LH][e % LH] = bf(W.W2[e]);
-  if (tid < LH) sm.w3[tid] = W.w3[tid];
-  {
-    static_assert(LF * T_ROWS == T_THREADS, "one input value a thread");
-    const int r = tid / LF, k = tid % LF;
+  ptx::grid_dependents_launch();
+  ptx::grid_dependency_wait();  // the weights and the activations are the step before's
+  for (int e = tid; e < (int)sizeof(TrainW) / 16; e += T_THREADS)
+    ptx::cp_async16_zfill(t_raw + e * 16, reinterpret_cast<const unsigned char*>(A.W) + e * 16, 16u);
+  ptx::cp_async_commit();
+  float b1[T_U], b2[T_U], w3[T_U];
+#pragma unroll
+  for (int j = 0; j < T_U; ++j) {
+    b1[j] = W.b1[u0 + T_US * j];
+    b2[j] = W.b2[u0 + T_US * j];
+    w3[j] = W.w3[u0 + T_US * j];
+    if (r0 == 0) sm.w3[u0 + T_US * j] = w3[j];
+  }
+  const float b3 = W.b3[0];
+  const float target = tid < live ? t[b0 + tid] : 0.f;
+  for (int e = tid; e < LF * T_ROWS; e += T_THREADS) {
+    const int r = e / LF, k = e % LF;
     sm.x[k][r] = r < live ? bf(X[(size_t)(b0 + r) * LF + k]) : 0.f;
   }
-  const float b1 = W.b1[u], b2 = W.b2[u];
+  ptx::cp_async_wait<0>();
   __syncthreads();
-  // sums of 4 rows over n inputs: s[r] = sum_k a[k][r0 + r] * w[k * step]
-  auto dot4 = [&](const float (*a)[T_ROWS], const float* w, int step, int n, float (&s)[4]) {
+  // one layer's activations: kept in z, rounded in h, out to the batch's arrays
+  auto finish = [&](float (&z)[T_U][4], const float (&bias)[T_U], float (*h)[T_ROWS], float* out) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) s[r] = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < n; ++k) {
-      const float wk = w[k * step];
-      const float4 v = *reinterpret_cast<const float4*>(&a[k][r0]);
-      s[0] = fmaf(v.x, wk, s[0]);
-      s[1] = fmaf(v.y, wk, s[1]);
-      s[2] = fmaf(v.z, wk, s[2]);
-      s[3] = fmaf(v.w, wk, s[3]);
+    for (int j = 0; j < T_U; ++j) {
+      float v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        z[j][r] = fmaxf(z[j][r] + bias[j], 0.f);
+        v[r] = bf(z[j][r]);
+      }
+      *reinterpret_cast<float4*>(&h[u0 + T_US * j][r0]) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r0 + r >= live) v[r] = 0.f;
+      *reinterpret_cast<float4*>(out + (size_t)(u0 + T_US * j) * A.ld + b0 + r0) = make_float4(v[0], v[1], v[2], v[3]);
     }
   };
-  const size_t at = (size_t)u * A.ld + b0 + r0;
-  auto layer = [&](const float (*a)[T_ROWS], const float* w, int n, float bias, float (*h)[T_ROWS],
-                   __nv_bfloat16* out, float (&z)[4]) {
-    dot4(a, w, 1, n, z);
-    float v[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      z[r] = fmaxf(z[r] + bias, 0.f);
-      v[r] = bf(z[r]);
-      h[u][r0 + r] = v[r];
-      if (r0 + r >= live) v[r] = 0.f;
-    }
-    *reinterpret_cast<uint2*>(out + at) = bf16x4(v);
-  };
-  float z1[4], z2[4];
-  layer(sm.x, sm.W1[u], LF, b1, sm.h1, A.H1, z1);
+  float z1[T_U][4], z2[T_U][4], d[T_U][4];
+  dot_rows<LF, LF + 4, true>(&sm.x[0][r0], sm.W.W1[u0], z1);
+  finish(z1, b1, sm.h1, A.H1);
   __syncthreads();
-  layer(sm.h1, sm.W2[u], LH, b2, sm.h2, A.H2, z2);
-  if (tid < LF) {
-    float v[4], w[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      v[r] = sm.x[tid][r];
-      w[r] = sm.x[tid][4 + r];
-    }
-    const uint2 lo = bf16x4(v), hi = bf16x4(w);
-    *reinterpret_cast<uint4*>(A.X + (size_t)tid * A.ld + b0) = make_uint4(lo.x, lo.y, hi.x, hi.y);
-  }
+  dot_rows<LH, LH + 4, true>(&sm.h1[0][r0], sm.W.W2[u0], z2);
+  finish(z2, b2, sm.h2, A.H2);
+  if (u0 < LF)
+    *reinterpret_cast<float4*>(A.X + (size_t)u0 * A.ld + b0 + r0) = *reinterpret_cast<const float4*>(&sm.x[u0][r0]);
   __syncthreads();
   if (tid < T_ROWS) {  // the output, its error and the row's part of mean((y - t)^2) / 2
-    float s = W.b3[0];
-#pragma unroll 16
-    for (int o = 0; o < LH; ++o) s = fmaf(sm.h2[o][tid], sm.w3[o], s);
+    float s = b3;
+#pragma unroll 4
+    for (int o = 0; o < LH; o += 8) {
+      const float4 wa = *reinterpret_cast<const float4*>(&sm.w3[o]), wb = *reinterpret_cast<const float4*>(&sm.w3[o + 4]);
+      s = fmaf(sm.h2[o][tid], wa.x, s);
+      s = fmaf(sm.h2[o + 1][tid], wa.y, s);
+      s = fmaf(sm.h2[o + 2][tid], wa.z, s);
+      s = fmaf(sm.h2[o + 3][tid], wa.w, s);
+      s = fmaf(sm.h2[o + 4][tid], wb.x, s);
+      s = fmaf(sm.h2[o + 5][tid], wb.y, s);
+      s = fmaf(sm.h2[o + 6][tid], wb.z, s);
+      s = fmaf(sm.h2[o + 7][tid], wb.w, s);
+    }
     float dy = 0.f, l = 0.f;
     if (tid < live) {
-      const float d = s - t[b0 + tid];
-      dy = d / B;
-      l = 0.5f * d * d / B;
+      const float e = s - target;
+      dy = e / B;
+      l = 0.5f * e * e / B;
     }
     sm.dy[tid] = dy;
     A.dy[b0 + tid] = dy;
@@ -798,16 +875,24 @@ __global__ void __launch_bounds__(T_THREADS) k_t_rows(const float* __restrict__ 
     if (tid == 0) atomicAdd(loss, l);
   }
   __syncthreads();
-  float d[4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) d[r] = z2[r] > 0.f ? sm.dy[r0 + r] * sm.w3[u] : 0.f;
-  *reinterpret_cast<float4*>(&sm.d2[u][r0]) = make_float4(d[0], d[1], d[2], d[3]);
-  *reinterpret_cast<float4*>(A.dZ2 + at) = make_float4(d[0], d[1], d[2], d[3]);
+  for (int j = 0; j < T_U; ++j) {
+    const int u = u0 + T_US * j;
+    float v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = z2[j][r] > 0.f ? sm.dy[r0 + r] * w3[j] : 0.f;
+    *reinterpret_cast<float4*>(&sm.d2[u][r0]) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(A.dZ2 + (size_t)u * A.ld + b0 + r0) = make_float4(v[0], v[1], v[2], v[3]);
+  }
   __syncthreads();
-  dot4(sm.d2, &sm.W2[0][u], LH + 1, LH, d);
+  dot_rows<LH, LH + 4, false>(&sm.d2[0][r0], &sm.W.W2[0][u0], d);
 #pragma unroll
-  for (int r = 0; r < 4; ++r) d[r] = z1[r] > 0.f ? d[r] : 0.f;
-  *reinterpret_cast<float4*>(A.dZ1 + at) = make_float4(d[0], d[1], d[2], d[3]);
+  for (int j = 0; j < T_U; ++j) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) d[j][r] = z1[j][r] > 0.f ? d[j][r] : 0.f;
+    *reinterpret_cast<float4*>(A.dZ1 + (size_t)(u0 + T_US * j) * A.ld + b0 + r0) =
+        make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
+  }
 }
 
 struct AdamArgs {
@@ -815,21 +900,24 @@ struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;
 };
 
-// dW[o][i] = sum_b dZ[o][b] * bf(A[i][b]), db[o] = sum_b dZ[o][b]: one sum a
-// thread, 16 x 8 of a layer's a block (the last layer: one row of 8), and one
-// warp for the biases beside the first 8 inputs.  kAdam: the step of Adam on
-// each sum instead of writing it to g.
-// Bound by the chain of B dependent FMAs (4 cycles each: 2 us at B = 1024),
-// so the tiles are as small as puts all 20865 sums on the chip at once (176
-// blocks), the rows come 8 to a 16-byte (activations) or two 16-byte loads,
-// and the copies of T_STAGES chunks of T_CB rows are in flight together.
+// dW[o][i] = sum_b dZ[o][b] * A[i][b], db[o] = sum_b dZ[o][b]: a block makes
+// 16 x 8 sums of a layer (the last layer: one row of 8) on two warps, two sums
+// a thread, and the biases beside the first 8 inputs on a third.  kAdam: the
+// step of Adam on each sum instead of writing it to g, its parameter and
+// moments loaded before the sums.
+// Every sum is a chain of B dependent FMAs (4 cycles each, 2 us at B = 1024),
+// so all 20865 run on the chip at once (176 blocks).  Bound by the words read
+// from shared memory (3 a row and warp) and one warp's issue rate: 8.4 cycles a
+// row.  One sum a thread on four warps and four on one warp took 12-13, as
+// did loading only 4 rows ahead.  The copies of T_STAGES chunks of T_CB rows
+// are in flight together.
 constexpr int T_TO = 16, T_TI = 8;    // units x inputs a block
 constexpr int T_CB = 256;             // rows of the batch a chunk
 constexpr int T_STAGES = 4;
-constexpr int T_W_THREADS = T_TO * T_TI + 32;
+constexpr int T_W_THREADS = 96;
 struct TrainWgradSmem {  // rows padded by 16 bytes: 8 rows' 16-byte pieces in different banks
-  float dz[T_STAGES][T_TO][T_CB + 4];
-  __nv_bfloat16 a[T_STAGES][T_TI][T_CB + 8];
+  float r[T_STAGES][T_TO + T_TI][T_CB + 4];  // the units' dz, then the inputs' a
+  float past[16];                            // the inner loop's last load runs past its row
 };
 constexpr int T_W2_TILES = (LH / T_TO) * (LH / T_TI), T_W1_TILES = (LH / T_TO) * (LF / T_TI), T_W3_TILES = LH / T_TI;
 constexpr int T_WGRAD_GRID = T_W2_TILES + T_W1_TILES + T_W3_TILES;
@@ -842,92 +930,146 @@ constexpr int L_OFF_W3 = L_OFF_B2 + LH;
 constexpr int L_OFF_B3 = L_OFF_W3 + LH;
 constexpr int L_NPARAM = L_OFF_B3 + 1;
 
+struct AdamState {
+  float p, m, v;
+};
+__device__ __forceinline__ AdamState adam_load(const AdamArgs& ad, int e) { return {ad.p[e], ad.m[e], ad.v[e]}; }
+__device__ __forceinline__ float adam_step(const AdamArgs& ad, int e, AdamState a, float s) {
+  a.m = fmaf(1.f - ad.b1, s, ad.b1 * a.m);
+  a.v = fmaf((1.f - ad.b2) * s, s, ad.b2 * a.v);
+  a.p -= ad.lr * (a.m / ad.c1) / (sqrtf(a.v / ad.c2) + ad.eps);
+  ad.m[e] = a.m;
+  ad.v[e] = a.v;
+  ad.p[e] = a.p;
+  return a.p;
+}
+
 template <bool kAdam>
 __global__ void __launch_bounds__(T_W_THREADS) k_t_wgrad(TrainActs A, float* g, AdamArgs ad) {
   extern __shared__ __align__(16) unsigned char t_raw[];
   TrainWgradSmem& sm = *reinterpret_cast<TrainWgradSmem*>(t_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
   // this block's tile: units o0 .. o0 + no - 1 of dz, inputs i0 .. i0 + 7 of a
-  int tile = blockIdx.x, I, offw, offb, no = T_TO;
-  const float* dz;
-  const __nv_bfloat16* a;
+  int tile = blockIdx.x, I, offw, offb, no = T_TO, layer;
+  const float *dz, *a;
   if (tile < T_W2_TILES) {
-    I = LH, offw = L_OFF_W2, offb = L_OFF_B2, dz = A.dZ2, a = A.H1;
+    layer = 2, I = LH, offw = L_OFF_W2, offb = L_OFF_B2, dz = A.dZ2, a = A.H1;
   } else if (tile < T_W2_TILES + T_W1_TILES) {
     tile -= T_W2_TILES;
-    I = LF, offw = L_OFF_W1, offb = L_OFF_B1, dz = A.dZ1, a = A.X;
+    layer = 1, I = LF, offw = L_OFF_W1, offb = L_OFF_B1, dz = A.dZ1, a = A.X;
   } else {
     tile -= T_W2_TILES + T_W1_TILES;
-    I = LH, offw = L_OFF_W3, offb = L_OFF_B3, dz = A.dy, a = A.H2, no = 1;
+    layer = 3, I = LH, offw = L_OFF_W3, offb = L_OFF_B3, dz = A.dy, a = A.H2, no = 1;
   }
   const int i0 = tile % (I / T_TI) * T_TI, o0 = tile / (I / T_TI) * T_TO;
   const int nchunk = (A.ld + T_CB - 1) / T_CB;
+  ptx::grid_dependents_launch();
+  ptx::grid_dependency_wait();
   auto load = [&](int c) {  // chunk c's rows, zeros past ld
-    if (c < nchunk) {
-      const int s = c % T_STAGES, b0 = c * T_CB;
-      for (int e = tid; e < no * (T_CB / 4); e += T_W_THREADS) {
-        const int o = e / (T_CB / 4), b = e % (T_CB / 4) * 4;
-        const bool in = b0 + b < A.ld;
-        ptx::cp_async16_zfill(&sm.dz[s][o][b], dz + (in ? (size_t)(o0 + o) * A.ld + b0 + b : 0), in ? 16u : 0u);
-      }
-      for (int e = tid; e < T_TI * (T_CB / 8); e += T_W_THREADS) {
-        const int i = e / (T_CB / 8), b = e % (T_CB / 8) * 8;
-        const bool in = b0 + b < A.ld;
-        ptx::cp_async16_zfill(&sm.a[s][i][b], a + (in ? (size_t)(i0 + i) * A.ld + b0 + b : 0), in ? 16u : 0u);
-      }
+    if (c < nchunk && tid < T_CB / 4) {  // warps 0 and 1: a thread's 4 columns of each row of the tile
+      const int b = c * T_CB + 4 * tid;
+      const uint32_t n = b < A.ld ? 16u : 0u;
+      float* dst = &sm.r[c % T_STAGES][0][4 * tid];
+      const float* src = dz + (size_t)o0 * A.ld + (n ? b : 0);
+      for (int r = 0; r < no; ++r) ptx::cp_async16_zfill(dst + r * (T_CB + 4), src + (size_t)r * A.ld, n);
+      dst += T_TO * (T_CB + 4);
+      src = a + (size_t)i0 * A.ld + (n ? b : 0);
+#pragma unroll
+      for (int r = 0; r < T_TI; ++r) ptx::cp_async16_zfill(dst + r * (T_CB + 4), src + (size_t)r * A.ld, n);
     }
     ptx::cp_async_commit();
   };
   for (int c = 0; c < T_STAGES - 1; ++c) load(c);
-  // threads 0 .. 127: unit 4 warp + lane / 8, input lane % 8; the last warp: the bias of unit `lane`
-  const bool bias = warp == T_TO * T_TI / 32;
-  const int o = bias ? lane : 4 * warp + (lane >> 3), i = lane & 7;
-  const bool on = o < no && (!bias || i0 == 0);
-  float s = 0.f;
+  // warps 0 and 1: units o, o + 8 and input i of each lane; warp 2: the bias of unit `lane`
+  const bool bias = tid >= 64;
+  const int o = bias ? min(lane, T_TO - 1) : lane >> 2, i = (lane & 3) + 4 * (tid >> 5 & 1);
+  const bool on = bias ? lane < no && i0 == 0 : o < no, two = on && !bias && no > 1;
+  const int e0 = bias ? offb + o0 + o : offw + (o0 + o) * I + i0 + i, e1 = e0 + 8 * I;  // the sums' parameters
+  AdamState st0{}, st1{};
+  if (kAdam && on) st0 = adam_load(ad, e0);
+  if (kAdam && two) st1 = adam_load(ad, e1);
+  float s0 = 0.f, s1 = 0.f;
   for (int c = 0; c < nchunk; ++c) {
     ptx::cp_async_wait<T_STAGES - 2>();
     __syncthreads();  // chunk c has landed, and nobody reads the stage that the next copy overwrites
     load(c + T_STAGES - 1);
     if (!on) continue;
-    const int n = min(T_CB, A.ld - c * T_CB);  // a multiple of 8
-    const float4* zr = reinterpret_cast<const float4*>(sm.dz[c % T_STAGES][o]);
-    const uint4* ar = reinterpret_cast<const uint4*>(sm.a[c % T_STAGES][i]);
+    const int n = min(T_CB, A.ld - c * T_CB) / 4;  // a multiple of 4
+    const float4* zr = reinterpret_cast<const float4*>(sm.r[c % T_STAGES][o]);
+    // 16 rows are loaded while the 16 before them are summed (the last load
+    // runs past the row and is not used)
     if (bias) {
-#pragma unroll 4
-      for (int b = 0; b < n / 4; ++b) {
-        const float4 z = zr[b];
-        s += z.x;
-        s += z.y;
-        s += z.z;
-        s += z.w;
+      float4 z[2][4];
+      auto fetch = [&](int b, int h) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) z[h][q] = zr[b + q];
+      };
+      auto add = [&](int h) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          s0 += z[h][q].x;
+          s0 += z[h][q].y;
+          s0 += z[h][q].z;
+          s0 += z[h][q].w;
+        }
+      };
+      fetch(0, 0);
+#pragma unroll 1
+      for (int b = 0; b < n; b += 8) {
+        fetch(b + 4, 1);
+        add(0);
+        if (b + 4 >= n) break;
+        fetch(b + 8, 0);
+        add(1);
       }
-    } else {
-#pragma unroll 4
-      for (int b = 0; b < n / 8; ++b) {
-        const float4 z0 = zr[2 * b], z1 = zr[2 * b + 1];
-        const uint4 v = ar[b];
-        s = fmaf(z0.x, __uint_as_float(v.x << 16), s);
-        s = fmaf(z0.y, __uint_as_float(v.x & 0xffff0000u), s);
-        s = fmaf(z0.z, __uint_as_float(v.y << 16), s);
-        s = fmaf(z0.w, __uint_as_float(v.y & 0xffff0000u), s);
-        s = fmaf(z1.x, __uint_as_float(v.z << 16), s);
-        s = fmaf(z1.y, __uint_as_float(v.z & 0xffff0000u), s);
-        s = fmaf(z1.z, __uint_as_float(v.w << 16), s);
-        s = fmaf(z1.w, __uint_as_float(v.w & 0xffff0000u), s);
+      continue;
+    }
+    // (the last layer has one unit: s1 is not used)
+    const float4* zr8 = reinterpret_cast<const float4*>(sm.r[c % T_STAGES][two ? o + 8 : o]);
+    const float4* ar = reinterpret_cast<const float4*>(sm.r[c % T_STAGES][T_TO + i]);
+    float4 z[2][4], y[2][4], v[2][4];
+    auto fetch = [&](int b, int h) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        z[h][q] = zr[b + q];
+        y[h][q] = zr8[b + q];
+        v[h][q] = ar[b + q];
       }
+    };
+    auto add = [&](int h) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        s0 = fmaf(z[h][q].x, v[h][q].x, s0);
+        s1 = fmaf(y[h][q].x, v[h][q].x, s1);
+        s0 = fmaf(z[h][q].y, v[h][q].y, s0);
+        s1 = fmaf(y[h][q].y, v[h][q].y, s1);
+        s0 = fmaf(z[h][q].z, v[h][q].z, s0);
+        s1 = fmaf(y[h][q].z, v[h][q].z, s1);
+        s0 = fmaf(z[h][q].w, v[h][q].w, s0);
+        s1 = fmaf(y[h][q].w, v[h][q].w, s1);
+      }
+    };
+    fetch(0, 0);
+#pragma unroll 1
+    for (int b = 0; b < n; b += 8) {
+      fetch(b + 4, 1);
+      add(0);
+      if (b + 4 >= n) break;
+      fetch(b + 8, 0);
+      add(1);
     }
   }
-  if (!on) return;
-  const int e = bias ? offb + o0 + o : offw + (o0 + o) * I + i0 + i;
-  if (!kAdam) {
-    g[e] = s;
-    return;
-  }
-  const float m = ad.b1 * ad.m[e] + (1.f - ad.b1) * s;
-  const float v = ad.b2 * ad.v[e] + (1.f - ad.b2) * s * s;
-  ad.m[e] = m;
-  ad.v[e] = v;
-  ad.p[e] -= ad.lr * (m / ad.c1) / (sqrtf(v / ad.c2) + ad.eps);
+  auto finish = [&](int e, const AdamState& st, float s, int oo) {
+    if (!kAdam) {
+      g[e] = s;
+      return;
+    }
+    const float w = adam_step(ad, e, st, s);
+    if (!bias && layer == 2) A.W->W2[oo][i0 + i] = bf(w);
+    else if (!bias && layer == 1) A.W->W1[oo][i0 + i] = bf(w);
+  };
+  if (on) finish(e0, st0, s0, o0 + o);
+  if (two) finish(e1, st1, s1, o0 + o + 8);
 }
 
 }  // namespace vnm
@@ -962,27 +1104,29 @@ static MlpW mlp_view(const vnm_mlp* n) {
 static size_t mlp_smem() { return sizeof(MlpSmem) + 1024; }
 
 // Arena bytes and storage of a step's activations (batches of B rows).
-static int train_ld(int B) { return (B + T_ROWS - 1) / T_ROWS * T_ROWS; }
+static int train_ld(int B) { return (B + 15) / 16 * 16; }
 static size_t train_bytes(int B) {
   const size_t ld = (size_t)train_ld(B);
-  return arena_bytes(ld * LF, 2) + 2 * arena_bytes(ld * LH, 2) + 2 * arena_bytes(ld * LH, 4) + arena_bytes(ld, 4);
+  return arena_bytes(ld * LF, 4) + 4 * arena_bytes(ld * LH, 4) + arena_bytes(ld, 4) + arena_bytes(1, sizeof(TrainW));
 }
-static vnm_status train_acts(vnm_ctx* ctx, int B, TrainActs& A) {
+static vnm_status train_acts(vnm_ctx* ctx, const vnm_mlp* n, int B, TrainActs& A) {
   A.ld = train_ld(B);
   const size_t ld = (size_t)A.ld;
-  A.X = arena_take<__nv_bfloat16>(ctx, ld * LF);
-  A.H1 = arena_take<__nv_bfloat16>(ctx, ld * LH);
-  A.H2 = arena_take<__nv_bfloat16>(ctx, ld * LH);
+  A.X = arena_take<float>(ctx, ld * LF);
+  A.H1 = arena_take<float>(ctx, ld * LH);
+  A.H2 = arena_take<float>(ctx, ld * LH);
   A.dZ1 = arena_take<float>(ctx, ld * LH);
   A.dZ2 = arena_take<float>(ctx, ld * LH);
   A.dy = arena_take<float>(ctx, ld);
-  if (!A.X || !A.H1 || !A.H2 || !A.dZ1 || !A.dZ2 || !A.dy) return VNM_ERR_NOMEM;
+  A.W = arena_take<TrainW>(ctx, 1);
+  if (!A.X || !A.H1 || !A.H2 || !A.dZ1 || !A.dZ2 || !A.dy || !A.W) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(TrainRowsSmem)));
   VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_wgrad<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(TrainWgradSmem)));
   VNM_CUDA_TRY(cudaFuncSetAttribute(k_t_wgrad<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(TrainWgradSmem)));
+  VNM_LAUNCH(ctx, k_t_round, 84, 256, 0, n->p + L_OFF_W1, n->p + L_OFF_W2, A.W);
   return VNM_OK;
 }
 
@@ -991,11 +1135,25 @@ static vnm_status train_acts(vnm_ctx* ctx, int B, TrainActs& A) {
 // n->g or, with `adam`, straight into a step of Adam.
 static vnm_status mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t, int B, const TrainActs& A,
                            float* d_loss, const AdamArgs* adam) {
-  VNM_LAUNCH(ctx, k_t_rows, A.ld / T_ROWS, T_THREADS, sizeof(TrainRowsSmem), X, t, B, mlp_view(n), A, d_loss);
-  if (adam)
-    VNM_LAUNCH(ctx, k_t_wgrad<true>, T_WGRAD_GRID, T_W_THREADS, sizeof(TrainWgradSmem), A, n->g, *adam);
-  else
-    VNM_LAUNCH(ctx, k_t_wgrad<false>, T_WGRAD_GRID, T_W_THREADS, sizeof(TrainWgradSmem), A, n->g, AdamArgs{});
+  // each kernel may be set up while the one before it runs; its own wait for
+  // that one (grid_dependency_wait) comes before its first access to memory
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(A.ld / T_ROWS);
+  cfg.blockDim = dim3(T_THREADS);
+  cfg.dynamicSmemBytes = sizeof(TrainRowsSmem);
+  VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_t_rows, X, t, B, mlp_view(n), A, d_loss));
+  cfg.gridDim = dim3(T_WGRAD_GRID);
+  cfg.blockDim = dim3(T_W_THREADS);
+  cfg.dynamicSmemBytes = sizeof(TrainWgradSmem);
+  VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, adam ? k_t_wgrad<true> : k_t_wgrad<false>, A, n->g,
+                                  adam ? *adam : AdamArgs{}));
+  ctx->launches += 2;
   return VNM_OK;
 }
 
@@ -1074,7 +1232,7 @@ vnm_status vnm_mlp_grad(vnm_ctx* ctx, vnm_mlp* n, const float* X, const float* t
   float* dl = arena_take<float>(ctx, 1);
   if (!dl) return VNM_ERR_NOMEM;
   TrainActs A;
-  VNM_TRY(train_acts(ctx, B, A));
+  VNM_TRY(train_acts(ctx, n, B, A));
   VNM_CUDA_TRY(cudaMemsetAsync(dl, 0, sizeof(float), ctx->stream));
   VNM_TRY(mlp_grad(ctx, n, dX, dt, B, A, dl, nullptr));
   VNM_CUDA_TRY(cudaMemcpyAsync(grads, n->g, sizeof(float) * L_NPARAM, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1099,7 +1257,7 @@ vnm_status vnm_mlp_train(vnm_ctx* ctx, vnm_mlp* net, const float* X, const float
   float* losses = arena_take<float>(ctx, nb + 1);
   if (!losses) return VNM_ERR_NOMEM;
   TrainActs A;
-  VNM_TRY(train_acts(ctx, B, A));
+  VNM_TRY(train_acts(ctx, net, B, A));
   AdamArgs ad{net->p, net->m, net->v, lr, 0.9f, 0.999f, 1e-8f, 0.f, 0.f};
   for (int e = 0; e < epochs; ++e) {
     VNM_CUDA_TRY(cudaMemsetAsync(losses, 0, sizeof(float) * nb, ctx->stream));

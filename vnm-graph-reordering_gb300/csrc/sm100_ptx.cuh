@@ -112,6 +112,12 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch: let the next kernel of the stream be set up
+// from here on, and wait until the kernels before this one have finished and
+// their writes are visible (both nothing in an ordinary launch).
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Arrive on `bar` once this thread's earlier cp.async copies have landed;
 // the arrival counts toward the barrier's expected count (.noinc).
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
