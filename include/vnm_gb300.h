@@ -340,9 +340,7 @@ vnm_status vnm_spmm_info(const vnm_spmm_matrix* A, long long* info, int n);
 /* C (nrows x n, FP32, row-major) = A * B with B (nrows x n, row-major, the
  * compressed dtype).  n must be a multiple of 64.  mem = where B and C are
  * (device: 16-byte aligned).  The tensor-core kernel works on column blocks
- * of 256, 128 or 64; the first call of a context for an operand shape (rows, K-steps)
- * and n times each width that divides n once and keeps the fastest for
- * later calls (up to 8 shapes per context).  VNM_SPMM_WIDTH=64|128|256 in
+ * of 256, 128 or 64, the widest that divides n; VNM_SPMM_WIDTH=64|128|256 in
  * the environment fixes the width where it divides n. */
 vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, int n, float* C, int mem);
 
@@ -351,10 +349,9 @@ vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, i
  * default stream) after the work the caller enqueued there, and the call
  * returns at once.  B (nrows x n, the operand's 16-bit type) and C (nrows x
  * n, FP32) are device memory, 16-byte aligned, valid until the stream
- * reaches the product.  Exceptions to "without waiting": the first call for
- * an operand shape and n times the tensor-core column-block widths
- * (synchronising `stream` once), and the first call with a larger n than
- * before allocates the operand's scratch (cudaMalloc).  Calls on one operand
+ * reaches the product.  Exception to "without waiting": the first call with
+ * a larger n than before may allocate the operand's scratch (cudaMalloc; it
+ * has room for n <= 256 from the start).  Calls on one operand
  * share that scratch, so they must run in order (one stream, or streams the
  * caller orders).  A bounded wait that ran out inside the tensor-core kernel
  * sets a flag on the operand; vnm_spmm_check reads it. */

@@ -69,10 +69,6 @@ struct vnm_ctx {
   int last_clusters_fit = 0;  // clusters of the launched size the GPU can hold at once (occupancy query)
   int launches = 0;
   int last_cluster = 1;  // blocks per job of the last NM round launch
-  // SpMM column-block widths measured fastest, by (rows, K-steps, B width)
-  long long spmm_tune_key[8][3] = {};
-  int spmm_tune_nt[8] = {};
-  int spmm_tune_next = 0;
   DeviceArena arena;
   vnm_spmm_spare* spare = nullptr;
   // pinned staging for small results

@@ -41,14 +41,16 @@
 //               no tensor-core work) gathers its B rows with 16-byte loads and
 //               writes its C row (or a partial row);
 //   k_spmm_fin  adds the partial rows of the split rows, in chunk order;
-//   k_spmm_vnm  tensor cores, one CTA per (tile with K-steps, column block of
-//               C).  A producer warp streams each K-step's A tile (one bulk
-//               copy) and copies its 16 B rows with 16-byte cp.async loads
-//               into the 128-byte swizzled layout, with the row ids loaded
-//               eight K-steps ahead; one thread issues the MMA per K-step;
-//               eight stages keep copies in flight while the MMAs run.  Four
-//               warps then read the FP32 accumulator out of tensor memory,
-//               scale it and store it, or add it to what the residual wrote.
+//   k_spmm_vnm  tensor cores, one CTA per (work item, column block of C), a
+//               work item being a tile's K-steps or a part of them.  Eight
+//               producer warps stream stages of several K-steps: the A tiles
+//               by one bulk copy, their B rows with 16-byte cp.async loads
+//               into the 128-byte swizzled layout, the row ids loaded
+//               several stages ahead; a ninth warp issues the MMAs.  The
+//               producers then read the FP32 accumulator out of tensor
+//               memory, scale it and store it, or add it to what the residual
+//               wrote, or leave a part's sums for
+//   k_spmm_tfin which adds the parts of the split tiles, in K order.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -67,8 +69,9 @@ struct vnm_spmm_matrix {
   long long nnz = 0, groups = 0, slices = 0, slices_padded = 0, valid_blocks = 0;
   // tensor-core part
   int ntt = 0;                 // tiles with at least one K-step
-  int* tile_step = nullptr;    // [ntiles + 1]
-  int2* tlist = nullptr;       // [ntt] {tile, 1 when the residual kernel wrote the tile's rows first}
+  int npart = 0, ntsplit = 0, ntslots = 0;
+  int4* part_list = nullptr;   // [npart] {2 tile + (1: the residual kernel wrote its rows first), begin, end, slot or -1}
+  int4* tsplit = nullptr;      // [ntsplit] tiles cut into several parts: {2 tile + .., first slot, parts, 0}
   int* cols = nullptr;         // [nsteps * 16], -1 = padding column
   unsigned char* a = nullptr;  // [nsteps * 4096]
   float* rscale = nullptr;     // [ntiles * 128]
@@ -82,9 +85,10 @@ struct vnm_spmm_matrix {
   void* base = nullptr;        // one allocation for all of the above
   size_t bytes = 0;            // its size
   vnm_spmm_spare* spare = nullptr;  // the compressing context's spare storage
-  // state of the asynchronous entry point, allocated on its first call
-  float* part = nullptr;       // partial rows of split rows, for the largest n seen
+  // state of the asynchronous entry point
+  float* part = nullptr;       // partial rows and tiles, for the largest n seen
   size_t part_floats = 0;
+  bool part_own = false;       // an allocation of its own (the first PART_COLS columns' worth lies in `base`)
   int* err = nullptr;          // sticky failure flag of the tensor-core kernel
 };
 
@@ -92,8 +96,9 @@ namespace vnm {
 
 constexpr int SP_TM = 128;        // rows per tile (MMA M)
 constexpr int SP_KSTEP_BYTES = 4096;
-constexpr int SP_THREADS = 128;
-constexpr uint32_t SP_WAIT_LIMIT = 1u << 22;  // polls before a wait gives up
+constexpr int SP_THREADS = 288;
+constexpr uint32_t SP_WAIT_LIMIT = 1u << 22;  // polls (each may suspend) before a wait gives up
+constexpr uint32_t SP_SPIN_LIMIT = 1u << 26;  // polls of a pipeline wait, which spins
 constexpr int RES_CHUNK = 256;    // residual nonzeros per task, at most
 constexpr int RES_THREADS = 256;
 constexpr int RES_U = 8;          // entries in flight per lane group (8 measured ahead of 4)
@@ -276,10 +281,96 @@ __global__ void k_cmp_count(const unsigned long long* skeys, const int* spos, co
   }
 }
 
-__global__ void k_cmp_pad(const int* tile_raw, int ntiles, int* tile_pad, int* tile_has) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
-    tile_pad[t] = (tile_raw[t] + 3) & ~3;
-    tile_has[t] = tile_raw[t] > 0 ? 1 : 0;
+// Exclusive block-wide sums of N values a thread (1024 threads), each over
+// all threads; `tot` gets the totals.
+template <int N>
+__device__ __forceinline__ void block_scan(int (&v)[N], int (&tot)[N]) {
+  __shared__ int wsum[N][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int incl[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    incl[k] = v[k];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl[k], o);
+      if (lane >= o) incl[k] += x;
+    }
+    if (lane == 31) wsum[k][w] = incl[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    int x = wsum[k][lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    tot[k] = __shfl_sync(0xffffffffu, x, 31);
+    const int before = __shfl_sync(0xffffffffu, x, w > 0 ? w - 1 : 0);
+    v[k] = incl[k] - v[k] + (w > 0 ? before : 0);
+  }
+  __syncthreads();  // wsum is free again
+}
+
+// How the tensor-core work of `steps` K-steps of a tile is cut: parts of
+// about `per` K-steps, so that a few heavy tiles fill the chip.
+__host__ __device__ __forceinline__ int tile_parts(int steps, int per) {
+  const int k = (steps + per / 2) / per;
+  return k < 1 ? 1 : k;
+}
+// K-steps a part: an even share of an SM, but no less than PART_MIN.  A part
+// costs a CTA's set-up and the write and read of its partial tile, about as
+// much as 30 K-steps: without parts, 32 tiles of 256 K-steps (4096 rows,
+// V:2:8, V = 64) left 120 SMs idle (55 us a product at n = 128), and a hub
+// tile of a Chung-Lu graph held the chip for 170 us.
+constexpr int PART_MIN = 32;
+constexpr int PART_COLS = 256;                       // columns whose partial sums an operand has room for from the start,
+constexpr size_t PART_BYTES_MAX = size_t(256) << 20;  // unless they would take more than this
+
+// One block plans the tiles: counters[2] = tiles with K-steps, counters[3] =
+// padded slices, [4] = work items, [5] = split tiles, [6] = partial slots; a
+// tile's first slice (padded, and as counted), and its first work item, its
+// place among the split tiles and its first partial slot.
+__global__ void __launch_bounds__(1024)
+    k_tile_plan(const int* tile_raw, int ntiles, int num_sms, int* tile_base, int* tile_rawbase, int4* tile_plan,
+                int* counters) {
+  int run_pad = 0, run_raw = 0, run_has = 0;
+  for (int t0 = 0; t0 <= ntiles; t0 += 1024) {
+    const int t = t0 + threadIdx.x;
+    const int raw = t < ntiles ? tile_raw[t] : 0;
+    int v[3] = {(raw + 3) & ~3, raw, raw > 0 ? 1 : 0}, tot[3];
+    block_scan<3>(v, tot);
+    if (t <= ntiles) {
+      tile_base[t] = run_pad + v[0];
+      tile_rawbase[t] = run_raw + v[1];
+    }
+    run_pad += tot[0];
+    run_raw += tot[1];
+    run_has += tot[2];
+  }
+  const int total = run_pad / 4;  // K-steps
+  const int share = (total + num_sms - 1) / num_sms, per = share > PART_MIN ? share : PART_MIN;
+  int np = 0, ns = 0, nslot = 0;
+  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
+    const int t = t0 + threadIdx.x;
+    const int steps = t < ntiles ? (tile_raw[t] + 3) / 4 : 0;
+    const int k = steps > 0 ? tile_parts(steps, per) : 0;
+    int v[3] = {k, k > 1 ? 1 : 0, k > 1 ? k : 0}, tot[3];
+    block_scan<3>(v, tot);
+    if (t < ntiles) tile_plan[t] = make_int4(np + v[0], k, ns + v[1], nslot + v[2]);
+    np += tot[0];
+    ns += tot[1];
+    nslot += tot[2];
+  }
+  if (threadIdx.x == 0) {
+    counters[2] = run_raw;
+    counters[3] = run_has;
+    counters[8] = run_pad;
+    counters[9] = np;
+    counters[10] = ns;
+    counters[11] = nslot;
   }
 }
 
@@ -310,11 +401,11 @@ __device__ __forceinline__ int res_chunks(int len, bool needed) {
   return len <= RES_CHUNK ? 1 : (len + RES_CHUNK - 1) / RES_CHUNK;
 }
 
-__global__ void k_res_task_count(const int* rptr, int R, const int* tile_has, const int* tile_res, int* nmt, int* nst,
+__global__ void k_res_task_count(const int* rptr, int R, const int* tile_raw, const int* tile_res, int* nmt, int* nst,
                                  int* nmr) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
     const int t = r / SP_TM;
-    const int nch = res_chunks(rptr[r + 1] - rptr[r], !(tile_has[t] && tile_res[t] == 0));
+    const int nch = res_chunks(rptr[r + 1] - rptr[r], !(tile_raw[t] > 0 && tile_res[t] == 0));
     nmt[r] = nch > 1 ? nch : 0;
     nst[r] = nch == 1 ? 1 : 0;
     nmr[r] = nch > 1 ? 1 : 0;
@@ -322,12 +413,12 @@ __global__ void k_res_task_count(const int* rptr, int R, const int* tile_has, co
 }
 
 // Split rows' chunks first (they are the longest tasks), then the others.
-__global__ void k_res_task_fill(const int* rptr, int R, const int* tile_has, const int* tile_res, const int* mt_off,
+__global__ void k_res_task_fill(const int* rptr, int R, const int* tile_raw, const int* tile_res, const int* mt_off,
                                 const int* st_off, const int* mr_off, int nmt_total, int4* task, int4* multi) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
     const int t = r / SP_TM;
     const int b = rptr[r], e = rptr[r + 1];
-    const int nch = res_chunks(e - b, !(tile_has[t] && tile_res[t] == 0));
+    const int nch = res_chunks(e - b, !(tile_raw[t] > 0 && tile_res[t] == 0));
     if (nch == 1) {
       task[nmt_total + st_off[r]] = make_int4(r, b, e, -1);
     } else if (nch > 1) {
@@ -341,9 +432,17 @@ __global__ void k_res_task_fill(const int* rptr, int R, const int* tile_has, con
   }
 }
 
-__global__ void k_tile_list(const int* tile_has, const int* tile_res, int ntiles, const int* tl_off, int2* tlist) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
-    if (tile_has[t]) tlist[tl_off[t]] = make_int2(t, tile_res[t] > 0 ? 1 : 0);
+// The work items of the tiles with K-steps, split tiles' parts in K order.
+__global__ void k_tile_parts(const int* tile_raw, const int* tile_res, int ntiles, const int* tile_base,
+                             const int4* tile_plan, int4* part, int4* tsplit) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
+    const int steps = (tile_raw[t] + 3) / 4, s0 = tile_base[t] / 4, x = 2 * t + (tile_res[t] > 0 ? 1 : 0);
+    const int4 pl = tile_plan[t];
+    for (int k = 0; k < pl.y; ++k)
+      part[pl.x + k] = make_int4(x, s0 + (int)((long long)steps * k / pl.y), s0 + (int)((long long)steps * (k + 1) / pl.y),
+                                 pl.y > 1 ? pl.w + k : -1);
+    if (pl.y > 1) tsplit[pl.z] = make_int4(x, pl.w, pl.y, 0);
+  }
 }
 
 template <class T>
@@ -415,12 +514,10 @@ __global__ void k_cmp_fill(const unsigned long long* skeys, const int* spos, con
   }
 }
 
-__global__ void k_cmp_rscale(const unsigned* bmax, int ntiles, int R, int V, float* rscale, const int* tile_base,
-                             int* tile_step) {
+__global__ void k_cmp_rscale(const unsigned* bmax, int ntiles, int R, int V, float* rscale) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntiles * SP_TM; i += gridDim.x * blockDim.x) {
     const unsigned m = i < R ? bmax[i / V] : 0u;
     rscale[i] = m ? __uint_as_float(m) : 1.0f;
-    if (i <= ntiles) tile_step[i] = tile_base[i] >> 2;
   }
 }
 
@@ -580,65 +677,74 @@ __global__ void __launch_bounds__(FIN_THREADS)
 // Tensor-core kernel
 // ---------------------------------------------------------------------------
 struct SpmmArgs {
-  const int2* tlist;
-  const int* tile_step;
+  const int4* part;        // work items {2 tile + add, first K-step, last + 1, partial slot or -1}
   const int* cols;
   const unsigned char* a;
   const unsigned char* B;  // dense operand, row-major, 16-bit values
   size_t ldb;              // its row stride in bytes
   const float* rscale;
   float* C;
+  float* P;                // partial tiles of 128 rows, row stride ldc
   int R, n, ldc;
   uint32_t idesc;
   int* err;
   uint32_t wait_limit;  // polls of a pipeline wait (copies <-> MMAs) before it gives up
 };
 
-// K-steps in flight per CTA (192 KB of stages at NT = 256).  On a full
-// V:2:8 operand (19456 rows, n=256) with three producer warps: 8 stages
-// 0.161 ms, 10 0.145, 12 0.143, 14 0.133, 16 0.128 (one producer warp had
-// been faster with 8: 0.25 against 0.29 ms).
-constexpr int SP_STAGES = 16;
-constexpr int SP_PF = 8;      // pairs of K-steps whose column ids are loaded ahead (the ids come from DRAM)
+// A stage holds KS K-steps (their A tiles, 4 KB each, come as one bulk copy)
+// and is handed over once: a wait, a proxy fence, KS MMAs and a commit.  With
+// a stage per K-step that chain of the issuing thread was the bound, 0.2 us a
+// K-step at any width: a full V:2:8 operand (19456 rows) took 129 / 126 / 124
+// us at n = 256 / 128 / 64; with the stages below 82 / 61 / 58 us, bound by
+// the A tiles from HBM (378 MB, 6.2 TB/s at n = 128) and, at 256, by the
+// 192 KB of copies in flight (4 producer warps: 143 us; stages of 2 K-steps:
+// 126).
+constexpr int SP_PF = 4;  // groups of stages whose column ids are loaded ahead (the ids come from DRAM)
+constexpr int SP_PW = 8;  // producer warps
 
-template <int NT>
+template <int NT, int KS, int ST>
 struct SpmmSmem {
   static constexpr int B_BYTES = 16 * NT * 2;  // K=16 rows x NT columns, 16-bit
-  alignas(1024) unsigned char b[SP_STAGES][B_BYTES];
-  alignas(1024) unsigned char a[SP_STAGES][SP_KSTEP_BYTES];
-  alignas(8) uint64_t full[SP_STAGES];
-  alignas(8) uint64_t empty[SP_STAGES];
+  alignas(1024) unsigned char b[ST][KS][B_BYTES];
+  alignas(1024) unsigned char a[ST][KS * SP_KSTEP_BYTES];
+  alignas(8) uint64_t full[ST];  // an arrival a producer lane, and the A copy's bytes
+  alignas(8) uint64_t empty[ST];
   alignas(8) uint64_t done;
-  int last_k[SP_STAGES];  // the last K-step whose copies were issued into each stage
+  int last_a;  // the last stage fill whose A copy was issued
   uint32_t tmem_base;
   int abort;
 };
 
-// Warps that issue the copies: every warp but warp 1, whose lane 0 issues
-// the MMAs.  K-step i is copied by producer i % SP_PRODUCERS.  One producer
-// warp left the tensor pipe idle ~80 % of the time on a full V:2:8 operand
-// (16 B-row copies, their shuffles and addresses per K-step on one warp).
-constexpr int SP_PRODUCERS = SP_THREADS / 32 - 1;
-
-template <int NT>
+// One CTA: one work item (a tile, or a part of its K-steps) and NT columns
+// of C.  The first SP_PW warps copy, each its share of the B rows of every
+// stage, and read the accumulator out at the end; one lane of the last warp
+// issues the MMAs.  That warp runs its loop whole, so that the descriptors
+// stay in uniform registers (on one lane of a divergent branch an MMA took 85
+// cycles to issue).
+template <int NT, int KS, int ST>
 __global__ void __launch_bounds__(SP_THREADS, 1)
     k_spmm_vnm(SpmmArgs p) {
+  static_assert(SP_THREADS == 32 * (SP_PW + 1), "the producer warps and the issuing warp");
+  constexpr int WR = KS * 16 / SP_PW;  // a stage's B rows a producer warp
   extern __shared__ unsigned char sp_raw[];
-  SpmmSmem<NT>& sm = *reinterpret_cast<SpmmSmem<NT>*>(
+  using Smem = SpmmSmem<NT, KS, ST>;
+  Smem& sm = *reinterpret_cast<Smem*>(
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sp_raw) + 1023) & ~uintptr_t(1023)));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int2 tl = p.tlist[blockIdx.x];
-  const int t = tl.x;
-  const bool add = tl.y != 0;  // the residual kernel wrote these rows first
+  const int4 item = p.part[blockIdx.x];
+  const int t = item.x >> 1;
+  const bool add = item.x & 1;  // the residual kernel wrote these rows first
   const int n0 = blockIdx.y * NT;
-  const int s0 = p.tile_step[t], nsteps = p.tile_step[t + 1] - s0;
+  const int s0 = item.y, nsteps = item.z - item.y;
+  const int nst = (nsteps + KS - 1) / KS;  // stage fills
+  ptx::grid_dependents_launch();
 
   if (tid == 0) {
-    for (int s = 0; s < SP_STAGES; ++s) {
-      ptx::mbar_init(&sm.full[s], 1 + 32);  // the A copy's expect-tx arrival + one per producer lane
+    for (int s = 0; s < ST; ++s) {
+      ptx::mbar_init(&sm.full[s], 32 * SP_PW + 1);
       ptx::mbar_init(&sm.empty[s], 1);
-      sm.last_k[s] = -1;
     }
+    sm.last_a = -1;
     ptx::mbar_init(&sm.done, 1);
     sm.abort = 0;
     ptx::fence_mbar_init();
@@ -652,147 +758,192 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   ptx::tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
 
-  if (nsteps > 0) {
-    if (warp != 1) {
-      // producer warps.  Producer pw copies K-steps pw, pw + P, pw + 2P, ...
-      // (P = SP_PRODUCERS), two at a time.  Lane l holds column id (l & 15)
-      // of the (l >> 4)-th K-step of each of the SP_PF pairs ahead
-      // (coalesced 64-byte loads issued well before use); lane 0 issues the
-      // A tile by bulk copy, and every lane copies its 16-byte pieces of the
-      // 16 B rows.
-      const int pw = warp == 0 ? 0 : warp - 1;
-      constexpr int P = SP_PRODUCERS;
-      const uint64_t pol_a = ptx::policy_evict_first(), pol_b = ptx::policy_evict_last();
-      int pf[SP_PF];
+  int filled = 0;  // stage fills that this thread has arrived for
+  if (warp < SP_PW) {
+    // producer warps.  Lane l holds the column id of this warp's row l % WR
+    // of the (l / WR)-th stage of each of the SP_PF groups of SG stages ahead
+    // (issued well before use); every lane copies its 16-byte pieces of the
+    // warp's B rows.
+    constexpr int SG = 32 / WR;
+    const uint64_t pol_a = ptx::policy_evict_first(), pol_b = ptx::policy_evict_last();
+    auto ids = [&](int j) {  // group j
+      const int k = (SG * j + lane / WR) * (KS * 16) + warp * WR + lane % WR;  // row of the item's operand
+      return k < nsteps * 16 ? p.cols[(size_t)s0 * 16 + k] : -1;
+    };
+    int pf[SP_PF];
 #pragma unroll
-      for (int q = 0; q < SP_PF; ++q) {
-        const int st = pw + P * (2 * q + (lane >> 4));
-        pf[q] = st < nsteps ? p.cols[(size_t)(s0 + st) * 16 + (lane & 15)] : 0;
-      }
-      bool stop = false;
-      for (int j = 0; pw + P * j < nsteps && !stop; j += 2) {
-        const int cur = pf[0];
+    for (int q = 0; q < SP_PF; ++q) pf[q] = ids(q);
+    bool stop = false;
+    for (int j = 0; SG * j < nst && !stop; ++j) {
+      const int cur = pf[0];
 #pragma unroll
-        for (int q = 0; q + 1 < SP_PF; ++q) pf[q] = pf[q + 1];
-        {
-          const int st = pw + P * (j + 2 * SP_PF + (lane >> 4));
-          pf[SP_PF - 1] = st < nsteps ? p.cols[(size_t)(s0 + st) * 16 + (lane & 15)] : 0;
-        }
-        for (int d = 0; d < 2; ++d) {
-          const int ii = pw + P * (j + d), s = ii % SP_STAGES;
-          if (ii >= nsteps) break;
-          int ok = 1;
+      for (int q = 0; q + 1 < SP_PF; ++q) pf[q] = pf[q + 1];
+      pf[SP_PF - 1] = ids(j + SP_PF);
+      for (int d = 0; d < SG; ++d) {
+        const int i = SG * j + d, s = i % ST;
+        if (i >= nst) break;
+        const bool ok = !*reinterpret_cast<volatile int*>(&sm.abort) &&
+                        (i < ST || ptx::mbar_spin(&sm.empty[s], ((i / ST) - 1) & 1, p.wait_limit));
+        if (!__all_sync(0xffffffffu, ok)) {
           if (lane == 0) {
-            if (*reinterpret_cast<volatile int*>(&sm.abort)) ok = 0;
-            else if (ii >= SP_STAGES)
-              ok = ptx::mbar_wait(&sm.empty[s], ((ii / SP_STAGES) - 1) & 1, p.wait_limit) ? 1 : 0;
+            atomicOr(p.err, 1);
+            sm.abort = 1;
           }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) {
-            if (lane == 0) {
-              atomicOr(p.err, 1);
-              sm.abort = 1;
-            }
-            stop = true;
-            break;
-          }
-          if (lane == 0) {
-            sm.last_k[s] = ii;
-            // A tiles are read once: evict-first, so that they do not push
-            // the B rows (read by every tile) out of L2
-            ptx::mbar_arrive_expect_tx(&sm.full[s], SP_KSTEP_BYTES);
-            ptx::bulk_g2s_hint(sm.a[s], p.a + (size_t)(s0 + ii) * SP_KSTEP_BYTES, SP_KSTEP_BYTES, &sm.full[s],
-                               pol_a);
-          }
-          // the 16 B rows: each lane copies 16-byte chunks into the
-          // 128-byte-swizzled layout of the MMA's B operand (atoms of 8 k-rows
-          // x 128 bytes, n-atoms 2048 bytes apart, k-atoms 1024 bytes apart,
-          // chunk j of k-row r stored at chunk j ^ (r % 8))
-          {
-            constexpr int CPR = NT / 8;       // 16-byte chunks per row
-            constexpr int RPI = 32 / CPR;     // rows per warp instruction
-            const int c = lane % CPR, sub = lane / CPR;
-            unsigned char* bs = sm.b[s];
-#pragma unroll
-            for (int kr0 = 0; kr0 < 16; kr0 += RPI) {
-              const int kr = kr0 + sub;
-              const int row = __shfl_sync(0xffffffffu, cur, d * 16 + kr);
-              // a padding column (-1): its A column is zero; fill zeros, read nothing
-              const unsigned char* src = p.B + (size_t)(row < 0 ? 0 : row) * p.ldb + (size_t)(n0 + 8 * c) * 2;
-              unsigned char* dst = bs + (c >> 3) * 2048 + (kr >> 3) * 1024 + (kr & 7) * 128 + (((c & 7) ^ (kr & 7)) << 4);
-              ptx::cp_async16_zfill_hint(dst, src, row < 0 ? 0u : 16u, pol_b);
-            }
-            ptx::cp_async_mbar_arrive(&sm.full[s]);
-          }
-          __syncwarp();
-        }
-      }
-    } else if (tid == 32) {
-      // MMA issuer
-      for (int i = 0; i < nsteps; ++i) {
-        const int s = i % SP_STAGES;
-        if (!ptx::mbar_wait(&sm.full[s], (i / SP_STAGES) & 1, p.wait_limit)) {
-          atomicOr(p.err, 2);
-          sm.abort = 1;
+          stop = true;
           break;
         }
-        // the B rows were written by the load/store path: order them before
-        // the tensor core reads shared memory
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        ptx::tc_fence_after();
-        const uint64_t adesc = ptx::smem_desc(ptx::smem_addr(sm.a[s]), 128, 256, 0);
-        const uint64_t bdesc = ptx::smem_desc(ptx::smem_addr(sm.b[s]), 2048, 1024, 2);
-        ptx::mma_f16(tmem, adesc, bdesc, p.idesc, i > 0 ? 1u : 0u);
-        ptx::mma_commit(&sm.empty[s]);
-      }
-      ptx::mma_commit(&sm.done);
-    }
-    __syncwarp();
-    // everybody waits for the last MMA
-    bool ok = ptx::mbar_wait(&sm.done, 0, SP_WAIT_LIMIT);
-    if (!ok && tid == 0) atomicOr(p.err, 4);
-    __syncthreads();
-    if (tid == 0 && (sm.abort || !ok)) {
-      // a wait gave up: let every stage's last issued copies land before exit
-      // (the last K-step of a stage is the only one whose phase can be open)
-      for (int s = 0; s < SP_STAGES; ++s)
-        if (sm.last_k[s] >= 0) ptx::mbar_wait(&sm.full[s], (sm.last_k[s] / SP_STAGES) & 1, SP_WAIT_LIMIT);
-    }
-    __syncthreads();
-    ptx::tc_fence_after();
-    if (ok && !sm.abort) {
-      // warp w reads TMEM lanes 32 (w % 4) ..; the SP_THREADS / 128 warps of
-      // a lane quarter split the columns
-      constexpr int EG = SP_THREADS / 128, CW = NT / EG;
-      const int row = t * SP_TM + (warp & 3) * 32 + lane;
-      const float sc = row < p.R ? p.rscale[row] : 0.f;
-#pragma unroll 1
-      for (int c0 = (warp >> 2) * CW; c0 < (warp >> 2) * CW + CW; c0 += 32) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
-        ptx::tmem_ld_wait();
-        if (row < p.R) {
-          float4* dst = reinterpret_cast<float4*>(p.C + (size_t)row * p.ldc + n0 + c0);
+        ++filled;
+        if (warp == 0 && lane == 0) {
+          // A tiles are read once: evict-first, so that they do not push
+          // the B rows (read by every tile) out of L2
+          const uint32_t bytes = (uint32_t)min(KS, nsteps - i * KS) * SP_KSTEP_BYTES;
+          sm.last_a = i;
+          ptx::mbar_arrive_expect_tx(&sm.full[s], bytes);
+          ptx::bulk_g2s_hint(sm.a[s], p.a + (size_t)(s0 + i * KS) * SP_KSTEP_BYTES, bytes, &sm.full[s], pol_a);
+        }
+        // the 16 B rows: each lane copies 16-byte chunks into the
+        // 128-byte-swizzled layout of the MMA's B operand (atoms of 8 k-rows
+        // x 128 bytes, n-atoms 2048 bytes apart, k-atoms 1024 bytes apart,
+        // chunk j of k-row r stored at chunk j ^ (r % 8))
+        // (rows past the item's last K-step land in places no MMA reads)
+        {
+          constexpr int CPR = NT / 8;                      // 16-byte chunks per row
+          constexpr int RPI = 32 / CPR;                    // rows per warp instruction
+          const int c = lane % CPR, sub = lane / CPR;
+          unsigned char* bs = &sm.b[s][0][0];
+          const unsigned char* bcol = p.B + (size_t)(n0 + 8 * c) * 2;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            float4 o = make_float4(__uint_as_float(v[4 * q]) * sc, __uint_as_float(v[4 * q + 1]) * sc,
-                                   __uint_as_float(v[4 * q + 2]) * sc, __uint_as_float(v[4 * q + 3]) * sc);
-            if (add) {
-              const float4 r = dst[q];
-              o.x += r.x;
-              o.y += r.y;
-              o.z += r.z;
-              o.w += r.w;
-            }
-            dst[q] = o;
+          for (int r0 = 0; r0 < WR; r0 += RPI) {
+            const int k = warp * WR + r0 + sub, kr = k % 16;  // row of the stage, of its K-step
+            const int row = __shfl_sync(0xffffffffu, cur, d * WR + r0 + sub);
+            // a padding column (-1): its A column is zero; fill zeros, read nothing
+            const unsigned char* src = bcol + (size_t)(row < 0 ? 0 : row) * p.ldb;
+            unsigned char* dst = bs + (k / 16) * Smem::B_BYTES + (c >> 3) * 2048 + (kr >> 3) * 1024 + (kr & 7) * 128 +
+                                 (((c & 7) ^ (kr & 7)) << 4);
+            ptx::cp_async16_zfill_hint(dst, src, row < 0 ? 0u : 16u, pol_b);
           }
         }
+        ptx::cp_async_mbar_arrive(&sm.full[s]);
+        __syncwarp();
       }
+    }
+    if (stop) ptx::cp_async_wait_all();  // nothing of this thread's is in flight when the CTA leaves
+  } else {
+    const bool leader = ptx::elect_one();
+    for (int i = 0; i < nst; ++i) {
+      const int s = i % ST;
+      const bool ok = ptx::mbar_spin(&sm.full[s], (i / ST) & 1, p.wait_limit);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (leader) {
+          atomicOr(p.err, 2);
+          sm.abort = 1;
+        }
+        break;
+      }
+      // the B rows were written by the load/store path: order them before
+      // the tensor core reads shared memory
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      ptx::tc_fence_after();
+      const uint64_t adesc = ptx::smem_desc(ptx::smem_addr(sm.a[s]), 128, 256, 0);
+      const uint64_t bdesc = ptx::smem_desc(ptx::smem_addr(sm.b[s]), 2048, 1024, 2);
+      const int ks = min(KS, nsteps - i * KS);
+      if (leader) {
+#pragma unroll
+        for (int k = 0; k < KS; ++k)
+          if (k < ks)
+            ptx::mma_f16(tmem, adesc + (uint64_t)(k * (SP_KSTEP_BYTES >> 4)),
+                         bdesc + (uint64_t)(k * (Smem::B_BYTES >> 4)), p.idesc, (i | k) > 0 ? 1u : 0u);
+        ptx::mma_commit(&sm.empty[s]);
+      }
+    }
+    if (leader) ptx::mma_commit(&sm.done);
+  }
+  __syncwarp();
+  // everybody waits for the last MMA
+  bool ok = ptx::mbar_wait(&sm.done, 0, SP_WAIT_LIMIT);
+  if (!ok && tid == 0) atomicOr(p.err, 4);
+  __syncthreads();
+  if (sm.abort || !ok) {
+    // a wait gave up: before the CTA leaves, every A copy lands.  The
+    // producers that stopped early arrive for the fills they missed (at most
+    // one a stage, as a stage is filled again only after it was used), which
+    // completes the phase of each stage's last fill.
+    if (warp < SP_PW)
+      for (int i = filled; i <= sm.last_a; ++i) ptx::mbar_arrive(&sm.full[i % ST]);
+    if (tid == 0)
+      for (int i = max(sm.last_a - ST + 1, 0); i <= sm.last_a; ++i)
+        ptx::mbar_wait(&sm.full[i % ST], (i / ST) & 1, SP_WAIT_LIMIT);
+  }
+  __syncthreads();
+  ptx::tc_fence_after();
+  if (ok && !sm.abort && warp < SP_PW) {
+    // warp w reads TMEM lanes 32 (w % 4) .. of half of the columns; a part of
+    // a split tile goes out as it is,
+    // through a 32 x 32 piece of shared memory (the stages are free now), so
+    // that a warp reads and writes whole 128-byte lines of C
+    constexpr int CW = NT / (SP_PW / 4), EP = 36;
+    static_assert(sizeof(sm.b) + sizeof(sm.a) >= SP_PW * 32 * EP * sizeof(float), "the pieces fit the stages");
+    float* piece = reinterpret_cast<float*>(&sm.b[0][0][0]) + warp * (32 * EP);
+    const bool whole = item.w < 0;
+    const int r0 = (warp & 3) * 32, row0 = t * SP_TM + r0;  // the warp's first row of the tile, of C
+    const float sc = whole ? (row0 + lane < p.R ? p.rscale[row0 + lane] : 0.f) : 1.f;
+    const int live = whole ? p.R - row0 : 32;  // rows of the warp that are written
+    float* out = whole ? p.C + (size_t)row0 * p.ldc : p.P + ((size_t)item.w * SP_TM + r0) * p.ldc;
+    out += (size_t)(lane >> 3) * p.ldc + n0 + (lane & 7) * 4;
+#pragma unroll 1
+    for (int c0 = (warp >> 2) * CW; c0 < (warp >> 2) * CW + CW; c0 += 32) {
+      float4 was[8];
+      if (whole && add) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (4 * q + (lane >> 3) < live) was[q] = *reinterpret_cast<const float4*>(out + (size_t)(4 * q) * p.ldc + c0);
+      }
+      uint32_t v[32];
+      ptx::tmem_ld_32x32b_x32(tmem + ((uint32_t)r0 << 16) + (uint32_t)c0, v);
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(piece + lane * EP + 4 * q) =
+            make_float4(__uint_as_float(v[4 * q]) * sc, __uint_as_float(v[4 * q + 1]) * sc,
+                        __uint_as_float(v[4 * q + 2]) * sc, __uint_as_float(v[4 * q + 3]) * sc);
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        float4 o = *reinterpret_cast<const float4*>(piece + (4 * q + (lane >> 3)) * EP + (lane & 7) * 4);
+        if (whole && add) add4(o, was[q]);
+        if (4 * q + (lane >> 3) < live) *reinterpret_cast<float4*>(out + (size_t)(4 * q) * p.ldc + c0) = o;
+      }
+      __syncwarp();
     }
   }
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 0) ptx::tmem_dealloc(tmem, NT);
+}
+
+// Rows of a split tile: the sum of its parts in order, scaled, added to what
+// the residual kernel wrote.  Bound by L2 (the parts were just written): one
+// float4 of C a thread, the parts' loads four in flight.
+__global__ void __launch_bounds__(256)
+    k_spmm_tfin(const int4* __restrict__ split, const float* __restrict__ P, const float* __restrict__ rscale, int R,
+                int n, float* __restrict__ C) {
+  ptx::grid_dependency_wait();
+  const int4 m = split[blockIdx.x];
+  const int t = m.x >> 1, nq = n / 4;
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < SP_TM * nq; e += gridDim.y * blockDim.x) {
+    const int rt = e / nq, q = e % nq, row = t * SP_TM + rt;
+    if (row >= R) break;
+    const float4* src = reinterpret_cast<const float4*>(P + ((size_t)m.y * SP_TM + rt) * n) + q;
+    const size_t step = (size_t)SP_TM * nq;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int k = 0; k < m.z; ++k) add4(s, src[k * step]);
+    const float sc = rscale[row];
+    float4 o = make_float4(s.x * sc, s.y * sc, s.z * sc, s.w * sc);
+    float4* dst = reinterpret_cast<float4*>(C + (size_t)row * n) + q;
+    if (m.x & 1) add4(o, *dst);
+    *dst = o;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -815,7 +966,7 @@ static uint32_t spmm_wait_limit() {
     const long v = atol(e);
     if (v > 0) return (uint32_t)v;
   }
-  return SP_WAIT_LIMIT;
+  return SP_SPIN_LIMIT;
 }
 
 // Arena bytes compress_t takes for nnz entries and R rows.
@@ -825,7 +976,7 @@ static size_t compress_scratch_bytes(int R, int nnz) {
   size_t b = arena_bytes(n, 8) + 6 * arena_bytes(n, 4);          // keys, flag, gstart, gsl, gofs, resflag, rpos
   b += arena_bytes(n, 8) + arena_bytes(n, 4);                    // residual keys and sources
   b += 2 * radix_sort_scratch_bytes(nnz);
-  b += 7 * arena_bytes(ntiles + 1, 4);                           // tile_raw/pad/has/base/rawbase/res, tl_off
+  b += 4 * arena_bytes(ntiles + 1, 4) + arena_bytes(ntiles + 1, 16);  // tile_raw/base/rawbase/res, tile_plan
   b += 5 * arena_bytes((size_t)R + 1, 4);                        // rowlen, rptr, nmt, nst, nmr
   b += 3 * arena_bytes((size_t)R + 1, 4);                        // their scans
   b += arena_bytes((size_t)R + 2, 4);                            // bmax (R / V + 1 entries at most)
@@ -851,12 +1002,10 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   int* resflag = arena_take<int>(ctx, n1);
   int* rpos = arena_take<int>(ctx, n1);
   int* tile_raw = arena_take<int>(ctx, ntiles + 1);
-  int* tile_pad = arena_take<int>(ctx, ntiles + 1);
-  int* tile_has = arena_take<int>(ctx, ntiles + 1);
+  int4* tile_plan = arena_take<int4>(ctx, ntiles + 1);
   int* tile_res = arena_take<int>(ctx, ntiles + 1);
   int* tile_base = arena_take<int>(ctx, ntiles + 1);
   int* tile_rawbase = arena_take<int>(ctx, ntiles + 1);
-  int* tl_off = arena_take<int>(ctx, ntiles + 1);
   int* rowlen = arena_take<int>(ctx, (size_t)R + 1);
   int* rptr = arena_take<int>(ctx, (size_t)R + 1);
   int* nmt = arena_take<int>(ctx, (size_t)R + 1);
@@ -867,14 +1016,12 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   int* mr_off = arena_take<int>(ctx, (size_t)R + 1);
   unsigned* bmax = arena_take<unsigned>(ctx, nbrow + 1);
   int* counters = arena_take<int>(ctx, 16);
-  if (!keys || !flag || !gstart || !gsl || !gofs || !resflag || !rpos || !tile_raw || !tile_pad || !tile_has ||
-      !tile_res || !tile_base || !tile_rawbase || !tl_off || !rowlen || !rptr || !nmt || !nst || !nmr || !mt_off ||
+  if (!keys || !flag || !gstart || !gsl || !gofs || !resflag || !rpos || !tile_raw || !tile_plan ||
+      !tile_res || !tile_base || !tile_rawbase || !rowlen || !rptr || !nmt || !nst || !nmr || !mt_off ||
       !st_off || !mr_off || !bmax || !counters)
     return VNM_ERR_NOMEM;
   cudaStream_t st = ctx->stream;
   VNM_CUDA_TRY(cudaMemsetAsync(tile_raw, 0, sizeof(int) * (ntiles + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(tile_pad, 0, sizeof(int) * (ntiles + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(tile_has, 0, sizeof(int) * (ntiles + 1), st));
   VNM_CUDA_TRY(cudaMemsetAsync(tile_res, 0, sizeof(int) * (ntiles + 1), st));
   VNM_CUDA_TRY(cudaMemsetAsync(rowlen, 0, sizeof(int) * ((size_t)R + 1), st));
   VNM_CUDA_TRY(cudaMemsetAsync(resflag, 0, sizeof(int) * n1, st));
@@ -897,22 +1044,22 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
                sh, nseg, bmax);
     VNM_LAUNCH(ctx, k_cmp_count, sp_grid(ctx, nnz, 128), 128, 0, skeys, spos, gstart, counters, nnz, M, V, nseg, bm,
                dense_min, gsl, tile_raw, counters + 1, resflag, rowlen, tile_res);
-    VNM_TRY(exclusive_scan(ctx, gsl, gofs, nnz, counters + 2));
+    VNM_TRY(exclusive_scan(ctx, gsl, gofs, nnz, nullptr));
   }
-  VNM_LAUNCH(ctx, k_cmp_pad, sp_grid(ctx, ntiles), 256, 0, tile_raw, ntiles, tile_pad, tile_has);
-  VNM_TRY(exclusive_scan(ctx, tile_pad, tile_base, ntiles + 1, nullptr));
-  VNM_TRY(exclusive_scan(ctx, tile_raw, tile_rawbase, ntiles + 1, nullptr));
-  VNM_TRY(exclusive_scan(ctx, tile_has, tl_off, ntiles, counters + 3));
+  VNM_LAUNCH(ctx, k_tile_plan, 1, 1024, 0, tile_raw, ntiles, ctx->num_sms, tile_base, tile_rawbase, tile_plan,
+             counters);
   VNM_TRY(exclusive_scan(ctx, resflag, rpos, nnz, counters + 4));
   VNM_TRY(exclusive_scan(ctx, rowlen, rptr, R + 1, nullptr));
-  VNM_LAUNCH(ctx, k_res_task_count, sp_grid(ctx, R), 256, 0, rptr, R, tile_has, tile_res, nmt, nst, nmr);
+  VNM_LAUNCH(ctx, k_res_task_count, sp_grid(ctx, R), 256, 0, rptr, R, tile_raw, tile_res, nmt, nst, nmr);
   VNM_TRY(exclusive_scan(ctx, nmt, mt_off, R, counters + 5));
   VNM_TRY(exclusive_scan(ctx, nst, st_off, R, counters + 6));
   VNM_TRY(exclusive_scan(ctx, nmr, mr_off, R, counters + 7));
-  VNM_CUDA_TRY(cudaMemcpyAsync(h, tile_base + ntiles, sizeof(int), cudaMemcpyDeviceToHost, st));
-  VNM_CUDA_TRY(cudaMemcpyAsync(h + 1, counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  VNM_CUDA_TRY(cudaMemcpyAsync(h + 1, counters, 12 * sizeof(int), cudaMemcpyDeviceToHost, st));
   VNM_CUDA_TRY(cudaStreamSynchronize(st));
-  const int padded = h[0];
+  const int padded = h[9];
+  out->npart = h[10];
+  out->ntsplit = h[11];
+  out->ntslots = h[12];
   const int ngroups = nnz > 0 ? h[1] : 0;
   out->valid_blocks = h[2];
   out->slices = ngroups > 0 ? h[3] : 0;
@@ -928,13 +1075,18 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   out->nsteps = padded / 4;
   out->ntiles = ntiles;
   // the matrix's own storage (kept across calls)
-  const size_t b_step = arena_bytes(ntiles + 1, 4), b_tl = arena_bytes((size_t)out->ntt + 1, 8),
+  const size_t b_pt = arena_bytes((size_t)out->npart + 1, 16), b_ts = arena_bytes((size_t)out->ntsplit + 1, 16),
                b_cols = arena_bytes((size_t)out->nsteps * 16 + 1, 4),
                b_a = arena_bytes((size_t)out->nsteps * SP_KSTEP_BYTES + 16, 1),
                b_sc = arena_bytes((size_t)ntiles * SP_TM, 4), b_rc = arena_bytes((size_t)out->nres + 1, 8),
                b_tk = arena_bytes((size_t)out->ntask + 1, 16),
                b_mu = arena_bytes((size_t)out->nmulti + 1, 16);
-  const size_t need = b_step + b_tl + b_cols + b_a + b_sc + b_rc + b_tk + b_mu;
+  // with room for the asynchronous entry point's flag and partial sums up to
+  // PART_COLS columns, so that a first product allocates nothing
+  size_t pfloats = ((size_t)out->nslots + (size_t)out->ntslots * SP_TM) * PART_COLS + 1;
+  if (pfloats * sizeof(float) > PART_BYTES_MAX) pfloats = 1;
+  const size_t b_err = arena_bytes(1, 4), b_part = arena_bytes(pfloats, 4);
+  const size_t need = b_pt + b_ts + b_cols + b_a + b_sc + b_rc + b_tk + b_mu + b_err + b_part;
   void* base = nullptr;
   size_t have = 0;
   if (ctx->spare) {  // a freed operand's storage, when large enough
@@ -954,10 +1106,10 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   out->bytes = have;
   char* pb = static_cast<char*>(base);
   size_t o = 0;
-  out->tile_step = reinterpret_cast<int*>(pb + o);
-  o += b_step;
-  out->tlist = reinterpret_cast<int2*>(pb + o);
-  o += b_tl;
+  out->part_list = reinterpret_cast<int4*>(pb + o);
+  o += b_pt;
+  out->tsplit = reinterpret_cast<int4*>(pb + o);
+  o += b_ts;
   out->cols = reinterpret_cast<int*>(pb + o);
   o += b_cols;
   out->a = reinterpret_cast<unsigned char*>(pb + o);
@@ -969,6 +1121,12 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   out->task = reinterpret_cast<int4*>(pb + o);
   o += b_tk;
   out->multi = reinterpret_cast<int4*>(pb + o);
+  o += b_mu;
+  out->err = reinterpret_cast<int*>(pb + o);
+  o += b_err;
+  out->part = reinterpret_cast<float*>(pb + o);
+  out->part_floats = pfloats;
+  VNM_CUDA_TRY(cudaMemsetAsync(out->err, 0, sizeof(int), st));
   // residual CSR: the residual entries in their original order, stably
   // sorted by row
   if (out->nres > 0) {
@@ -982,32 +1140,32 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
     VNM_LAUNCH(ctx, k_res_gather, sp_grid(ctx, out->nres), 256, 0, ss, d_col, d_val, (int)out->nres, out->rcv);
   }
   if (out->ntask > 0)
-    VNM_LAUNCH(ctx, k_res_task_fill, sp_grid(ctx, R), 256, 0, rptr, R, tile_has, tile_res, mt_off, st_off, mr_off,
+    VNM_LAUNCH(ctx, k_res_task_fill, sp_grid(ctx, R), 256, 0, rptr, R, tile_raw, tile_res, mt_off, st_off, mr_off,
                nmt_total, out->task, out->multi);
   if (out->ntt > 0)
-    VNM_LAUNCH(ctx, k_tile_list, sp_grid(ctx, ntiles), 256, 0, tile_has, tile_res, ntiles, tl_off, out->tlist);
+    VNM_LAUNCH(ctx, k_tile_parts, sp_grid(ctx, ntiles), 256, 0, tile_raw, tile_res, ntiles, tile_base, tile_plan,
+               out->part_list, out->tsplit);
   VNM_CUDA_TRY(cudaMemsetAsync(out->cols, 0xff, b_cols, st));  // -1: padding columns
   VNM_CUDA_TRY(cudaMemsetAsync(out->a, 0, b_a, st));
   if (ngroups > 0 && out->nsteps > 0)
     VNM_LAUNCH(ctx, k_cmp_fill<T>, sp_grid(ctx, ngroups, 128), 128, 0, skeys, spos, d_val, gstart, ngroups, nnz, M,
                V, nseg, bm, dense_min, gofs, tile_base, tile_rawbase, bmax, out->cols, out->a);
-  VNM_LAUNCH(ctx, k_cmp_rscale, sp_grid(ctx, (long long)ntiles * SP_TM), 256, 0, bmax, ntiles, R, V, out->rscale,
-             tile_base, out->tile_step);
+  VNM_LAUNCH(ctx, k_cmp_rscale, sp_grid(ctx, (long long)ntiles * SP_TM), 256, 0, bmax, ntiles, R, V, out->rscale);
   return VNM_OK;
 }
 
-template <int NT>
+template <int NT, int KS, int ST>
 static vnm_status launch_spmm(vnm_ctx* ctx, const vnm_spmm_matrix* A, SpmmArgs& p) {
   // enough shared memory that at most 512 / NT CTAs share an SM: their NT
   // column accumulators then fit the SM's 512 tensor-memory columns, so an
   // allocation never waits for another CTA (228 KB of shared memory per SM)
   constexpr size_t floor_bytes = (228u << 10) / (512 / NT + 1) + 1024;
-  size_t smem = sizeof(SpmmSmem<NT>) + 1024;
+  size_t smem = sizeof(SpmmSmem<NT, KS, ST>) + 1024;
   if (smem < floor_bytes) smem = floor_bytes;
-  dim3 grid(A->ntt, p.n / NT);
-  VNM_CUDA_TRY(cudaFuncSetAttribute(k_spmm_vnm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  dim3 grid(A->npart, p.n / NT);
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_spmm_vnm<NT, KS, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   p.idesc = ptx::idesc_f16(A->dtype == 1 ? 1u : 0u, 0u, 1u, SP_TM, NT);
-  VNM_LAUNCH(ctx, k_spmm_vnm<NT>, grid, SP_THREADS, smem, p);
+  VNM_LAUNCH(ctx, (k_spmm_vnm<NT, KS, ST>), grid, SP_THREADS, smem, p);
   return VNM_OK;
 }
 
@@ -1069,8 +1227,7 @@ vnm_status vnm_spmm_info(const vnm_spmm_matrix* A, long long* info, int n) {
 vnm_status vnm_spmm_free(vnm_spmm_matrix* A) {
   if (!A) return VNM_ERR_ARG;
   cudaSetDevice(A->device);
-  if (A->part) cudaFree(A->part);
-  if (A->err) cudaFree(A->err);
+  if (A->part_own) cudaFree(A->part);
   bool last = false;
   if (A->spare) {
     // keep the storage for the context's next compression (the larger of
@@ -1091,20 +1248,18 @@ vnm_status vnm_spmm_free(vnm_spmm_matrix* A) {
 }
 
 // Enqueue one product on ctx->stream: the residual kernels, then the tensor
-// kernel at the column-block width the context measured fastest for this
-// operand shape and n (timed here, which synchronises the stream, on the
-// first call for a shape).  dB, dC, P and err are device memory.
+// kernel and the sum of its split tiles.  dB, dC, P and err are device memory.
 static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* dB, int n, float* dC, float* P,
                                int* err, bool timed) {
   SpmmArgs p;
-  p.tlist = A->tlist;
-  p.tile_step = A->tile_step;
+  p.part = A->part_list;
   p.cols = A->cols;
   p.a = A->a;
   p.B = static_cast<const unsigned char*>(dB);
   p.ldb = (size_t)n * 2;
   p.rscale = A->rscale;
   p.C = dC;
+  p.P = P + (size_t)A->nslots * n;  // after the residual's partial rows
   p.R = A->R;
   p.n = n;
   p.ldc = n;
@@ -1136,50 +1291,37 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
     if (A->nmulti > 0) VNM_LAUNCH(ctx, k_spmm_fin, A->nmulti, FIN_THREADS, 0, A->multi, P, n, dC, n, n);
     return VNM_OK;
   };
-  const long long key[3] = {A->R, A->nsteps, n};
-  int nt = 0;
-  if (const char* e = getenv("VNM_SPMM_WIDTH")) {  // a fixed width (64, 128 or 256) that divides n
+  // The widest column block that divides n: its A tiles are read fewest
+  // times.  VNM_SPMM_WIDTH (64, 128 or 256) in the environment fixes it where
+  // it divides n.
+  int nt = n % 256 == 0 ? 256 : n % 128 == 0 ? 128 : 64;
+  if (const char* e = getenv("VNM_SPMM_WIDTH")) {
     const int w = atoi(e);
     if ((w == 64 || w == 128 || w == 256) && n % w == 0) nt = w;
   }
-  for (int q = 0; q < 8 && nt == 0; ++q)
-    if (ctx->spmm_tune_nt[q] && ctx->spmm_tune_key[q][0] == key[0] && ctx->spmm_tune_key[q][1] == key[1] &&
-        ctx->spmm_tune_key[q][2] == key[2])
-      nt = ctx->spmm_tune_nt[q];
-  auto launch_nt = [&](int w) -> vnm_status {
+  auto launch_nt = [&]() -> vnm_status {
     if (A->ntt == 0) return VNM_OK;
-    if (w == 256) return launch_spmm<256>(ctx, A, p);
-    if (w == 128) return launch_spmm<128>(ctx, A, p);
-    return launch_spmm<64>(ctx, A, p);
+    if (nt == 256) VNM_TRY((launch_spmm<256, 4, 4>(ctx, A, p)));
+    else if (nt == 128) VNM_TRY((launch_spmm<128, 8, 3>(ctx, A, p)));
+    else VNM_TRY((launch_spmm<64, 8, 4>(ctx, A, p)));
+    if (A->ntsplit == 0) return VNM_OK;
+    cudaLaunchAttribute attr[1];  // set up while the parts are made
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(A->ntsplit, (SP_TM * (n / 4) + 1023) / 1024);
+    cfg.blockDim = dim3(256);
+    VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmm_tfin, (const int4*)A->tsplit, (const float*)p.P,
+                                    (const float*)A->rscale, A->R, n, dC));
+    ctx->launches++;
+    return VNM_OK;
   };
-  if (nt == 0 && A->ntt == 0) nt = 64;  // no tensor-core work: nothing to tune
-  if (nt == 0) {
-    // the tensor kernel adds into rows the residual kernel wrote: time each
-    // width on that state (the final launches below write C afresh)
-    VNM_TRY(launch_res());
-    const int cand[3] = {256, 128, 64};
-    float best = 0.f;
-    for (int w : cand) {
-      if (n % w) continue;
-      VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-      VNM_TRY(launch_nt(w));
-      VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
-      VNM_CUDA_TRY(cudaEventSynchronize(ctx->ev_main1));
-      float ms = 0.f;
-      VNM_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev_main0, ctx->ev_main1));
-      if (nt == 0 || ms < best) {
-        best = ms;
-        nt = w;
-      }
-    }
-    const int slot = ctx->spmm_tune_next;
-    ctx->spmm_tune_next = (slot + 1) % 8;
-    for (int k = 0; k < 3; ++k) ctx->spmm_tune_key[slot][k] = key[k];
-    ctx->spmm_tune_nt[slot] = nt;
-  }
   if (timed) VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
   VNM_TRY(launch_res());
-  VNM_TRY(launch_nt(nt));
+  VNM_TRY(launch_nt());
   if (timed) VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   return VNM_OK;
 }
@@ -1189,7 +1331,8 @@ vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, i
   if (mem != VNM_MEM_HOST && mem != VNM_MEM_DEVICE) return VNM_ERR_ARG;
   if (A->device != ctx->device) return VNM_ERR_ARG;
   const size_t bbytes = (size_t)A->R * n * 2, cbytes = (size_t)A->R * n * sizeof(float);
-  const size_t pbytes = arena_bytes((size_t)A->nslots * n + 1, sizeof(float));
+  const size_t pfloats = ((size_t)A->nslots + (size_t)A->ntslots * SP_TM) * n + 1;
+  const size_t pbytes = arena_bytes(pfloats, sizeof(float));
   VNM_TRY(arena_reserve(ctx, (mem == VNM_MEM_HOST ? bbytes + cbytes + 512 : 0) + pbytes + 4096));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
@@ -1204,7 +1347,7 @@ vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, i
   }
   if ((reinterpret_cast<uintptr_t>(dB) & 15) != 0 || (reinterpret_cast<uintptr_t>(dC) & 15) != 0)
     return VNM_ERR_ARG;
-  float* P = arena_take<float>(ctx, (size_t)A->nslots * n + 1);
+  float* P = arena_take<float>(ctx, pfloats);
   int* err = arena_take<int>(ctx, 1);
   if (!err || !P) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
@@ -1223,17 +1366,15 @@ vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, i
   if (A->device != ctx->device) return VNM_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(B) & 15) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0) return VNM_ERR_ARG;
   VNM_CUDA_TRY(cudaSetDevice(ctx->device));
-  const size_t need = (size_t)A->nslots * n + 1;
-  if (!A->err) {
-    VNM_CUDA_TRY(cudaMalloc(&A->err, sizeof(int)));
-    VNM_CUDA_TRY(cudaMemset(A->err, 0, sizeof(int)));
-  }
+  const size_t need = ((size_t)A->nslots + (size_t)A->ntslots * SP_TM) * n + 1;
   if (need > A->part_floats) {  // the first call for a larger n: make room (this waits for the device)
-    if (A->part) VNM_CUDA_TRY(cudaFree(A->part));
+    if (A->part_own) VNM_CUDA_TRY(cudaFree(A->part));
     A->part = nullptr;
     A->part_floats = 0;
+    A->part_own = false;
     VNM_CUDA_TRY(cudaMalloc(&A->part, need * sizeof(float)));
     A->part_floats = need;
+    A->part_own = true;
   }
   ctx->launches = 0;
   ctx->last_ms = ctx->main_ms = 0.f;
@@ -1247,7 +1388,6 @@ vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, i
 vnm_status vnm_spmm_check(vnm_spmm_matrix* A, void* stream, int* failed) {
   if (!A || !failed) return VNM_ERR_ARG;
   *failed = 0;
-  if (!A->err) return VNM_OK;
   VNM_CUDA_TRY(cudaSetDevice(A->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int h = 0;

@@ -378,7 +378,7 @@ class SpmmMatrix:
     def run_async(self, B, C=None, stream=None):
         """C = A B enqueued on a CUDA stream (torch's current stream of B's
         device by default) without waiting; B and C are CUDA tensors.  The
-        first call for an operand shape and n times the kernel widths once."""
+        first call with n > 256 may allocate the operand's scratch."""
         import torch
         n = B.shape[1]
         if C is None:

@@ -18,8 +18,7 @@ D^-1/2 A D^-1/2 of an undirected graph is).
 Every aggregation is enqueued on PyTorch's current stream of X's device
 (vnm_spmm_run_async) after the work that produced X, and the op returns
 without waiting for it, so a training loop does not stall the host at each
-layer.  The first aggregation of an operand shape and feature width times
-the kernel's widths once (a one-time wait).
+layer.
 """
 import numpy as np
 
