@@ -18,13 +18,23 @@
 //      order.  Done by refinement: sort rows by (group of the previous
 //      pass, k-th token) with the stable radix sort until no group of equal
 //      rows can still be split.
+// For m <= 65536 rows and nseg <= 16384 segments nothing is sorted by entry
+// and a round is four kernels: the entries stay in the original matrix's rows
+// (a round only composes the node map), one warp per row turns its columns
+// into the token list (k_vs_tokens), and one thread-block cluster holds all
+// rows in its shared memory and refines their order there (k_vs_order).
 // Token order: comparing the dense hash tuples of two rows is the same as
 // comparing their lists of (segment, hash) tokens, where token (s, h) ranks
 // by  h > 0: +(nseg - s),  h < 0: -(nseg - s),  end of row: 0, then by h.
+#include <cooperative_groups.h>
+
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace vnm {
 
@@ -369,6 +379,458 @@ static vnm_status vnm_args(vnm_ctx* ctx, int m, int n, int nnz, const int* row, 
   return VNM_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Rounds on the original rows
+// ---------------------------------------------------------------------------
+constexpr int VO_MAX_ROWS = 65536, VO_MAX_SEG = 16384;
+
+__device__ __forceinline__ unsigned vs_token(unsigned bits, int s, int nseg) {
+  const int h = __popc(bits) <= 2 ? gray_rank(bits) : -gray_rank(bits);
+  const int rank = h > 0 ? (nseg - s) : -(nseg - s);
+  return ((unsigned)(rank + nseg) << 9) | (unsigned)(h + 256);
+}
+
+// Entries per row; lanes of a warp with the same row add once.
+__global__ void k_vs_rowcount(const int* row, int nnz, int* count) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
+    const int r = row[i];
+    const unsigned peers = __match_any_sync(__activemask(), r);
+    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&count[r], __popc(peers));
+  }
+}
+
+// Columns by row (any order inside a row; `fill` zero on entry).
+__global__ void k_vs_rowfill(const int* row, const int* col, int nnz, const int* rowptr, int* fill, int* ccol) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
+    const int r = row[i], lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(__activemask(), r);
+    const int lead = __ffs(peers) - 1;
+    int at = 0;
+    if (lane == lead) at = atomicAdd(&fill[r], __popc(peers));
+    at = __shfl_sync(peers, at, lead);
+    ccol[rowptr[r] + at + __popc(peers & ((1u << lane) - 1u))] = col[i];
+  }
+}
+
+// The composed map (identity without prev) and where its value lies:
+// segment << 3 | place in the segment.
+__global__ void k_vs_map(const int* prev, const int* new_id, int m, int M, int* comp, int* packed) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    const int c = prev ? new_id[prev[i]] : i;
+    comp[i] = c;
+    packed[i] = (c / M) << 3 | (c % M);
+  }
+}
+
+// Token list of every row, at the row's place in the column list, and the
+// V-block tables; one warp a row.  A row of at most 32 entries is sorted in
+// registers; a longer one sets its bits in a bitmap of one byte a segment in
+// shared memory and reads the touched parts back in order.  Bound by the
+// gathers of `packed` and the atomics of the tables: 16384 rows, 262144
+// entries take 13 us, where sorting the entries by (row, column) took 130.
+constexpr int VT_WARPS = 8;
+__global__ void __launch_bounds__(VT_WARPS * 32)
+    k_vs_tokens(const int* __restrict__ rowptr, const int* __restrict__ ccol, const int* __restrict__ comp,
+                const int* __restrict__ packed, int m, int M, int nseg, int V, int2* tlist, unsigned* gtok,
+                unsigned* ortab, unsigned* badtab) {
+  extern __shared__ unsigned vt_bitmap[];
+  const int nw = (nseg + 3) / 4;                          // words of a row's bitmap
+  const int part = ((nw + 31) / 32 + 31) / 32 * 32;       // words a bit of the touched mask stands for
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned* bm = vt_bitmap + warp * nw;
+  for (int w = lane; w < nw; w += 32) bm[w] = 0u;
+  __syncwarp();
+  for (int q = blockIdx.x * VT_WARPS + warp; q < m; q += gridDim.x * VT_WARPS) {
+    const int b = rowptr[q], len = rowptr[q + 1] - b, cr = comp[q];
+    const long long cell0 = (long long)(cr / V) * nseg;
+    auto emit = [&](int s, unsigned bits, int at) {
+      gtok[b + at] = vs_token(bits, s, nseg);
+      const long long cell = cell0 + s;
+      atomicOr(&ortab[cell >> 2], bits << ((cell & 3) * 8));
+      if (__popc(bits) > 2) atomicOr(&badtab[cell >> 2], 1u << ((cell & 3) * 8));
+    };
+    int n = 0;
+    if (len <= 32) {
+      unsigned key = lane < len ? (unsigned)packed[ccol[b + lane]] : ~0u;
+#pragma unroll
+      for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+          const unsigned other = __shfl_xor_sync(0xffffffffu, key, j);
+          const bool up = (lane & k) == 0, low = (lane & j) == 0;
+          key = (low == up) ? min(key, other) : max(key, other);
+        }
+      const unsigned s = key >> 3;
+      const bool valid = key != ~0u;
+      unsigned bits = valid ? 1u << (M - 1 - (int)(key & 7u)) : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {  // OR over the lanes of the same segment from here on
+        const unsigned t = __shfl_down_sync(0xffffffffu, bits, o), ts = __shfl_down_sync(0xffffffffu, s, o);
+        if (lane + o < 32 && ts == s) bits |= t;
+      }
+      const unsigned ps = __shfl_up_sync(0xffffffffu, s, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, valid && (lane == 0 || ps != s));
+      if ((heads >> lane) & 1u) emit((int)s, bits, __popc(heads & ((1u << lane) - 1u)));
+      n = __popc(heads);
+    } else {
+      unsigned touched = 0;
+      for (int e = lane; e < len; e += 32) {
+        const int p = packed[ccol[b + e]], s = p >> 3;
+        atomicOr(&bm[s >> 2], (1u << (M - 1 - (p & 7))) << ((s & 3) * 8));
+        touched |= 1u << ((s >> 2) / part);
+      }
+      touched = __reduce_or_sync(0xffffffffu, touched);
+      __syncwarp();
+      for (; touched; touched &= touched - 1) {
+        const int w0 = (__ffs(touched) - 1) * part, w1 = min(w0 + part, nw);
+        for (int w = w0 + lane; w - lane < w1; w += 32) {
+          unsigned word = 0;
+          if (w < w1) {
+            word = bm[w];
+            bm[w] = 0u;
+          }
+          if (!__any_sync(0xffffffffu, word != 0u)) continue;
+          int c = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) c += ((word >> (8 * k)) & 0xffu) ? 1 : 0;
+          int incl = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          int at = n + incl - c;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned bits = (word >> (8 * k)) & 0xffu;
+            if (bits) emit(4 * w + k, bits, at++);
+          }
+          n += __shfl_sync(0xffffffffu, incl, 31);
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) tlist[cr] = make_int2(b, n);
+  }
+}
+
+// The stable order of the rows by their token lists, in the shared memory of
+// one thread-block cluster: position p lives in block p / cap (cap a power of
+// two).  Level k sorts the rows by (start of the row's group so far, k-th
+// token) with a stable radix sort of VO_BITS-bit digits, then splits the
+// groups; rows alone in their group, or at the end of their list, keep their
+// place.  A digit takes two cluster barriers: each warp ranks its 32-row
+// chunks with __match_any, the blocks exchange their digit counts, and every
+// row goes straight to its place in the other buffer, in whichever block.
+// Bound by latency: a digit takes about 2 us at 16384 rows on 16 blocks, where
+// a pass of the multi-kernel radix sort took 23.
+constexpr int VO_BITS = 9, VO_BINS = 1 << VO_BITS, VO_THREADS = 1024, VO_WARPS = 32, VO_ITEMS = 4, VO_MAX_CTAS = 16;
+constexpr int VO_MAX_CAP = VO_THREADS * VO_ITEMS;
+static_assert(VO_MAX_CAP * VO_MAX_CTAS == VO_MAX_ROWS, "all rows fit the largest cluster");
+struct alignas(16) OrderSmem {
+  uint16_t whist[VO_WARPS][VO_BINS];       // a warp's digit counts, then the counts of the warps before it
+  uint32_t tot[VO_BINS / 2];               // this block's digit counts, two to a word
+  uint32_t ctot[VO_MAX_CTAS][VO_BINS / 2]; // every block's
+  int base[VO_BINS];                       // where this block's rows of a digit go
+  int wsum[VO_WARPS];
+  int cmax[VO_MAX_CTAS];                   // every block's last group start
+  int act[VO_MAX_CTAS];                    // whether a block has rows to split
+};
+
+__global__ void __launch_bounds__(VO_THREADS, 1)
+    k_vs_order(const int2* __restrict__ tlist, const unsigned* __restrict__ gtok, int m, int nseg, int tokbits,
+               int grpbits, int cap, int* order) {
+  extern __shared__ __align__(16) unsigned char vo_raw[];
+  OrderSmem& sm = *reinterpret_cast<OrderSmem*>(vo_raw);
+  auto* const key0 = reinterpret_cast<unsigned long long*>(vo_raw + sizeof(OrderSmem));  // [2][cap]
+  auto* const row0 = reinterpret_cast<int*>(key0 + 2 * cap);                             // [2][cap]
+  cg::cluster_group cl = cg::this_cluster();
+  const int nct = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int capb = 31 - __clz(cap);
+  const int items = cap >= VO_THREADS ? cap / VO_THREADS : 1;  // 32-row chunks a warp
+  // slot of this lane's item j; with fewer rows than threads the first warps have them
+  auto slot_of = [&](int j) { return (w * items + j) * 32 + lane; };
+  auto live_of = [&](int j) { return slot_of(j) < cap && rank * cap + slot_of(j) < m; };
+  const unsigned endtok = ((unsigned)nseg << 9) | 256u;
+  const unsigned long long tmask = (1ull << tokbits) - 1;
+  int grp[VO_ITEMS];      // start of the group of each of this lane's positions
+  unsigned settled = 0;   // bit j: position j keeps its row
+#pragma unroll
+  for (int j = 0; j < VO_ITEMS; ++j) {
+    grp[j] = 0;
+    if (j < items && live_of(j)) row0[slot_of(j)] = rank * cap + slot_of(j);
+  }
+  int cur = 0;
+  __syncthreads();
+  for (int k = 0;; ++k) {
+    unsigned long long* key = key0 + cur * cap;
+    int act = 0;
+#pragma unroll
+    for (int j = 0; j < VO_ITEMS; ++j)
+      if (j < items && live_of(j)) {
+        unsigned tok = 0;
+        if (!((settled >> j) & 1u)) {
+          const int2 t = tlist[row0[cur * cap + slot_of(j)]];
+          tok = k < t.y ? gtok[t.x + k] : endtok;
+          act = 1;
+        }
+        key[slot_of(j)] = (unsigned long long)(unsigned)grp[j] << tokbits | tok;
+      }
+    act = __syncthreads_or(act);
+    if (tid < nct) *cl.map_shared_rank(&sm.act[rank], tid) = act;
+    const int bits = tokbits + (k > 0 ? grpbits : 0);  // one group at first
+    bool any = true;
+    for (int shift = 0; shift < bits; shift += VO_BITS) {
+      key = key0 + cur * cap;
+      int* row = row0 + cur * cap;
+      uint32_t* wh = reinterpret_cast<uint32_t*>(&sm.whist[0][0]);
+      for (int i = tid; i < VO_WARPS * VO_BINS / 2; i += VO_THREADS) wh[i] = 0u;
+      __syncthreads();
+      int dig[VO_ITEMS], at[VO_ITEMS];
+#pragma unroll
+      for (int j = 0; j < VO_ITEMS; ++j) {
+        if (j >= items) break;
+        const bool live = live_of(j);
+        dig[j] = live ? (int)(key[slot_of(j)] >> shift) & (VO_BINS - 1) : VO_BINS + lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, dig[j]);
+        at[j] = live ? sm.whist[w][dig[j]] + __popc(peers & ((1u << lane) - 1u)) : 0;
+        __syncwarp();
+        if (live && lane == __ffs(peers) - 1) sm.whist[w][dig[j]] += (uint16_t)__popc(peers);
+        __syncwarp();
+      }
+      __syncthreads();
+      if (tid < VO_BINS / 2) {  // counts of the warps before, two digits a thread (no carry: at most cap)
+        uint32_t run = 0;
+#pragma unroll 8
+        for (int v = 0; v < VO_WARPS; ++v) {
+          const uint32_t c = wh[v * (VO_BINS / 2) + tid];
+          wh[v * (VO_BINS / 2) + tid] = run;
+          run += c;
+        }
+        sm.tot[tid] = run;
+      }
+      __syncthreads();
+      for (int i = tid; i < nct * (VO_BINS / 2); i += VO_THREADS)
+        *cl.map_shared_rank(&sm.ctot[rank][i % (VO_BINS / 2)], i / (VO_BINS / 2)) = sm.tot[i % (VO_BINS / 2)];
+      cl.sync();
+      if (shift == 0) {
+        int a = 0;
+        for (int c = 0; c < nct; ++c) a |= sm.act[c];
+        any = a != 0;
+        if (!any) break;  // the same in every block
+      }
+      if (tid < VO_BINS / 2) {
+        int lo = 0, hi = 0, blo = 0, bhi = 0;  // all blocks' counts, and of the blocks before this one
+        for (int c = 0; c < nct; ++c) {
+          const uint32_t x = sm.ctot[c][tid];
+          if (c == rank) {
+            blo = lo;
+            bhi = hi;
+          }
+          lo += (int)(x & 0xffffu);
+          hi += (int)(x >> 16);
+        }
+        int incl = lo + hi;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
+        }
+        if (lane == 31) sm.wsum[w] = incl;
+        sm.base[2 * tid] = incl - lo - hi + blo;
+        sm.base[2 * tid + 1] = incl - hi + bhi;
+      }
+      __syncthreads();
+      {
+        unsigned long long* const okey = key0 + (cur ^ 1) * cap;
+        int* const orow = row0 + (cur ^ 1) * cap;
+#pragma unroll
+        for (int j = 0; j < VO_ITEMS; ++j)
+          if (j < items && live_of(j)) {
+            int before = 0;
+            for (int v = 0; v < dig[j] >> 6; ++v) before += sm.wsum[v];
+            const int dst = sm.base[dig[j]] + before + sm.whist[w][dig[j]] + at[j];
+            const int blk = dst >> capb, sl = dst & (cap - 1);
+            *cl.map_shared_rank(okey + sl, blk) = key[slot_of(j)];
+            *cl.map_shared_rank(orow + sl, blk) = row[slot_of(j)];
+          }
+      }
+      cl.sync();
+      cur ^= 1;
+    }
+    if (!any) break;
+    // split the groups: a row starts one when its key differs from the one before
+    key = key0 + cur * cap;
+    int last = -1;  // the last group start up to here, of this warp
+    unsigned alone = 0, done = 0;
+#pragma unroll
+    for (int j = 0; j < VO_ITEMS; ++j) {
+      if (j >= items) break;
+      const int sl = slot_of(j), pos = rank * cap + sl;
+      int start = -1;
+      if (live_of(j)) {
+        const unsigned long long me = key[sl];
+        const bool head = pos == 0 || me != (sl > 0 ? key[sl - 1] : *cl.map_shared_rank(key + cap - 1, rank - 1));
+        const bool tail =
+            pos == m - 1 || me != (sl + 1 < cap ? key[sl + 1] : *cl.map_shared_rank(key, rank + 1));
+        const unsigned tok = (unsigned)(me & tmask);
+        if (head) start = pos;
+        if (head && tail) alone |= 1u << j;
+        if (tok == endtok || tok == 0u) done |= 1u << j;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, start, o);
+        if (lane >= o) start = max(start, t);
+      }
+      grp[j] = max(start, last);
+      last = max(last, __shfl_sync(0xffffffffu, start, 31));
+    }
+    settled = alone | done;
+    if (lane == 0) sm.wsum[w] = last;
+    __syncthreads();
+    int mine = sm.wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, mine, o);
+      if (lane >= o) mine = max(mine, t);
+    }
+    const int all = __shfl_sync(0xffffffffu, mine, 31);
+    int before = __shfl_sync(0xffffffffu, mine, w > 0 ? w - 1 : 0);
+    if (w == 0) before = -1;
+    if (tid < nct) *cl.map_shared_rank(&sm.cmax[rank], tid) = all;
+    cl.sync();
+    for (int c = 0; c < rank; ++c) before = max(before, sm.cmax[c]);
+#pragma unroll
+    for (int j = 0; j < VO_ITEMS; ++j) grp[j] = max(grp[j], before);
+  }
+#pragma unroll
+  for (int j = 0; j < VO_ITEMS; ++j)
+    if (j < items && live_of(j)) order[rank * cap + slot_of(j)] = row0[cur * cap + slot_of(j)];
+}
+
+struct VnmRows {  // the original matrix by rows, and the state of the rounds
+  int m, M, V, nseg, tokbits;
+  long long ncells;
+  int *rowptr, *ccol, *packed;
+  int2* tlist;
+  unsigned *gtok, *ortab, *badtab;
+  int *counts, *order;
+};
+
+static size_t vnm_rows_bytes(int mp, int np, int nnz, long long ncells) {
+  const int nodes = mp > np ? mp : np;
+  return arena_bytes(mp + 1, 4) * 2 + arena_bytes(nnz + 1, 4) * 2 + arena_bytes(nodes, 4) + arena_bytes(mp, 8) +
+         2 * arena_bytes((ncells + 3) / 4 + 1, 4) + arena_bytes(2, 4) + arena_bytes(mp, 4) + scan_scratch_bytes(mp + 1) +
+         4096;
+}
+
+static vnm_status vnm_rows_build(vnm_ctx* ctx, int mp, int np, int nnz, const int* row, const int* col, int M, int V,
+                                 VnmRows& W) {
+  W.m = mp;
+  W.M = M;
+  W.V = V;
+  W.nseg = np / M;
+  W.ncells = (long long)((mp + V - 1) / V) * W.nseg;
+  W.tokbits = bits_for(2ll * W.nseg) + 9;
+  W.rowptr = arena_take<int>(ctx, mp + 1);
+  int* fill = arena_take<int>(ctx, mp + 1);
+  W.ccol = arena_take<int>(ctx, nnz + 1);
+  W.gtok = arena_take<unsigned>(ctx, nnz + 1);
+  W.packed = arena_take<int>(ctx, mp > np ? mp : np);
+  W.tlist = arena_take<int2>(ctx, mp);
+  W.ortab = arena_take<unsigned>(ctx, (W.ncells + 3) / 4 + 1);
+  W.badtab = arena_take<unsigned>(ctx, (W.ncells + 3) / 4 + 1);
+  W.counts = arena_take<int>(ctx, 2);
+  W.order = arena_take<int>(ctx, mp);
+  if (!W.rowptr || !fill || !W.ccol || !W.gtok || !W.packed || !W.tlist || !W.ortab || !W.badtab || !W.counts ||
+      !W.order)
+    return VNM_ERR_NOMEM;
+  VNM_CUDA_TRY(cudaMemsetAsync(W.rowptr, 0, sizeof(int) * (mp + 1), ctx->stream));
+  VNM_CUDA_TRY(cudaMemsetAsync(fill, 0, sizeof(int) * (mp + 1), ctx->stream));
+  if (nnz) VNM_LAUNCH(ctx, k_vs_rowcount, vs_grid(ctx, nnz), VS_NT, 0, row, nnz, W.rowptr);
+  VNM_TRY(exclusive_scan(ctx, W.rowptr, W.rowptr, mp + 1, nullptr));
+  if (nnz) VNM_LAUNCH(ctx, k_vs_rowfill, vs_grid(ctx, nnz), VS_NT, 0, row, col, nnz, W.rowptr, fill, W.ccol);
+  return VNM_OK;
+}
+
+// Tokens and V-block counts under the map `comp` (W.packed holds its places);
+// the counts come back in h[0..1].
+static vnm_status vnm_rows_analyse(vnm_ctx* ctx, VnmRows& W, const int* comp, int* h) {
+  const size_t tab = ((W.ncells + 3) / 4) * 4, smem = (size_t)VT_WARPS * ((W.nseg + 3) / 4) * 4;
+  VNM_CUDA_TRY(cudaMemsetAsync(W.counts, 0, 2 * sizeof(int), ctx->stream));
+  VNM_CUDA_TRY(cudaMemsetAsync(W.ortab, 0, tab, ctx->stream));
+  VNM_CUDA_TRY(cudaMemsetAsync(W.badtab, 0, tab, ctx->stream));
+  if (W.m > 0) {
+    VNM_CUDA_TRY(cudaFuncSetAttribute(k_vs_tokens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VNM_LAUNCH(ctx, k_vs_tokens, vs_grid(ctx, (long long)W.m * 32), VT_WARPS * 32, smem, W.rowptr, W.ccol, comp,
+               W.packed, W.m, W.M, W.nseg, W.V, W.tlist, W.gtok, W.ortab, W.badtab);
+  }
+  VNM_LAUNCH(ctx, k_vs_count, vs_grid(ctx, (W.ncells + 3) / 4), VS_NT, 0, W.ortab, W.badtab, W.ncells, W.counts);
+  VNM_CUDA_TRY(cudaMemcpyAsync(h, W.counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return VNM_OK;
+}
+
+// Launch shape of k_vs_order for m rows: a block for each 1024 rows (1, 2, 4,
+// 8 or 16, then more rows a block), fewer blocks where the GPU cannot hold
+// the cluster; false when the rows do not fit any it can hold.
+static bool vnm_order_shape(vnm_ctx* ctx, int m, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int& cap) {
+  int nct = 1;
+  while (nct < VO_MAX_CTAS && nct * VO_THREADS < m) nct *= 2;
+  cfg = cudaLaunchConfig_t{};
+  cfg.blockDim = dim3(VO_THREADS);
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  for (; nct >= 1; nct /= 2) {
+    cap = VO_THREADS;
+    while (nct * cap < m) cap *= 2;
+    if (cap > VO_MAX_CAP) break;
+    cfg.gridDim = dim3(nct);
+    cfg.dynamicSmemBytes = sizeof(OrderSmem) + (size_t)2 * cap * (sizeof(unsigned long long) + sizeof(int));
+    attr[0].val.clusterDim.x = (unsigned)nct;
+    int fit = 0;
+    if (cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
+            cudaSuccess &&
+        (nct <= 8 || cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                         cudaSuccess) &&
+        cudaOccupancyMaxActiveClusters(&fit, k_vs_order, &cfg) == cudaSuccess && fit >= 1)
+      return true;
+    (void)cudaGetLastError();
+  }
+  return false;
+}
+
+// W.order = the stable row order of reordering.py:219 for the analysed rows.
+static vnm_status vnm_rows_order(vnm_ctx* ctx, VnmRows& W) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  int cap = 0;
+  if (!vnm_order_shape(ctx, W.m, cfg, attr, cap)) return VNM_ERR_CUDA;
+  VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_vs_order, (const int2*)W.tlist, (const unsigned*)W.gtok, W.m, W.nseg,
+                                  W.tokbits, bits_for(W.m - 1), cap, W.order));
+  ctx->launches++;
+  return VNM_OK;
+}
+
+// Whether a call runs on the original rows: all rows fit a cluster the GPU
+// can hold, and every column's new place (the row map's) lies in a segment.
+// VNM_VS_ROWS=0 in the environment takes every call to the general path.
+static bool vnm_rows_fit(vnm_ctx* ctx, int mp, int np, int M) {
+  if (const char* e = getenv("VNM_VS_ROWS"))
+    if (atoi(e) == 0) return false;
+  if (mp > VO_MAX_ROWS || mp > np || np / M > VO_MAX_SEG || cudaSetDevice(ctx->device) != cudaSuccess) return false;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  int cap = 0;
+  return vnm_order_shape(ctx, mp, cfg, attr, cap);
+}
+
 }  // namespace vnm
 
 using namespace vnm;
@@ -381,7 +843,10 @@ vnm_status vnm_vnm_eval(vnm_ctx* ctx, int m, int n, int nnz, const int* row, con
   if (!out2) return VNM_ERR_ARG;
   const int mp = (m + M - 1) / M * M, np = (n + M - 1) / M * M;
   const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
-  VNM_TRY(arena_reserve(ctx, vnm_bytes(mp, nnz, ncells) + 2 * arena_bytes(nnz, 4)));
+  const bool rows = vnm_rows_fit(ctx, mp, np, M);
+  VNM_TRY(arena_reserve(ctx, (rows ? vnm_rows_bytes(mp, np, nnz, ncells) + arena_bytes(mp > np ? mp : np, 4)
+                                   : vnm_bytes(mp, nnz, ncells)) +
+                                 2 * arena_bytes(nnz, 4) + arena_bytes(1, 4)));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
   const int *d_row, *d_col;
@@ -394,11 +859,89 @@ vnm_status vnm_vnm_eval(vnm_ctx* ctx, int m, int n, int nnz, const int* row, con
   VNM_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (ctx->h_pinned[0]) return VNM_ERR_RANGE;
-  VnmWork W;
-  VNM_TRY(vnm_setup(ctx, m, n, nnz, M, V, W));
-  VNM_TRY(vnm_analyse(ctx, d_row, d_col, W, ctx->h_pinned));
+  if (rows) {
+    VnmRows W;
+    VNM_TRY(vnm_rows_build(ctx, mp, np, nnz, d_row, d_col, M, V, W));
+    const int nodes = mp > np ? mp : np;
+    int* comp = arena_take<int>(ctx, nodes);
+    if (!comp) return VNM_ERR_NOMEM;
+    VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, nodes), VS_NT, 0, nullptr, nullptr, nodes, M, comp, W.packed);
+    VNM_TRY(vnm_rows_analyse(ctx, W, comp, ctx->h_pinned));
+  } else {
+    VnmWork W;
+    VNM_TRY(vnm_setup(ctx, m, n, nnz, M, V, W));
+    VNM_TRY(vnm_analyse(ctx, d_row, d_col, W, ctx->h_pinned));
+  }
   out2[0] = ctx->h_pinned[0];
   out2[1] = ctx->h_pinned[1];
+  return end_call(ctx);
+}
+
+// vnm_vnm_reorder on the original rows: prev (accepted) and cur (candidate)
+// are node maps; the entries are relabelled once, at the end.
+static vnm_status reorder_rows(vnm_ctx* ctx, int mp, int np, int nnz, int* row, int* col, int mem, int M, int V,
+                               int maxiter, int* out5, int* newpos) {
+  const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
+  VNM_TRY(arena_reserve(ctx, vnm_rows_bytes(mp, np, nnz, ncells) + 2 * arena_bytes(nnz + 1, 4) +
+                                 2 * arena_bytes(mp > np ? mp : np, 4) + arena_bytes(1, 4)));
+  VNM_TRY(pinned_reserve(ctx, 64));
+  VNM_TRY(begin_call(ctx));
+  int* h = ctx->h_pinned;
+  const int nodes = mp > np ? mp : np;
+  int *d_row = row, *d_col = col;
+  if (mem == VNM_MEM_HOST && nnz) {
+    d_row = arena_take<int>(ctx, nnz);
+    d_col = arena_take<int>(ctx, nnz);
+    if (!d_row || !d_col) return VNM_ERR_NOMEM;
+    VNM_CUDA_TRY(cudaMemcpyAsync(d_row, row, sizeof(int) * nnz, cudaMemcpyHostToDevice, ctx->stream));
+    VNM_CUDA_TRY(cudaMemcpyAsync(d_col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  int* prev = arena_take<int>(ctx, nodes);
+  int* cur = arena_take<int>(ctx, nodes);
+  int* err = arena_take<int>(ctx, 1);
+  if (!prev || !cur || !err) return VNM_ERR_NOMEM;
+  VNM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  // columns index new_id[] (m entries), as in reordering.py:175-176
+  if (nnz) VNM_LAUNCH(ctx, k_vs_check, vs_grid(ctx, nnz), VS_NT, 0, d_row, d_col, nnz, mp, mp < np ? mp : np, err);
+  VNM_CUDA_TRY(cudaMemcpyAsync(h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (h[0]) return VNM_ERR_RANGE;
+  VnmRows W;
+  VNM_TRY(vnm_rows_build(ctx, mp, np, nnz, d_row, d_col, M, V, W));
+  VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, mp), VS_NT, 0, nullptr, nullptr, mp, M, prev, W.packed);
+  VNM_TRY(vnm_rows_analyse(ctx, W, prev, h));
+  const int init_inv = h[0], init_strict = h[1];
+  int inv = init_inv, prev_inv = init_inv, prev_strict = init_strict;
+  int round = 1;
+  const int MAXITER = init_inv > maxiter ? init_inv : maxiter;  // reordering.py:209-210
+  bool early = false;
+  while (inv > 0 && round <= MAXITER) {
+    VNM_TRY(vnm_rows_order(ctx, W));  // new_id[i] = sorted_data[i][0]
+    VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, mp), VS_NT, 0, prev, W.order, mp, M, cur, W.packed);
+    VNM_TRY(vnm_rows_analyse(ctx, W, cur, h));
+    inv = h[0];
+    if (inv > prev_inv) {  // reordering.py:242-246: keep the previous state
+      early = true;
+      break;
+    }
+    prev_inv = inv;
+    prev_strict = h[1];
+    std::swap(prev, cur);
+    round += 1;
+  }
+  out5[0] = init_inv;
+  out5[1] = init_strict;
+  out5[2] = prev_inv;
+  out5[3] = prev_strict;
+  out5[4] = early ? round : round - 1;
+  if (nnz) {
+    VNM_LAUNCH(ctx, k_vs_apply, vs_grid(ctx, nnz), VS_NT, 0, d_row, d_col, nnz, prev);
+    if (mem == VNM_MEM_HOST) {
+      VNM_CUDA_TRY(cudaMemcpyAsync(row, d_row, sizeof(int) * nnz, cudaMemcpyDeviceToHost, ctx->stream));
+      VNM_CUDA_TRY(cudaMemcpyAsync(col, d_col, sizeof(int) * nnz, cudaMemcpyDeviceToHost, ctx->stream));
+    }
+  }
+  if (newpos) VNM_CUDA_TRY(cudaMemcpyAsync(newpos, prev, sizeof(int) * mp, cudaMemcpyDeviceToHost, ctx->stream));
   return end_call(ctx);
 }
 
@@ -408,6 +951,7 @@ vnm_status vnm_vnm_reorder(vnm_ctx* ctx, int m, int n, int nnz, int* row, int* c
   if (!out5) return VNM_ERR_ARG;
   const int mp = (m + M - 1) / M * M, np = (n + M - 1) / M * M;
   const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
+  if (vnm_rows_fit(ctx, mp, np, M)) return reorder_rows(ctx, mp, np, nnz, row, col, mem, M, V, maxiter, out5, newpos);
   VNM_TRY(arena_reserve(ctx, vnm_bytes(mp, nnz, ncells)));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
