@@ -111,11 +111,14 @@ __global__ void k_vs_groups(const unsigned long long* keys, const int* gpos, int
   }
 }
 
-__global__ void k_vs_count(const unsigned* ortab, const unsigned* badtab, long long ncells, int* out2) {
+// `clear`: the tables are left zero for the next round.
+__global__ void k_vs_count(unsigned* ortab, unsigned* badtab, long long ncells, int* out2, bool clear) {
   int inv = 0, strict = 0;
   for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < (ncells + 3) / 4;
        w += (long long)gridDim.x * blockDim.x) {
     const unsigned o = ortab[w], b = badtab[w];
+    if (clear && o) ortab[w] = 0u;
+    if (clear && b) badtab[w] = 0u;
     for (int q = 0; q < 4; ++q) {
       if (w * 4 + q >= ncells) break;
       const unsigned ob = (o >> (8 * q)) & 0xffu;
@@ -124,14 +127,17 @@ __global__ void k_vs_count(const unsigned* ortab, const unsigned* badtab, long l
       strict += a || ((b >> (8 * q)) & 0xffu);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    inv += __shfl_xor_sync(0xffffffffu, inv, o);
-    strict += __shfl_xor_sync(0xffffffffu, strict, o);
+  __shared__ int sum[2];
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  inv = __reduce_add_sync(0xffffffffu, inv);
+  strict = __reduce_add_sync(0xffffffffu, strict);
+  if ((threadIdx.x & 31) == 0 && strict) {  // (an invalid block is also a strictly invalid one)
+    atomicAdd(&sum[0], inv);
+    atomicAdd(&sum[1], strict);
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&out2[0], inv);
-    atomicAdd(&out2[1], strict);
-  }
+  __syncthreads();
+  if (threadIdx.x < 2 && sum[threadIdx.x]) atomicAdd(&out2[threadIdx.x], sum[threadIdx.x]);
 }
 
 // first group of each row (groups are sorted by row)
@@ -275,7 +281,7 @@ static vnm_status vnm_analyse(vnm_ctx* ctx, const int* row, const int* col, VnmW
                W.gseg, W.gtok, W.ortab, W.badtab);
     VNM_CUDA_TRY(cudaMemcpyAsync(h2 + 2, d_ng, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   }
-  VNM_LAUNCH(ctx, k_vs_count, vs_grid(ctx, (W.ncells + 3) / 4), VS_NT, 0, W.ortab, W.badtab, W.ncells, W.counts);
+  VNM_LAUNCH(ctx, k_vs_count, vs_grid(ctx, (W.ncells + 3) / 4), VS_NT, 0, W.ortab, W.badtab, W.ncells, W.counts, false);
   VNM_CUDA_TRY(cudaMemcpyAsync(h2, W.counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (nnz > 0) W.ng = h2[2];
@@ -384,10 +390,11 @@ static vnm_status vnm_args(vnm_ctx* ctx, int m, int n, int nnz, const int* row, 
 // ---------------------------------------------------------------------------
 constexpr int VO_MAX_ROWS = 65536, VO_MAX_SEG = 16384;
 
+// A token of the rows' order, in bits_for(2 nseg) + 8 bits and never 0:
+// (rank + nseg) << 8, then h, or 256 + h of a negative one.
 __device__ __forceinline__ unsigned vs_token(unsigned bits, int s, int nseg) {
-  const int h = __popc(bits) <= 2 ? gray_rank(bits) : -gray_rank(bits);
-  const int rank = h > 0 ? (nseg - s) : -(nseg - s);
-  return ((unsigned)(rank + nseg) << 9) | (unsigned)(h + 256);
+  const int h = gray_rank(bits);
+  return __popc(bits) <= 2 ? (unsigned)(2 * nseg - s) << 8 | (unsigned)h : (unsigned)s << 8 | (unsigned)(256 - h);
 }
 
 // Entries per row; lanes of a warp with the same row add once.
@@ -425,116 +432,197 @@ __global__ void k_vs_map(const int* prev, const int* new_id, int m, int M, int* 
 // Token list of every row, at the row's place in the column list, and the
 // V-block tables; one warp a row.  A row of at most 32 entries is sorted in
 // registers; a longer one sets its bits in a bitmap of one byte a segment in
-// shared memory and reads the touched parts back in order.  Bound by the
-// gathers of `packed` and the atomics of the tables: 16384 rows, 262144
-// entries take 13 us, where sorting the entries by (row, column) took 130.
-constexpr int VT_WARPS = 8;
+// shared memory and reads the touched parts back in order; one of more than
+// VT_LONG takes a block of its own, the first `nlb` blocks walking the list of
+// those rows (on one warp a hub row's chain of gathers, and in one block the
+// hubs that share their low bits, set the kernel's time: 27 us at 16384 rows,
+// 262144 entries, 18 now).  Bound by the gathers of `packed` and the
+// atomics of the tables.
+constexpr int VT_WARPS = 8, VT_LONG = 128;
+// The rows of more than VT_LONG entries; *n counts them (zero on entry).
+__global__ void k_vs_long(const int* rowptr, int m, int* list, int* n) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
+    if (rowptr[r + 1] - rowptr[r] > VT_LONG) list[atomicAdd(n, 1)] = r;
+}
+
 __global__ void __launch_bounds__(VT_WARPS * 32)
     k_vs_tokens(const int* __restrict__ rowptr, const int* __restrict__ ccol, const int* __restrict__ comp,
-                const int* __restrict__ packed, int m, int M, int nseg, int V, int2* tlist, unsigned* gtok,
-                unsigned* ortab, unsigned* badtab) {
+                const int* __restrict__ packed, const int* __restrict__ longs, const int* __restrict__ nlong, int nlb,
+                int m, int M, int nseg, int V, int2* tlist, unsigned* gtok, unsigned* ortab, unsigned* badtab) {
   extern __shared__ unsigned vt_bitmap[];
-  const int nw = (nseg + 3) / 4;                          // words of a row's bitmap
-  const int part = ((nw + 31) / 32 + 31) / 32 * 32;       // words a bit of the touched mask stands for
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int wsum[VT_WARPS];
+  const int nw = (nseg + 3) / 4;                     // words of a row's bitmap
+  const int part = ((nw + 31) / 32 + 31) / 32 * 32;  // words a bit of the touched mask stands for
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned* bm = vt_bitmap + warp * nw;
-  for (int w = lane; w < nw; w += 32) bm[w] = 0u;
-  __syncwarp();
-  for (int q = blockIdx.x * VT_WARPS + warp; q < m; q += gridDim.x * VT_WARPS) {
-    const int b = rowptr[q], len = rowptr[q + 1] - b, cr = comp[q];
-    const long long cell0 = (long long)(cr / V) * nseg;
-    auto emit = [&](int s, unsigned bits, int at) {
-      gtok[b + at] = vs_token(bits, s, nseg);
-      const long long cell = cell0 + s;
-      atomicOr(&ortab[cell >> 2], bits << ((cell & 3) * 8));
-      if (__popc(bits) > 2) atomicOr(&badtab[cell >> 2], 1u << ((cell & 3) * 8));
-    };
-    int n = 0;
-    if (len <= 32) {
-      unsigned key = lane < len ? (unsigned)packed[ccol[b + lane]] : ~0u;
+  auto emit = [&](int b, long long cell0, int s, unsigned bits, int at) {
+    gtok[b + at] = vs_token(bits, s, nseg);
+    const long long cell = cell0 + s;
+    atomicOr(&ortab[cell >> 2], bits << ((cell & 3) * 8));
+    if (__popc(bits) > 2) atomicOr(&badtab[cell >> 2], 1u << ((cell & 3) * 8));
+  };
+  // entries first, first + step, ... of row b .. b + len into the bitmap t; the parts of it that were touched
+  auto set_bits = [&](unsigned* t, int b, int len, int first, int step) {
+    constexpr int U = 4;  // entries a lane in flight
+    unsigned touched = 0;
+    for (int e0 = first; e0 < len; e0 += step * U) {
+      int c[U], p[U];
 #pragma unroll
-      for (int k = 2; k <= 32; k <<= 1)
+      for (int u = 0; u < U; ++u) c[u] = e0 + step * u < len ? ccol[b + e0 + step * u] : -1;
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          const unsigned other = __shfl_xor_sync(0xffffffffu, key, j);
-          const bool up = (lane & k) == 0, low = (lane & j) == 0;
-          key = (low == up) ? min(key, other) : max(key, other);
+      for (int u = 0; u < U; ++u) p[u] = c[u] >= 0 ? packed[c[u]] : 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) {
+          const int s = p[u] >> 3;
+          atomicOr(&t[s >> 2], (1u << (M - 1 - (p[u] & 7))) << ((s & 3) * 8));
+          touched |= 1u << ((s >> 2) / part);
         }
-      const unsigned s = key >> 3;
-      const bool valid = key != ~0u;
-      unsigned bits = valid ? 1u << (M - 1 - (int)(key & 7u)) : 0u;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {  // OR over the lanes of the same segment from here on
-        const unsigned t = __shfl_down_sync(0xffffffffu, bits, o), ts = __shfl_down_sync(0xffffffffu, s, o);
-        if (lane + o < 32 && ts == s) bits |= t;
-      }
-      const unsigned ps = __shfl_up_sync(0xffffffffu, s, 1);
-      const unsigned heads = __ballot_sync(0xffffffffu, valid && (lane == 0 || ps != s));
-      if ((heads >> lane) & 1u) emit((int)s, bits, __popc(heads & ((1u << lane) - 1u)));
-      n = __popc(heads);
-    } else {
-      unsigned touched = 0;
-      for (int e = lane; e < len; e += 32) {
-        const int p = packed[ccol[b + e]], s = p >> 3;
-        atomicOr(&bm[s >> 2], (1u << (M - 1 - (p & 7))) << ((s & 3) * 8));
-        touched |= 1u << ((s >> 2) / part);
-      }
-      touched = __reduce_or_sync(0xffffffffu, touched);
-      __syncwarp();
-      for (; touched; touched &= touched - 1) {
-        const int w0 = (__ffs(touched) - 1) * part, w1 = min(w0 + part, nw);
-        for (int w = w0 + lane; w - lane < w1; w += 32) {
-          unsigned word = 0;
-          if (w < w1) {
-            word = bm[w];
-            bm[w] = 0u;
-          }
-          if (!__any_sync(0xffffffffu, word != 0u)) continue;
-          int c = 0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) c += ((word >> (8 * k)) & 0xffu) ? 1 : 0;
-          int incl = c;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-          }
-          int at = n + incl - c;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const unsigned bits = (word >> (8 * k)) & 0xffu;
-            if (bits) emit(4 * w + k, bits, at++);
-          }
-          n += __shfl_sync(0xffffffffu, incl, 31);
-        }
-      }
-      __syncwarp();
     }
-    if (lane == 0) tlist[cr] = make_int2(b, n);
+    return touched;
+  };
+  auto nonzero_bytes = [](unsigned word) {
+    int c = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c += ((word >> (8 * k)) & 0xffu) ? 1 : 0;
+    return c;
+  };
+  auto warp_incl = [&](int v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
+    }
+    return v;
+  };
+  if ((int)blockIdx.x < nlb) {  // the long rows, in the first warp's bitmap
+    const int nl = *nlong;
+    if ((int)blockIdx.x >= nl) return;
+    for (int w = tid; w < nw; w += VT_WARPS * 32) vt_bitmap[w] = 0u;
+    for (int i = blockIdx.x; i < nl; i += nlb) {
+      const int q = longs[i], b = rowptr[q], cr = comp[q];
+      const long long cell0 = (long long)(cr / V) * nseg;
+      __syncthreads();
+      set_bits(vt_bitmap, b, rowptr[q + 1] - b, tid, VT_WARPS * 32);
+      __syncthreads();
+      int n = 0;
+      for (int w0 = 0; w0 < nw; w0 += VT_WARPS * 32) {
+        const int w = w0 + tid;
+        unsigned word = 0;
+        if (w < nw) {
+          word = vt_bitmap[w];
+          vt_bitmap[w] = 0u;
+        }
+        const int c = nonzero_bytes(word), incl = warp_incl(c);
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int at = n + incl - c;
+#pragma unroll
+        for (int u = 0; u < VT_WARPS; ++u) {
+          if (u < warp) at += wsum[u];
+          n += wsum[u];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned bits = (word >> (8 * k)) & 0xffu;
+          if (bits) emit(b, cell0, 4 * w + k, bits, at++);
+        }
+        __syncthreads();
+      }
+      if (tid == 0) tlist[cr] = make_int2(b, n);
+    }
+    return;
+  }
+  bool clean = false;  // this warp's bitmap is zero
+  for (int q = ((int)blockIdx.x - nlb) * VT_WARPS + warp; q < m; q += ((int)gridDim.x - nlb) * VT_WARPS) {
+    const int b = rowptr[q], len = rowptr[q + 1] - b;
+    if (len > VT_LONG) continue;
+    {
+      const int cr = comp[q];
+      const long long cell0 = (long long)(cr / V) * nseg;
+      int n = 0;
+      if (len <= 32) {
+        unsigned key = lane < len ? (unsigned)packed[ccol[b + lane]] : ~0u;
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+          for (int j = k >> 1; j > 0; j >>= 1) {
+            const unsigned other = __shfl_xor_sync(0xffffffffu, key, j);
+            const bool up = (lane & k) == 0, low = (lane & j) == 0;
+            key = (low == up) ? min(key, other) : max(key, other);
+          }
+        const unsigned s = key >> 3;
+        const bool valid = key != ~0u;
+        unsigned bits = valid ? 1u << (M - 1 - (int)(key & 7u)) : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {  // OR over the lanes of the same segment from here on
+          const unsigned t = __shfl_down_sync(0xffffffffu, bits, o), ts = __shfl_down_sync(0xffffffffu, s, o);
+          if (lane + o < 32 && ts == s) bits |= t;
+        }
+        const unsigned ps = __shfl_up_sync(0xffffffffu, s, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, valid && (lane == 0 || ps != s));
+        if ((heads >> lane) & 1u) emit(b, cell0, (int)s, bits, __popc(heads & ((1u << lane) - 1u)));
+        n = __popc(heads);
+      } else {
+        if (!clean)
+          for (int w = lane; w < nw; w += 32) bm[w] = 0u;
+        clean = true;
+        __syncwarp();
+        unsigned touched = __reduce_or_sync(0xffffffffu, set_bits(bm, b, len, lane, 32));
+        __syncwarp();
+        for (; touched; touched &= touched - 1) {
+          const int w0 = (__ffs(touched) - 1) * part, w1 = min(w0 + part, nw);
+          for (int w = w0 + lane; w - lane < w1; w += 32) {
+            unsigned word = 0;
+            if (w < w1) {
+              word = bm[w];
+              bm[w] = 0u;
+            }
+            if (!__any_sync(0xffffffffu, word != 0u)) continue;
+            const int c = nonzero_bytes(word), incl = warp_incl(c);
+            int at = n + incl - c;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const unsigned bits = (word >> (8 * k)) & 0xffu;
+              if (bits) emit(b, cell0, 4 * w + k, bits, at++);
+            }
+            n += __shfl_sync(0xffffffffu, incl, 31);
+          }
+        }
+        __syncwarp();
+      }
+      if (lane == 0) tlist[cr] = make_int2(b, n);
+    }
   }
 }
 
 // The stable order of the rows by their token lists, in the shared memory of
 // one thread-block cluster: position p lives in block p / cap (cap a power of
-// two).  Level k sorts the rows by (start of the row's group so far, k-th
-// token) with a stable radix sort of VO_BITS-bit digits, then splits the
-// groups; rows alone in their group, or at the end of their list, keep their
-// place.  A digit takes two cluster barriers: each warp ranks its 32-row
-// chunks with __match_any, the blocks exchange their digit counts, and every
-// row goes straight to its place in the other buffer, in whichever block.
-// Bound by latency: a digit takes about 2 us at 16384 rows on 16 blocks, where
-// a pass of the multi-kernel radix sort took 23.
+// two).  A row is one 64-bit word, its sort key above its id (16 bits).
+// First all rows are sorted by their first two tokens; then each level sorts
+// the rows of a group (rows equal so far) by their next token and splits the
+// groups; a row alone in its group, or at the end of its list, keeps its
+// place.  Sorting is a stable radix sort of VO_BITS-bit digits (two cluster
+// barriers a digit: each warp ranks its 32-row chunks with __match_any, the
+// blocks exchange their digit counts, and every row goes straight to its
+// place in the other buffer, in whichever block), or, where the largest group
+// has at most VO_COUNT rows (on R-MAT 16384 76 after two tokens, 9 after
+// three), every row counts the rows of its group that come before it.
+// Bound by latency and the scattered stores between the blocks.  At 16384
+// rows on 16 blocks VO_MEASURED.
 constexpr int VO_BITS = 9, VO_BINS = 1 << VO_BITS, VO_THREADS = 1024, VO_WARPS = 32, VO_ITEMS = 4, VO_MAX_CTAS = 16;
+constexpr int VO_COUNT = 256, VO_ID = 16;
 constexpr int VO_MAX_CAP = VO_THREADS * VO_ITEMS;
-static_assert(VO_MAX_CAP * VO_MAX_CTAS == VO_MAX_ROWS, "all rows fit the largest cluster");
+static_assert(VO_MAX_CAP * VO_MAX_CTAS == VO_MAX_ROWS && VO_MAX_ROWS <= 1 << VO_ID, "all rows fit the largest cluster");
 struct alignas(16) OrderSmem {
   uint16_t whist[VO_WARPS][VO_BINS];       // a warp's digit counts, then the counts of the warps before it
   uint32_t tot[VO_BINS / 2];               // this block's digit counts, two to a word
   uint32_t ctot[VO_MAX_CTAS][VO_BINS / 2]; // every block's
   int base[VO_BINS];                       // where this block's rows of a digit go
   int wsum[VO_WARPS];
-  int cmax[VO_MAX_CTAS];                   // every block's last group start
-  int act[VO_MAX_CTAS];                    // whether a block has rows to split
+  int wbig[VO_WARPS];
+  int cmax[VO_MAX_CTAS];                   // every block's last group start,
+  int cbig[VO_MAX_CTAS];                   // largest group that can still be split (0: none)
 };
 
 __global__ void __launch_bounds__(VO_THREADS, 1)
@@ -542,57 +630,33 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
                int grpbits, int cap, int* order) {
   extern __shared__ __align__(16) unsigned char vo_raw[];
   OrderSmem& sm = *reinterpret_cast<OrderSmem*>(vo_raw);
-  auto* const key0 = reinterpret_cast<unsigned long long*>(vo_raw + sizeof(OrderSmem));  // [2][cap]
-  auto* const row0 = reinterpret_cast<int*>(key0 + 2 * cap);                             // [2][cap]
+  auto* const buf = reinterpret_cast<unsigned long long*>(vo_raw + sizeof(OrderSmem));  // [2][cap]
   cg::cluster_group cl = cg::this_cluster();
   const int nct = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int capb = 31 - __clz(cap);
-  const int items = cap >= VO_THREADS ? cap / VO_THREADS : 1;  // 32-row chunks a warp
-  // slot of this lane's item j; with fewer rows than threads the first warps have them
-  auto slot_of = [&](int j) { return (w * items + j) * 32 + lane; };
-  auto live_of = [&](int j) { return slot_of(j) < cap && rank * cap + slot_of(j) < m; };
-  const unsigned endtok = ((unsigned)nseg << 9) | 256u;
-  const unsigned long long tmask = (1ull << tokbits) - 1;
-  int grp[VO_ITEMS];      // start of the group of each of this lane's positions
-  unsigned settled = 0;   // bit j: position j keeps its row
-#pragma unroll
-  for (int j = 0; j < VO_ITEMS; ++j) {
-    grp[j] = 0;
-    if (j < items && live_of(j)) row0[slot_of(j)] = rank * cap + slot_of(j);
-  }
+  const int items = cap / VO_THREADS;  // 32-row chunks a warp
+  auto slot_of = [&](int j) { return (w * items + j) * 32 + lane; };  // of this lane's item j
+  auto live_of = [&](int j) { return rank * cap + slot_of(j) < m; };
+  const unsigned endtok = (unsigned)nseg << 8, idmask = (1u << VO_ID) - 1u;
   int cur = 0;
-  __syncthreads();
-  for (int k = 0;; ++k) {
-    unsigned long long* key = key0 + cur * cap;
-    int act = 0;
-#pragma unroll
-    for (int j = 0; j < VO_ITEMS; ++j)
-      if (j < items && live_of(j)) {
-        unsigned tok = 0;
-        if (!((settled >> j) & 1u)) {
-          const int2 t = tlist[row0[cur * cap + slot_of(j)]];
-          tok = k < t.y ? gtok[t.x + k] : endtok;
-          act = 1;
-        }
-        key[slot_of(j)] = (unsigned long long)(unsigned)grp[j] << tokbits | tok;
-      }
-    act = __syncthreads_or(act);
-    if (tid < nct) *cl.map_shared_rank(&sm.act[rank], tid) = act;
-    const int bits = tokbits + (k > 0 ? grpbits : 0);  // one group at first
-    bool any = true;
-    for (int shift = 0; shift < bits; shift += VO_BITS) {
-      key = key0 + cur * cap;
-      int* row = row0 + cur * cap;
+
+  // stable radix sort of the current buffer by bits VO_ID .. VO_ID + bits - 1
+  auto radix = [&](int bits) {
+    for (int shift = VO_ID; shift < VO_ID + bits; shift += VO_BITS) {
+      const unsigned long long* key = buf + cur * cap;
       uint32_t* wh = reinterpret_cast<uint32_t*>(&sm.whist[0][0]);
-      for (int i = tid; i < VO_WARPS * VO_BINS / 2; i += VO_THREADS) wh[i] = 0u;
+      for (int i = tid; i < VO_WARPS * VO_BINS / 8; i += VO_THREADS)
+        reinterpret_cast<uint4*>(wh)[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
+      unsigned long long v[VO_ITEMS];
       int dig[VO_ITEMS], at[VO_ITEMS];
 #pragma unroll
       for (int j = 0; j < VO_ITEMS; ++j) {
         if (j >= items) break;
         const bool live = live_of(j);
-        dig[j] = live ? (int)(key[slot_of(j)] >> shift) & (VO_BINS - 1) : VO_BINS + lane;
+        v[j] = live ? key[slot_of(j)] : 0ull;
+        dig[j] = live ? (int)(v[j] >> shift) & (VO_BINS - 1) : VO_BINS + lane;
         const unsigned peers = __match_any_sync(0xffffffffu, dig[j]);
         at[j] = live ? sm.whist[w][dig[j]] + __popc(peers & ((1u << lane) - 1u)) : 0;
         __syncwarp();
@@ -603,9 +667,9 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
       if (tid < VO_BINS / 2) {  // counts of the warps before, two digits a thread (no carry: at most cap)
         uint32_t run = 0;
 #pragma unroll 8
-        for (int v = 0; v < VO_WARPS; ++v) {
-          const uint32_t c = wh[v * (VO_BINS / 2) + tid];
-          wh[v * (VO_BINS / 2) + tid] = run;
+        for (int u = 0; u < VO_WARPS; ++u) {
+          const uint32_t c = wh[u * (VO_BINS / 2) + tid];
+          wh[u * (VO_BINS / 2) + tid] = run;
           run += c;
         }
         sm.tot[tid] = run;
@@ -614,12 +678,6 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
       for (int i = tid; i < nct * (VO_BINS / 2); i += VO_THREADS)
         *cl.map_shared_rank(&sm.ctot[rank][i % (VO_BINS / 2)], i / (VO_BINS / 2)) = sm.tot[i % (VO_BINS / 2)];
       cl.sync();
-      if (shift == 0) {
-        int a = 0;
-        for (int c = 0; c < nct; ++c) a |= sm.act[c];
-        any = a != 0;
-        if (!any) break;  // the same in every block
-      }
       if (tid < VO_BINS / 2) {
         int lo = 0, hi = 0, blo = 0, bhi = 0;  // all blocks' counts, and of the blocks before this one
         for (int c = 0; c < nct; ++c) {
@@ -642,42 +700,44 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
         sm.base[2 * tid + 1] = incl - hi + bhi;
       }
       __syncthreads();
-      {
-        unsigned long long* const okey = key0 + (cur ^ 1) * cap;
-        int* const orow = row0 + (cur ^ 1) * cap;
+      unsigned long long* const out = buf + (cur ^ 1) * cap;
 #pragma unroll
-        for (int j = 0; j < VO_ITEMS; ++j)
-          if (j < items && live_of(j)) {
-            int before = 0;
-            for (int v = 0; v < dig[j] >> 6; ++v) before += sm.wsum[v];
-            const int dst = sm.base[dig[j]] + before + sm.whist[w][dig[j]] + at[j];
-            const int blk = dst >> capb, sl = dst & (cap - 1);
-            *cl.map_shared_rank(okey + sl, blk) = key[slot_of(j)];
-            *cl.map_shared_rank(orow + sl, blk) = row[slot_of(j)];
-          }
-      }
+      for (int j = 0; j < VO_ITEMS; ++j)
+        if (j < items && live_of(j)) {
+          int before = 0;
+          for (int u = 0; u < dig[j] >> 6; ++u) before += sm.wsum[u];
+          const int dst = sm.base[dig[j]] + before + sm.whist[w][dig[j]] + at[j];
+          *cl.map_shared_rank(out + (dst & (cap - 1)), dst >> capb) = v[j];
+        }
       cl.sync();
       cur ^= 1;
     }
-    if (!any) break;
-    // split the groups: a row starts one when its key differs from the one before
-    key = key0 + cur * cap;
+  };
+
+  int grp[VO_ITEMS];     // start of the group of each of this lane's positions
+  unsigned settled = 0;  // bit j: position j keeps its row
+  // Split the groups: a row starts one when its key differs from the one
+  // before, and is settled when it is alone in it or its list has ended
+  // (ended(key)).  Returns the size of the largest group left to split.
+  auto split = [&](auto&& ended) -> int {
+    const unsigned long long* key = buf + cur * cap;
     int last = -1;  // the last group start up to here, of this warp
-    unsigned alone = 0, done = 0;
+    unsigned alone = 0, done = 0, tails = 0;
 #pragma unroll
     for (int j = 0; j < VO_ITEMS; ++j) {
       if (j >= items) break;
       const int sl = slot_of(j), pos = rank * cap + sl;
       int start = -1;
       if (live_of(j)) {
-        const unsigned long long me = key[sl];
-        const bool head = pos == 0 || me != (sl > 0 ? key[sl - 1] : *cl.map_shared_rank(key + cap - 1, rank - 1));
+        const unsigned long long me = key[sl] >> VO_ID;
+        const bool head =
+            pos == 0 || me != (sl > 0 ? key[sl - 1] : *cl.map_shared_rank(key + cap - 1, rank - 1)) >> VO_ID;
         const bool tail =
-            pos == m - 1 || me != (sl + 1 < cap ? key[sl + 1] : *cl.map_shared_rank(key, rank + 1));
-        const unsigned tok = (unsigned)(me & tmask);
+            pos == m - 1 || me != (sl + 1 < cap ? key[sl + 1] : *cl.map_shared_rank(key, rank + 1)) >> VO_ID;
         if (head) start = pos;
+        if (tail) tails |= 1u << j;
         if (head && tail) alone |= 1u << j;
-        if (tok == endtok || tok == 0u) done |= 1u << j;
+        if (ended(me)) done |= 1u << j;
       }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -702,12 +762,86 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
     if (tid < nct) *cl.map_shared_rank(&sm.cmax[rank], tid) = all;
     cl.sync();
     for (int c = 0; c < rank; ++c) before = max(before, sm.cmax[c]);
+    int big = 0;
 #pragma unroll
-    for (int j = 0; j < VO_ITEMS; ++j) grp[j] = max(grp[j], before);
+    for (int j = 0; j < VO_ITEMS; ++j) {
+      if (j >= items) break;
+      grp[j] = max(grp[j], before);
+      if (((tails & ~settled) >> j) & 1u) big = max(big, rank * cap + slot_of(j) - grp[j] + 1);
+    }
+    big = __reduce_max_sync(0xffffffffu, big);
+    if (lane == 0) sm.wbig[w] = big;
+    __syncthreads();
+    if (tid < nct) {
+      int b = 0;
+      for (int u = 0; u < VO_WARPS; ++u) b = max(b, sm.wbig[u]);
+      *cl.map_shared_rank(&sm.cbig[rank], tid) = b;
+    }
+    cl.sync();
+    int b = 0;
+    for (int c = 0; c < nct; ++c) b = max(b, sm.cbig[c]);
+    return b;
+  };
+
+#pragma unroll
+  for (int j = 0; j < VO_ITEMS; ++j)
+    if (j < items && live_of(j)) {
+      const int r = rank * cap + slot_of(j);
+      const int2 t = tlist[r];
+      const unsigned t0 = t.y > 0 ? gtok[t.x] : endtok, t1 = t.y > 1 ? gtok[t.x + 1] : t.y == 1 ? endtok : 0u;
+      buf[slot_of(j)] = ((unsigned long long)t0 << tokbits | t1) << VO_ID | (unsigned)r;
+    }
+  cl.sync();  // every block has started before any remote access
+  radix(2 * tokbits);
+  const unsigned tmask = (1u << tokbits) - 1u;
+  int big = split([&](unsigned long long k) { return ((unsigned)k & tmask) == endtok || ((unsigned)k & tmask) == 0u; });
+  for (int k = 2; big > 1; ++k) {
+    // keys: the group, the next token (0 for a settled row)
+    unsigned long long* key = buf + cur * cap;
+    unsigned tok[VO_ITEMS];
+#pragma unroll
+    for (int j = 0; j < VO_ITEMS; ++j)
+      if (j < items && live_of(j)) {
+        const unsigned r = (unsigned)key[slot_of(j)] & idmask;
+        tok[j] = 0;
+        if (!((settled >> j) & 1u)) {
+          const int2 t = tlist[r];
+          tok[j] = k < t.y ? gtok[t.x + k] : endtok;
+        }
+        key[slot_of(j)] = ((unsigned long long)(unsigned)grp[j] << tokbits | tok[j]) << VO_ID | r;
+      }
+    cl.sync();
+    if (big > VO_COUNT) {
+      radix(tokbits + grpbits);
+    } else {
+      unsigned long long* const out = buf + (cur ^ 1) * cap;
+#pragma unroll
+      for (int j = 0; j < VO_ITEMS; ++j)
+        if (j < items && live_of(j)) {
+          const int pos = rank * cap + slot_of(j);
+          int dst = pos;
+          if (!((settled >> j) & 1u)) {
+            auto at = [&](int p) {
+              return (p >> capb) == rank ? key[p & (cap - 1)] : *cl.map_shared_rank(key + (p & (cap - 1)), p >> capb);
+            };
+            dst = grp[j];
+            for (int p = grp[j]; p < pos; ++p) dst += ((unsigned)(at(p) >> VO_ID) & tmask) <= tok[j] ? 1 : 0;
+            for (int p = pos + 1; p < m; ++p) {
+              const unsigned long long o = at(p) >> VO_ID;
+              if ((int)(o >> tokbits) != grp[j]) break;
+              dst += ((unsigned)o & tmask) < tok[j] ? 1 : 0;
+            }
+          }
+          *cl.map_shared_rank(out + (dst & (cap - 1)), dst >> capb) = key[slot_of(j)];
+        }
+      cl.sync();
+      cur ^= 1;
+    }
+    big = split([&](unsigned long long q) { return ((unsigned)q & tmask) == endtok || ((unsigned)q & tmask) == 0u; });
   }
 #pragma unroll
   for (int j = 0; j < VO_ITEMS; ++j)
-    if (j < items && live_of(j)) order[rank * cap + slot_of(j)] = row0[cur * cap + slot_of(j)];
+    if (j < items && live_of(j)) order[rank * cap + slot_of(j)] = (int)((unsigned)buf[cur * cap + slot_of(j)] & idmask);
 }
 
 struct VnmRows {  // the original matrix by rows, and the state of the rounds
@@ -717,12 +851,18 @@ struct VnmRows {  // the original matrix by rows, and the state of the rounds
   int2* tlist;
   unsigned *gtok, *ortab, *badtab;
   int *counts, *order;
+  int* longs;                 // how many rows of more than VT_LONG entries, and the rows
+  int round = 0;              // analyses so far
+  cudaLaunchConfig_t cfg;     // launch shape of k_vs_order
+  cudaLaunchAttribute attr[1];
+  int cap = 0;
 };
+constexpr int VO_COUNTS = 64;
 
 static size_t vnm_rows_bytes(int mp, int np, int nnz, long long ncells) {
   const int nodes = mp > np ? mp : np;
-  return arena_bytes(mp + 1, 4) * 2 + arena_bytes(nnz + 1, 4) * 2 + arena_bytes(nodes, 4) + arena_bytes(mp, 8) +
-         2 * arena_bytes((ncells + 3) / 4 + 1, 4) + arena_bytes(2, 4) + arena_bytes(mp, 4) + scan_scratch_bytes(mp + 1) +
+  return arena_bytes(mp + 1, 4) * 3 + arena_bytes(nnz + 1, 4) * 2 + arena_bytes(nodes, 4) + arena_bytes(mp, 8) +
+         2 * arena_bytes((ncells + 3) / 4 + 1, 4) + arena_bytes(64, 4) + arena_bytes(mp, 4) + scan_scratch_bytes(mp + 1) +
          4096;
 }
 
@@ -733,7 +873,7 @@ static vnm_status vnm_rows_build(vnm_ctx* ctx, int mp, int np, int nnz, const in
   W.V = V;
   W.nseg = np / M;
   W.ncells = (long long)((mp + V - 1) / V) * W.nseg;
-  W.tokbits = bits_for(2ll * W.nseg) + 9;
+  W.tokbits = bits_for(2ll * W.nseg) + 8;
   W.rowptr = arena_take<int>(ctx, mp + 1);
   int* fill = arena_take<int>(ctx, mp + 1);
   W.ccol = arena_take<int>(ctx, nnz + 1);
@@ -742,33 +882,38 @@ static vnm_status vnm_rows_build(vnm_ctx* ctx, int mp, int np, int nnz, const in
   W.tlist = arena_take<int2>(ctx, mp);
   W.ortab = arena_take<unsigned>(ctx, (W.ncells + 3) / 4 + 1);
   W.badtab = arena_take<unsigned>(ctx, (W.ncells + 3) / 4 + 1);
-  W.counts = arena_take<int>(ctx, 2);
+  W.counts = arena_take<int>(ctx, VO_COUNTS);
   W.order = arena_take<int>(ctx, mp);
-  if (!W.rowptr || !fill || !W.ccol || !W.gtok || !W.packed || !W.tlist || !W.ortab || !W.badtab || !W.counts ||
+  W.longs = arena_take<int>(ctx, mp + 1);
+  if (!W.longs || !W.rowptr || !fill || !W.ccol || !W.gtok || !W.packed || !W.tlist || !W.ortab || !W.badtab || !W.counts ||
       !W.order)
     return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemsetAsync(W.rowptr, 0, sizeof(int) * (mp + 1), ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(fill, 0, sizeof(int) * (mp + 1), ctx->stream));
+  VNM_CUDA_TRY(cudaMemsetAsync(W.ortab, 0, ((W.ncells + 3) / 4) * 4, ctx->stream));
+  VNM_CUDA_TRY(cudaMemsetAsync(W.badtab, 0, ((W.ncells + 3) / 4) * 4, ctx->stream));
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_vs_tokens, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    VT_WARPS * ((VO_MAX_SEG + 3) / 4) * 4));
   if (nnz) VNM_LAUNCH(ctx, k_vs_rowcount, vs_grid(ctx, nnz), VS_NT, 0, row, nnz, W.rowptr);
   VNM_TRY(exclusive_scan(ctx, W.rowptr, W.rowptr, mp + 1, nullptr));
   if (nnz) VNM_LAUNCH(ctx, k_vs_rowfill, vs_grid(ctx, nnz), VS_NT, 0, row, col, nnz, W.rowptr, fill, W.ccol);
+  VNM_CUDA_TRY(cudaMemsetAsync(W.longs, 0, sizeof(int), ctx->stream));
+  if (mp) VNM_LAUNCH(ctx, k_vs_long, vs_grid(ctx, mp), VS_NT, 0, W.rowptr, mp, W.longs + 1, W.longs);
   return VNM_OK;
 }
 
 // Tokens and V-block counts under the map `comp` (W.packed holds its places);
 // the counts come back in h[0..1].
 static vnm_status vnm_rows_analyse(vnm_ctx* ctx, VnmRows& W, const int* comp, int* h) {
-  const size_t tab = ((W.ncells + 3) / 4) * 4, smem = (size_t)VT_WARPS * ((W.nseg + 3) / 4) * 4;
-  VNM_CUDA_TRY(cudaMemsetAsync(W.counts, 0, 2 * sizeof(int), ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(W.ortab, 0, tab, ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(W.badtab, 0, tab, ctx->stream));
-  if (W.m > 0) {
-    VNM_CUDA_TRY(cudaFuncSetAttribute(k_vs_tokens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    VNM_LAUNCH(ctx, k_vs_tokens, vs_grid(ctx, (long long)W.m * 32), VT_WARPS * 32, smem, W.rowptr, W.ccol, comp,
-               W.packed, W.m, W.M, W.nseg, W.V, W.tlist, W.gtok, W.ortab, W.badtab);
-  }
-  VNM_LAUNCH(ctx, k_vs_count, vs_grid(ctx, (W.ncells + 3) / 4), VS_NT, 0, W.ortab, W.badtab, W.ncells, W.counts);
-  VNM_CUDA_TRY(cudaMemcpyAsync(h, W.counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  if (W.m > 0)
+    VNM_LAUNCH(ctx, k_vs_tokens, 2 * ctx->num_sms + vs_grid(ctx, (long long)W.m * 32), VT_WARPS * 32,
+               (size_t)VT_WARPS * ((W.nseg + 3) / 4) * 4, W.rowptr, W.ccol, comp, W.packed, W.longs + 1, W.longs,
+               2 * ctx->num_sms, W.m, W.M, W.nseg, W.V,
+               W.tlist, W.gtok, W.ortab, W.badtab);
+  int* counts = W.counts + 2 * W.round++ % VO_COUNTS;  // a pair of its own for each of the next rounds
+  if (counts == W.counts) VNM_CUDA_TRY(cudaMemsetAsync(W.counts, 0, VO_COUNTS * sizeof(int), ctx->stream));
+  VNM_LAUNCH(ctx, k_vs_count, vs_grid(ctx, (W.ncells + 3) / 4), VS_NT, 0, W.ortab, W.badtab, W.ncells, counts, true);
+  VNM_CUDA_TRY(cudaMemcpyAsync(h, counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return VNM_OK;
 }
@@ -792,7 +937,7 @@ static bool vnm_order_shape(vnm_ctx* ctx, int m, cudaLaunchConfig_t& cfg, cudaLa
     while (nct * cap < m) cap *= 2;
     if (cap > VO_MAX_CAP) break;
     cfg.gridDim = dim3(nct);
-    cfg.dynamicSmemBytes = sizeof(OrderSmem) + (size_t)2 * cap * (sizeof(unsigned long long) + sizeof(int));
+    cfg.dynamicSmemBytes = sizeof(OrderSmem) + (size_t)2 * cap * sizeof(unsigned long long);
     attr[0].val.clusterDim.x = (unsigned)nct;
     int fit = 0;
     if (cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
@@ -808,12 +953,8 @@ static bool vnm_order_shape(vnm_ctx* ctx, int m, cudaLaunchConfig_t& cfg, cudaLa
 
 // W.order = the stable row order of reordering.py:219 for the analysed rows.
 static vnm_status vnm_rows_order(vnm_ctx* ctx, VnmRows& W) {
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  int cap = 0;
-  if (!vnm_order_shape(ctx, W.m, cfg, attr, cap)) return VNM_ERR_CUDA;
-  VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_vs_order, (const int2*)W.tlist, (const unsigned*)W.gtok, W.m, W.nseg,
-                                  W.tokbits, bits_for(W.m - 1), cap, W.order));
+  VNM_CUDA_TRY(cudaLaunchKernelEx(&W.cfg, k_vs_order, (const int2*)W.tlist, (const unsigned*)W.gtok, W.m, W.nseg,
+                                  W.tokbits, bits_for(W.m - 1), W.cap, W.order));
   ctx->launches++;
   return VNM_OK;
 }
@@ -821,14 +962,11 @@ static vnm_status vnm_rows_order(vnm_ctx* ctx, VnmRows& W) {
 // Whether a call runs on the original rows: all rows fit a cluster the GPU
 // can hold, and every column's new place (the row map's) lies in a segment.
 // VNM_VS_ROWS=0 in the environment takes every call to the general path.
-static bool vnm_rows_fit(vnm_ctx* ctx, int mp, int np, int M) {
+static bool vnm_rows_fit(vnm_ctx* ctx, int mp, int np, int M, VnmRows& W) {
   if (const char* e = getenv("VNM_VS_ROWS"))
     if (atoi(e) == 0) return false;
   if (mp > VO_MAX_ROWS || mp > np || np / M > VO_MAX_SEG || cudaSetDevice(ctx->device) != cudaSuccess) return false;
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  int cap = 0;
-  return vnm_order_shape(ctx, mp, cfg, attr, cap);
+  return vnm_order_shape(ctx, mp, W.cfg, W.attr, W.cap);
 }
 
 }  // namespace vnm
@@ -843,7 +981,8 @@ vnm_status vnm_vnm_eval(vnm_ctx* ctx, int m, int n, int nnz, const int* row, con
   if (!out2) return VNM_ERR_ARG;
   const int mp = (m + M - 1) / M * M, np = (n + M - 1) / M * M;
   const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
-  const bool rows = vnm_rows_fit(ctx, mp, np, M);
+  VnmRows R;
+  const bool rows = vnm_rows_fit(ctx, mp, np, M, R);
   VNM_TRY(arena_reserve(ctx, (rows ? vnm_rows_bytes(mp, np, nnz, ncells) + arena_bytes(mp > np ? mp : np, 4)
                                    : vnm_bytes(mp, nnz, ncells)) +
                                  2 * arena_bytes(nnz, 4) + arena_bytes(1, 4)));
@@ -860,13 +999,12 @@ vnm_status vnm_vnm_eval(vnm_ctx* ctx, int m, int n, int nnz, const int* row, con
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (ctx->h_pinned[0]) return VNM_ERR_RANGE;
   if (rows) {
-    VnmRows W;
-    VNM_TRY(vnm_rows_build(ctx, mp, np, nnz, d_row, d_col, M, V, W));
+    VNM_TRY(vnm_rows_build(ctx, mp, np, nnz, d_row, d_col, M, V, R));
     const int nodes = mp > np ? mp : np;
     int* comp = arena_take<int>(ctx, nodes);
     if (!comp) return VNM_ERR_NOMEM;
-    VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, nodes), VS_NT, 0, nullptr, nullptr, nodes, M, comp, W.packed);
-    VNM_TRY(vnm_rows_analyse(ctx, W, comp, ctx->h_pinned));
+    VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, nodes), VS_NT, 0, nullptr, nullptr, nodes, M, comp, R.packed);
+    VNM_TRY(vnm_rows_analyse(ctx, R, comp, ctx->h_pinned));
   } else {
     VnmWork W;
     VNM_TRY(vnm_setup(ctx, m, n, nnz, M, V, W));
@@ -879,8 +1017,8 @@ vnm_status vnm_vnm_eval(vnm_ctx* ctx, int m, int n, int nnz, const int* row, con
 
 // vnm_vnm_reorder on the original rows: prev (accepted) and cur (candidate)
 // are node maps; the entries are relabelled once, at the end.
-static vnm_status reorder_rows(vnm_ctx* ctx, int mp, int np, int nnz, int* row, int* col, int mem, int M, int V,
-                               int maxiter, int* out5, int* newpos) {
+static vnm_status reorder_rows(vnm_ctx* ctx, VnmRows& W, int mp, int np, int nnz, int* row, int* col, int mem, int M,
+                               int V, int maxiter, int* out5, int* newpos) {
   const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
   VNM_TRY(arena_reserve(ctx, vnm_rows_bytes(mp, np, nnz, ncells) + 2 * arena_bytes(nnz + 1, 4) +
                                  2 * arena_bytes(mp > np ? mp : np, 4) + arena_bytes(1, 4)));
@@ -906,7 +1044,6 @@ static vnm_status reorder_rows(vnm_ctx* ctx, int mp, int np, int nnz, int* row, 
   VNM_CUDA_TRY(cudaMemcpyAsync(h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (h[0]) return VNM_ERR_RANGE;
-  VnmRows W;
   VNM_TRY(vnm_rows_build(ctx, mp, np, nnz, d_row, d_col, M, V, W));
   VNM_LAUNCH(ctx, k_vs_map, vs_grid(ctx, mp), VS_NT, 0, nullptr, nullptr, mp, M, prev, W.packed);
   VNM_TRY(vnm_rows_analyse(ctx, W, prev, h));
@@ -951,7 +1088,9 @@ vnm_status vnm_vnm_reorder(vnm_ctx* ctx, int m, int n, int nnz, int* row, int* c
   if (!out5) return VNM_ERR_ARG;
   const int mp = (m + M - 1) / M * M, np = (n + M - 1) / M * M;
   const long long ncells = (long long)((mp + V - 1) / V) * (np / M);
-  if (vnm_rows_fit(ctx, mp, np, M)) return reorder_rows(ctx, mp, np, nnz, row, col, mem, M, V, maxiter, out5, newpos);
+  VnmRows R;
+  if (vnm_rows_fit(ctx, mp, np, M, R))
+    return reorder_rows(ctx, R, mp, np, nnz, row, col, mem, M, V, maxiter, out5, newpos);
   VNM_TRY(arena_reserve(ctx, vnm_bytes(mp, nnz, ncells)));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
