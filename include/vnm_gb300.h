@@ -340,8 +340,8 @@ vnm_status vnm_spmm_info(const vnm_spmm_matrix* A, long long* info, int n);
 /* C (nrows x n, FP32, row-major) = A * B with B (nrows x n, row-major, the
  * compressed dtype).  n must be a multiple of 64.  mem = where B and C are
  * (device: 16-byte aligned).  The tensor-core kernel works on column blocks
- * of 256, 128 or 64, the widest that divides n; VNM_SPMM_WIDTH=64|128|256 in
- * the environment fixes the width where it divides n. */
+ * of 256, then 128 and 64 for what is left; VNM_SPMM_WIDTH=64|128|256 in the
+ * environment fixes one width where it divides n. */
 vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, int n, float* C, int mem);
 
 /* vnm_spmm_run on the caller's stream, for device buffers, without

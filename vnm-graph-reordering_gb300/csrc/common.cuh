@@ -82,20 +82,6 @@ struct vnm_ctx {
 
 namespace vnm {
 
-// Lanes of a converged warp whose low BITS bits of d are this lane's (`ok`
-// lanes only), by one vote a bit: a match instruction is slower than 8 votes.
-template <int BITS>
-__device__ __forceinline__ unsigned warp_peers(unsigned d, bool ok) {
-  unsigned peers = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-  for (int b = 0; b < BITS; ++b) {
-    const bool on = (d >> b) & 1u;
-    const unsigned v = __ballot_sync(0xffffffffu, on);
-    peers &= on ? v : ~v;
-  }
-  return peers;
-}
-
 // Reserve `bytes` (256-byte aligned) of the arena; valid until arena_reset.
 vnm_status arena_reserve(vnm_ctx* ctx, size_t total_bytes);
 template <class T>

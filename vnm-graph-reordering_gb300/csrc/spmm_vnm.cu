@@ -165,15 +165,17 @@ __device__ __forceinline__ unsigned low2(unsigned m) {  // the lowest two set bi
 }
 
 // Counters of a compression.
-enum { CC_GROUPS, CC_VALID, CC_SLICES, CC_TILES, CC_RES, CC_MULTI_TASKS, CC_TASKS, CC_MULTI_ROWS, CC_PADDED, CC_PARTS,
-       CC_SPLIT, CC_SLOTS, CC_DENSE, CC_UNSORTED, CC_N };
+constexpr int TASK_CLASSES = 7;  // of residual tasks, by length (task_class)
+enum { CC_GROUPS, CC_VALID, CC_SLICES, CC_TILES, CC_RES, CC_MULTI_ROWS, CC_PADDED, CC_PARTS, CC_SPLIT, CC_SLOTS,
+       CC_DENSE, CC_UNSORTED, CC_CLASS, CC_CURSOR = CC_CLASS + TASK_CLASSES, CC_MULTI_CURSOR = CC_CURSOR + TASK_CLASSES,
+       CC_N };
 
 // The blocks, each walked by the thread of its first entry (neighbouring
 // threads walk neighbouring keys, so the walk lives in L1).  A block of fewer
 // than dense_min nonzeros is residual: its entries are flagged (by original
 // position) and counted per row, its tile marked.  A denser one goes to the
 // list of dense blocks, which warps take over.  228 K entries in 200 K
-// blocks: GROUPS_US us, where scanning block heads into a start table and one
+// blocks: 22 us, where scanning block heads into a start table and one
 // thread a block, dense ones included, took 115.
 __global__ void __launch_bounds__(256)
     k_cmp_groups(const unsigned long long* __restrict__ skeys, const int* __restrict__ spos, int nnz, int V, int nseg,
@@ -460,66 +462,78 @@ __device__ __forceinline__ int res_chunks(int len, bool needed) {
   return len <= RES_CHUNK ? 1 : (len + RES_CHUNK - 1) / RES_CHUNK;
 }
 
-// The residual rows' entries and tasks, in tiles of RP_TILE rows: sums[t] =
-// {entries, tasks of split rows, tasks of whole rows, split rows} of tile t,
-// the task totals in the counters.
+// Class of a row's tasks, the longest first: the chunks of a split row, then
+// whole rows by length.  The task list holds the classes in turn (the order
+// inside one does not matter), so that the warps that walk it with one stride
+// work on tasks of like length: with whole rows in row order the last warps of
+// a Chung-Lu 262144 product ran 18 % longer than the average.
+__device__ __forceinline__ int task_class(int len, int nch) {
+  return nch > 1 ? 0 : len > 64 ? 1 : len > 32 ? 2 : len > 16 ? 3 : len > 8 ? 4 : len > 4 ? 5 : 6;
+}
+
+// The residual rows in tiles of RP_TILE rows: sums[t] = entries of tile t;
+// tasks of each class, entries and split rows in the counters.
 constexpr int RP_TILE = 1024;
-__device__ __forceinline__ int4 res_of_row(int r, int R, const int* rowlen, const int* tile_raw, const int* tile_res) {
-  if (r >= R) return make_int4(0, 0, 0, 0);
+__device__ __forceinline__ int2 res_of_row(int r, int R, const int* rowlen, const int* tile_raw, const int* tile_res) {
+  if (r >= R) return make_int2(0, 0);
   const int t = r / SP_TM, len = rowlen[r];
-  const int nch = res_chunks(len, !(tile_raw[t] > 0 && tile_res[t] == 0));
-  return make_int4(len, nch > 1 ? nch : 0, nch == 1 ? 1 : 0, nch > 1 ? 1 : 0);
+  return make_int2(len, res_chunks(len, !(tile_raw[t] > 0 && tile_res[t] == 0)));
 }
 
 __global__ void __launch_bounds__(RP_TILE)
-    k_res_plan(const int* rowlen, int R, const int* tile_raw, const int* tile_res, int4* sums, int* counters) {
-  int v[4] = {0, 0, 0, 0}, tot[4];
-  const int4 x = res_of_row(blockIdx.x * RP_TILE + threadIdx.x, R, rowlen, tile_raw, tile_res);
-  v[0] = x.x;
-  v[1] = x.y;
-  v[2] = x.z;
-  v[3] = x.w;
-  block_scan<4>(v, tot);
-  if (threadIdx.x == 0) {
-    sums[blockIdx.x] = make_int4(tot[0], tot[1], tot[2], tot[3]);
-    if (tot[0]) atomicAdd(&counters[CC_RES], tot[0]);
-    if (tot[1]) atomicAdd(&counters[CC_MULTI_TASKS], tot[1]);
-    if (tot[2]) atomicAdd(&counters[CC_TASKS], tot[2]);
-    if (tot[3]) atomicAdd(&counters[CC_MULTI_ROWS], tot[3]);
-  }
+    k_res_plan(const int* rowlen, int R, const int* tile_raw, const int* tile_res, int* sums, int* counters) {
+  __shared__ int cls[TASK_CLASSES + 2];
+  if (threadIdx.x < TASK_CLASSES + 2) cls[threadIdx.x] = 0;
+  __syncthreads();
+  const int2 x = res_of_row(blockIdx.x * RP_TILE + threadIdx.x, R, rowlen, tile_raw, tile_res);
+  if (x.y) atomicAdd(&cls[task_class(x.x, x.y)], x.y);
+  if (x.y > 1) atomicAdd(&cls[TASK_CLASSES], 1);
+  const int len = __reduce_add_sync(0xffffffffu, x.x);
+  if ((threadIdx.x & 31) == 0 && len) atomicAdd(&cls[TASK_CLASSES + 1], len);
+  __syncthreads();
+  if (threadIdx.x < TASK_CLASSES + 2 && cls[threadIdx.x])
+    atomicAdd(&counters[threadIdx.x < TASK_CLASSES ? CC_CLASS + threadIdx.x
+                        : threadIdx.x == TASK_CLASSES ? CC_MULTI_ROWS : CC_RES], cls[threadIdx.x]);
+  if (threadIdx.x == 0) sums[blockIdx.x] = cls[TASK_CLASSES + 1];
 }
 
-// The tasks.  Split rows' chunks first (they are the longest), then the others.
+// The tasks; a split row's chunks are neighbours, and its partial slots are
+// their places in the list.
 __global__ void __launch_bounds__(RP_TILE)
-    k_res_tasks(const int* rowlen, int R, const int* tile_raw, const int* tile_res, const int4* sums, int nmt_total,
+    k_res_tasks(const int* rowlen, int R, const int* tile_raw, const int* tile_res, const int* sums, int* counters,
                 int4* task, int4* multi) {
-  int run[4];
-  {  // the tiles before this one
-    int v[4] = {0, 0, 0, 0};
-    for (int t = threadIdx.x; t < (int)blockIdx.x; t += 1024) {
-      const int4 x = sums[t];
-      v[0] += x.x;
-      v[1] += x.y;
-      v[2] += x.z;
-      v[3] += x.w;
-    }
-    block_scan<4>(v, run);
-  }
+  __shared__ int cls[TASK_CLASSES + 1], at[TASK_CLASSES + 1];
+  int before[1] = {0}, off[1], tot[1];
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += RP_TILE) before[0] += sums[t];
+  block_scan<1>(before, off);  // entries of the tiles before this one
+  if (threadIdx.x <= TASK_CLASSES) cls[threadIdx.x] = 0;
+  __syncthreads();
   const int r = blockIdx.x * RP_TILE + threadIdx.x;
-  const int4 x = res_of_row(r, R, rowlen, tile_raw, tile_res);
-  int v[4] = {x.x, x.y, x.z, x.w}, tot[4];
-  block_scan<4>(v, tot);
-  const int b = run[0] + v[0], e = b + x.x;
-  if (x.z) {
-    task[nmt_total + run[2] + v[2]] = make_int4(r, b, e, -1);
-  } else if (x.y) {
-    const int base = run[1] + v[1], csz = (e - b + x.y - 1) / x.y;
-    for (int j = 0; j < x.y; ++j) {
-      const int cb = min(b + j * csz, e), ce = min(cb + csz, e);
-      task[base + j] = make_int4(r, cb, ce, base + j);
-    }
-    multi[run[3] + v[3]] = make_int4(r, base, x.y, 0);
+  const int2 x = res_of_row(r, R, rowlen, tile_raw, tile_res);
+  const int c = task_class(x.x, x.y);
+  const int in = x.y ? atomicAdd(&cls[c], x.y) : 0, inm = x.y > 1 ? atomicAdd(&cls[TASK_CLASSES], 1) : 0;
+  int v[1] = {x.x};
+  block_scan<1>(v, tot);
+  if (threadIdx.x <= TASK_CLASSES) {
+    int start = 0;
+    for (int k = 0; k < (int)threadIdx.x && threadIdx.x < TASK_CLASSES; ++k) start += counters[CC_CLASS + k];
+    const int n = cls[threadIdx.x];
+    at[threadIdx.x] =
+        start + (n ? atomicAdd(&counters[threadIdx.x < TASK_CLASSES ? CC_CURSOR + threadIdx.x : CC_MULTI_CURSOR], n) : 0);
   }
+  __syncthreads();
+  if (!x.y) return;
+  const int b = off[0] + v[0], e = b + x.x, base = at[c] + in;
+  if (x.y == 1) {
+    task[base] = make_int4(r, b, e, -1);
+    return;
+  }
+  const int csz = (x.x + x.y - 1) / x.y;
+  for (int j = 0; j < x.y; ++j) {
+    const int cb = min(b + j * csz, e), ce = min(cb + csz, e);
+    task[base + j] = make_int4(r, cb, ce, base + j);
+  }
+  multi[at[TASK_CLASSES] + inm] = make_int4(r, base, x.y, 0);
 }
 
 // The residual records of entries that are sorted by row already.
@@ -637,87 +651,109 @@ __device__ __forceinline__ void fma8(unsigned long long (&acc)[4], uint4 b, unsi
   }
 }
 
-// Groups of LW lanes (32 / LW per warp) walk the task list with a stride
-// of every group of the grid (one wave of resident blocks); each lane owns 8
-// consecutive columns of the block's 8 * LW.  The records of a task are read
-// LW at a time, lane l of the group holding record l, and handed to the
-// lanes by shuffles; every lane gathers its 16 bytes of each B row, RES_U
-// rows in flight.  The next batch of records, and the next task with its
-// first batch, are loaded while the current ones are worked on, so a short
-// task costs about one round trip for its B rows.  Loop trip counts are the
-// warp's maximum; a group past its end reads a zero weight and a zero row,
-// so the arithmetic needs no predicate.
+// A warp walks the task list with a stride of every warp of the grid (one
+// wave of resident blocks); LW lanes cover the block's 8 * LW columns, 8
+// consecutive ones a lane, and the G = 32 / LW groups of lanes take the
+// task's records in turn, two at a time, their sums added at the end.  The
+// records come 32 at a time, one a lane, through shared memory (a 16-byte
+// read hands a group two of them; handing out columns and weights by shuffles
+// cost two a record), the next 32, and the next task with its first 32, loaded
+// ahead.  Every lane gathers its 16 bytes of RES_U rows before the first is
+// used; a short rest of a task issues half as many.
+// Bound by instructions issued (unpacking 16-bit values, packed FMAs, an
+// address and a load a record and lane) and, next, the gathers from L2: 4.2 M
+// records, n = 256 (Chung-Lu 262144): 234 us, 9.2 TB/s of gathered rows, 361
+// with the records handed out by shuffles, padded batches of 8 and whole rows
+// in row order (task_class).
+template <bool BF16, int NU, bool FULL, int G>
+__device__ __forceinline__ void res_step(unsigned long long (&acc)[4], const int4* rec, int grp, int left,
+                                         const unsigned char* bcol, unsigned ldb) {
+  uint4 b[NU];
+  int w[NU];
+#pragma unroll
+  for (int u = 0; u < NU; u += 2) {
+    const int4 r = rec[u / 2 * G + grp];  // records u * G + 2 grp and the one after it
+    const int k = u * G + 2 * grp;
+    const unsigned char *p0, *p1;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(p0) : "r"(r.x), "r"(ldb), "l"(bcol));
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(p1) : "r"(r.z), "r"(ldb), "l"(bcol));
+    b[u] = FULL || k < left ? __ldg(reinterpret_cast<const uint4*>(p0)) : make_uint4(0, 0, 0, 0);
+    b[u + 1] = FULL || k + 1 < left ? __ldg(reinterpret_cast<const uint4*>(p1)) : make_uint4(0, 0, 0, 0);
+    w[u] = r.y;
+    w[u + 1] = r.w;
+  }
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    unsigned long long ww;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "r"(w[u]));
+    fma8<BF16>(acc, b[u], ww);
+  }
+}
+
 template <int LW, bool BF16>
 __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS_PER_SM)
     k_spmm_res(const int4* __restrict__ task, int ntask, const int2* __restrict__ rcv,
-               const unsigned char* __restrict__ B, size_t ldb, float* __restrict__ C, int ldc,
+               const unsigned char* __restrict__ B, unsigned ldb, float* __restrict__ C, int ldc,
                float* __restrict__ P, int ldp) {
   constexpr int G = 32 / LW;
+  __shared__ __align__(16) int2 recs[RES_THREADS / 32][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / LW, lid = lane % LW;
-  const int stride = gridDim.x * (RES_THREADS / 32) * G;
-  int t = (blockIdx.x * (RES_THREADS / 32) + warp) * G + grp;
+  const int stride = gridDim.x * (RES_THREADS / 32);
   const int cb = blockIdx.y * (8 * LW) + lid * 8;  // this lane's first column
   const unsigned char* bcol = B + (size_t)cb * 2;
-  int4 tk = t < ntask ? task[t] : make_int4(0, 0, 0, -1);
-  int2 rc = tk.y + lid < tk.z ? __ldg(rcv + tk.y + lid) : make_int2(0, 0);
+  int t = blockIdx.x * (RES_THREADS / 32) + warp, par = 0;
+  if (t >= ntask) return;
+  int4 tk = task[t];
+  int2 rc = tk.y + lane < tk.z ? __ldg(rcv + tk.y + lane) : make_int2(0, 0);
   int4 tkn = t + stride < ntask ? task[t + stride] : make_int4(0, 0, 0, -1);
-  while (__any_sync(0xffffffffu, t < ntask)) {
-    const int len = tk.z - tk.y;  // 0 past the end
-    const int maxlen = G == 1 ? len : __reduce_max_sync(0xffffffffu, len);
+  for (; t < ntask; t += stride) {
+    const int len = tk.z - tk.y;
     // the next task's first records, and the task after it
-    const int2 rc1 = tkn.y + lid < tkn.z ? __ldg(rcv + tkn.y + lid) : make_int2(0, 0);
+    const int2 rc1 = tkn.y + lane < tkn.z ? __ldg(rcv + tkn.y + lane) : make_int2(0, 0);
     const int4 tk2 = t + 2 * stride < ntask ? task[t + 2 * stride] : make_int4(0, 0, 0, -1);
     unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};  // FP32 pairs
-    for (int k0 = 0; k0 < maxlen; k0 += LW) {
-      const int kn = k0 + LW + lid;
-      const int2 rcn = kn < len ? __ldg(rcv + tk.y + kn) : make_int2(0, 0);
+    for (int k0 = 0; k0 < len; k0 += 32) {
+      recs[warp][par][lane] = rc;
+      const int kn = k0 + 32 + lane;
+      rc = kn < len ? __ldg(rcv + tk.y + kn) : make_int2(0, 0);
+      __syncwarp();
+      const int cnt = min(32, len - k0);
+      const int4* rec = reinterpret_cast<const int4*>(recs[warp][par]);
 #pragma unroll 1
-      for (int u0 = 0; u0 < LW; u0 += RES_U) {
-        if (k0 + u0 >= maxlen) break;
-        uint4 b[RES_U];
-#pragma unroll
-        for (int u = 0; u < RES_U; ++u) {
-          const int col = __shfl_sync(0xffffffffu, rc.x, grp * LW + u0 + u);
-          b[u] = k0 + u0 + u < len ? __ldg(reinterpret_cast<const uint4*>(bcol + (size_t)col * ldb))
-                                   : make_uint4(0, 0, 0, 0);
-        }
-        // the weights are fetched once the rows are in flight
-#pragma unroll
-        for (int u = 0; u < RES_U; ++u) {
-          const int vbits = __shfl_sync(0xffffffffu, rc.y, grp * LW + u0 + u);
-          const uint32_t w = k0 + u0 + u < len ? (uint32_t)vbits : 0u;
-          unsigned long long ww;
-          asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "r"(w));
-          fma8<BF16>(acc, b[u], ww);
-        }
+      for (int s = 0; s < cnt; s += RES_U * G) {
+        const int left = cnt - s;
+        if (left >= RES_U * G) res_step<BF16, RES_U, true, G>(acc, rec + s / 2, grp, left, bcol, ldb);
+        else if (left > RES_U * G / 2) res_step<BF16, RES_U, false, G>(acc, rec + s / 2, grp, left, bcol, ldb);
+        else res_step<BF16, RES_U / 2, false, G>(acc, rec + s / 2, grp, left, bcol, ldb);
       }
-      rc = rcn;
+      par ^= 1;  // (the other half is read before this one is written again)
     }
-    if (t < ntask) {
-      float* dst = tk.w < 0 ? C + (size_t)tk.x * ldc + cb : P + (size_t)tk.w * ldp + cb;
-      float f[8];
+    float f[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float((uint32_t)acc[i]);
-        f[2 * i + 1] = __uint_as_float((uint32_t)(acc[i] >> 32));
-      }
-      reinterpret_cast<float4*>(dst)[0] = make_float4(f[0], f[1], f[2], f[3]);
-      reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
+    for (int i = 0; i < 4; ++i) {
+      f[2 * i] = __uint_as_float((uint32_t)acc[i]);
+      f[2 * i + 1] = __uint_as_float((uint32_t)(acc[i] >> 32));
     }
-    t += stride;
+#pragma unroll
+    for (int o = 16; o >= LW; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] += __shfl_xor_sync(0xffffffffu, f[i], o);
+    float4* dst = reinterpret_cast<float4*>(tk.w < 0 ? C + (size_t)tk.x * ldc + cb : P + (size_t)tk.w * ldp + cb);
+    if (G == 1 || grp == 0) dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+    if (G == 1 || grp == 1) dst[1] = make_float4(f[4], f[5], f[6], f[7]);
     tk = tkn;
     tkn = tk2;
     rc = rc1;
   }
 }
 
-// C row of a split row = the sum of its partial rows in a fixed order: the
-// block's threads cover the row's float4 columns qpb at a time, and the
-// ng = FIN_THREADS / qpb thread groups of a column sum every ng-th chunk
-// (group g: chunks g, g + ng, ...) before the group sums are added in group
-// order.  A row of a few hundred chunks (a hub of a power-law graph) is then
-// not one thread's serial chain of loads.
-constexpr int FIN_THREADS = 256;
+// C row of a split row = the sum of its partial rows in a fixed order: a
+// block takes FIN_COLS float4 columns of a row, and its thread groups every
+// ng-th chunk each (group g: chunks g, g + ng, ...) before the group sums are
+// added in group order.  A row of a few hundred chunks (a hub of a power-law
+// graph) is then not one thread's serial chain of loads: with all of a row's
+// columns in one block, four groups, the hubs of Chung-Lu 262144 took 15 us.
+constexpr int FIN_THREADS = 256, FIN_COLS = 16;
 __device__ __forceinline__ void add4(float4& s, const float4 x) {
   s.x += x.x;
   s.y += x.y;
@@ -725,38 +761,31 @@ __device__ __forceinline__ void add4(float4& s, const float4 x) {
   s.w += x.w;
 }
 __global__ void __launch_bounds__(FIN_THREADS)
-    k_spmm_fin(const int4* __restrict__ multi, const float* __restrict__ P, int ldp, float* C, int ldc, int n) {
+    k_spmm_fin(const int4* __restrict__ multi, const float* __restrict__ P, int ldp, float* C, int ldc) {
   __shared__ float4 red[FIN_THREADS];
   const int4 m = multi[blockIdx.x];
-  const int nq = n / 4;
-  const int qpb = nq < FIN_THREADS ? nq : FIN_THREADS;
-  const int ng = FIN_THREADS / qpb;
-  const int g = threadIdx.x / qpb, qi = threadIdx.x % qpb;
-  for (int q0 = 0; q0 < nq; q0 += qpb) {
-    const int q = q0 + qi;
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (g < ng && q < nq) {
-      const float4* src = reinterpret_cast<const float4*>(P + (size_t)m.y * ldp) + q;
-      const size_t step = (size_t)ng * (ldp / 4);
-      int j = g;
-      for (; j + 3 * ng < m.z; j += 4 * ng) {  // four loads in flight, added in chunk order
-        const float4 x0 = src[(size_t)j * (ldp / 4)], x1 = src[(size_t)j * (ldp / 4) + step],
-                     x2 = src[(size_t)j * (ldp / 4) + 2 * step], x3 = src[(size_t)j * (ldp / 4) + 3 * step];
-        add4(s, x0);
-        add4(s, x1);
-        add4(s, x2);
-        add4(s, x3);
-      }
-      for (; j < m.z; j += ng) add4(s, src[(size_t)j * (ldp / 4)]);
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    if (g == 0 && q < nq) {
-      float4 t = red[qi];
-      for (int h = 1; h < ng; ++h) add4(t, red[h * qpb + qi]);
-      reinterpret_cast<float4*>(C + (size_t)m.x * ldc)[q] = t;
-    }
-    __syncthreads();
+  constexpr int ng = FIN_THREADS / FIN_COLS;
+  const int g = threadIdx.x / FIN_COLS, qi = threadIdx.x % FIN_COLS;
+  const int q = blockIdx.y * FIN_COLS + qi;  // n is a multiple of 64: whole blocks
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4* src = reinterpret_cast<const float4*>(P + (size_t)m.y * ldp) + q;
+  const size_t row = ldp / 4, step = (size_t)ng * row;
+  int j = g;
+  for (; j + 3 * ng < m.z; j += 4 * ng) {  // four loads in flight, added in chunk order
+    const float4* x = src + (size_t)j * row;
+    const float4 x0 = x[0], x1 = x[step], x2 = x[2 * step], x3 = x[3 * step];
+    add4(s, x0);
+    add4(s, x1);
+    add4(s, x2);
+    add4(s, x3);
+  }
+  for (; j < m.z; j += ng) add4(s, src[(size_t)j * row]);
+  red[threadIdx.x] = s;
+  __syncthreads();
+  if (g == 0) {
+    const int used = m.z < ng ? m.z : ng;
+    for (int h = 1; h < used; ++h) add4(s, red[h * FIN_COLS + qi]);
+    reinterpret_cast<float4*>(C + (size_t)m.x * ldc)[q] = s;
   }
 }
 
@@ -773,6 +802,7 @@ struct SpmmArgs {
   float* C;
   float* P;                // partial tiles of 128 rows, row stride ldc
   int R, n, ldc;
+  int col0;                // first column of the launch
   uint32_t idesc;
   int* err;
   uint32_t wait_limit;  // polls of a pipeline wait (copies <-> MMAs) before it gives up
@@ -821,7 +851,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   const int4 item = p.part[blockIdx.x];
   const int t = item.x >> 1;
   const bool add = item.x & 1;  // the residual kernel wrote these rows first
-  const int n0 = blockIdx.y * NT;
+  const int n0 = p.col0 + blockIdx.y * NT;
   const int s0 = item.y, nsteps = item.z - item.y;
   const int nst = (nsteps + KS - 1) / KS;  // stage fills
   ptx::grid_dependents_launch();
@@ -1010,20 +1040,20 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
 
 // Rows of a split tile: the sum of its parts in order, scaled, added to what
 // the residual kernel wrote.  Bound by L2 (the parts were just written): one
-// float4 of C a thread, the parts' loads four in flight.
+// float4 of C a thread, the parts' loads eight in flight.
 __global__ void __launch_bounds__(256)
     k_spmm_tfin(const int4* __restrict__ split, const float* __restrict__ P, const float* __restrict__ rscale, int R,
                 int n, float* __restrict__ C) {
   ptx::grid_dependency_wait();
   const int4 m = split[blockIdx.x];
   const int t = m.x >> 1, nq = n / 4;
-  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < SP_TM * nq; e += gridDim.y * blockDim.x) {
-    const int rt = e / nq, q = e % nq, row = t * SP_TM + rt;
-    if (row >= R) break;
+  const int e = blockIdx.y * blockDim.x + threadIdx.x, rt = e / nq, q = e % nq, row = t * SP_TM + rt;
+  if (row >= R) return;
+  {
     const float4* src = reinterpret_cast<const float4*>(P + ((size_t)m.y * SP_TM + rt) * n) + q;
     const size_t step = (size_t)SP_TM * nq;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 8
     for (int k = 0; k < m.z; ++k) add4(s, src[k * step]);
     const float sc = rscale[row];
     float4 o = make_float4(s.x * sc, s.y * sc, s.z * sc, s.w * sc);
@@ -1089,7 +1119,7 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   int* tile_base = arena_take<int>(ctx, ntiles + 1);
   int* tile_rawbase = arena_take<int>(ctx, ntiles + 1);
   int4* tile_plan = arena_take<int4>(ctx, ntiles + 1);
-  int4* sums = arena_take<int4>(ctx, rtiles);
+  int* sums = arena_take<int>(ctx, rtiles);
   const size_t zero0 = ctx->arena.used;  // zeroed together from here
   int* gsl = arena_take<int>(ctx, n1);
   int* resflag = arena_take<int>(ctx, n1);
@@ -1130,9 +1160,9 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   out->slices = h[CC_SLICES];
   out->ntt = h[CC_TILES];
   out->nres = h[CC_RES];
-  const int nmt_total = h[CC_MULTI_TASKS], nst_total = h[CC_TASKS];
-  out->nslots = nmt_total;
-  out->ntask = nmt_total + nst_total;
+  out->nslots = h[CC_CLASS];
+  out->ntask = 0;
+  for (int k = 0; k < TASK_CLASSES; ++k) out->ntask += h[CC_CLASS + k];
   out->nmulti = h[CC_MULTI_ROWS];
   out->dense_min = dense_min;
   out->slices_padded = padded;
@@ -1210,7 +1240,7 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
     }
   }
   if (out->ntask > 0)
-    VNM_LAUNCH(ctx, k_res_tasks, rtiles, RP_TILE, 0, rowlen, R, tile_raw, tile_res, sums, nmt_total, out->task,
+    VNM_LAUNCH(ctx, k_res_tasks, rtiles, RP_TILE, 0, rowlen, R, tile_raw, tile_res, sums, counters, out->task,
                out->multi);
   if (out->ntt > 0)
     VNM_LAUNCH(ctx, k_tile_parts, sp_grid(ctx, ntiles), 256, 0, tile_raw, tile_res, ntiles, tile_base, tile_plan,
@@ -1227,14 +1257,15 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
 }
 
 template <int NT, int KS, int ST>
-static vnm_status launch_spmm(vnm_ctx* ctx, const vnm_spmm_matrix* A, SpmmArgs& p) {
+static vnm_status launch_spmm(vnm_ctx* ctx, const vnm_spmm_matrix* A, SpmmArgs& p, int col0, int blocks) {
   // enough shared memory that at most 512 / NT CTAs share an SM: their NT
   // column accumulators then fit the SM's 512 tensor-memory columns, so an
   // allocation never waits for another CTA (228 KB of shared memory per SM)
   constexpr size_t floor_bytes = (228u << 10) / (512 / NT + 1) + 1024;
   size_t smem = sizeof(SpmmSmem<NT, KS, ST>) + 1024;
   if (smem < floor_bytes) smem = floor_bytes;
-  dim3 grid(A->npart, p.n / NT);
+  p.col0 = col0;
+  dim3 grid(A->npart, blocks);
   VNM_CUDA_TRY(cudaFuncSetAttribute(k_spmm_vnm<NT, KS, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   p.idesc = ptx::idesc_f16(A->dtype == 1 ? 1u : 0u, 0u, 1u, SP_TM, NT);
   VNM_LAUNCH(ctx, (k_spmm_vnm<NT, KS, ST>), grid, SP_THREADS, smem, p);
@@ -1337,45 +1368,55 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
   p.ldc = n;
   p.err = err;
   p.wait_limit = spmm_wait_limit();
-  // the CUDA-core part: lanes per task so that 8 columns a lane tile n
+  // the CUDA-core part: 8 columns a lane, in blocks of 256 columns, then 128
+  // and 64 where they are left
   auto launch_res = [&]() -> vnm_status {
     if (A->ntask > 0) {
-      const int lw = (n % 256) == 0 ? 32 : (n % 128) == 0 ? 16 : 8;
       // one wave of resident blocks (the task list is walked with a stride)
-      const int per_block = (RES_THREADS / 32) * (32 / lw);
+      const int per_block = RES_THREADS / 32;
       int bx = (A->ntask + per_block - 1) / per_block;
       if (bx > ctx->num_sms * RES_BLOCKS_PER_SM) bx = ctx->num_sms * RES_BLOCKS_PER_SM;
-      dim3 grid((unsigned)bx, (unsigned)(n / (8 * lw)));
-#define VNM_RES(LWV, BFV)                                                                                   \
-  VNM_LAUNCH(ctx, (k_spmm_res<LWV, BFV>), grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B, p.ldb, dC, \
-             n, P, n)
-      if (A->dtype == 1) {
-        if (lw == 32) VNM_RES(32, true);
-        else if (lw == 16) VNM_RES(16, true);
-        else VNM_RES(8, true);
-      } else {
-        if (lw == 32) VNM_RES(32, false);
-        else if (lw == 16) VNM_RES(16, false);
-        else VNM_RES(8, false);
-      }
+      int col = 0;
+#define VNM_RES(LWV, COUNT)                                                                                          \
+  do {                                                                                                               \
+    const int count_ = (COUNT);                                                                                      \
+    if (count_ > 0) {                                                                                                \
+      const dim3 grid((unsigned)bx, (unsigned)count_);                                                               \
+      if (A->dtype == 1)                                                                                             \
+        VNM_LAUNCH(ctx, (k_spmm_res<LWV, true>), grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B + 2 * col,     \
+                   (unsigned)p.ldb, dC + col, n, P + col, n);                                                        \
+      else                                                                                                           \
+        VNM_LAUNCH(ctx, (k_spmm_res<LWV, false>), grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B + 2 * col,    \
+                   (unsigned)p.ldb, dC + col, n, P + col, n);                                                        \
+      col += count_ * 8 * LWV;                                                                                       \
+    }                                                                                                                \
+  } while (0)
+      VNM_RES(32, n / 256);
+      VNM_RES(16, (n % 256) / 128);
+      VNM_RES(8, (n % 128) / 64);
 #undef VNM_RES
     }
-    if (A->nmulti > 0) VNM_LAUNCH(ctx, k_spmm_fin, A->nmulti, FIN_THREADS, 0, A->multi, P, n, dC, n, n);
+    if (A->nmulti > 0)
+      VNM_LAUNCH(ctx, k_spmm_fin, dim3(A->nmulti, n / (4 * FIN_COLS)), FIN_THREADS, 0, A->multi, P, n, dC, n);
     return VNM_OK;
   };
-  // The widest column block that divides n: its A tiles are read fewest
-  // times.  VNM_SPMM_WIDTH (64, 128 or 256) in the environment fixes it where
-  // it divides n.
-  int nt = n % 256 == 0 ? 256 : n % 128 == 0 ? 128 : 64;
+  // Column blocks of 256, then one of 128 and one of 64 where they are left:
+  // the operand is read once a block (n = 192 as 128 + 64 instead of three
+  // times 64).  VNM_SPMM_WIDTH (64, 128 or 256) in the environment fixes the
+  // tensor kernel's width where it divides n.
+  int fixed = 0;
   if (const char* e = getenv("VNM_SPMM_WIDTH")) {
     const int w = atoi(e);
-    if ((w == 64 || w == 128 || w == 256) && n % w == 0) nt = w;
+    if ((w == 64 || w == 128 || w == 256) && n % w == 0) fixed = w;
   }
   auto launch_nt = [&]() -> vnm_status {
     if (A->ntt == 0) return VNM_OK;
-    if (nt == 256) VNM_TRY((launch_spmm<256, 4, 4>(ctx, A, p)));
-    else if (nt == 128) VNM_TRY((launch_spmm<128, 8, 3>(ctx, A, p)));
-    else VNM_TRY((launch_spmm<64, 8, 4>(ctx, A, p)));
+    const int n256 = fixed == 256 ? n / 256 : fixed ? 0 : n / 256;
+    const int n128 = fixed == 128 ? n / 128 : fixed ? 0 : (n % 256) / 128;
+    const int n64 = fixed == 64 ? n / 64 : fixed ? 0 : (n % 128) / 64;
+    if (n256) VNM_TRY((launch_spmm<256, 4, 4>(ctx, A, p, 0, n256)));
+    if (n128) VNM_TRY((launch_spmm<128, 8, 3>(ctx, A, p, n256 * 256, n128)));
+    if (n64) VNM_TRY((launch_spmm<64, 8, 4>(ctx, A, p, n256 * 256 + n128 * 128, n64)));
     if (A->ntsplit == 0) return VNM_OK;
     cudaLaunchAttribute attr[1];  // set up while the parts are made
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1384,7 +1425,7 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3(A->ntsplit, (SP_TM * (n / 4) + 1023) / 1024);
+    cfg.gridDim = dim3(A->ntsplit, SP_TM * (n / 4) / 256);
     cfg.blockDim = dim3(256);
     VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmm_tfin, (const int4*)A->tsplit, (const float*)p.P,
                                     (const float*)A->rscale, A->R, n, dC));

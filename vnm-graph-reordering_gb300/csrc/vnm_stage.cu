@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(VT_WARPS * 32)
 // the rows of a group (rows equal so far) by their next token and splits the
 // groups; a row alone in its group, or at the end of its list, keeps its
 // place.  Sorting is a stable radix sort of VO_BITS-bit digits (two cluster
-// barriers a digit: each warp ranks its 32-row chunks by votes, the
+// barriers a digit: each warp ranks its 32-row chunks with __match_any, the
 // blocks exchange their digit counts, and every row goes straight to its
 // place in the other buffer, in whichever block), or, where the largest group
 // has at most VO_COUNT rows (on R-MAT 16384 76 after two tokens, 9 after
@@ -657,8 +657,8 @@ __global__ void __launch_bounds__(VO_THREADS, 1)
         if (j >= items) break;
         const bool live = live_of(j);
         v[j] = live ? key[slot_of(j)] : 0ull;
-        dig[j] = (int)(v[j] >> shift) & (VO_BINS - 1);
-        const unsigned peers = warp_peers<VO_BITS>((unsigned)dig[j], live);
+        dig[j] = live ? (int)(v[j] >> shift) & (VO_BINS - 1) : VO_BINS + lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, dig[j]);
         at[j] = live ? sm.whist[w][dig[j]] + __popc(peers & ((1u << lane) - 1u)) : 0;
         __syncwarp();
         if (live && lane == __ffs(peers) - 1) sm.whist[w][dig[j]] += (uint16_t)__popc(peers);
