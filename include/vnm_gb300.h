@@ -357,6 +357,14 @@ vnm_status vnm_spmm_run(vnm_ctx* ctx, const vnm_spmm_matrix* A, const void* B, i
  * sets a flag on the operand; vnm_spmm_check reads it. */
 vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, int n, float* C, void* stream);
 
+/* vnm_spmm_run_async for features of another type or width: X (nrows x F
+ * device memory, row stride ldx elements, xtype 0 FP16, 1 BF16, 2 FP32) is
+ * rounded to the operand's type into B (nrows x n, 16-byte aligned device
+ * memory the caller provides; columns F .. n - 1 become zero), which is then
+ * multiplied; F <= n, n a multiple of 64. */
+vnm_status vnm_spmm_run_cast_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* X, int xtype, long long ldx, int F,
+                                   void* B, int n, float* C, void* stream);
+
 /* Waits for `stream`; *failed = 1 when a vnm_spmm_run_async of A failed
  * inside a kernel since the last check (the flag is cleared), else 0. */
 vnm_status vnm_spmm_check(vnm_spmm_matrix* A, void* stream, int* failed);

@@ -38,3 +38,28 @@ def test_split_tiles_match_float64(ctx, V, n, dtype):
         assert torch.equal(A.run_async(Bd), C)
     A.check()
     A.close()
+
+
+@pytest.mark.parametrize("F", [1, 7, 64, 100, 130])
+@pytest.mark.parametrize("xdtype,dtype", [("float32", "bf16"), ("float32", "fp16"), ("bfloat16", "fp16"),
+                                          ("float16", "fp16")])
+def test_cast_product_matches_torch_rounding(ctx, F, xdtype, dtype):
+    """Features rounded and padded by the library give bit for bit the product
+    of the features rounded and padded by torch, whatever their stride and
+    alignment, infinities and overflowing values among them."""
+    import torch
+    import vnm_gb300
+    from vnm_gb300 import gcn, synth
+    n, r, c, v = synth.chung_lu(1000, 2.1, 8.0, 3)
+    A = vnm_gb300.SpmmMatrix(ctx, n, r, c, v, 8, 128, dtype)
+    g = torch.Generator().manual_seed(F)
+    X = (100 * torch.randn((n, F), generator=g)).to(getattr(torch, xdtype))
+    X[5, 0], X[6, F - 1], X[7, 0] = float("inf"), 70000.0, float("-inf")
+    X = X.cuda()
+    wide = torch.zeros((n, F + 3), dtype=X.dtype, device="cuda")
+    wide[:, 3:] = X
+    Xp, _ = gcn._pad_cols(X.to(torch.bfloat16 if dtype == "bf16" else torch.float16))
+    want = A.run_async(Xp)[:, :F]
+    for x in (X, wide[:, 3:]):
+        assert torch.equal(torch.nan_to_num(A.run_cast_async(x), nan=1.25), torch.nan_to_num(want, nan=1.25))
+    A.close()

@@ -789,6 +789,34 @@ __global__ void __launch_bounds__(FIN_THREADS)
   }
 }
 
+// The dense operand from features of another type or width: out (R x n, 16
+// bits, row-major) = X (R x F, row stride ldx) rounded to nearest, columns F
+// .. n - 1 zero; 8 columns a thread.  Bound by HBM: 65536 x 100 FP32 to 128
+// FP16 columns 9 us.  vec: rows of X are 16-byte aligned.
+template <class S, class D>
+__global__ void __launch_bounds__(256)
+    k_spmm_cast(const S* __restrict__ X, long long ldx, int R, int F, int n, bool vec, D* __restrict__ out) {
+  const int nc = n / 8;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)R * nc;
+       e += (long long)gridDim.x * blockDim.x) {
+    const long long r = e / nc;
+    const int c = (int)(e - r * nc) * 8;
+    const S* src = X + r * ldx + c;
+    alignas(16) S v[8];
+    if (vec && c + 8 <= F) {
+#pragma unroll
+      for (int q = 0; q < (int)sizeof(v) / 16; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(src)[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = c + q < F ? src[q] : S(0.f);
+    }
+    alignas(16) D o[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) o[q] = to_t<D>((float)v[q]);
+    *reinterpret_cast<uint4*>(out + r * n + c) = *reinterpret_cast<const uint4*>(o);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Tensor-core kernel
 // ---------------------------------------------------------------------------
@@ -1496,6 +1524,36 @@ vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, i
   const vnm_status st = spmm_enqueue(ctx, A, B, n, C, A->part, A->err, false);
   ctx->stream = own;
   return st;
+}
+
+vnm_status vnm_spmm_run_cast_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* X, int xtype, long long ldx, int F,
+                                   void* B, int n, float* C, void* stream) {
+  if (!ctx || !A || !X || !B || xtype < 0 || xtype > 2 || F <= 0 || ldx < F || n < F || (n % 64) != 0)
+    return VNM_ERR_ARG;
+  if (A->device != ctx->device || (reinterpret_cast<uintptr_t>(B) & 15) != 0) return VNM_ERR_ARG;
+  VNM_CUDA_TRY(cudaSetDevice(ctx->device));
+  const size_t xsize = xtype == 2 ? 4 : 2;
+  const bool vec = (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (ldx * xsize) % 16 == 0;
+  long long g = ((long long)A->R * (n / 8) + 255) / 256;
+  if (g > (long long)ctx->num_sms * 32) g = (long long)ctx->num_sms * 32;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define VNM_CAST(S)                                                                                              \
+  do {                                                                                                           \
+    if (A->dtype == 1)                                                                                           \
+      k_spmm_cast<S, __nv_bfloat16><<<(unsigned)g, 256, 0, st>>>(static_cast<const S*>(X), ldx, A->R, F, n, vec, \
+                                                                 static_cast<__nv_bfloat16*>(B));                \
+    else                                                                                                         \
+      k_spmm_cast<S, __half><<<(unsigned)g, 256, 0, st>>>(static_cast<const S*>(X), ldx, A->R, F, n, vec,        \
+                                                          static_cast<__half*>(B));                              \
+  } while (0)
+  if (xtype == 0) VNM_CAST(__half);
+  else if (xtype == 1) VNM_CAST(__nv_bfloat16);
+  else VNM_CAST(float);
+#undef VNM_CAST
+  if (cudaGetLastError() != cudaSuccess) return VNM_ERR_CUDA;
+  const vnm_status s = vnm_spmm_run_async(ctx, A, B, n, C, stream);
+  ctx->launches++;
+  return s;
 }
 
 vnm_status vnm_spmm_check(vnm_spmm_matrix* A, void* stream, int* failed) {

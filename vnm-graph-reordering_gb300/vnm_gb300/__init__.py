@@ -335,6 +335,8 @@ class SpmmMatrix:
             L.vnm_spmm_free.argtypes = [_vp]
             L.vnm_spmm_run_async.argtypes = [_vp, _vp, _vp, ctypes.c_int, _vp, _vp]
             L.vnm_spmm_check.argtypes = [_vp, _vp, _i32p]
+            L.vnm_spmm_run_cast_async.argtypes = [_vp, _vp, _vp, ctypes.c_int, ctypes.c_longlong, ctypes.c_int, _vp,
+                                                  ctypes.c_int, _vp, _vp]
             L._spmm_typed = True
         self.ctx = ctx
         self.nrows = nrows
@@ -389,6 +391,21 @@ class SpmmMatrix:
                                         ctypes.c_void_p(C.data_ptr()), ctypes.c_void_p(stream.cuda_stream)),
                "vnm_spmm_run_async")
         return C
+
+    def run_cast_async(self, X):
+        """A X as FP32 (nrows x F) for a CUDA tensor X of FP32, FP16 or BF16
+        with contiguous rows, rounded to the operand's type, enqueued on
+        torch's current stream of X's device without waiting."""
+        import torch
+        F, dev = X.shape[1], X.device
+        n = (F + 63) // 64 * 64
+        xtype = 2 if X.dtype == torch.float32 else 1 if X.dtype == torch.bfloat16 else 0
+        B = torch.empty((self.nrows, n), dtype=torch.bfloat16 if self.dtype == "bf16" else torch.float16, device=dev)
+        C = torch.empty((self.nrows, n), dtype=torch.float32, device=dev)
+        st = lib().vnm_spmm_run_cast_async(self.ctx.h, self.h, X.data_ptr(), xtype, X.stride(0), F, B.data_ptr(), n,
+                                           C.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+        _check(st, "vnm_spmm_run_cast_async")
+        return C if n == F else C[:, :F]
 
     def check(self, stream=None):
         """Wait for the stream; raise if an asynchronous product failed in a kernel."""

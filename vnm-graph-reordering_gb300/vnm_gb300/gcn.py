@@ -70,8 +70,15 @@ class VnmAdjacency:
         """A @ X (or A^T @ X) as FP32, X an n x F CUDA tensor."""
         import torch
         assert X.is_cuda and X.dim() == 2 and X.shape[0] == self.n
+        op = self.bwd if transpose else self.fwd
+        # rounding and padding in one launch where X is not the operand's
+        # input already; the general way for other types and strides
+        ready = X.dtype == self.torch_dtype and X.shape[1] % 64 == 0
+        if not ready and X.stride(1) == 1 and X.stride(0) >= X.shape[1] > 0 and X.dtype in (
+                torch.float32, torch.float16, torch.bfloat16):
+            return op.run_cast_async(X)
         Xp, F = _pad_cols(X.detach().to(self.torch_dtype))
-        Y = (self.bwd if transpose else self.fwd).run_async(Xp, stream=torch.cuda.current_stream(X.device))
+        Y = op.run_async(Xp, stream=torch.cuda.current_stream(X.device))
         return Y[:, :F] if Y.shape[1] != F else Y
 
     def close(self):
