@@ -40,6 +40,7 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -98,6 +99,7 @@ __host__ __device__ __forceinline__ int row_group(int row) {
 
 struct NMJob {
   int R;              // padded rows = columns
+  int row0;           // first row id in crow (a batch's matrices share one id range)
   int nseg;           // R / M
   int sched;          // 0..3
   int maxiter;        // reorderUtil MAXITER before it is raised to init_size
@@ -257,12 +259,12 @@ struct RoundSmem {
   int ts_max;       // slots of `table` (a power of two) or 0
   int ts_shift;     // 32 - log2(ts_max)
   int use_table;    // this round's records are in `table` (else in J.rec)
-  int* tlist;       // the slots of `table` claimed this round, densely (ts_max entries)
+  int dslots;       // > 0: `table` has a slot of its own for every row the block owns (a multiple of 32)
+  int wcnt[NW];     // touched slots of each warp's share of them
+  uint16_t* tlist;  // the slots of `table` in use this round, densely
   int tcount;       // how many
   int toff;         // this block's part of J.touched
   unsigned long long acc[4];  // leader: the helpers' work counters, added at the end
-  uint4* rcache;    // the process phase's first pass of touched rows, kept for the apply phase
-  int* rcrow;       //   (NM_THREADS x 4 records and their rows), or null
   int status;
   int nswaps;
   int hprog[K * K];  // pops of each ordered pair's heap written to ord so far
@@ -274,10 +276,9 @@ struct RoundSmem {
   int CR[NPAIR][MM];           //                              right-side corrections
   static constexpr int HSTR = (K * K + 31) / 32 * 32;  // heaps, rounded up to whole warps
   // Scratch at the head of dynamic shared memory, used by three phases in
-  // turn: the process phase's per-warp row masks (2 x K x M words a warp),
-  // the heap phase's slots [MM][HSTR] and entries [MM][HSTR] (4 B each), and
-  // the apply phase's bit-move table (K x ceil(M/4) x 16 x 16 B, less than
-  // the row masks).
+  // turn: the process phase's row masks (2 x K x M words a 32-row chunk, at
+  // least a chunk a warp at a time), the heap phase's slots [MM][HSTR] and
+  // entries [MM][HSTR] (4 B each), and the row masks again in the apply phase.
   static constexpr int PROC_BYTES = NW * 2 * K * M * 4;
   static constexpr int HEAP_BYTES = MM * HSTR * 8;
   static constexpr int SCR_U4 = ((PROC_BYTES > HEAP_BYTES ? PROC_BYTES : HEAP_BYTES) + 15) / 16;
@@ -290,6 +291,7 @@ struct RoundSmem {
     uint32_t dest_w[DEST_W];   // the same bytes as words, for copies to other blocks
   };
   int newinv[K], newpres[K];
+  uint8_t from[K * M];         // the column (xi * M + k) whose bits a column holds after the swaps
   int swaps[2 * K * M];        // committed swaps (positions)
   unsigned long long wtop[2][NW][K];
   unsigned long long sel_top[15][2][K];  // leader: each helper's scan (top K both orders) ...
@@ -599,13 +601,18 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
   }
 }
 
+// Slots of the direct table, at most: 65536 rows on 16 blocks, 8192 on 2 (and
+// the run of 16 rows that a range not starting at a multiple of 16 adds).
+constexpr int DIRECT_MAX = 4352;
+
 // OR the bitmaps of the round's segments into the records of the rows this
 // block owns.  Every column's rows are stored grouped by row_group (csplit),
 // so the block's entries of a column are one contiguous run of it, and no
 // other block touches these records: the process and apply phases that
 // follow need no cluster barrier.  The records go to the block's
-// shared-memory table when its entries fill at most 3/4 of it, else to
-// J.rec in global memory.
+// shared-memory table, where every row the block owns has its slot when there
+// are at most DIRECT_MAX of them; else they are hashed when the block's entries
+// fill at most 3/4 of the table, and go to J.rec in global memory when not.
 template <int M>
 __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{0, 1}) {
   constexpr int K = M + 1;
@@ -643,11 +650,75 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
     if (tid == 31) {
       sm.colpre[KM] = incl;
       sm.E = incl;
-      sm.use_table = sm.ts_max > 0 && incl <= (sm.ts_max >> 2) * 3;
+      sm.use_table = sm.dslots > 0 || (sm.ts_max > 0 && incl <= (sm.ts_max >> 2) * 3);
     }
   }
   __syncthreads();
   const int E = sm.E;
+  if (sm.dslots > 0) {
+    // A slot of its own for every row: one atomic an entry, no key and no
+    // probing; then each warp lists the touched slots of its share.  (With the
+    // hashed table below, or the records in global memory once the entries
+    // might fill it, a round of R-MAT 65536 2:8 took 21 us here at schedule 0,
+    // GATHER_US now.)
+    unsigned* tw = reinterpret_cast<unsigned*>(sm.table);
+    const int run0 = J.row0 >> 4, gpb = ROW_GROUPS / sl.cs;
+    constexpr int U = 4;  // entries a thread in flight
+    for (int base = tid; base < E; base += NM_THREADS * U) {
+      int rows[U], qs[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = base + u * NM_THREADS;
+        rows[u] = -1;
+        qs[u] = 0;
+        if (e < E) {
+          int lo = 0, hi = KM - 1;  // last q with colpre[q] <= e
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (sm.colpre[mid] <= e) lo = mid;
+            else hi = mid - 1;
+          }
+          qs[u] = lo;
+          rows[u] = J.crow[sm.colstart[lo] + (e - sm.colpre[lo])];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (rows[u] >= 0) {
+          const int xi = qs[u] / M, k = qs[u] % M;
+          const int slot = ((rows[u] >> 4) - run0) * gpb + row_group(rows[u]) - g0;
+          atomicOr(&tw[4 * slot + (xi >> 2)], (1u << k) << ((xi & 3) * 8));
+        }
+    }
+    __syncthreads();
+    constexpr int NW = NM_THREADS / 32;
+    const int lane = tid & 31, w = tid >> 5;
+    // the list, in slot order: lane q of a warp keeps the mask of the q-th
+    // 32-slot chunk of the warp's share
+    const int nch = sm.dslots / 32, per = (nch + NW - 1) / NW;
+    static_assert(DIRECT_MAX / 32 <= 32 * NW, "a lane a chunk of the warp's share");
+    unsigned mask = 0u;
+#pragma unroll 1
+    for (int q = 0; q < per && w * per + q < nch; ++q) {
+      const uint4 v = sm.table[(w * per + q) * 32 + lane];
+      const unsigned m = __ballot_sync(FULL, (v.x | v.y | v.z) != 0u);
+      if (lane == q) mask = m;
+    }
+    const int cnt = __reduce_add_sync(FULL, __popc(mask));
+    if (lane == 0) sm.wcnt[w] = cnt;
+    __syncthreads();
+    const int mine = sm.wcnt[lane];
+    int at = __reduce_add_sync(FULL, lane < w ? mine : 0);
+    if (w == NW - 1 && lane == 0) sm.tcount = sm.ntouched = at + cnt;
+#pragma unroll 1
+    for (int q = 0; q < per && w * per + q < nch; ++q) {
+      const unsigned m = __shfl_sync(FULL, mask, q);
+      if ((m >> lane) & 1u) sm.tlist[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((w * per + q) * 32 + lane);
+      at += __popc(m);
+    }
+    __syncthreads();
+    return;
+  }
   if (sm.use_table) {
     // open addressing, linear probing; a slot is claimed by CAS on its row
     // key and appended to the list of claimed slots, which the process and
@@ -686,7 +757,7 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
           const unsigned cur = atomicCAS(&tw[4 * h + 3], 0u, key);
           if (cur == 0u || cur == key) {
             atomicOr(&tw[4 * h + (xi >> 2)], (1u << k) << ((xi & 3) * 8));
-            if (cur == 0u) sm.tlist[atomicAdd(&sm.tcount, 1)] = (int)h;
+            if (cur == 0u) sm.tlist[atomicAdd(&sm.tcount, 1)] = (uint16_t)h;
             placed = true;
             break;
           }
@@ -742,127 +813,119 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
   __syncthreads();
 }
 
-__device__ __forceinline__ unsigned rec_byte(const uint4& w, int xi) {
-  const unsigned word = xi < 4 ? w.x : (xi < 8 ? w.y : w.z);
-  return (word >> ((xi & 3) * 8)) & 0xffu;
+// The touched row of place i in this round's list: its record, and its slot
+// or row id (for clearing it), -1 and zeros past the end.
+template <int M>
+__device__ __forceinline__ uint4 round_record(const RoundSmem<M>& sm, const NMJob& J, int i, int n, int& id) {
+  id = -1;
+  if (i >= n) return make_uint4(0u, 0u, 0u, 0u);
+  if (sm.use_table) {
+    id = sm.tlist[i];
+    return sm.table[id];
+  }
+  id = J.touched[sm.toff + i];
+  return J.rec[id];
 }
 
-// Run f(row, record, valid) over the touched rows, one row per lane, with
-// every lane of a warp calling f the same number of times (lanes past the
-// end get valid = false and a zero record) so f may use warp votes.  Each
-// lane first loads the records of TOUCH_U rows so their L2 round trips
-// overlap.
-// CM = 1: keep the records of the first pass in shared memory (process
-// phase); CM = 2: take them from there (apply phase), saving two dependent
-// L2 loads.  Both phases deal the rows to threads the same way, and the
-// touched rows and their records do not change in between.
-constexpr int TOUCH_U = 4;
-template <int M, int CM, class F>
-__device__ __forceinline__ void for_touched_warp(const RoundSmem<M>& sm, const NMJob& J, F&& f) {
-  constexpr int NW = NM_THREADS / 32;
-  const int nt = sm.ntouched;
-  const int* tl = J.touched + sm.toff;  // the rows this block owns and the round touched
-  // 32-row chunks dealt round-robin over the block's warps
-  constexpr int NWt = NW;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  bool first = true;
-  for (int c0 = w; c0 * 32 < nt; c0 += NWt * TOUCH_U) {
-    int rv[TOUCH_U];
-    uint4 wv[TOUCH_U];
-    if (CM == 2 && first && sm.rcache) {
-#pragma unroll
-      for (int u = 0; u < TOUCH_U; ++u) {
-        rv[u] = sm.rcrow[u * NM_THREADS + threadIdx.x];
-        wv[u] = sm.rcache[u * NM_THREADS + threadIdx.x];
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < TOUCH_U; ++u) {
-        const int t = (c0 + u * NWt) * 32 + lane;
-        rv[u] = t < nt ? tl[t] : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < TOUCH_U; ++u) wv[u] = rv[u] >= 0 ? J.rec[rv[u]] : make_uint4(0u, 0u, 0u, 0u);
-      if (CM == 1 && first && sm.rcache) {
-#pragma unroll
-        for (int u = 0; u < TOUCH_U; ++u) {
-          sm.rcrow[u * NM_THREADS + threadIdx.x] = rv[u];
-          sm.rcache[u * NM_THREADS + threadIdx.x] = wv[u];
-        }
-      }
-    }
-    first = false;
+// 4 bits from the top bits of 4 bytes.
+__device__ __forceinline__ unsigned byte_tops(unsigned z) { return ((z >> 7) & 0x01010101u) * 0x10204080u >> 28; }
+
+// The row masks of chunks c0 .. c1 - 1 (32 rows each), a warp a chunk, chunk
+// c's at scratch + (c - c0) * 2KM: VL[x][k] = rows with bit k of segment x, at
+// 2 x * M + k, and VE[x][k] = rows with bit k of eL (below), at (2 x + 1) * M
+// + k.  A word of the records holds 4 segments, so one transpose of 32 x 32
+// bits (lane b gets bit b of every lane's word) makes the masks of 4 segments
+// on all 32 lanes, where a vote for every bit, kept by one lane, took four
+// times the instructions; which rows have N+1 or N bits in a segment comes
+// from byte-wise population counts and one more transpose.  Bound by fetching
+// its own code once a round, so it is one copy of short loops for both phases
+// that use it: inlined and unrolled a chunk took 3.8 K cycles on an idle SM,
+// CHUNK_CYCLES now.
+template <int M>
+__device__ __noinline__ void masks_of_chunks(const RoundSmem<M>& sm, const NMJob& J, int N, int c0, int c1, int n,
+                                             unsigned* scratch) {
+  constexpr int K = M + 1, NWD = (K + 3) / 4, NW = NM_THREADS / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, Kn = sm.K_;
+  int id;
+  uint4 next = round_record<M>(sm, J, (c0 + w) * 32 + lane, c0 + w < c1 ? n : 0, id);
 #pragma unroll 1
-    for (int u = 0; u < TOUCH_U && (c0 + u * NWt) * 32 < nt; ++u) f(rv[u], wv[u], rv[u] >= 0, c0 + u * NWt);
-  }
-}
-
-// Run f(index, record, valid) over this round's row records: the table
-// slots (index = slot) when the records are in shared memory, else the
-// touched rows (index = row).  Warp-uniform like for_touched_warp.
-template <int M, int CM, class F>
-__device__ __forceinline__ void for_rows_warp(const RoundSmem<M>& sm, const NMJob& J, F&& f) {
-  if (sm.use_table) {  // the rows this block's table holds, from its list of claimed slots
-    constexpr int NW = NM_THREADS / 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int n = sm.tcount;
-    for (int base = w * 32; base < n; base += NW * 32) {
-      const int i = base + lane;
-      const int slot = i < n ? sm.tlist[i] : 0;
-      const uint4 v = i < n ? sm.table[slot] : make_uint4(0u, 0u, 0u, 0u);
-      f(slot, v, i < n, base >> 5);
+  for (int c = c0 + w; c < c1; c += NW) {
+    const uint4 rec = next;
+    next = round_record<M>(sm, J, (c + NW) * 32 + lane, c + NW < c1 ? n : 0, id);
+    unsigned t[NWD + 1];  // the record's words, and the flags: bit x N+1 bits in segment x, bit 16 + x N bits
+    t[NWD] = 0;
+#pragma unroll
+    for (int j = 0; j < NWD; ++j) {
+      const unsigned word = j == 0 ? rec.x : j == 1 ? rec.y : rec.z;
+      unsigned p = word - ((word >> 1) & 0x55555555u);
+      p = (p & 0x33333333u) + ((p >> 2) & 0x33333333u);
+      p = (p + (p >> 4)) & 0x0f0f0f0fu;
+      // bytes equal to N + 1 and to N: their difference is zero (no carry: it is below 16)
+      t[NWD] |= byte_tops(~((p ^ (unsigned)(N + 1) * 0x01010101u) + 0x7f7f7f7fu)) << (4 * j);
+      t[NWD] |= byte_tops(~((p ^ (unsigned)N * 0x01010101u) + 0x7f7f7f7fu)) << (16 + 4 * j);
+      t[j] = word;
     }
-  } else {
-    for_touched_warp<M, CM>(sm, J, f);
+    unsigned m = 0x0000ffffu;  // bits b with !(b & s)
+#pragma unroll 1
+    for (int s = 16; s > 0; s >>= 1, m ^= m << s) {
+      const bool high = lane & s;
+      const unsigned keep = high ? ~m : m, rot = high ? 32 - s : s;
+#pragma unroll
+      for (int j = 0; j <= NWD; ++j) {
+        const unsigned y = __shfl_xor_sync(FULL, t[j], s);
+        t[j] = (t[j] & keep) | (__funnelshift_l(y, y, rot) & ~keep);
+      }
+    }
+    unsigned* vw = scratch + (c - c0) * (2 * K * M);
+    const int k = lane & 7;
+#pragma unroll
+    for (int j = 0; j < NWD; ++j) {
+      const int xi = 4 * j + (lane >> 3);
+      const unsigned p1 = __shfl_sync(FULL, t[NWD], xi), p0 = __shfl_sync(FULL, t[NWD], 16 + xi);
+      if (xi < Kn && k < M) {
+        vw[(2 * xi) * M + k] = t[j];
+        vw[(2 * xi + 1) * M + k] = (t[j] & p1) | (~t[j] & p0);
+      }
+    }
   }
 }
 
-// Solo terms and pair corrections (fact 3), accumulated with warp votes:
-// for 32 rows at a time, a count over rows of a product of two per-row bit
-// conditions is popc(ballot(first) & ballot(second)), and one lane adds it
-// to shared memory.  For the pair (a, c) with L = bits in a, R = bits in c,
-// over rows where both are non-empty:
+// Chunks whose masks fit the scratch.
+template <int M>
+__host__ __device__ constexpr int mask_chunks() {
+  return RoundSmem<M>::SCR_U4 * 16 / (2 * (M + 1) * M * 4);
+}
+
+// Solo terms and pair corrections (fact 3) from the row masks: a count over
+// rows of a product of two per-row bit conditions is the population count of
+// the AND of two masks.  For the pair (a, c) with L = bits in a, R = bits in
+// c, over rows where both are non-empty (the others have no bits in VE[a] and
+// VL[a], or in VL[c] and VE[c]):
 //   CL(i, j) = sum  R_j * eL_i,   eL = L if pL == N+1, ~L if pL == N, else 0
 //   CR(i, j) = sum  L_i * eR_j,   eR = R if pR == N+1, ~R if pR == N, else 0
-//   S_a(k)   = sum over all rows of [L_k and pL == N+1]
+//   S_a(k)   = sum over all rows of [L_k and pL == N+1] = popc(VL & VE)
+// The chunks' masks go to the scratch, as many as fit, and are summed over
+// all of them once an entry.
 template <int M>
 __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl = Slice{0, 1}) {
   constexpr int K = M + 1;
   constexpr int MM = M * M;
-  const int Kn = sm.K_;
-  const bool self = sm.mode == 2;
-  const int lane = threadIdx.x & 31;
-  // this warp's row masks: VL[x][k] at vw[2x * M + k], VE[x][k] at vw[(2x + 1) * M + k]
+  constexpr int NP = RoundSmem<M>::NPAIR;
+  constexpr int NCH = mask_chunks<M>();
+  static_assert(NCH >= NM_THREADS / 32, "one chunk a warp fits the scratch");
   extern __shared__ uint4 smem_heap[];
-  unsigned* vw_warp = reinterpret_cast<unsigned*>(smem_heap) + (threadIdx.x >> 5) * (2 * K * M);
+  unsigned* const scratch = reinterpret_cast<unsigned*>(smem_heap);
+  const int Kn = sm.K_;
+  const int n = sm.use_table ? sm.tcount : sm.ntouched;
   const bool tmain = threadIdx.x == 0 && sl.rank == 0 && J.timed;  // the leader's thread 0 times (when asked)
   const unsigned long long t_in = tmain ? global_ns() : 0ull;
-  // When every 32-row chunk's masks fit the scratch, each chunk leaves them
-  // there and the sums are made afterwards over all chunks (gathered),
-  // instead of a shared atomic per chunk, pair and entry: those atomics, and
-  // the mask loads queued behind them, were 90 % of the process phase at
-  // R-MAT 16384 2:4.
-  constexpr int NCH = RoundSmem<M>::SCR_U4 * 16 / (2 * K * M * 4);  // chunks whose masks fit the scratch
-  static_assert(NCH >= NM_THREADS / 32, "one chunk a warp fits the scratch");
-  const int nchunks = ((sm.use_table ? sm.tcount : sm.ntouched) + 31) / 32;
-  const bool gathered = !self && nchunks <= NCH;
-  for_rows_warp<M, 1>(sm, J, [&](int r, const uint4& w, bool valid, int chunk) {
-    (void)r;
-    // chunk c's masks at c * 2KM when they are summed afterwards, else this warp's
-    unsigned* vw = gathered ? reinterpret_cast<unsigned*>(smem_heap) + chunk * (2 * K * M) : vw_warp;
-    const unsigned long long t_a = tmain ? global_ns() : 0ull;
-    unsigned b[K];
-    int p[K];
-#pragma unroll
-    for (int xi = 0; xi < K; ++xi) {
-      b[xi] = (valid && xi < Kn) ? rec_byte(w, xi) : 0u;
-      p[xi] = __popc(b[xi]);
-    }
-    if (self) {
-      // reference kernel lines 108-121 with lval == rval: direct per (i, j)
-      const unsigned L = b[0];
-      const int pl = p[0];
-      if (L == 0) return;
+  if (sm.mode == 2) {
+    // one segment with itself, reference kernel lines 108-121 with lval == rval: direct per (i, j)
+    for (int i0 = threadIdx.x; i0 < n; i0 += NM_THREADS) {
+      int id;
+      const unsigned L = round_record<M>(sm, J, i0, n, id).x & 0xffu;
+      const int pl = __popc(L);
+      if (L == 0) continue;
       for (int i = 0; i < M; ++i) {
         const unsigned li = (L >> i) & 1u;
         for (int j = 0; j < M; ++j) {
@@ -873,101 +936,28 @@ __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl 
           if (rr) atomicAdd(&sm.CR[0][i * M + j], rr);
         }
       }
-      return;
     }
-    // Per segment x of the round, over the chunk's rows: VL[x][k] = rows
-    // with bit k, VE[x][k] = rows with bit k of eL, and the solo terms.
-    // With P1 = rows of popcount N+1 and P0 = rows of popcount N,
-    // VE[x][k] = (VL[x][k] & P1) | (~VL[x][k] & P0) and the solo rows of
-    // bit k are VL[x][k] & P1.  Lane k < M keeps the masks of bit k in this
-    // warp's scratch.
-#pragma unroll
-    for (int xi = 0; xi < K; ++xi) {
-      if (xi >= Kn) break;
-      const unsigned bx = valid ? rec_byte(w, xi) : 0u;
-      if (__ballot_sync(FULL, bx != 0u) == 0u) {
-        if (gathered && lane < M) vw[(2 * xi) * M + lane] = vw[(2 * xi + 1) * M + lane] = 0u;
-        continue;
-      }
-      const int px = __popc(bx);
-      const unsigned p1 = __ballot_sync(FULL, px == N + 1), p0 = __ballot_sync(FULL, px == N);
-      unsigned vl = 0u;
-#pragma unroll
-      for (int k = 0; k < M; ++k) {
-        const unsigned l = __ballot_sync(FULL, (bx >> k) & 1u);
-        if (lane == k) vl = l;
-      }
-      if (lane < M) {
-        const unsigned so = vl & p1;
-        if (so && !gathered) atomicAdd(&sm.S[xi][lane], __popc(so));
-        vw[(2 * xi) * M + lane] = vl;
-        vw[(2 * xi + 1) * M + lane] = so | (~vl & p0);
-      }
-    }
-    __syncwarp();
-    // Pair corrections, over the segment pairs that some row of this chunk
-    // holds both of.  For the pair (a, c) the masks restricted to rows with
-    // both segments non-empty are VE[a][i] & NZ[c] and VL[c][j] & NZ[a];
-    // VE[a][i] lies inside NZ[a] (eL is empty when L is) and VL[c][j] inside
-    // NZ[c], so CL(i, j) = popc(VE[a][i] & VL[c][j]) and likewise
-    // CR(i, j) = popc(VL[a][i] & VE[c][j]).
-    const bool timed = tmain;
-    const unsigned long long t_b = timed ? global_ns() : 0ull;
-    if (timed) s_tin[4] += t_b - t_a;
-    if (gathered) {  // the masks stay in this warp's scratch for the sums below
-      __syncwarp();
-      return;
-    }
-    unsigned segs = 0;
-#pragma unroll
-    for (int xi = 0; xi < K; ++xi) segs |= (b[xi] != 0u ? 1u : 0u) << xi;
-    unsigned wsegs = __popc(segs) >= 2 ? segs : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) wsegs |= __shfl_xor_sync(FULL, wsegs, o);
-    constexpr int U = (MM + 31) / 32;  // (i, j) entries per lane
-#pragma unroll 1
-    for (unsigned sa = wsegs; sa; sa &= sa - 1) {
-      const int a = __ffs(sa) - 1;
-      unsigned ea[U], la[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = (lane + 32 * u < MM ? lane + 32 * u : 0) / M;
-        ea[u] = vw[(2 * a + 1) * M + i];
-        la[u] = vw[(2 * a) * M + i];
-      }
-#pragma unroll 1
-      for (unsigned sc = sa & (sa - 1); sc; sc &= sc - 1) {
-        const int c = __ffs(sc) - 1;
-        const int pid = pair_id<M>(a, c);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int idx = lane + 32 * u;
-          if (idx < MM) {
-            const int j = idx % M;
-            const int cl = __popc(ea[u] & vw[(2 * c) * M + j]);
-            const int cr = __popc(la[u] & vw[(2 * c + 1) * M + j]);
-            if (cl) atomicAdd(&sm.CL[pid][idx], cl);
-            if (cr) atomicAdd(&sm.CR[pid][idx], cr);
-          }
-        }
-      }
-    }
-    __syncwarp();  // the masks are read before the next chunk writes them
-    if (timed) s_tin[5] += global_ns() - t_b;
-  });
-  __syncthreads();
-  if (gathered) {
-    // sums over the chunks' masks (chunk c's at c * 2KM)
-    const unsigned long long t_g = tmain ? global_ns() : 0ull;
-    const unsigned* vb = reinterpret_cast<const unsigned*>(smem_heap);
-    constexpr int NP = RoundSmem<M>::NPAIR;
+    __syncthreads();
+    return;
+  }
+  const int nchunks = (n + 31) / 32;
+  for (int c0 = 0; c0 < nchunks; c0 += NCH) {
+    const int nb = min(NCH, nchunks - c0);
+    const unsigned long long t_a = tmain ? global_ns() : 0ull;
+    if (c0 > 0) __syncthreads();  // the sums of the chunks before have been read
+    masks_of_chunks<M>(sm, J, N, c0, c0 + nb, n, scratch);
+    __syncthreads();
+    const unsigned long long t_b = tmain ? global_ns() : 0ull;
+    if (tmain) s_tin[4] += t_b - t_a;
     if constexpr (M % 4 == 0 && M >= 8) {
       // thread (pair, i) makes CL(i, .) and CR(i, .) of its pair from
-      // VE[a][i], VL[a][i] and the 16-byte rows VL[c][.], VE[c][.] of each
-      // chunk; the K * M threads after them make S[x][k] = popc(VL & VE)
+      // VE[a][i], VL[a][i] and the 16-byte rows VL[c][.], VE[c][.] of every
+      // SPL-th chunk; the K * M threads after them make S[x][k]
+      constexpr int SPL = (NM_THREADS - K * M) / (NP * M);
+      static_assert(SPL >= 1, "a thread a (pair, i) and an S entry");
       const int t = threadIdx.x;
-      if (t < NP * M) {
-        const int pid = t / M, i = t % M;
+      if (t < SPL * NP * M) {
+        const int h = t / (NP * M), pid = t % (NP * M) / M, i = t % M;
         int a = 0, q = pid;  // pair (a, c), a < c, of pair_id
         while (q >= K - 1 - a) {
           q -= K - 1 - a;
@@ -978,21 +968,22 @@ __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl 
           int cl[M], cr[M];
 #pragma unroll
           for (int j = 0; j < M; ++j) cl[j] = cr[j] = 0;
-          for (int w = 0; w < nchunks; ++w) {
-            const unsigned* v = vb + w * (2 * K * M);
+#pragma unroll 2
+          for (int w = h; w < nb; w += SPL) {
+            const unsigned* v = scratch + w * (2 * K * M);
             const unsigned ea = v[(2 * a + 1) * M + i], la = v[(2 * a) * M + i];
 #pragma unroll
-            for (int h = 0; h < M / 4; ++h) {
-              const uint4 x = reinterpret_cast<const uint4*>(v + (2 * c) * M)[h];
-              const uint4 y = reinterpret_cast<const uint4*>(v + (2 * c + 1) * M)[h];
-              cl[4 * h] += __popc(ea & x.x);  // VE[a][i] & VL[c][j]
-              cl[4 * h + 1] += __popc(ea & x.y);
-              cl[4 * h + 2] += __popc(ea & x.z);
-              cl[4 * h + 3] += __popc(ea & x.w);
-              cr[4 * h] += __popc(la & y.x);  // VL[a][i] & VE[c][j]
-              cr[4 * h + 1] += __popc(la & y.y);
-              cr[4 * h + 2] += __popc(la & y.z);
-              cr[4 * h + 3] += __popc(la & y.w);
+            for (int hh = 0; hh < M / 4; ++hh) {
+              const uint4 x = reinterpret_cast<const uint4*>(v + (2 * c) * M)[hh];
+              const uint4 y = reinterpret_cast<const uint4*>(v + (2 * c + 1) * M)[hh];
+              cl[4 * hh] += __popc(ea & x.x);  // VE[a][i] & VL[c][j]
+              cl[4 * hh + 1] += __popc(ea & x.y);
+              cl[4 * hh + 2] += __popc(ea & x.z);
+              cl[4 * hh + 3] += __popc(ea & x.w);
+              cr[4 * hh] += __popc(la & y.x);  // VL[a][i] & VE[c][j]
+              cr[4 * hh + 1] += __popc(la & y.y);
+              cr[4 * hh + 2] += __popc(la & y.z);
+              cr[4 * hh + 3] += __popc(la & y.w);
             }
           }
 #pragma unroll
@@ -1001,27 +992,29 @@ __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl 
             if (cr[j]) atomicAdd(&sm.CR[pid][i * M + j], cr[j]);
           }
         }
-      } else if (t < NP * M + K * M) {
-        const int e = t - NP * M, xi = e / M, k = e % M;
+      } else if (t < SPL * NP * M + K * M) {
+        const int e = t - SPL * NP * M, xi = e / M, k = e % M;
         int sum = 0;
         if (xi < Kn)
-          for (int w = 0; w < nchunks; ++w) {
-            const unsigned* v = vb + w * (2 * K * M);
+          for (int w = 0; w < nb; ++w) {
+            const unsigned* v = scratch + w * (2 * K * M);
             sum += __popc(v[(2 * xi) * M + k] & v[(2 * xi + 1) * M + k]);
           }
         if (sum) atomicAdd(&sm.S[xi][k], sum);
       }
-      static_assert(RoundSmem<M>::NPAIR * M + (M + 1) * M <= NM_THREADS, "a thread a (pair, i) and an S entry");
     } else {
-      // one thread an entry of S, CL, CR (in that order, as laid out)
+      // a thread an entry of S, CL, CR (in that order, as laid out) and every
+      // SPL-th chunk, or more entries a thread where there are more
       constexpr int NSUM = K * M + 2 * NP * MM;
-      for (int e = threadIdx.x; e < NSUM; e += NM_THREADS) {
+      constexpr int SPL = NSUM <= NM_THREADS ? NM_THREADS / NSUM : 1;
+      const int h = SPL > 1 ? threadIdx.x / NSUM : 0;
+      for (int e = SPL > 1 ? threadIdx.x % NSUM : threadIdx.x; e < NSUM && h < SPL; e += SPL > 1 ? NSUM : NM_THREADS) {
         int sum = 0;
-        if (e < K * M) {  // S[x][k] = rows with bit k and popcount N+1 = popc(VL & VE)
+        if (e < K * M) {
           const int xi = e / M, k = e % M;
           if (xi < Kn)
-            for (int w = 0; w < nchunks; ++w) {
-              const unsigned* v = vb + w * (2 * K * M);
+            for (int w = h; w < nb; w += SPL) {
+              const unsigned* v = scratch + w * (2 * K * M);
               sum += __popc(v[(2 * xi) * M + k] & v[(2 * xi + 1) * M + k]);
             }
           if (sum) atomicAdd(&sm.S[xi][k], sum);
@@ -1035,8 +1028,8 @@ __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl 
           }
           const int c = a + 1 + q;
           if (c < Kn)
-            for (int w = 0; w < nchunks; ++w) {
-              const unsigned* v = vb + w * (2 * K * M);
+            for (int w = h; w < nb; w += SPL) {
+              const unsigned* v = scratch + w * (2 * K * M);
               sum += side == 0 ? __popc(v[(2 * a + 1) * M + i] & v[(2 * c) * M + j])   // CL: VE[a][i] & VL[c][j]
                                : __popc(v[(2 * a) * M + i] & v[(2 * c + 1) * M + j]);  // CR: VL[a][i] & VE[c][j]
             }
@@ -1044,9 +1037,9 @@ __device__ void process_phase(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl 
         }
       }
     }
-    if (tmain) s_tin[5] += global_ns() - t_g;
-    __syncthreads();
+    if (tmain) s_tin[5] += global_ns() - t_b;
   }
+  __syncthreads();
   if (tmain) s_tin[2] += global_ns() - t_in;
 }
 
@@ -1458,64 +1451,74 @@ __device__ void apply_recount(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl)
     J.orig[v1] = o2;
     J.orig[v2] = o1;
   }
-  const int Kn = sm.K_;
-  const int lane = tid & 31;
-  // where the bits of each nibble of each segment's group go, packed like
-  // the record (4 segments per word): one table entry per (segment, nibble
-  // position, nibble value)
-  constexpr int NH = (M + 3) / 4;
+  // A swap moves whole columns of bits, so the rows' groups afterwards are
+  // the same column masks in other places: a thread takes a segment and a
+  // chunk, reads the masks of the columns it now holds, and counts the rows
+  // that are not empty, and those with more than N bits by a bit-sliced sum.
+  // A helper still has the process phase's masks in its scratch; the leader's
+  // made way for the heaps and are made again.
+  constexpr int NCH = mask_chunks<M>();
   extern __shared__ uint4 smem_heap[];
-  uint4 (*bitmove)[NH][16] = reinterpret_cast<uint4 (*)[NH][16]>(smem_heap);  // [K][NH][16]
-  static_assert((M + 1) * NH * 16 * 16 <= RoundSmem<M>::PROC_BYTES, "bit-move table fits the scratch");
-  for (int t = tid; t < Kn * NH * 16; t += NM_THREADS) {
-    const int xi = t / (NH * 16), h = (t / 16) % NH, v = t % 16;
-    unsigned o[3] = {0u, 0u, 0u};
-    for (int q = 0; q < 4; ++q) {
-      const int k = 4 * h + q;
-      if (k < M && ((v >> q) & 1)) {
-        const int d = sm.dest[xi][k];
-        const int dx = d >> 4, dk = d & 15;
-        o[dx >> 2] |= (1u << dk) << ((dx & 3) * 8);
-      }
-    }
-    bitmove[xi][h][v] = make_uint4(o[0], o[1], o[2], 0u);
+  unsigned* const scratch = reinterpret_cast<unsigned*>(smem_heap);
+  const int Kn = sm.K_;
+  const int n = sm.use_table ? sm.tcount : sm.ntouched;
+  const int nchunks = (n + 31) / 32;
+  if (tid < Kn * M) {
+    const int d = sm.dest[tid / M][tid % M];
+    sm.from[(d >> 4) * M + (d & 15)] = (uint8_t)tid;
   }
-  __syncthreads();
   const bool tmain = threadIdx.x == 0 && sl.rank == 0 && J.timed;
   const unsigned long long t_in = tmain ? global_ns() : 0ull;
-  for_rows_warp<M, 2>(sm, J, [&](int r, const uint4& w, bool valid, int chunk) {
-    (void)chunk;
-    // the row's groups after the swaps, packed like the record
-    unsigned n0 = 0, n1 = 0, n2 = 0;
+  const bool kept = sl.rank != 0 && nchunks <= NCH && sm.mode != 2;
+  constexpr int PER = NM_THREADS / K;  // threads a segment
+  const int xi = tid / PER, ti = tid % PER;
+  int inv = 0, pres = 0;
+  for (int c0 = 0; c0 < nchunks; c0 += NCH) {
+    const int nb = min(NCH, nchunks - c0);
+    if (c0 > 0) __syncthreads();
+    if (!kept) masks_of_chunks<M>(sm, J, N, c0, c0 + nb, n, scratch);
+    __syncthreads();
+    if (xi < Kn) {
+      int at[M];  // the masks of this segment's columns
 #pragma unroll
-    for (int xi = 0; xi < K; ++xi) {
-      const unsigned bb = (valid && xi < Kn) ? rec_byte(w, xi) : 0u;
+      for (int k = 0; k < M; ++k) {
+        const int f = sm.from[xi * M + k];
+        at[k] = (2 * (f / M)) * M + f % M;
+      }
+      for (int c = ti; c < nb; c += PER) {
+        const unsigned* v = scratch + c * (2 * K * M);
+        unsigned s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // bits of the rows' counts
 #pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        const unsigned nib = (bb >> (4 * h)) & 15u;
-        if (nib) {
-          const uint4 m = bitmove[xi][h][nib];
-          n0 |= m.x;
-          n1 |= m.y;
-          n2 |= m.z;
+        for (int k = 0; k < M; ++k) {
+          const unsigned m = v[at[k]], c1 = s0 & m, c2 = s1 & c1;
+          s0 ^= m;
+          s1 ^= c1;
+          s3 |= s2 & c2;
+          s2 ^= c2;
         }
+        unsigned gt = 0u, eq = ~0u;  // count > N
+        const unsigned bit[4] = {s3, s2, s1, s0};
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          if ((N >> (3 - b)) & 1) {
+            eq &= bit[b];
+          } else {
+            gt |= eq & bit[b];
+            eq &= ~bit[b];
+          }
+        }
+        inv += __popc(gt);
+        pres += __popc(s0 | s1 | s2 | s3);
       }
     }
-    // non-empty and invalid groups per segment, one shared add per warp
-#pragma unroll
-    for (int xi = 0; xi < K; ++xi) {
-      if (xi >= Kn) break;
-      const unsigned nb = ((xi < 4 ? n0 : (xi < 8 ? n1 : n2)) >> ((xi & 3) * 8)) & 0xffu;
-      const unsigned pres = __ballot_sync(FULL, nb != 0u);
-      const unsigned inv = __ballot_sync(FULL, __popc(nb) > N);
-      if (lane == 0 && pres) atomicAdd(&sm.newpres[xi], __popc(pres));
-      if (lane == 0 && inv) atomicAdd(&sm.newinv[xi], __popc(inv));
-    }
-    if (valid) {
-      if (sm.use_table) sm.table[r] = make_uint4(0u, 0u, 0u, 0u);
-      else J.rec[r] = make_uint4(0u, 0u, 0u, 0u);
-    }
-  });
+  }
+  if (pres) atomicAdd(&sm.newpres[xi], pres);
+  if (inv) atomicAdd(&sm.newinv[xi], inv);
+  // the records are zero between rounds
+  for (int i = tid; i < n; i += NM_THREADS) {
+    if (sm.use_table) sm.table[sm.tlist[i]] = make_uint4(0u, 0u, 0u, 0u);
+    else J.rec[J.touched[sm.toff + i]] = make_uint4(0u, 0u, 0u, 0u);
+  }
   if (tmain) s_tin[3] += global_ns() - t_in;
   __syncthreads();
   if (threadIdx.x == 0) sm.tcount = 0;  // the table is empty again (before the next round's inserts)
@@ -1575,7 +1578,7 @@ __device__ void cluster_push(cg::cluster_group& cl, int* mine, int n) {
 // round is copied to every block before the barrier that opens it.
 template <int M>
 __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __restrict__ jobs, int N,
-                                                              int cnt_in_smem, int ts_max, int cs, int rcache_on) {
+                                                              int cnt_in_smem, int ts_max, int dslots, int cs) {
   constexpr int K = M + 1;
   __shared__ RoundSmem<M> sm;
   static_assert(offsetof(RoundSmem<M>, CL) == offsetof(RoundSmem<M>, S) + sizeof(int) * K * M, "S, CL adjacent");
@@ -1584,15 +1587,13 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
   static_assert(offsetof(RoundSmem<M>, newpres) == offsetof(RoundSmem<M>, newinv) + sizeof(int) * K,
                 "newinv, newpres adjacent");
   constexpr int NSUM = K * M + 2 * RoundSmem<M>::NPAIR * RoundSmem<M>::MM;
-  // dynamic shared memory: [heap scratch][row-record table: ts_max x 16 B]
-  // [claimed-slot list: ts_max x 4 B][record cache: NM_THREADS x TOUCH_U x
-  // (16 + 4) B, when on][segment counts]
+  // dynamic shared memory: [scratch][row-record table: its slots x 16 B][list
+  // of the slots in use: slots x 2 B][segment counts]
   extern __shared__ uint4 smem_heap[];
+  const int slots = dslots > 0 ? dslots : ts_max;
   uint4* smem_dyn = smem_heap + RoundSmem<M>::SCR_U4;
-  int* smem_list = reinterpret_cast<int*>(smem_dyn + ts_max);
-  uint4* smem_rcache = reinterpret_cast<uint4*>(smem_list + ts_max);
-  int* smem_rcrow = reinterpret_cast<int*>(smem_rcache + (rcache_on ? NM_THREADS * TOUCH_U : 0));
-  int* smem_cnt = smem_rcrow + (rcache_on ? NM_THREADS * TOUCH_U : 0);
+  uint16_t* smem_list = reinterpret_cast<uint16_t*>(smem_dyn + slots);
+  int* smem_cnt = reinterpret_cast<int*>(smem_list + slots);
   cg::cluster_group cl = cg::this_cluster();
   const int rank = cs > 1 ? (int)cl.block_rank() : 0;
   const bool lead = rank == 0;
@@ -1605,13 +1606,12 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
   int* cnt = cnt_in_smem ? smem_cnt : J.cnt;
   if (lead && cnt_in_smem)
     for (int s = tid; s < J.nseg; s += NM_THREADS) smem_cnt[s] = J.cnt[s];
-  for (int i = tid; i < ts_max; i += NM_THREADS) smem_dyn[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = tid; i < slots; i += NM_THREADS) smem_dyn[i] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) {
     sm.status = JOB_OK;
-    sm.table = ts_max > 0 ? smem_dyn : nullptr;
-    sm.tlist = ts_max > 0 ? smem_list : nullptr;
-    sm.rcache = rcache_on ? smem_rcache : nullptr;
-    sm.rcrow = rcache_on ? smem_rcrow : nullptr;
+    sm.table = slots > 0 ? smem_dyn : nullptr;
+    sm.tlist = slots > 0 ? smem_list : nullptr;
+    sm.dslots = dslots;
     sm.tcount = 0;
     sm.toff = rank * ((J.R + ROW_GROUPS - 1) / ROW_GROUPS + 1) * (ROW_GROUPS / cs);
     for (int q = 0; q < 4; ++q) sm.acc[q] = 0ull;
@@ -1807,8 +1807,7 @@ __global__ void __launch_bounds__(NM_THREADS) k_pair_score(NMJob J, int N, int s
     sm.ts_max = 0;
     sm.use_table = 0;
     sm.toff = 0;
-    sm.rcache = nullptr;
-    sm.rcrow = nullptr;
+    sm.dslots = 0;
     sm.xseg[0] = s1;
     sm.xcnt[0] = 0;
     if (s1 == s2) {
@@ -1950,6 +1949,7 @@ size_t job_bytes(int R) {
 // Carve one job's state out of the arena and initialise it.
 static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J) {
   J.R = P.R;
+  J.row0 = 0;
   J.nseg = P.nseg;
   J.sched = sched;
   J.maxiter = maxiter;
@@ -1987,12 +1987,43 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   return VNM_OK;
 }
 
-// Shared memory beyond RoundSmem: the swap-heap scratch, the segment counts when
-// they are small (<= 64 KB), and a row-record table of up to 8192 16-byte
-// slots in what is left of a 150 KB budget (the rest of the SM's 256 KB is L1,
-// which the gather phase's reads of the column pattern live on: 200 KB ran the
-// 256-matrix 2:8 batch 4 % slower when it used one block per job).
+// Shared memory beyond RoundSmem: the scratch, the segment counts when they
+// are small (<= 64 KB), and the row records: a slot for every row a block owns
+// when those are at most DIRECT_MAX (up to 78 KB), else a hashed table of up
+// to 8192 slots in what is left of a 150 KB budget (the rest of the SM's 256
+// KB is L1, which the gather phase's reads of the column pattern live on: 200
+// KB ran the 256-matrix 2:8 batch 4 % slower when it used one block per job
+// and its records lay in global memory).
 constexpr size_t NM_SMEM_BUDGET = 150u << 10;
+
+// How the blocks of a cluster of cs hold their records: dslots > 0 or ts > 0.
+struct RoundShape {
+  int dslots, ts;
+  size_t dyn;
+};
+template <int M>
+static RoundShape round_shape(int max_nseg, int max_runs, int cs) {
+  const size_t cbytes = (size_t)max_nseg * sizeof(int);
+  const bool in_smem = cbytes <= (64u << 10);
+  const size_t hbytes = (size_t)RoundSmem<M>::SCR_U4 * sizeof(uint4);
+  const size_t fixed = sizeof(RoundSmem<M>) + hbytes + (in_smem ? cbytes : 0);
+  constexpr size_t SLOT = sizeof(uint4) + sizeof(uint16_t);  // a table slot and its list entry
+  RoundShape f{0, 0, 0};
+  const long long own = ((long long)max_runs * (ROW_GROUPS / cs) + 31) / 32 * 32;
+  // VNM_NM_ROW_TABLE=0 keeps every round's records in global memory, for measurement.
+  const char* e = getenv("VNM_NM_ROW_TABLE");
+  if (!e || atoi(e) != 0) {
+    if (own <= DIRECT_MAX) {
+      f.dslots = (int)own;
+    } else {
+      f.ts = 8192;
+      while (f.ts >= 1024 && fixed + (size_t)f.ts * SLOT > NM_SMEM_BUDGET) f.ts >>= 1;
+      if (f.ts < 1024) f.ts = 0;
+    }
+  }
+  f.dyn = hbytes + (size_t)(f.dslots + f.ts) * SLOT + (in_smem ? cbytes : 0);
+  return f;
+}
 
 // k_nm_rounds<M>'s dynamic shared-memory ceiling depends on the call (the
 // segment counts and the table size), and it is a property of the function
@@ -2002,33 +2033,18 @@ constexpr size_t NM_SMEM_BUDGET = 150u << 10;
 static std::mutex g_round_launch_mu;
 
 template <int M>
-static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int max_nseg, int cs) {
+static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int max_nseg, int max_runs,
+                                  int cs) {
   std::lock_guard<std::mutex> launch_lock(g_round_launch_mu);
   ctx->last_clusters_fit = 0;
-  const size_t cbytes = (size_t)max_nseg * sizeof(int);
-  const int in_smem = cbytes <= (64u << 10) ? 1 : 0;
-  const size_t hbytes = (size_t)RoundSmem<M>::SCR_U4 * sizeof(uint4);
-  const size_t fixed = sizeof(RoundSmem<M>) + hbytes + (in_smem ? cbytes : 0);
-  constexpr size_t SLOT = sizeof(uint4) + sizeof(int);  // a table slot and its list entry
-  int ts = 8192;
-  while (ts >= 1024 && fixed + (size_t)ts * SLOT > NM_SMEM_BUDGET) ts >>= 1;
-  if (ts < 1024) ts = 0;
-  // Each block keeps the records of the rows it owns in its own table (a
-  // round whose entries would fill more than 3/4 of it uses J.rec in global
-  // memory instead).  VNM_NM_ROW_TABLE=0 keeps every round's records in
-  // global memory, for measurement.
-  if (const char* e = getenv("VNM_NM_ROW_TABLE"))
-    if (atoi(e) == 0) ts = 0;
-
-  // the record cache of the apply phase, when the budget allows it
-  constexpr size_t RCACHE = (size_t)NM_THREADS * TOUCH_U * (sizeof(uint4) + sizeof(int));
-  int rc = fixed + (size_t)ts * SLOT + RCACHE <= NM_SMEM_BUDGET ? 1 : 0;
-  const size_t dyn = hbytes + (size_t)ts * SLOT + (rc ? RCACHE : 0) + (in_smem ? cbytes : 0);
-  // static + dynamic shared memory may pass the 48 KB a launch gets without
-  // opting in (RoundSmem<8> alone is ~30 KB)
-  VNM_CUDA_TRY(cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  const int in_smem = (size_t)max_nseg * sizeof(int) <= (64u << 10) ? 1 : 0;
   if (cs > 8)
     VNM_CUDA_TRY(cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  // static + dynamic shared memory may pass the 48 KB a launch gets without
+  // opting in (RoundSmem<8> alone is ~30 KB)
+  auto set_dyn = [&](const RoundShape& f) {
+    return cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.dyn);
+  };
   if (cs > 1) {
     // How many clusters of a size the GPU can hold at once depends on the
     // SMs of each of its GPCs; take the largest size (halving from cs) at
@@ -2036,7 +2052,6 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
     // fits at all.
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(NM_THREADS);
-    cfg.dynamicSmemBytes = dyn;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2046,10 +2061,12 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
     cfg.numAttrs = 1;
     int pick = 1, fallback = 1;
     for (int c = cs; c > 1; c >>= 1) {
+      const RoundShape f = round_shape<M>(max_nseg, max_runs, c);
       attr[0].val.clusterDim.x = (unsigned)c;
       cfg.gridDim = dim3((unsigned)(njobs * c));
+      cfg.dynamicSmemBytes = f.dyn;
       int nclusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, k_nm_rounds<M>, &cfg) != cudaSuccess) {
+      if (set_dyn(f) != cudaSuccess || cudaOccupancyMaxActiveClusters(&nclusters, k_nm_rounds<M>, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         continue;
       }
@@ -2065,19 +2082,21 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
     }
     if (pick == 1) pick = fallback;
     if (pick > 1) {
+      const RoundShape f = round_shape<M>(max_nseg, max_runs, pick);
+      VNM_CUDA_TRY(set_dyn(f));
       attr[0].val.clusterDim.x = (unsigned)pick;
       cfg.gridDim = dim3((unsigned)(njobs * pick));
-      VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_nm_rounds<M>, d_jobs, N, in_smem, ts, pick, rc));
+      cfg.dynamicSmemBytes = f.dyn;
+      VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_nm_rounds<M>, d_jobs, N, in_smem, f.ts, f.dslots, pick));
       ctx->launches++;
       ctx->last_cluster = pick;
       return VNM_OK;
     }
-    // no cluster fits: one block per job
-    VNM_LAUNCH(ctx, k_nm_rounds<M>, njobs, NM_THREADS, dyn, d_jobs, N, in_smem, ts, 1, rc);
-    ctx->last_cluster = 1;
-    return VNM_OK;
   }
-  VNM_LAUNCH(ctx, k_nm_rounds<M>, njobs, NM_THREADS, dyn, d_jobs, N, in_smem, ts, 1, rc);
+  // one block per job (asked for, or no cluster fits)
+  const RoundShape f = round_shape<M>(max_nseg, max_runs, 1);
+  VNM_CUDA_TRY(set_dyn(f));
+  VNM_LAUNCH(ctx, k_nm_rounds<M>, njobs, NM_THREADS, f.dyn, d_jobs, N, in_smem, f.ts, f.dslots, 1);
   ctx->last_cluster = 1;
   return VNM_OK;
 }
@@ -2097,16 +2116,17 @@ static int nm_cluster_size(long long np) {
   return np >= (1ll << 17) ? 16 : 8;
 }
 
-static vnm_status launch_rounds(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int M, int max_nseg,
-                                int cs = 1) {
+// max_runs: aligned runs of 16 rows a job's rows lie in, at most.
+static vnm_status launch_rounds(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int M, int max_nseg, int max_runs,
+                                int cs) {
   switch (M) {
-    case 2: return launch_rounds_t<2>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 3: return launch_rounds_t<3>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 4: return launch_rounds_t<4>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 5: return launch_rounds_t<5>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 6: return launch_rounds_t<6>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 7: return launch_rounds_t<7>(ctx, d_jobs, njobs, N, max_nseg, cs);
-    case 8: return launch_rounds_t<8>(ctx, d_jobs, njobs, N, max_nseg, cs);
+    case 2: return launch_rounds_t<2>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 3: return launch_rounds_t<3>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 4: return launch_rounds_t<4>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 5: return launch_rounds_t<5>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 6: return launch_rounds_t<6>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 7: return launch_rounds_t<7>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 8: return launch_rounds_t<8>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
   }
   return VNM_ERR_ARG;
 }
@@ -2218,7 +2238,7 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
   // the stored entries stand in for the pattern's (nonzero-valued) entries
   // when sizing the clusters: their count is known without a readback
-  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, nm_cluster_size(nnz)));
+  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, nm_cluster_size(nnz)));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hp = ctx->h_pinned;
   for (int s = 0; s < nsched; ++s)
@@ -2415,10 +2435,11 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   VNM_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(uint4) * (R > 0 ? R : 1), ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(res, 0, sizeof(int) * JOB_RES * nmat, ctx->stream));
   std::vector<NMJob> hj(nmat);
-  int max_nseg = 0;
+  int max_nseg = 0, max_runs = 0;
   for (int b = 0; b < nmat; ++b) {
     NMJob& J = hj[b];
     J.R = nrows[b];
+    J.row0 = row_off[b];
     J.nseg = nrows[b] / M;
     J.sched = sched;
     J.maxiter = maxiter;
@@ -2440,6 +2461,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     J.err = nullptr;
     J.timed = ctx->phase_timing ? 1 : 0;
     if (J.nseg > max_nseg) max_nseg = J.nseg;
+    if (J.R > 0) max_runs = std::max(max_runs, ((row_off[b] + J.R - 1) >> 4) - (row_off[b] >> 4) + 1);
   }
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, hj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
   VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, d_soff);
@@ -2448,7 +2470,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   // jobs, and two SMs each shorten them more than the extra waves cost
   // (GB300, 256 R-MAT matrices 256-8192 rows at 2:8: 88 ms with one block
   // per job, 63 ms with 2, 69 ms with 4)
-  VNM_TRY(launch_rounds(ctx, d_jobs, nmat, N, M, max_nseg, 2));
+  VNM_TRY(launch_rounds(ctx, d_jobs, nmat, N, M, max_nseg, max_runs, 2));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hres = ctx->h_pinned + 256;
   VNM_CUDA_TRY(cudaMemcpyAsync(hres, res, sizeof(int) * JOB_RES * nmat, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2717,7 +2739,7 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   VNM_CUDA_TRY(cudaMemcpyAsync(d_job, &hj, sizeof(NMJob), cudaMemcpyHostToDevice, c.stream));
   // the same launch shape as vnm_nm_reorder (a cluster of blocks per job);
   // the scratch it needs does not depend on the cluster size
-  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, nm_cluster_size(P.np)));
+  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, nm_cluster_size(P.np)));
   VNM_CUDA_TRY(cudaMemcpyAsync(hs, hj.res, sizeof(int) * 16, cudaMemcpyDeviceToHost, c.stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(c.stream));
   if (hs[5] != 0) return VNM_ERR_INTERNAL;
