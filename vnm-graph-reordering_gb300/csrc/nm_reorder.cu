@@ -1232,10 +1232,12 @@ __device__ void heap_sift(RoundSmem<M>& sm) {
 // a lane mask; each step is a few warp votes and shuffles:
 //   - primary: the largest list key among the list's lanes; its visited
 //     bits then live in a register of every lane for the pass;
-//   - targets: each lane's position in traversal order by comparing keys,
-//     inverted once per pass into a list of the targets' lanes;
+//   - targets: each lane's position in traversal order by comparing keys;
+//     for the pass lane x holds the x-th target's state, so that a step's
+//     shuffles do not wait for one another;
 //   - the first unvisited swap of a pair's pop order: the unique largest
-//     qualifying key read off the entries, else a ballot over the pops;
+//     qualifying key, which carries its swap and its gains, read off the
+//     entries, else a ballot over the pops;
 //   - each committed swap's bit moves go straight into dest.
 __device__ __forceinline__ unsigned order_key_hi(int c, bool rev) {  // count, order-preserving
   const unsigned u = (unsigned)c ^ 0x80000000u;
@@ -1328,105 +1330,100 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
         const unsigned qh = __shfl_sync(FULL, th, q), ql = __shfl_sync(FULL, tl, q);
         pos += (((Tm >> q) & 1u) && (qh > th || (qh == th && ql > tl))) ? 1 : 0;
       }
-      // lane x: the lane of the x-th target
+      // lane x: the x-th target's lane, counts and visited bits for the pass
       int tx = 0;
 #pragma unroll
       for (int q = 0; q < K; ++q) {
         const int pq = __shfl_sync(FULL, pos, q);
         if (((Tm >> q) & 1u) && pq == lane) tx = q;
       }
+      const int tseg = __shfl_sync(FULL, seg, tx), tcol = pxi * K + tx;
+      int tcnt = __shfl_sync(FULL, cnt, tx);
+      unsigned tvis = __shfl_sync(FULL, vis, tx);
       const int nT = __popc(Tm);
-      unsigned Um = 0;
+      unsigned Ux = 0;  // bit x: the x-th target stays in the list
       for (int x = 0; x < nT; ++x) {
         if (pc <= 0 || vp == FULLM) break;
-        const int txi = __shfl_sync(FULL, tx, x);
-        const unsigned vt = __shfl_sync(FULL, vis, txi);
-        int tc = __shfl_sync(FULL, cnt, txi);
+        const int col = __shfl_sync(FULL, tcol, x);
+        const unsigned vt = __shfl_sync(FULL, tvis, x);
         // First pop of the pair whose two nodes are both unvisited.  A heap
         // pops in non-increasing key order, so that is the qualifying swap of
         // largest key when only one has it (read off the entries); on a tie
         // it is the first of them in the pops published so far, waiting for
         // more while none qualifies.
-        const int col = pxi * K + txi;
-        const uint8_t* ord = ord0 + col;
-        int pick = -1, seen = 0;
-        unsigned pe = ~0u;  // the pick's entry word, when read off the entries
-        {
-          unsigned eo[U];  // this lane's entries: entry k holds swap k
-          unsigned kq[U];  // key + 1 of this lane's qualifying swaps, else 0
-          unsigned best = 0;
+        unsigned kq[U], most = 0;  // (key + 1) << 6 | swap of this lane's qualifying swaps, else 0
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int k = lane + 32 * u;
-            const unsigned e = k < MM ? ent[k * HS + col] : 0u;
-            eo[u] = e;
-            const bool ok = k < MM && !((vp >> (k / M)) & 1u) && !((vt >> (k % M)) & 1u);
-            kq[u] = ok ? (e >> 8) + 1u : 0u;
-            best = max(best, __reduce_max_sync(FULL, kq[u]));
-          }
-          int nbest = 0, who = -1;
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const unsigned bb = __ballot_sync(FULL, best != 0u && kq[u] == best);
-            nbest += __popc(bb);
-            if (bb && who < 0) who = 32 * u + __ffs(bb) - 1;
-          }
-          if (nbest == 1) {  // swap index == entry position
-            pick = who;
-            unsigned ep = eo[0];
-#pragma unroll
-            for (int u = 1; u < U; ++u)
-              if ((pick >> 5) == u) ep = eo[u];
-            pe = __shfl_sync(FULL, ep, pick & 31);
-          }
+        for (int u = 0; u < U; ++u) {
+          const int k = lane + 32 * u;  // entry k holds swap k
+          const unsigned e = k < MM ? ent[k * HS + col] : 0u;
+          const bool ok = k < MM && !((vp >> (k / M)) & 1u) && !((vt >> (k % M)) & 1u);
+          kq[u] = ok ? ((e >> 8) + 1u) << 6 | (unsigned)k : 0u;
+          most = max(most, kq[u]);
         }
-        while (pick < 0 && !dead) {
-          if (seen >= MM) {  // unreachable: a scored target always has an unvisited node
-            if (lane == 0) sm.status |= JOB_EMPTY_HEAP;
-            pick = ord[(MM - 1) * HS];
-            break;
+        const bool small = sm.hsmall[col];
+        const unsigned best = __reduce_max_sync(FULL, most);
+        int nbest = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) nbest += __popc(__ballot_sync(FULL, kq[u] >> 6 == best >> 6));
+        int pick = (int)(best & 63u);
+        unsigned key = (best >> 6) - 1u;
+        if (best == 0u || nbest != 1) {
+          const uint8_t* ord = ord0 + col;
+          int seen = 0;
+          pick = -1;
+          while (pick < 0 && !dead) {
+            if (seen >= MM) {  // unreachable: a scored target always has an unvisited node
+              if (lane == 0) sm.status |= JOB_EMPTY_HEAP;
+              pick = ord[(MM - 1) * HS];
+              break;
+            }
+            const int avail = wait_pops(col, seen + 1);
+            if (avail < 0) {
+              dead = true;
+              break;
+            }
+            for (int k0 = seen; k0 < avail && pick < 0; k0 += 32) {
+              const int k = k0 + lane;
+              const int e = k < avail ? ord[k * HS] : 0;
+              const bool ok = k < avail && !((vp >> (e / M)) & 1u) && !((vt >> (e % M)) & 1u);
+              const unsigned bal = __ballot_sync(FULL, ok);
+              if (bal) pick = __shfl_sync(FULL, e, __ffs(bal) - 1);
+            }
+            seen = avail;
           }
-          const int avail = wait_pops(col, seen + 1);
-          if (avail < 0) {
-            dead = true;
-            break;
-          }
-          for (int k0 = seen; k0 < avail && pick < 0; k0 += 32) {
-            const int k = k0 + lane;
-            const int e = k < avail ? ord[k * HS] : 0;
-            const bool ok = k < avail && !((vp >> (e / M)) & 1u) && !((vt >> (e % M)) & 1u);
-            const unsigned bal = __ballot_sync(FULL, ok);
-            if (bal) pick = __shfl_sync(FULL, e, __ffs(bal) - 1);
-          }
-          seen = avail;
+          if (dead) pick = 0;
+          key = ent[pick * HS + col] >> 8;
         }
-        if (dead) pick = 0;
         int l, r;
-        if (sm.hsmall[col]) {  // the gains are the pick's key: (l + r + 2048) << 12 | (r + 2048)
-          if (pe == ~0u || dead) pe = ent[pick * HS + col];  // picked from the pops
-          const unsigned key = pe >> 8;
+        if (small) {  // the gains are the pick's key: (l + r + 2048) << 12 | (r + 2048)
           r = (int)(key & 4095u) - 2048;
           l = (int)(key >> 12) - 2048 - r;
         } else {
-          pair_gains<M>(sm, pxi, txi, pick, l, r);
+          pair_gains<M>(sm, pxi, col - pxi * K, pick, l, r);
         }
         const int i = pick / M, j = pick % M;
-        if (lane == 0) {
+        if (lane == x) {
           sm.swaps[2 * nsw] = sp * M + i;
-          sm.swaps[2 * nsw + 1] = sm.xseg[txi] * M + j;
-          sm.dest[pxi][i] = (uint8_t)((txi << 4) | j);
-          sm.dest[txi][j] = (uint8_t)((pxi << 4) | i);
+          sm.swaps[2 * nsw + 1] = tseg * M + j;
+          sm.dest[pxi][i] = (uint8_t)((tx << 4) | j);
+          sm.dest[tx][j] = (uint8_t)((pxi << 4) | i);
+          tvis |= 1u << j;
+          tcnt -= r;
         }
         ++nsw;
         vp |= 1u << i;
-        if (lane == txi) vis |= 1u << j;
         pc -= l;
-        tc -= r;
-        if (lane == txi) cnt = tc;
-        if (tc > 0) Um |= 1u << txi;
+        if (__shfl_sync(FULL, tcnt, x) > 0) Ux |= 1u << x;
+      }
+      // back to the segments' lanes
+      const int c1 = __shfl_sync(FULL, tcnt, pos);
+      const unsigned v1 = __shfl_sync(FULL, tvis, pos);
+      if (isT) {
+        cnt = c1;
+        vis = v1;
       }
       if (lane == pxi) vis = vp;
-      Wm = Um;
+      Wm = __ballot_sync(FULL, isT && ((Ux >> pos) & 1u));
     }
   }
   if (lane == 0) {
