@@ -1232,9 +1232,8 @@ __device__ void heap_sift(RoundSmem<M>& sm) {
 // a lane mask; each step is a few warp votes and shuffles:
 //   - primary: the largest list key among the list's lanes; its visited
 //     bits then live in a register of every lane for the pass;
-//   - targets: each lane's position in traversal order by comparing keys;
-//     for the pass lane x holds the x-th target's state, so that a step's
-//     shuffles do not wait for one another;
+//   - targets: the largest traversal key among the lanes left, the next one
+//     found while the current one is worked on;
 //   - the first unvisited swap of a pair's pop order: the unique largest
 //     qualifying key, which carries its swap and its gains, read off the
 //     entries, else a ballot over the pops;
@@ -1310,42 +1309,50 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
     int cnt = lane < Kn ? sm.xcnt[lane] : 0;
     unsigned vis = 0;
     unsigned Wm = (1u << Kn) - 1u;
+    // the lane of `lanes` (not empty) with the largest (hi, lo); lo is looked
+    // at only where several share the largest hi
+    auto top_lane = [&](unsigned lanes, unsigned hi, unsigned lo) -> int {
+      const bool in = (lanes >> lane) & 1u;
+      const unsigned mh = __reduce_max_sync(FULL, in ? hi : 0u);
+      unsigned at = __ballot_sync(FULL, in && hi == mh);
+      if (at & (at - 1u)) {
+        const bool tied = (at >> lane) & 1u;
+        const unsigned ml = __reduce_max_sync(FULL, tied ? lo : 0u);
+        at = __ballot_sync(FULL, tied && lo == ml);
+      }
+      return __ffs(at) - 1;
+    };
     while (__popc(Wm) >= 2) {
-      const bool inW = (Wm >> lane) & 1u;
-      // primary = top of the list (largest key; 0 marks lanes outside it)
-      const unsigned lh = inW ? order_key_hi(cnt, rev_list) : 0u, ll = inW ? order_key_lo(seg, rev_list) : 0u;
-      const unsigned mh = __reduce_max_sync(FULL, lh);
-      const unsigned ml = __reduce_max_sync(FULL, lh == mh ? ll : 0u);
-      const int pxi = __ffs(__ballot_sync(FULL, inW && lh == mh && ll == ml)) - 1;
+      // primary = top of the list
+      const int pxi = top_lane(Wm, order_key_hi(cnt, rev_list), order_key_lo(seg, rev_list));
       int pc = __shfl_sync(FULL, cnt, pxi);
       unsigned vp = __shfl_sync(FULL, vis, pxi);  // the primary's visited bits, on every lane
       const int sp = __shfl_sync(FULL, seg, pxi);
-      // targets: the rest of the list, by position in traversal order
-      const unsigned Tm = Wm & ~(1u << pxi);
-      const bool isT = (Tm >> lane) & 1u;
-      const unsigned th = isT ? order_key_hi(cnt, trav_rev) : 0u, tl = isT ? order_key_lo(seg, trav_rev) : 0u;
-      int pos = 0;
+      // targets: the rest of the list in traversal order, by their counts at
+      // the start of the pass; the next target, its state and its entries are
+      // fetched while the current one is worked on
+      unsigned left = Wm & ~(1u << pxi);
+      const unsigned th = order_key_hi(cnt, trav_rev), tl = order_key_lo(seg, trav_rev);
+      int ntx = 0, ntc = 0;
+      unsigned nvt = 0, ne[U];
+      bool nsmall = false;
+      auto fetch = [&]() {
+        ntx = top_lane(left, th, tl);
+        nvt = __shfl_sync(FULL, vis, ntx);
+        ntc = __shfl_sync(FULL, cnt, ntx);
+        const int c = pxi * K + ntx;
 #pragma unroll
-      for (int q = 0; q < K; ++q) {
-        const unsigned qh = __shfl_sync(FULL, th, q), ql = __shfl_sync(FULL, tl, q);
-        pos += (((Tm >> q) & 1u) && (qh > th || (qh == th && ql > tl))) ? 1 : 0;
-      }
-      // lane x: the x-th target's lane, counts and visited bits for the pass
-      int tx = 0;
-#pragma unroll
-      for (int q = 0; q < K; ++q) {
-        const int pq = __shfl_sync(FULL, pos, q);
-        if (((Tm >> q) & 1u) && pq == lane) tx = q;
-      }
-      const int tseg = __shfl_sync(FULL, seg, tx), tcol = pxi * K + tx;
-      int tcnt = __shfl_sync(FULL, cnt, tx);
-      unsigned tvis = __shfl_sync(FULL, vis, tx);
-      const int nT = __popc(Tm);
-      unsigned Ux = 0;  // bit x: the x-th target stays in the list
-      for (int x = 0; x < nT; ++x) {
+        for (int u = 0; u < U; ++u) ne[u] = lane + 32 * u < MM ? ent[(lane + 32 * u) * HS + c] : 0u;
+        nsmall = sm.hsmall[c];
+      };
+      fetch();
+      unsigned Um = 0;
+      while (left) {
         if (pc <= 0 || vp == FULLM) break;
-        const int col = __shfl_sync(FULL, tcol, x);
-        const unsigned vt = __shfl_sync(FULL, tvis, x);
+        const int txi = ntx, col = pxi * K + txi;
+        const unsigned vt = nvt;
+        int tc = ntc;
+        const bool small = nsmall;
         // First pop of the pair whose two nodes are both unvisited.  A heap
         // pops in non-increasing key order, so that is the qualifying swap of
         // largest key when only one has it (read off the entries); on a tie
@@ -1355,13 +1362,13 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int k = lane + 32 * u;  // entry k holds swap k
-          const unsigned e = k < MM ? ent[k * HS + col] : 0u;
           const bool ok = k < MM && !((vp >> (k / M)) & 1u) && !((vt >> (k % M)) & 1u);
-          kq[u] = ok ? ((e >> 8) + 1u) << 6 | (unsigned)k : 0u;
+          kq[u] = ok ? ((ne[u] >> 8) + 1u) << 6 | (unsigned)k : 0u;
           most = max(most, kq[u]);
         }
-        const bool small = sm.hsmall[col];
         const unsigned best = __reduce_max_sync(FULL, most);
+        left &= ~(1u << txi);
+        if (left) fetch();
         int nbest = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u) nbest += __popc(__ballot_sync(FULL, kq[u] >> 6 == best >> 6));
@@ -1399,31 +1406,25 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
           r = (int)(key & 4095u) - 2048;
           l = (int)(key >> 12) - 2048 - r;
         } else {
-          pair_gains<M>(sm, pxi, col - pxi * K, pick, l, r);
+          pair_gains<M>(sm, pxi, txi, pick, l, r);
         }
         const int i = pick / M, j = pick % M;
-        if (lane == x) {
+        tc -= r;
+        pc -= l;
+        vp |= 1u << i;
+        if (tc > 0) Um |= 1u << txi;
+        if (lane == txi) {
           sm.swaps[2 * nsw] = sp * M + i;
-          sm.swaps[2 * nsw + 1] = tseg * M + j;
-          sm.dest[pxi][i] = (uint8_t)((tx << 4) | j);
-          sm.dest[tx][j] = (uint8_t)((pxi << 4) | i);
-          tvis |= 1u << j;
-          tcnt -= r;
+          sm.swaps[2 * nsw + 1] = seg * M + j;
+          sm.dest[pxi][i] = (uint8_t)((txi << 4) | j);
+          sm.dest[txi][j] = (uint8_t)((pxi << 4) | i);
+          vis |= 1u << j;
+          cnt = tc;
         }
         ++nsw;
-        vp |= 1u << i;
-        pc -= l;
-        if (__shfl_sync(FULL, tcnt, x) > 0) Ux |= 1u << x;
-      }
-      // back to the segments' lanes
-      const int c1 = __shfl_sync(FULL, tcnt, pos);
-      const unsigned v1 = __shfl_sync(FULL, tvis, pos);
-      if (isT) {
-        cnt = c1;
-        vis = v1;
       }
       if (lane == pxi) vis = vp;
-      Wm = __ballot_sync(FULL, isT && ((Ux >> pos) & 1u));
+      Wm = Um;
     }
   }
   if (lane == 0) {
