@@ -2100,7 +2100,7 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
 }
 
 // Blocks per job for calls with few jobs (one matrix, or its four
-// schedules); batches run clusters of 2 (run_batch).  Measured on GB300 (find_best,
+// schedules); batches have their own rule (run_batch).  Measured on GB300 (find_best,
 // four jobs) with 4 / 8 / 16 blocks: R-MAT 2048 2:8 (26 K entries) 6.7 /
 // 6.8 / 7.3 ms, R-MAT 16384 2:4 (228 K entries) 17.1 / 12.9 / 12.4 ms,
 // R-MAT 65536 2:8 (1.8 M entries) 472 / 295 / 209 ms; so 16 (a non-portable
@@ -2385,7 +2385,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   if (nnz > 0 && (!row || !col || !val)) return VNM_ERR_ARG;
   const int R = (int)totR, n = (int)nnz;
   size_t need = pattern_bytes(R, n) + 5 * arena_bytes(n, sizeof(int)) + arena_bytes(nmat + 1, 8) +
-                3 * arena_bytes(nmat + 1, sizeof(int)) + arena_bytes(nmat, sizeof(NMJob)) +
+                3 * arena_bytes(nmat + 1, sizeof(int)) + 2 * arena_bytes(nmat, sizeof(NMJob)) +
                 arena_bytes(R, sizeof(int)) + arena_bytes((size_t)R + (size_t)2 * ROW_GROUPS * nmat, sizeof(int)) +
                 arena_bytes(R, sizeof(uint4)) + 2 * arena_bytes(R / M + nmat, sizeof(int)) +
                 arena_bytes((size_t)JOB_RES * nmat, sizeof(int)) + arena_bytes(R, sizeof(int)) + 8192;
@@ -2461,14 +2461,31 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     if (J.nseg > max_nseg) max_nseg = J.nseg;
     if (J.R > 0) max_runs = std::max(max_runs, ((row_off[b] + J.R - 1) >> 4) - (row_off[b] >> 4) + 1);
   }
+  // The rounds run in the order of the matrices' entries, most first: the
+  // batch lasts as long as its largest jobs, which must not start late (256
+  // R-MAT matrices 256-8192 rows at 2:8: 36.8 -> 27.1 ms).
+  std::vector<int> by_size(nmat);
+  for (int b = 0; b < nmat; ++b) by_size[b] = b;
+  std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int y) {
+    return nnz_offset[x + 1] - nnz_offset[x] > nnz_offset[y + 1] - nnz_offset[y];
+  });
+  std::vector<NMJob> sj(nmat);
+  for (int b = 0; b < nmat; ++b) sj[b] = hj[by_size[b]];
+  NMJob* d_sorted = arena_take<NMJob>(ctx, nmat);
+  if (!d_sorted) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, hj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
+  VNM_CUDA_TRY(cudaMemcpyAsync(d_sorted, sj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
   VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, d_soff);
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  // clusters of 2 blocks per job: the batch's time is its largest matrices'
+  // Clusters of 2 blocks per job: the batch's time is its largest matrices'
   // jobs, and two SMs each shorten them more than the extra waves cost
-  // (GB300, 256 R-MAT matrices 256-8192 rows at 2:8: 88 ms with one block
-  // per job, 63 ms with 2, 69 ms with 4)
-  VNM_TRY(launch_rounds(ctx, d_jobs, nmat, N, M, max_nseg, max_runs, 2));
+  // (88 ms with one block per job, 63 ms with 2, 69 ms with 4, measured on
+  // an earlier form of the kernel).  Clusters of 4 or 8 where all jobs may
+  // still run at once (launch_rounds halves them if they do not): 12 matrices
+  // of 2048-8192 rows 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms,
+  // 12 of 256-512 rows 2.25 ms either way.
+  const int cs = nmat * 8 <= ctx->num_sms ? 8 : nmat * 4 <= ctx->num_sms ? 4 : 2;
+  VNM_TRY(launch_rounds(ctx, d_sorted, nmat, N, M, max_nseg, max_runs, cs));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hres = ctx->h_pinned + 256;
   VNM_CUDA_TRY(cudaMemcpyAsync(hres, res, sizeof(int) * JOB_RES * nmat, cudaMemcpyDeviceToHost, ctx->stream));
