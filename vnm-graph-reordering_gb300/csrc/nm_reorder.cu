@@ -274,6 +274,8 @@ struct RoundSmem {
   int S[K][M];                 // S_x(k): rows with bit k set and popcount == N+1
   int CL[NPAIR][MM];           // per unordered pair (a < b): left-side corrections
   int CR[NPAIR][MM];           //                              right-side corrections
+  unsigned CLR[NPAIR][MM];     // leader: the helpers' packed corrections, CL + (CR << 16), zero between rounds
+  int packed;                  // leader: some came
   static constexpr int HSTR = (K * K + 31) / 32 * 32;  // heaps, rounded up to whole warps
   // Scratch at the head of dynamic shared memory, used by three phases in
   // turn: the process phase's row masks (2 x K x M words a 32-row chunk, at
@@ -590,6 +592,7 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
   for (int i = threadIdx.x; i < RoundSmem<M>::NPAIR * RoundSmem<M>::MM; i += NM_THREADS) {
     (&sm.CL[0][0])[i] = 0;
     (&sm.CR[0][0])[i] = 0;
+    (&sm.CLR[0][0])[i] = 0u;
   }
   if (threadIdx.x < K) {
     sm.newinv[threadIdx.x] = 0;
@@ -660,7 +663,7 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
     // probing; then each warp lists the touched slots of its share.  (With the
     // hashed table below, or the records in global memory once the entries
     // might fill it, a round of R-MAT 65536 2:8 took 21 us here at schedule 0,
-    // GATHER_US now.)
+    // 9.5 us now.)
     unsigned* tw = reinterpret_cast<unsigned*>(sm.table);
     const int run0 = J.row0 >> 4, gpb = ROW_GROUPS / sl.cs;
     constexpr int U = 4;  // entries a thread in flight
@@ -840,7 +843,7 @@ __device__ __forceinline__ unsigned byte_tops(unsigned z) { return ((z >> 7) & 0
 // from byte-wise population counts and one more transpose.  Bound by fetching
 // its own code once a round, so it is one copy of short loops for both phases
 // that use it: inlined and unrolled a chunk took 3.8 K cycles on an idle SM,
-// CHUNK_CYCLES now.
+// 1.2 K now.
 template <int M>
 __device__ __noinline__ void masks_of_chunks(const RoundSmem<M>& sm, const NMJob& J, int N, int c0, int c1, int n,
                                              unsigned* scratch) {
@@ -1564,6 +1567,63 @@ __device__ void cluster_push(cg::cluster_group& cl, int* mine, int n) {
   }
 }
 
+// Helper block: add its partial scores into the leader's copy and clear them.
+// With more scores than threads, the corrections of a pair go two to a word:
+// what bounds the push is the remote atomics that the leader's shared memory
+// takes in (all of them singly were 8 us of a 57 us round at R-MAT 65536 2:8,
+// 4.5 us packed).  Each counts entries of one column that the block gathered,
+// so with no more than PACK_MAX of them the sums of 15 helpers fit 16 bits.
+// Blocks with longer columns send theirs singly, and so do those with a
+// segment paired with itself (mode 2: signed) and those of so few entries
+// that most scores are 0 anyway, where the leader's pass over the packed
+// words would cost more than it saves (0.5 us of a 23 us round at R-MAT 512).
+constexpr int PACK_MAX = 4095, PACK_MIN_ENTRIES = 1024;
+static_assert(15 * PACK_MAX < 1 << 16, "packed corrections do not carry");
+template <int M>
+__host__ __device__ constexpr bool scores_packed() {
+  return RoundSmem<M>::NPAIR * RoundSmem<M>::MM * 2 > NM_THREADS;
+}
+template <int M>
+__device__ void score_push(cg::cluster_group& cl, RoundSmem<M>& sm) {
+  constexpr int KM = (M + 1) * M, NC = RoundSmem<M>::NPAIR * RoundSmem<M>::MM;
+  if constexpr (!scores_packed<M>()) {
+    cluster_push(cl, &sm.S[0][0], KM + 2 * NC);
+  } else {
+    bool single = sm.mode == 2 || sm.E < PACK_MIN_ENTRIES;
+    for (int q = threadIdx.x; q < sm.K_ * M; q += NM_THREADS) single |= sm.colpre[q + 1] - sm.colpre[q] > PACK_MAX;
+    if (__syncthreads_or(single)) {
+      cluster_push(cl, &sm.S[0][0], KM + 2 * NC);
+      return;
+    }
+    RoundSmem<M>* lead = cl.map_shared_rank(&sm, 0);
+    if (threadIdx.x == 0) lead->packed = 1;
+    cluster_push(cl, &sm.S[0][0], KM);
+    int *CL = &sm.CL[0][0], *CR = &sm.CR[0][0];
+    for (int i = threadIdx.x; i < NC; i += NM_THREADS) {
+      const int l = CL[i], r = CR[i];
+      if (!(l | r)) continue;
+      atomicAdd(&lead->CLR[0][0] + i, (unsigned)l | (unsigned)r << 16);
+      CL[i] = CR[i] = 0;
+    }
+  }
+}
+
+// Leader block, after the barrier: the packed corrections, if any came, to
+// the others.
+template <int M>
+__device__ void score_unpack(RoundSmem<M>& sm) {
+  if (!sm.packed) return;
+  for (int i = threadIdx.x; i < RoundSmem<M>::NPAIR * RoundSmem<M>::MM; i += NM_THREADS) {
+    const unsigned v = (&sm.CLR[0][0])[i];
+    if (!v) continue;
+    (&sm.CL[0][0])[i] += (int)(v & 0xffffu);
+    (&sm.CR[0][0])[i] += (int)(v >> 16);
+    (&sm.CLR[0][0])[i] = 0u;
+  }
+  __syncthreads();  // (and the flag has been read)
+  if (threadIdx.x == 0) sm.packed = 0;
+}
+
 // All rounds of a job.  With cs == 1 one thread block runs the job; with
 // cs > 1 the job runs on a thread-block cluster of cs blocks: the leader
 // (rank 0) runs the sequential parts (segment choice, heaps, walk, counts)
@@ -1584,7 +1644,6 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
                                                                               RoundSmem<M>::MM, "CL, CR adjacent");
   static_assert(offsetof(RoundSmem<M>, newpres) == offsetof(RoundSmem<M>, newinv) + sizeof(int) * K,
                 "newinv, newpres adjacent");
-  constexpr int NSUM = K * M + 2 * RoundSmem<M>::NPAIR * RoundSmem<M>::MM;
   // dynamic shared memory: [scratch][row-record table: its slots x 16 B][list
   // of the slots in use: slots x 2 B][segment counts]
   extern __shared__ uint4 smem_heap[];
@@ -1616,6 +1675,7 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
     sm.ts_max = ts_max;
     sm.ts_shift = 32 - (31 - __clz(ts_max > 0 ? ts_max : 1));
     sm.use_table = 0;
+    sm.packed = 0;
     sm.go = 0;
   }
   clear_round_smem<M>(sm);
@@ -1697,7 +1757,7 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
       // (the leader pulling the helpers' sums over DSMEM instead was slower:
       // 8.92 against 8.55 ms at R-MAT 16384 2:4, 200.5 against 197.2 ms at
       // R-MAT 65536 2:8)
-      if (!lead) cluster_push(cl, &sm.S[0][0], NSUM);
+      if (!lead) score_push<M>(cl, sm);
       cl.sync();
       if (!lead) {  // while the leader runs the heaps and the walk: next round's scan
         const int nh = cs - 1, hr = rank - 1;
@@ -1712,6 +1772,7 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
     }
     VNM_PHASE(3);
     if (lead) {
+      if constexpr (scores_packed<M>()) score_unpack<M>(sm);
       rank_phase<M>(sm);
       VNM_PHASE(4);
       const unsigned long long t_in = (tid == NM_THREADS - 32 && timed) ? global_ns() : 0ull;
