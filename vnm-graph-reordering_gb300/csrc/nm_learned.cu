@@ -66,69 +66,89 @@ __global__ void k_l_build_G(const int* prow, const int* pcol, int np, int M, int
   }
 }
 
-// hist / cnt from the sorted pattern (runs of equal (row, col/M) are groups)
-__global__ void k_l_hist(const int* prow, const int* pcol, int np, int M, int N, int* hist, int* cnt) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const int r = prow[i], s = pcol[i] / M;
-    if (i + 1 < np && prow[i + 1] == r && pcol[i + 1] / M == s) continue;
-    int len = 1;
-    for (int b = 1; b < M && i - b >= 0 && prow[i - b] == r && pcol[i - b] / M == s; ++b) len++;
-    atomicAdd(&hist[s * 9 + len], 1);
-    if (len > N) atomicAdd(&cnt[s], 1);
+// hist / cnt of a segment from its columns' histograms: a group of k bits is
+// counted by each of its k columns.  (Counting runs of the sorted pattern with
+// atomics took 44 us at 65536 rows, 2 M entries; this takes 5.)
+__global__ void k_l_seg_hist(LMat L) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < L.nseg; s += gridDim.x * blockDim.x) {
+    int h[9], t = 0, c = 0;
+#pragma unroll
+    for (int k = 1; k <= 8; ++k) h[k] = 0;
+    for (int i = 0; i < L.M; ++i) {
+      const int u = L.orig[s * L.M + i];
+#pragma unroll
+      for (int k = 1; k <= 8; ++k) h[k] += L.colh[u * 9 + k];
+    }
+#pragma unroll
+    for (int k = 1; k <= 8; ++k) {
+      h[k] /= k;
+      L.hist[s * 9 + k] = h[k];
+      t += h[k];
+      c += k > L.N ? h[k] : 0;
+    }
+    L.hist[s * 9] = L.R - t;
+    L.cnt[s] = c;
   }
 }
 
-__global__ void k_l_hist_zero(int* hist, int nseg, int R) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
-    int t = 0;
-    for (int k = 1; k <= 8; ++k) t += hist[s * 9 + k];
-    hist[s * 9] = R - t;
-  }
-}
-
-// colh of the columns at the given positions.  A column's rows are cut into
-// chunks of L_CHUNK, one warp per chunk, so a hub column spreads over many
-// warps: k_l_colh_prep zeroes each column's histogram and counts its
-// chunks, an exclusive scan turns the counts into offsets, and
-// k_l_colh_rows adds each chunk's histogram.
+// colh of the columns at some positions.  A column's rows are cut into chunks
+// of L_CHUNK, one warp a chunk, so a hub column spreads over many warps.
+// take_column zeroes a column's histogram and appends its chunks to the work
+// list, k_l_colh_rows adds each chunk's histogram.  (The sums are of
+// integers, so the list's order does not matter, and it is made by one atomic
+// a warp; with chunk counts, a scan of them over all R columns and a search
+// in the offsets for each chunk, a round of the search took five launches
+// and 25 us more at 65536 rows.)
 constexpr int L_CHUNK = 256;
 
-__global__ void k_l_colh_prep(LMat L, const int* positions, const int* npos_p, int npos_fixed, int cap,
-                              int* nchunk) {
-  const int npos = npos_p ? *npos_p : npos_fixed;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < cap; q += gridDim.x * blockDim.x) {
-    int c = 0;
-    if (q < npos) {
-      const int u = L.orig[positions ? positions[q] : q];
+// Counters of a call, on the device.
+enum { LC_ACTIVE, LC_ACC, LC_SWAP_ITEMS, LC_DUMP, LC_ERR, LC_COL_ITEMS, LC_N = 8 };
+
+__device__ __forceinline__ int chunks_of(const LMat& L, int u) {
+  return (L.cptr[u + 1] - L.cptr[u] + L_CHUNK - 1) / L_CHUNK;
+}
+
+// Where a lane's n items go in a list of *len: whole warps call.
+__device__ __forceinline__ int warp_append(int n, int* len) {
+  const int lane = threadIdx.x & 31;
+  int incl = n;
 #pragma unroll
-      for (int z = 0; z < 9; ++z) L.colh[u * 9 + z] = 0;
-      c = (L.cptr[u + 1] - L.cptr[u] + L_CHUNK - 1) / L_CHUNK;
-    }
-    nchunk[q] = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
+  int base = 0;
+  if (lane == 31 && incl > 0) base = atomicAdd(len, incl);
+  return __shfl_sync(0xffffffffu, base, 31) + incl - n;
 }
 
-// the entry of a sorted offset table that holds `item`: last q with offs[q] <= item
-__device__ __forceinline__ int chunk_owner(const int* offs, int n, int item) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (offs[mid] <= item) lo = mid;
-    else hi = mid - 1;
+// items: (position, chunk); whole warps call, lanes without a column with live = false
+__device__ __forceinline__ void take_column(const LMat& L, int a, bool live, int2* items, int* nitems) {
+  int c = 0;
+  if (live) {
+    const int u = L.orig[a];
+#pragma unroll
+    for (int z = 0; z < 9; ++z) L.colh[u * 9 + z] = 0;
+    c = chunks_of(L, u);
   }
-  return lo;
+  const int at = warp_append(c, nitems);
+  for (int k = 0; k < c; ++k) items[at + k] = make_int2(a, k);
 }
 
-__global__ void k_l_colh_rows(LMat L, const int* positions, const int* npos_p, int npos_fixed, const int* offs,
-                              const int* ntot) {
+__global__ void k_l_all_columns(LMat L, int2* items, int* nitems) {
+  const int lane = threadIdx.x & 31;
+  for (int a0 = blockIdx.x * blockDim.x + threadIdx.x - lane; a0 < L.R; a0 += gridDim.x * blockDim.x)
+    take_column(L, a0 + lane, a0 + lane < L.R, items, nitems);
+}
+
+__global__ void k_l_colh_rows(LMat L, const int2* items, const int* nitems) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
-  const int npos = npos_p ? *npos_p : npos_fixed, tot = *ntot;
+  const int tot = *nitems;
   for (int item = warp; item < tot; item += nw) {
-    const int q = chunk_owner(offs, npos, item);
-    const int a = positions ? positions[q] : q;
-    const int u = L.orig[a], s = a / L.M;
-    const int beg = L.cptr[u] + (item - offs[q]) * L_CHUNK;
+    const int2 it = items[item];
+    const int u = L.orig[it.x], s = it.x / L.M;
+    const int beg = L.cptr[u] + it.y * L_CHUNK;
     const int end = min(beg + L_CHUNK, L.cptr[u + 1]);
     int h[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int e = beg + lane; e < end; e += 32) {
@@ -142,6 +162,52 @@ __global__ void k_l_colh_rows(LMat L, const int* positions, const int* npos_p, i
       const int v = __reduce_add_sync(0xffffffffu, h[z]);
       if (lane == z && v) atomicAdd(&L.colh[u * 9 + z], v);
     }
+  }
+}
+
+// The round's start: the segments that hold an invalid group in ascending
+// order to `active` (block 0, a tile of its threads x 4 at a time: 8192
+// segments are two tiles), the round's counters and the best and claim words
+// cleared (the other blocks).  One launch where a scan took four and 18 us.
+constexpr int L_START_THREADS = 1024;
+__global__ void __launch_bounds__(L_START_THREADS)
+    k_l_round_start(LMat L, int* active, int* ci, unsigned long long* best, unsigned long long* claim) {
+  if (blockIdx.x > 0) {
+    for (int s = (blockIdx.x - 1) * blockDim.x + threadIdx.x; s < L.nseg; s += (gridDim.x - 1) * blockDim.x)
+      best[s] = claim[s] = 0ull;
+    return;
+  }
+  __shared__ int wsum[L_START_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (int t0 = 0; t0 < L.nseg; t0 += 4 * L_START_THREADS) {
+    const int s0 = t0 + 4 * (int)threadIdx.x;
+    unsigned on = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (s0 + k < L.nseg && L.cnt[s0 + k] > 0) on |= 1u << k;
+    const int n = __popc(on);
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    const int w = wsum[lane];  // 32 warps, a sum a lane
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+    const int all = __reduce_add_sync(0xffffffffu, w);
+    int at = base + before + incl - n;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if ((on >> k) & 1u) active[at++] = s0 + k;
+    base += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    ci[LC_ACTIVE] = base;
+    ci[LC_ACC] = ci[LC_SWAP_ITEMS] = ci[LC_COL_ITEMS] = 0;
   }
 }
 
@@ -526,69 +592,81 @@ __global__ void k_l_claim(LMat L, const int* active, const int* nactive_p, int r
   }
 }
 
-// winners: swaps that hold the claim on both of their segments, so accepted
-// swaps touch disjoint segments and their exact gains add up
-__global__ void k_l_accept(LMat L, const int* active, const int* nactive_p, int round, unsigned seed,
-                           const unsigned long long* best, const unsigned long long* claim, int4* acc, int* nacc,
-                           unsigned long long* gain_sum) {
-  const int nactive = *nactive_p;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nactive; a += gridDim.x * blockDim.x) {
-    const unsigned long long b = best[a];
-    if (!b) continue;
-    const int c = (int)((1ull << 40) - 1 - (b & ((1ull << 40) - 1)));
-    int q, i, j;
-    cand_of(c, L.M, q, i, j);
-    const int p = active[a], t = target_of(p, q, round, L.nseg, seed);
-    const unsigned long long key = (b & ~((1ull << 40) - 1)) | (unsigned long long)(unsigned)a;
-    if (claim[p] == key && claim[t] == key) {
-      const int s = atomicAdd(nacc, 1);
-      acc[s] = make_int4(p, i, t, j);
-      atomicAdd(gain_sum, b >> 40);
+// Winners: swaps that hold the claim on both of their segments, so accepted
+// swaps touch disjoint segments and their exact gains add up.  A winner's
+// nodes exchange places here, and the chunks of its two columns go to the
+// work list of k_l_apply_rows as (swap, chunk), the first column's first.
+__global__ void k_l_accept(LMat L, const int* active, int* ci, int round, unsigned seed,
+                           const unsigned long long* best, const unsigned long long* claim, int4* acc, int2* uw,
+                           int2* items, unsigned long long* gain_sum) {
+  const int nactive = ci[LC_ACTIVE], lane = threadIdx.x & 31;
+  for (int a0 = blockIdx.x * blockDim.x + threadIdx.x - lane; a0 < nactive; a0 += gridDim.x * blockDim.x) {
+    const int a = a0 + lane;
+    const unsigned long long b = a < nactive ? best[a] : 0ull;
+    int n = 0, nitems = 0;
+    int4 sw;
+    int2 nodes;
+    if (b) {
+      const int c = (int)((1ull << 40) - 1 - (b & ((1ull << 40) - 1)));
+      int q, i, j;
+      cand_of(c, L.M, q, i, j);
+      const int p = active[a], t = target_of(p, q, round, L.nseg, seed);
+      const unsigned long long key = (b & ~((1ull << 40) - 1)) | (unsigned long long)(unsigned)a;
+      if (claim[p] == key && claim[t] == key) {
+        n = 1;
+        sw = make_int4(p, i, t, j);
+        const int x = p * L.M + i, y = t * L.M + j;
+        const int u = L.orig[x], w = L.orig[y];
+        nodes = make_int2(u, w);
+        nitems = chunks_of(L, u) + chunks_of(L, w);
+        L.orig[x] = w;
+        L.orig[y] = u;
+        L.pos[w] = x;
+        L.pos[u] = y;
+        atomicAdd(gain_sum, b >> 40);
+      }
+    }
+    const int s = warp_append(n, ci + LC_ACC), at = warp_append(nitems, ci + LC_SWAP_ITEMS);
+    if (n) {
+      acc[s] = sw;
+      uw[s] = nodes;
+      for (int k = 0; k < nitems; ++k) items[at + k] = make_int2(s, k);
     }
   }
 }
 
 // Apply accepted swaps: flip the two bits of every row that holds exactly one
-// of the two columns, keep hist / cnt in step, and exchange the nodes.
-// Accepted swaps touch disjoint segments, and a row holding both columns
-// moves nothing, so the rows of the two columns are independent: they are
-// cut into chunks of L_CHUNK, one warp per chunk.  k_l_apply_prep records
-// each swap's two nodes, counts their chunks and exchanges the nodes;
-// k_l_apply_rows moves the bits, summing a chunk's hist / cnt changes in
-// registers and adding them once per warp.
-__global__ void k_l_apply_prep(LMat L, const int4* acc, const int* nacc, int cap, int2* uw, int* nchunk) {
-  const int n = *nacc;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < cap; s += gridDim.x * blockDim.x) {
-    int c = 0;
-    if (s < n) {
-      const int4 sw = acc[s];
-      const int a = sw.x * L.M + sw.y, b = sw.z * L.M + sw.w;
-      const int u = L.orig[a], w = L.orig[b];
-      uw[s] = make_int2(u, w);
-      c = (L.cptr[u + 1] - L.cptr[u] + L_CHUNK - 1) / L_CHUNK + (L.cptr[w + 1] - L.cptr[w] + L_CHUNK - 1) / L_CHUNK;
-      L.orig[a] = w;
-      L.orig[b] = u;
-      L.pos[w] = a;
-      L.pos[u] = b;
-    }
-    nchunk[s] = c;
-  }
-}
-
-__global__ void k_l_apply_rows(LMat L, const int4* acc, const int* nacc, const int2* uw, const int* offs,
-                               const int* ntot) {
-  const int n = *nacc, tot = *ntot;
+// of the two columns and keep hist / cnt in step.  Accepted swaps touch
+// disjoint segments, and a row holding both columns moves nothing, so the
+// rows of the two columns are independent: they are cut into chunks of
+// L_CHUNK, one warp a chunk, which sums its hist / cnt changes in registers
+// and adds them once.  The columns of the swaps' segments are listed for
+// their new histograms on the side: that reads nothing that changes here.
+__global__ void k_l_apply_rows(LMat L, const int4* acc, int* ci, const int2* uw, const int2* items,
+                               int2* col_items) {
+  const int n = ci[LC_ACC], tot = ci[LC_SWAP_ITEMS];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int e0 = 32 * warp; e0 < n * 2 * L.M; e0 += 32 * nw) {  // n * 2M <= R
+    const int e = e0 + lane;
+    const bool live = e < n * 2 * L.M;
+    int a = 0;
+    if (live) {
+      const int4 sw = acc[e / (2 * L.M)];
+      const int k = e % (2 * L.M);
+      a = (k < L.M ? sw.x : sw.z) * L.M + k % L.M;
+    }
+    take_column(L, a, live, col_items, ci + LC_COL_ITEMS);
+  }
   unsigned* Gw = reinterpret_cast<unsigned*>(L.G);
   for (int item = warp; item < tot; item += nw) {
-    const int s = chunk_owner(offs, n, item);
+    const int s = items[item].x;
     const int4 sw = acc[s];
     const int p = sw.x, i = sw.y, t = sw.z, j = sw.w;
     const int u = uw[s].x, w = uw[s].y;
     const unsigned bi = 1u << i, bj = 1u << j;
-    const int cu = (L.cptr[u + 1] - L.cptr[u] + L_CHUNK - 1) / L_CHUNK;
-    int k = item - offs[s];
+    const int cu = chunks_of(L, u);
+    int k = items[item].y;
     const int col = k < cu ? u : w;
     if (k >= cu) k -= cu;
     const int beg = L.cptr[col] + k * L_CHUNK, end = min(beg + L_CHUNK, L.cptr[col + 1]);
@@ -623,26 +701,6 @@ __global__ void k_l_apply_rows(LMat L, const int4* acc, const int* nacc, const i
     if (lane == 0 && vcp) atomicAdd(&L.cnt[p], vcp);
     if (lane == 0 && vct) atomicAdd(&L.cnt[t], vct);
   }
-}
-
-// positions of all columns of the segments touched by accepted swaps
-__global__ void k_l_touched_cols(const int4* acc, const int* nacc, int M, int* cols, int* ncols) {
-  const int n = *nacc;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *ncols = n * 2 * M;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * 2 * M; e += gridDim.x * blockDim.x) {
-    const int s = e / (2 * M), k = e % (2 * M);
-    const int4 sw = acc[s];
-    cols[e] = (k < M ? sw.x : sw.z) * M + (k % M);
-  }
-}
-
-__global__ void k_l_flags(const int* cnt, int nseg, int* flags) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) flags[s] = cnt[s] > 0;
-}
-
-__global__ void k_l_scatter_active(const int* cnt, const int* idx, int nseg, int* active) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x)
-    if (cnt[s] > 0) active[idx[s]] = s;
 }
 
 // totals from the segment histograms: [0] invalid groups, [1] retained nonzeros
@@ -1356,14 +1414,13 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   const int R = nrows, nseg = R / M;
   const long long gbytes = ((long long)R * nseg + 3) & ~3ll;
   const int dcap = prm->dump_every > 0 ? prm->dump_cap : 0;
+  // chunks that columns, each in the list once at most, can have
+  const size_t chunk_cap = (size_t)R + (size_t)nnz / L_CHUNK + 1;
   size_t need = pattern_bytes(R, nnz) + 3 * arena_bytes(nnz, 4) + arena_bytes(gbytes, 1) +
                 arena_bytes((size_t)nseg * 9, 4) + arena_bytes(nseg, 4) + arena_bytes((size_t)R * 9, 4) +
-                3 * arena_bytes(R, 4) + 3 * arena_bytes(nseg + 1, 4) + arena_bytes((size_t)nseg * LTOP, 4) +
-                2 * arena_bytes(nseg, 8) + arena_bytes(nseg, 16) + arena_bytes(2 * (size_t)R, 4) +
-                arena_bytes(16, 4) + arena_bytes(8, 8) + arena_bytes(R + 1, 4) + arena_bytes(nseg + 1, 8) +
-                // scratch of the scans, given back every round: the active list, the applied
-                // swaps and the column histograms (the first histograms' scan before the loop)
-                scan_scratch_bytes(R + 1) + 2 * scan_scratch_bytes(nseg + 1) +
+                3 * arena_bytes(R + 1, 4) + 2 * arena_bytes(nseg + 1, 4) + arena_bytes((size_t)nseg * LTOP, 4) +
+                2 * arena_bytes(nseg + 1, 8) + arena_bytes(nseg + 1, 16) + arena_bytes(nseg + 1, 8) +
+                arena_bytes(LC_N + 8 * 2, 4) + 2 * arena_bytes(chunk_cap, 8) +
                 arena_bytes((size_t)dcap * LF, 4) + arena_bytes(dcap, 4) + 8192;
   VNM_TRY(arena_reserve(ctx, need));
   VNM_TRY(pinned_reserve(ctx, 256));
@@ -1374,7 +1431,7 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   VNM_TRY(stage_in(ctx, col, nnz, mem, &d_col));
   VNM_TRY(stage_in(ctx, val, nnz, mem, &d_val));
   Pattern P;
-  VNM_TRY(build_pattern(ctx, R, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned));
+  VNM_TRY(build_pattern(ctx, R, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned, false, false));
   LMat L;
   L.R = R;
   L.M = M;
@@ -1389,47 +1446,38 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   L.colh = arena_take<int>(ctx, (size_t)R * 9 + 1);
   L.orig = arena_take<int>(ctx, R + 1);
   L.pos = arena_take<int>(ctx, R + 1);
-  int* flags = arena_take<int>(ctx, nseg + 1);
   int* active = arena_take<int>(ctx, nseg + 1);
   int* top = arena_take<int>(ctx, (size_t)nseg * LTOP + 1);
   unsigned long long* best = arena_take<unsigned long long>(ctx, nseg + 1);
   unsigned long long* claim = arena_take<unsigned long long>(ctx, nseg + 1);
   int4* acc = arena_take<int4>(ctx, nseg + 1);
-  int* cols = arena_take<int>(ctx, 2 * (size_t)R + 1);
-  int* chunks = arena_take<int>(ctx, R + 1);     // per column (or swap) chunk counts, then their offsets
-  int2* uw = arena_take<int2>(ctx, nseg + 1);    // the two nodes of each accepted swap
-  int* ci = arena_take<int>(ctx, 16);  // [0] nactive [1] nacc [2] ncols [3] ndump [4] err [5..6] chunk totals
-  unsigned long long* cu = arena_take<unsigned long long>(ctx, 8);  // [0] gain [1] scored [2..3] totals
+  int2* uw = arena_take<int2>(ctx, nseg + 1);            // the two nodes of each accepted swap
+  int2* swap_items = arena_take<int2>(ctx, chunk_cap);  // chunks of accepted swaps' columns
+  int2* col_items = arena_take<int2>(ctx, chunk_cap);   // chunks of columns to be counted
+  // sums (cu: [0] gain [1] scored [2..3] totals) and counters, read back in one copy
+  unsigned long long* cu = arena_take<unsigned long long>(ctx, 8 + LC_N / 2);
+  int* ci = reinterpret_cast<int*>(cu + 8);
   float* dx = dcap ? arena_take<float>(ctx, (size_t)dcap * LF) : nullptr;
   float* dy = dcap ? arena_take<float>(ctx, dcap) : nullptr;
   int* d_newpos = arena_take<int>(ctx, R + 1);
-  if (!L.G || !L.hist || !L.cnt || !L.colh || !L.orig || !L.pos || !flags || !active || !top || !best || !claim ||
-      !acc || !cols || !chunks || !uw || !ci || !cu || !d_newpos || (dcap && (!dx || !dy)))
+  if (!L.G || !L.hist || !L.cnt || !L.colh || !L.orig || !L.pos || !active || !top || !best || !claim ||
+      !acc || !uw || !swap_items || !col_items || !cu || !d_newpos || (dcap && (!dx || !dy)))
     return VNM_ERR_NOMEM;
   cudaStream_t st = ctx->stream;
   VNM_CUDA_TRY(cudaMemsetAsync(L.G, 0, gbytes > 0 ? gbytes : 4, st));
-  VNM_CUDA_TRY(cudaMemsetAsync(L.hist, 0, sizeof(int) * ((size_t)nseg * 9 + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(L.cnt, 0, sizeof(int) * (nseg + 1), st));
-  VNM_CUDA_TRY(cudaMemsetAsync(ci, 0, sizeof(int) * 16, st));
-  VNM_CUDA_TRY(cudaMemsetAsync(cu, 0, sizeof(unsigned long long) * 8, st));
+  VNM_CUDA_TRY(cudaMemsetAsync(cu, 0, 8 * sizeof(unsigned long long) + LC_N * sizeof(int), st));
   if (R > 0) VNM_LAUNCH(ctx, k_l_iota2, lgrid(ctx, R), 256, 0, L.orig, L.pos, R);
-  if (P.np > 0) {
+  if (P.np > 0)
     VNM_LAUNCH(ctx, k_l_build_G, lgrid(ctx, P.np), 256, 0, P.prow, P.pcol, P.np, M, nseg,
                reinterpret_cast<unsigned*>(L.G));
-    VNM_LAUNCH(ctx, k_l_hist, lgrid(ctx, P.np), 256, 0, P.prow, P.pcol, P.np, M, N, L.hist, L.cnt);
-  }
   if (nseg > 0) {
-    VNM_LAUNCH(ctx, k_l_hist_zero, lgrid(ctx, nseg), 256, 0, L.hist, nseg, R);
+    VNM_LAUNCH(ctx, k_l_all_columns, lgrid(ctx, R), 256, 0, L, col_items, ci + LC_COL_ITEMS);
+    VNM_LAUNCH(ctx, k_l_colh_rows, lgrid(ctx, (long long)R * 32), 256, 0, L, col_items, ci + LC_COL_ITEMS);
+    VNM_LAUNCH(ctx, k_l_seg_hist, lgrid(ctx, nseg), 256, 0, L);
     VNM_LAUNCH(ctx, k_l_totals, lgrid(ctx, nseg), 256, 0, L.hist, nseg, N, cu + 2);
   }
-  const size_t round_mark = ctx->arena.used;  // scan scratch from here on is given back every round
-  if (R > 0) {  // every column's histogram
-    VNM_LAUNCH(ctx, k_l_colh_prep, lgrid(ctx, R), 256, 0, L, nullptr, nullptr, R, R, chunks);
-    VNM_TRY(exclusive_scan(ctx, chunks, chunks, R, ci + 5));
-    VNM_LAUNCH(ctx, k_l_colh_rows, lgrid(ctx, (long long)R * 32), 256, 0, L, nullptr, nullptr, R, chunks, ci + 5);
-  }
   unsigned long long* hcu = reinterpret_cast<unsigned long long*>(ctx->h_pinned);  // 8 words
-  int* hci = ctx->h_pinned + 32;                                                    // 16 ints
+  int* hci = reinterpret_cast<int*>(hcu + 8);                                       // LC_N ints, as on the device
   VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
   VNM_CUDA_TRY(cudaStreamSynchronize(st));
   out->init_invalid = out->final_invalid = (long long)hcu[2];
@@ -1439,47 +1487,36 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   const MlpW W = net ? mlp_view(net) : MlpW{};
   const int pgrid = 2 * ctx->num_sms;
   const int egrid = ctx->num_sms * 8;
+  const size_t state_bytes = 8 * sizeof(unsigned long long) + LC_N * sizeof(int);
   int idle = 0, rounds = 0, swaps = 0;
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, st));
   for (int round = 0; round < prm->max_rounds && nseg >= 2 && P.np > 0; ++round) {
-    ctx->arena.used = round_mark;
-    VNM_CUDA_TRY(cudaMemsetAsync(ci + 1, 0, sizeof(int) * 2, st));
-    VNM_CUDA_TRY(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * nseg, st));
-    VNM_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(unsigned long long) * nseg, st));
-    VNM_LAUNCH(ctx, k_l_flags, lgrid(ctx, nseg), 256, 0, L.cnt, nseg, flags);
-    VNM_TRY(exclusive_scan(ctx, flags, flags, nseg, ci));
-    VNM_LAUNCH(ctx, k_l_scatter_active, lgrid(ctx, nseg), 256, 0, L.cnt, flags, nseg, active);
+    VNM_LAUNCH(ctx, k_l_round_start, 1 + lgrid(ctx, nseg, L_START_THREADS), L_START_THREADS, 0, L, active, ci, best,
+               claim);
     if (mode == VNM_LEARNED_MLP)
       VNM_LAUNCH(ctx, k_l_mlp<false>, pgrid, L_THREADS, smem, L, W, active, ci, KT, round, prm->seed, top, nullptr,
-                 0, nullptr, ci + 4);
+                 0, nullptr, ci + LC_ERR);
     VNM_LAUNCH(ctx, k_l_exact, egrid, 256, 0, L, active, ci, KT, round, prm->seed, top, mode, prm->topk, best, dx, dy,
-               prm->dump_every, ci + 3, dcap, cu + 1);
+               prm->dump_every, ci + LC_DUMP, dcap, cu + 1);
     VNM_LAUNCH(ctx, k_l_claim, lgrid(ctx, nseg), 256, 0, L, active, ci, round, prm->seed, best, claim);
-    VNM_LAUNCH(ctx, k_l_accept, lgrid(ctx, nseg), 256, 0, L, active, ci, round, prm->seed, best, claim, acc, ci + 1,
-               cu);
-    VNM_LAUNCH(ctx, k_l_apply_prep, lgrid(ctx, nseg), 256, 0, L, acc, ci + 1, nseg, uw, chunks);
-    VNM_TRY(exclusive_scan(ctx, chunks, chunks, nseg, ci + 6));
-    VNM_LAUNCH(ctx, k_l_apply_rows, egrid, 256, 0, L, acc, ci + 1, uw, chunks, ci + 6);
-    VNM_LAUNCH(ctx, k_l_touched_cols, lgrid(ctx, 2 * (long long)R), 256, 0, acc, ci + 1, M, cols, ci + 2);
-    VNM_LAUNCH(ctx, k_l_colh_prep, lgrid(ctx, R), 256, 0, L, cols, ci + 2, 0, R, chunks);
-    VNM_TRY(exclusive_scan(ctx, chunks, chunks, R, ci + 5));
-    VNM_LAUNCH(ctx, k_l_colh_rows, egrid, 256, 0, L, cols, ci + 2, 0, chunks, ci + 5);
-    VNM_CUDA_TRY(cudaMemcpyAsync(hci, ci, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
-    VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    VNM_LAUNCH(ctx, k_l_accept, lgrid(ctx, nseg), 256, 0, L, active, ci, round, prm->seed, best, claim, acc, uw,
+               swap_items, cu);
+    VNM_LAUNCH(ctx, k_l_apply_rows, egrid, 256, 0, L, acc, ci, uw, swap_items, col_items);
+    VNM_LAUNCH(ctx, k_l_colh_rows, egrid, 256, 0, L, col_items, ci + LC_COL_ITEMS);
+    VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, state_bytes, cudaMemcpyDeviceToHost, st));
     VNM_CUDA_TRY(cudaStreamSynchronize(st));
-    if (hci[4]) return VNM_ERR_INTERNAL;
+    if (hci[LC_ERR]) return VNM_ERR_INTERNAL;
     rounds = round + 1;
-    if (hci[0] == 0) break;  // no segment holds an invalid group
-    swaps += hci[1];
-    idle = hci[1] == 0 ? idle + 1 : 0;
+    if (hci[LC_ACTIVE] == 0) break;  // no segment holds an invalid group
+    swaps += hci[LC_ACC];
+    idle = hci[LC_ACC] == 0 ? idle + 1 : 0;
     if (idle >= prm->patience) break;
     if (prm->stop_gain > 0 && (long long)hcu[0] >= prm->stop_gain) break;
   }
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, st));
   VNM_CUDA_TRY(cudaMemsetAsync(cu + 2, 0, sizeof(unsigned long long) * 2, st));
   if (nseg > 0) VNM_LAUNCH(ctx, k_l_totals, lgrid(ctx, nseg), 256, 0, L.hist, nseg, N, cu + 2);
-  VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
-  VNM_CUDA_TRY(cudaMemcpyAsync(hci, ci, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
+  VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, state_bytes, cudaMemcpyDeviceToHost, st));
   VNM_CUDA_TRY(cudaStreamSynchronize(st));
   VNM_CUDA_TRY(cudaEventElapsedTime(&ctx->main_ms, ctx->ev_main0, ctx->ev_main1));
   out->final_invalid = (long long)hcu[2];
@@ -1488,7 +1525,7 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   out->exact_scored = (long long)hcu[1];
   out->rounds = rounds;
   out->swaps = swaps;
-  out->ndump = hci[3] < dcap ? hci[3] : dcap;
+  out->ndump = hci[LC_DUMP] < dcap ? hci[LC_DUMP] : dcap;
   for (int q = 0; q < 28; ++q) ctx->stats[q] = 0;
   ctx->stats[0] = rounds;
   ctx->stats[1] = out->exact_scored;

@@ -1945,7 +1945,7 @@ size_t pattern_bytes(int R, int nnz) {
 
 template <int M>
 static vnm_status build_pattern_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, const int* d_col,
-                                  const float* d_val, int N, Pattern& P, int* h_scratch, bool deferred) {
+                                  const float* d_val, int N, Pattern& P, int* h_scratch, bool deferred, bool counts) {
   P.R = R;
   P.nseg = R / M;
   int* err = arena_take<int>(ctx, 2);  // [0] the input check's flag, [1] the pattern's entry count
@@ -1995,7 +1995,8 @@ static vnm_status build_pattern_t(vnm_ctx* ctx, int R, int nnz, const int* d_row
     if (nnz > 0) {
       VNM_LAUNCH(ctx, k_csc_scatter, grid_for(ctx, nnz), 256, 0, P.prow, P.pcol, d_np, P.csplit, cfill, P.crow,
                  err);
-      VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, nnz), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
+      if (counts)
+        VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, nnz), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
     }
     return VNM_OK;
   }
@@ -2005,21 +2006,22 @@ static vnm_status build_pattern_t(vnm_ctx* ctx, int R, int nnz, const int* d_row
   if (P.np > 0) {
     VNM_LAUNCH(ctx, k_csc_scatter, grid_for(ctx, P.np), 256, 0, P.prow, P.pcol, d_np, P.csplit, cfill, P.crow,
                err);
-    VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, P.np), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
+    if (counts)
+      VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, P.np), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
   }
   return VNM_OK;
 }
 
 vnm_status build_pattern(vnm_ctx* ctx, int R, int nnz, const int* d_row, const int* d_col, const float* d_val,
-                         int N, int M, Pattern& P, int* h_scratch, bool deferred) {
+                         int N, int M, Pattern& P, int* h_scratch, bool deferred, bool counts) {
   switch (M) {
-    case 2: return build_pattern_t<2>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 3: return build_pattern_t<3>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 4: return build_pattern_t<4>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 5: return build_pattern_t<5>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 6: return build_pattern_t<6>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 7: return build_pattern_t<7>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
-    case 8: return build_pattern_t<8>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred);
+    case 2: return build_pattern_t<2>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 3: return build_pattern_t<3>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 4: return build_pattern_t<4>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 5: return build_pattern_t<5>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 6: return build_pattern_t<6>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 7: return build_pattern_t<7>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
+    case 8: return build_pattern_t<8>(ctx, R, nnz, d_row, d_col, d_val, N, P, h_scratch, deferred, counts);
   }
   return VNM_ERR_ARG;
 }
