@@ -40,7 +40,6 @@ namespace vnm {
 constexpr int LF = 32;       // features
 constexpr int LH = 128;      // hidden width
 constexpr int LTOP = 8;      // proposals per segment that are scored exactly
-constexpr int L_THREADS = 128;
 constexpr uint32_t L_WAIT = 1u << 22;
 
 struct LMat {  // one matrix's state
@@ -321,207 +320,311 @@ __device__ __forceinline__ int kmaj_off(int r, int k, int K) {
   return (r >> 3) * (K * 16) + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2;
 }
 
+// A block is four groups of 128 threads with a tile of 128 candidates each in
+// flight, on one copy of the weights.
+constexpr int MG = 4;              // groups a block
+constexpr int ML_THREADS = MG * 128;
+// Staged columns of a tile: its target slots' (at most 32 slots, 64 columns),
+// the segment's own from ML_OWN on.
+constexpr int ML_OWN = 72, ML_COLS = ML_OWN + 8, ML_SLOTS = 32;
+
+struct MlpGroup {
+  alignas(1024) unsigned char A[128 * LH * 2];  // a tile's features (8 KB of it), then its first layer's output
+  unsigned key[2048];                            // the segment's scores, order-preserving (0: NaN)
+  uint4 colf[ML_COLS], slotf[ML_SLOTS];          // features of a column or a slot in BF16: eight of the histogram
+  unsigned colx[ML_COLS], slotx[ML_SLOTS];       // ... and the rest: degree | N+1 rows << 16; ninth of the histogram
+  unsigned own;                                  // the segment's two features
+};
 struct MlpSmem {
-  alignas(1024) unsigned char W1[LH * LF * 2];    // 8 KB
-  alignas(1024) unsigned char W2[LH * LH * 2];    // 32 KB
-  alignas(1024) unsigned char A1[128 * LF * 2];   // 8 KB
-  alignas(1024) unsigned char A2[128 * LH * 2];   // 32 KB
-  float b1[LH], b2[LH], w3[LH];
-  float score[2048];
-  alignas(8) uint64_t bar1, bar2;
+  alignas(1024) unsigned char W1[LH * LF * 2];  // 8 KB
+  alignas(1024) unsigned char W2[LH * LH * 2];  // 32 KB
+  MlpGroup g[MG];                               // 42 KB each
+  float b1[LH], b2[LH], w3[LH];                 // plain mode
+  alignas(8) uint64_t bar[MG];
   uint32_t tmem;
   int err;
+};
+
+// The biases and the last layer as a kernel argument: read in unrolled code
+// they are operands from the constant bank.
+struct MlpTail {
+  float b1[LH];
+  float b2[LH], w3[LH], b3;  // as in the parameter vector
 };
 
 __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
+__device__ __forceinline__ unsigned bf2(float lo, float hi) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const unsigned*>(&h);
+}
+// ReLU of two values, rounded to BF16: as rounding the ReLU, for NaN (0) too
+__device__ __forceinline__ unsigned relu_bf2(float lo, float hi) {
+  const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(lo, hi), __floats2bfloat162_rn(0.f, 0.f));
+  return *reinterpret_cast<const unsigned*>(&h);
+}
 
-// The MLP on tcgen05.  Candidate mode (kPlain = false): one CTA per active
-// segment at a time scores all of its candidates and keeps the best LTOP ids
+// The MLP on tcgen05.  Candidate mode (kPlain = false): a group takes an active
+// segment at a time, scores all of its candidates and keeps the best LTOP ids
 // in top[a], at most one per target segment (ties to the lower id), so the
-// exactly scored proposals are not near-copies of one swap.  Plain mode: rows of X in tiles of 128,
-// scores to Y (the inference path on given features, for tests and timing).
-// Per tile of 128 candidates: features -> A1 (bf16, K-major), MMA 128x128x32
-// into tensor-memory columns 0..127, bias + ReLU -> A2, MMA 128x128x128 into
-// columns 128..255, bias + ReLU + dot with w3 in registers.  Thread t owns
-// candidate t of the tile, which is TMEM lane t.
+// exactly scored proposals are not near-copies of one swap.  Plain mode: rows
+// of X in tiles of 128, scores to Y (the inference path on given features, for
+// tests and timing).  Per tile: features -> A (bf16, K-major), MMA 128x128x32
+// into the group's 128 tensor-memory columns, bias + ReLU -> A, MMA
+// 128x128x128 into the same columns, bias + ReLU + dot with w3 in registers in
+// ascending order.  Thread t owns candidate t of the tile, which is TMEM lane
+// t.
+//
+// Bound by issue: some 800 instructions a warp and tile, four warps to a
+// scheduler.  What made the form before this one (a group a block, two blocks
+// an SM) 2.5 times slower was the shared-memory pipe: the biases and w3 read
+// by every thread (an LDS costs a cycle for 32 lanes' word, broadcast or not),
+// first-layer stores of 4 bytes with four-way conflicts, and every candidate
+// making all of its features.  Now the biases come from the constant bank, a
+// thread stores 16 bytes of its row at a time (eight lanes' pieces are
+// contiguous), and a column's or slot's features are made once a tile by one
+// thread and copied.  At 8192 segments x 256 candidates: 176 -> 58 us.
 template <bool kPlain>
-__global__ void __launch_bounds__(L_THREADS, 1)
-    k_l_mlp(LMat L, MlpW W, const int* active, const int* nactive_p, int KT, int round, unsigned seed, int* top,
-            const float* X, int nX, float* Y, int* err) {
+__global__ void __launch_bounds__(ML_THREADS, 1)
+    k_l_mlp(LMat L, MlpW W, const __grid_constant__ MlpTail T, const int* active, const int* nactive_p, int KT,
+            int round, unsigned seed, int* top, const float* X, int nX, float* Y, int* err) {
   extern __shared__ unsigned char l_raw[];
   MlpSmem& sm = *reinterpret_cast<MlpSmem*>(
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(l_raw) + 1023) & ~uintptr_t(1023)));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // weights -> canonical layouts (B operands: rows = output features, K-major)
-  for (int e = tid; e < LH * LF; e += L_THREADS) {
-    const int n = e / LF, k = e % LF;
-    *reinterpret_cast<__nv_bfloat16*>(sm.W1 + kmaj_off(n, k, LF)) = __float2bfloat16_rn(W.W1[e]);
-  }
-  for (int e = tid; e < LH * LH; e += L_THREADS) {
-    const int n = e / LH, k = e % LH;
-    *reinterpret_cast<__nv_bfloat16*>(sm.W2 + kmaj_off(n, k, LH)) = __float2bfloat16_rn(W.W2[e]);
-  }
-  for (int e = tid; e < LH; e += L_THREADS) {
-    sm.b1[e] = W.b1[e];
-    sm.b2[e] = W.b2[e];
-    sm.w3[e] = W.w3[e];
-  }
+  const int tid = threadIdx.x, g = tid >> 7, t = tid & 127;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int nwork = kPlain ? (nX + 127) / 128 : *nactive_p;
+  if ((int)blockIdx.x >= nwork) return;
+  // weights -> canonical layouts (B operands: rows = output features, K-major), 16 bytes at a time
+  auto weights = [&](const float* w, unsigned char* dst, int K) {
+    for (int e = tid; e < LH * K / 8; e += ML_THREADS) {
+      float x[8];  // (the parameter vector is 4-byte aligned only where a layer starts)
+#pragma unroll
+      for (int z = 0; z < 8; ++z) x[z] = w[8 * e + z];
+      const int n = 8 * e / K, k = 8 * e % K;
+      *reinterpret_cast<uint4*>(dst + kmaj_off(n, k, K)) =
+          make_uint4(bf2(x[0], x[1]), bf2(x[2], x[3]), bf2(x[4], x[5]), bf2(x[6], x[7]));
+    }
+  };
+  weights(W.W1, sm.W1, LF);
+  weights(W.W2, sm.W2, LH);
+  if (kPlain)
+    for (int e = tid; e < LH; e += ML_THREADS) {
+      sm.b1[e] = W.b1[e];
+      sm.b2[e] = W.b2[e];
+      sm.w3[e] = W.w3[e];
+    }
   if (tid == 0) {
-    ptx::mbar_init(&sm.bar1, 1);
-    ptx::mbar_init(&sm.bar2, 1);
+    for (int k = 0; k < MG; ++k) ptx::mbar_init(&sm.bar[k], 1);
     sm.err = 0;
     ptx::fence_mbar_init();
   }
   if (warp == 0) {
-    ptx::tmem_alloc(&sm.tmem, 256);
+    ptx::tmem_alloc(&sm.tmem, MG * LH);
     ptx::tmem_relinquish();
   }
   fence_async_smem();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tm = sm.tmem;
+  MlpGroup& G = sm.g[g];
+  uint64_t* const bar = &sm.bar[g];
+  const uint32_t tm = sm.tmem + (uint32_t)(g * LH), tl = tm + ((uint32_t)((warp & 3) * 32) << 16);
   const uint32_t idesc = ptx::idesc_f16(1u, 0u, 0u, 128, LH);
-  const float b3 = W.b3[0];
-  const int ncand = kPlain ? 0 : KT * L.M * L.M;
-  const int nwork = kPlain ? (nX + 127) / 128 : *nactive_p;
+  const float b3 = kPlain ? W.b3[0] : T.b3;
+  const int MM = L.M * L.M;
+  const int ncand = kPlain ? 0 : KT * MM;
   const int ntile = kPlain ? 1 : (ncand + 127) / 128;
+  const int step = MG * gridDim.x;
   uint32_t phase = 0;
-  // this thread's features of candidate `tid` of tile (a, tile); the next
-  // tile's are computed while the tensor core runs the current one's first
-  // layer, so their loads' latency is hidden behind it
-  auto feats = [&](int a, int tile, float (&f)[LF]) {
-    const int c = kPlain ? a * 128 + tid : tile * 128 + tid;
-    const bool live = a < nwork && (kPlain ? c < nX : c < ncand);
-    if (!live) {
+  // What this thread makes of tile (a, tile)'s features: of one column (v, x),
+  // one slot (v, x), the segment's two (x), or in plain mode its row's.  The
+  // next tile's are loaded while the tensor core runs the current one's first
+  // layer, so their loads' latency is hidden behind it.
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  unsigned x = 0u;
+  float f[kPlain ? LF : 1];
+  auto load = [&](int a, int tile) {
+    if (a >= nwork) return;
+    if constexpr (kPlain) {
+      const int c = a * 128 + t;
 #pragma unroll
-      for (int k = 0; k < LF; ++k) f[k] = 0.f;
-    } else if (kPlain) {
-#pragma unroll
-      for (int k = 0; k < LF; ++k) f[k] = X[(size_t)c * LF + k];
+      for (int k = 0; k < LF; ++k) f[k] = c < nX ? X[(size_t)c * LF + k] : 0.f;
     } else {
-      int q, i, j;
-      cand_of(c, L.M, q, i, j);
-      const int p = active[a];
-      features(L, p, i, target_of(p, q, round, L.nseg, seed), j, f);
+      const int p = active[a], slot0 = tile * 128 / MM;
+      const int nslot = (min(ncand, tile * 128 + 128) - 1) / MM - slot0 + 1;
+      const float iR = 1.0f / (float)L.R;
+      int at = -1;  // position of this thread's column
+      if (t < nslot * L.M) at = target_of(p, slot0 + t / L.M, round, L.nseg, seed) * L.M + t % L.M;
+      else if (t >= ML_OWN && t < ML_OWN + L.M && tile == 0) at = p * L.M + t - ML_OWN;
+      if (at >= 0) {
+        const int u = L.orig[at], d = L.cptr[u + 1] - L.cptr[u];
+        const float id = 1.0f / (float)max(d, 1);
+        float h[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) h[k] = k + 1 <= L.M ? L.colh[u * 9 + k + 1] * id : 0.f;
+        v = make_uint4(bf2(h[0], h[1]), bf2(h[2], h[3]), bf2(h[4], h[5]), bf2(h[6], h[7]));
+        x = bf2(log2f(1.0f + d) * (1.0f / 16), L.colh[u * 9 + L.N + 1] * (1.0f / 16));
+      } else if (t >= ML_COLS && t < ML_COLS + nslot) {
+        const int* hs = L.hist + (size_t)target_of(p, slot0 + t - ML_COLS, round, L.nseg, seed) * 9;
+        float h[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) h[k] = hs[k] * iR;
+        v = make_uint4(bf2(h[0], h[1]), bf2(h[2], h[3]), bf2(h[4], h[5]), bf2(h[6], h[7]));
+        x = bf2(h[8], 0.f);
+      } else if (t == 127) {
+        x = bf2(L.hist[p * 9 + L.N] * iR, L.hist[p * 9 + L.N + 1] * iR);
+      }
     }
   };
-  float f[LF];
-  feats(blockIdx.x, 0, f);
-  for (int a = blockIdx.x; a < nwork; a += gridDim.x) {
+  const int a0 = g * gridDim.x + blockIdx.x;
+  load(a0, 0);
+  for (int a = a0; a < nwork; a += step) {
     for (int tile = 0; tile < ntile; ++tile) {
-      const int c = kPlain ? a * 128 + tid : tile * 128 + tid;
+      const int c = kPlain ? a * 128 + t : tile * 128 + t;
       const bool live = kPlain ? c < nX : c < ncand;
+      // (A: the second layer of the tile before has read it, as every thread
+      // has waited for; the staged features: read before the barrier that
+      // followed)
+      uint4 row[4];
+      if constexpr (kPlain) {
 #pragma unroll
-      for (int k = 0; k < LF; k += 2)
-        *reinterpret_cast<__nv_bfloat162*>(sm.A1 + kmaj_off(tid, k, LF)) = __floats2bfloat162_rn(f[k], f[k + 1]);
+        for (int k = 0; k < 4; ++k)
+          row[k] = make_uint4(bf2(f[8 * k], f[8 * k + 1]), bf2(f[8 * k + 2], f[8 * k + 3]),
+                              bf2(f[8 * k + 4], f[8 * k + 5]), bf2(f[8 * k + 6], f[8 * k + 7]));
+      } else {
+        const int slot0 = tile * 128 / MM;
+        const int nslot = (min(ncand, tile * 128 + 128) - 1) / MM - slot0 + 1;
+        if (t < nslot * L.M || (t >= ML_OWN && t < ML_OWN + L.M && tile == 0)) {
+          G.colf[t] = v;
+          G.colx[t] = x;
+        } else if (t >= ML_COLS && t < ML_COLS + nslot) {
+          G.slotf[t - ML_COLS] = v;
+          G.slotx[t - ML_COLS] = x;
+        } else if (t == 127) {
+          G.own = x;
+        }
+        group_sync(g);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) row[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (live) {
+          int q, i, j;
+          cand_of(c, L.M, q, i, j);
+          const int z = q - slot0, w = z * L.M + j;
+          const unsigned xu = G.colx[ML_OWN + i], xw = G.colx[w], xp = G.own;
+          row[0] = G.colf[ML_OWN + i];
+          row[1] = G.colf[w];
+          row[2] = G.slotf[z];
+          row[3] = make_uint4((G.slotx[z] & 0xffffu) | xu << 16, (xw & 0xffffu) | xp << 16,
+                              xp >> 16 | (xu & 0xffff0000u), xw >> 16 | bf2(0.f, 1.f));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(G.A + kmaj_off(t, 8 * k, LF)) = row[k];
       fence_async_smem();
       ptx::tc_fence_before();
-      __syncthreads();
+      group_sync(g);
       ptx::tc_fence_after();
-      if (tid == 0) {
+      if (t == 0) {
         for (int kk = 0; kk < LF / 16; ++kk) {
-          const uint64_t ad = ptx::smem_desc(ptx::smem_addr(sm.A1) + kk * 256, 128, LF * 16, 0);
+          const uint64_t ad = ptx::smem_desc(ptx::smem_addr(G.A) + kk * 256, 128, LF * 16, 0);
           const uint64_t bd = ptx::smem_desc(ptx::smem_addr(sm.W1) + kk * 256, 128, LF * 16, 0);
           ptx::mma_f16(tm, ad, bd, idesc, kk > 0 ? 1u : 0u);
         }
-        ptx::mma_commit(&sm.bar1);
+        ptx::mma_commit(bar);
       }
-      // the next tile's features (A1 is rewritten only after this tile's
-      // second barrier, by which time the first layer has read it)
-      if (tile + 1 < ntile) feats(a, tile + 1, f);
-      else feats(a + gridDim.x, 0, f);
-      if (!ptx::mbar_wait(&sm.bar1, phase, L_WAIT)) sm.err = 1;
+      if (tile + 1 < ntile) load(a, tile + 1);
+      else load(a + step, 0);
+      if (!ptx::mbar_wait(bar, phase, L_WAIT)) sm.err = 1;
+      phase ^= 1u;
       ptx::tc_fence_after();
-      // layer 1 epilogue: bias, ReLU, BF16 -> A2
-#pragma unroll 1
-      for (int c0 = 0; c0 < LH; c0 += 32) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-        ptx::tmem_ld_wait();
+      // layer 1 epilogue: bias, ReLU, BF16 -> A (the first layer has read it)
 #pragma unroll
-        for (int z = 0; z < 32; z += 2) {
-          const float h0 = fmaxf(__uint_as_float(v[z]) + sm.b1[c0 + z], 0.f);
-          const float h1 = fmaxf(__uint_as_float(v[z + 1]) + sm.b1[c0 + z + 1], 0.f);
-          *reinterpret_cast<__nv_bfloat162*>(sm.A2 + kmaj_off(tid, c0 + z, LH)) = __floats2bfloat162_rn(h0, h1);
-        }
+      for (int c0 = 0; c0 < LH; c0 += 32) {
+        uint32_t d[32];
+        ptx::tmem_ld_32x32b_x32(tl + (uint32_t)c0, d);
+        ptx::tmem_ld_wait();
+        auto b = [&](int z) { return kPlain ? sm.b1[c0 + z] : T.b1[c0 + z]; };
+        auto h = [&](int z) {
+          return relu_bf2(__uint_as_float(d[z]) + b(z), __uint_as_float(d[z + 1]) + b(z + 1));
+        };
+#pragma unroll
+        for (int z = 0; z < 32; z += 8)
+          *reinterpret_cast<uint4*>(G.A + kmaj_off(t, c0 + z, LH)) = make_uint4(h(z), h(z + 2), h(z + 4), h(z + 6));
       }
       fence_async_smem();
       ptx::tc_fence_before();
-      __syncthreads();
+      group_sync(g);
       ptx::tc_fence_after();
-      if (tid == 0) {
+      if (t == 0) {
         for (int kk = 0; kk < LH / 16; ++kk) {
-          const uint64_t ad = ptx::smem_desc(ptx::smem_addr(sm.A2) + kk * 256, 128, LH * 16, 0);
+          const uint64_t ad = ptx::smem_desc(ptx::smem_addr(G.A) + kk * 256, 128, LH * 16, 0);
           const uint64_t bd = ptx::smem_desc(ptx::smem_addr(sm.W2) + kk * 256, 128, LH * 16, 0);
-          ptx::mma_f16(tm + 128, ad, bd, idesc, kk > 0 ? 1u : 0u);
+          ptx::mma_f16(tm, ad, bd, idesc, kk > 0 ? 1u : 0u);
         }
-        ptx::mma_commit(&sm.bar2);
+        ptx::mma_commit(bar);
       }
-      if (!ptx::mbar_wait(&sm.bar2, phase, L_WAIT)) sm.err = 1;
+      if (!ptx::mbar_wait(bar, phase, L_WAIT)) sm.err = 1;
+      phase ^= 1u;
       ptx::tc_fence_after();
       float y = b3;
-#pragma unroll 1
-      for (int c0 = 0; c0 < LH; c0 += 32) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tm + ((uint32_t)(warp * 32) << 16) + 128u + (uint32_t)c0, v);
-        ptx::tmem_ld_wait();
 #pragma unroll
-        for (int z = 0; z < 32; ++z) {
-          const float h = fmaxf(__uint_as_float(v[z]) + sm.b2[c0 + z], 0.f);
-          y = fmaf(__bfloat162float(__float2bfloat16_rn(h)), sm.w3[c0 + z], y);
+      for (int c0 = 0; c0 < LH; c0 += 32) {
+        uint32_t d[32];
+        ptx::tmem_ld_32x32b_x32(tl + (uint32_t)c0, d);
+        ptx::tmem_ld_wait();
+        auto b = [&](int z) { return kPlain ? sm.b2[c0 + z] : T.b2[c0 + z]; };
+        auto w3 = [&](int z) { return kPlain ? sm.w3[c0 + z] : T.w3[c0 + z]; };
+#pragma unroll
+        for (int z = 0; z < 32; z += 2) {
+          const unsigned h = relu_bf2(__uint_as_float(d[z]) + b(z), __uint_as_float(d[z + 1]) + b(z + 1));
+          y = fmaf(__uint_as_float(h << 16), w3(z), y);
+          y = fmaf(__uint_as_float(h & 0xffff0000u), w3(z + 1), y);
         }
       }
       if (kPlain) {
         if (live) Y[c] = y;
       } else if (live) {
-        sm.score[c] = y;
+        const unsigned bits = __float_as_uint(y + 0.f);  // (-0 equals 0)
+        G.key[c] = y != y ? 0u : (bits >> 31 ? ~bits : bits | 0x80000000u);
       }
-      phase ^= 1u;
-      ptx::tc_fence_before();
-      __syncthreads();
-      ptx::tc_fence_after();
     }
     if (!kPlain) {
-      // top LTOP of this segment (ties to the lower id); warp 0
-      if (warp == 0) {
+      // top LTOP of this segment (ties to the lower id); the group's first
+      // warp (the others write scores again only past barriers that it joins)
+      group_sync(g);
+      if (t < 32) {
+        const unsigned dropped = ~0xff800000u;  // the key of -infinity
         for (int k = 0; k < LTOP; ++k) {
-          float best = -INFINITY;
+          unsigned best = 0u;
           int bid = 0x7fffffff;
           for (int c = lane; c < ncand; c += 32) {
-            const float s = sm.score[c];
-            if (s > best || (s == best && c < bid)) {
+            const unsigned s = G.key[c];
+            if (s > best) {
               best = s;
               bid = c;
             }
           }
-          for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bid, o);
-            if (ob > best || (ob == best && oi < bid)) {
-              best = ob;
-              bid = oi;
-            }
-          }
+          const unsigned m = __reduce_max_sync(0xffffffffu, best);
+          bid = __reduce_min_sync(0xffffffffu, m != 0u && best == m ? bid : 0x7fffffff);
           if (lane == 0) top[a * LTOP + k] = bid < ncand ? bid : -1;
           // one proposal per target segment: drop the rest of the winner's slot
           if (bid < ncand) {
-            const int mm = L.M * L.M, q0 = bid / mm;
-            for (int z = lane; z < mm; z += 32) sm.score[q0 * mm + z] = -INFINITY;
+            const int q0 = bid / MM;
+            for (int z = lane; z < MM; z += 32) G.key[q0 * MM + z] = dropped;
           }
           __syncwarp();
         }
       }
-      __syncthreads();
     }
   }
-  if (tid == 0 && sm.err) atomicOr(err, 8);
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  if (warp == 0) ptx::tmem_dealloc(tm, 256);
+  if (tid == 0 && sm.err) atomicOr(err, 8);
+  if (warp == 0) ptx::tmem_dealloc(sm.tmem, MG * LH);
 }
 
 // ---------------------------------------------------------------------------
@@ -1381,10 +1484,10 @@ vnm_status vnm_mlp_forward(vnm_ctx* ctx, const vnm_mlp* net, const float* X, int
   VNM_TRY(mlp_launch_prep(smem));
   LMat L{};
   const int tiles = (n + 127) / 128;
-  const int grid = tiles < 2 * ctx->num_sms ? tiles : 2 * ctx->num_sms;
+  const int grid = tiles < ctx->num_sms ? tiles : ctx->num_sms;
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  VNM_LAUNCH(ctx, k_l_mlp<true>, grid, L_THREADS, smem, L, mlp_view(net), nullptr, nullptr, 0, 0, 0u, nullptr, dX,
-             n, dY, err);
+  VNM_LAUNCH(ctx, k_l_mlp<true>, grid, ML_THREADS, smem, L, mlp_view(net), MlpTail{}, nullptr, nullptr, 0, 0, 0u,
+             nullptr, dX, n, dY, err);
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(Y, dY, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1423,7 +1526,7 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
                 arena_bytes(LC_N + 8 * 2, 4) + 2 * arena_bytes(chunk_cap, 8) +
                 arena_bytes((size_t)dcap * LF, 4) + arena_bytes(dcap, 4) + 8192;
   VNM_TRY(arena_reserve(ctx, need));
-  VNM_TRY(pinned_reserve(ctx, 256));
+  VNM_TRY(pinned_reserve(ctx, 512));
   VNM_TRY(begin_call(ctx));
   const int *d_row, *d_col;
   const float* d_val;
@@ -1479,13 +1582,21 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   unsigned long long* hcu = reinterpret_cast<unsigned long long*>(ctx->h_pinned);  // 8 words
   int* hci = reinterpret_cast<int*>(hcu + 8);                                       // LC_N ints, as on the device
   VNM_CUDA_TRY(cudaMemcpyAsync(hcu, cu, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
+  float* hb = reinterpret_cast<float*>(ctx->h_pinned + 64);
+  if (mode == VNM_LEARNED_MLP) {
+    VNM_CUDA_TRY(cudaMemcpyAsync(hb, net->p + L_OFF_B1, sizeof(float) * LH, cudaMemcpyDeviceToHost, st));
+    VNM_CUDA_TRY(cudaMemcpyAsync(hb + LH, net->p + L_OFF_B2, sizeof(float) * (2 * LH + 1), cudaMemcpyDeviceToHost, st));
+  }
   VNM_CUDA_TRY(cudaStreamSynchronize(st));
+  MlpTail T{};
+  static_assert(sizeof(T) == sizeof(float) * (3 * LH + 1), "the tail as copied");
+  if (mode == VNM_LEARNED_MLP) memcpy(&T, hb, sizeof(T));
   out->init_invalid = out->final_invalid = (long long)hcu[2];
   out->init_retained = out->final_retained = (long long)hcu[3];
   const size_t smem = mlp_smem();
   if (mode == VNM_LEARNED_MLP) VNM_TRY(mlp_launch_prep(smem));
   const MlpW W = net ? mlp_view(net) : MlpW{};
-  const int pgrid = 2 * ctx->num_sms;
+  const int pgrid = ctx->num_sms;  // the blocks beyond the active segments return at once
   const int egrid = ctx->num_sms * 8;
   const size_t state_bytes = 8 * sizeof(unsigned long long) + LC_N * sizeof(int);
   int idle = 0, rounds = 0, swaps = 0;
@@ -1494,8 +1605,8 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
     VNM_LAUNCH(ctx, k_l_round_start, 1 + lgrid(ctx, nseg, L_START_THREADS), L_START_THREADS, 0, L, active, ci, best,
                claim);
     if (mode == VNM_LEARNED_MLP)
-      VNM_LAUNCH(ctx, k_l_mlp<false>, pgrid, L_THREADS, smem, L, W, active, ci, KT, round, prm->seed, top, nullptr,
-                 0, nullptr, ci + LC_ERR);
+      VNM_LAUNCH(ctx, k_l_mlp<false>, pgrid, ML_THREADS, smem, L, W, T, active, ci + LC_ACTIVE, KT, round,
+                 prm->seed, top, nullptr, 0, nullptr, ci + LC_ERR);
     VNM_LAUNCH(ctx, k_l_exact, egrid, 256, 0, L, active, ci, KT, round, prm->seed, top, mode, prm->topk, best, dx, dy,
                prm->dump_every, ci + LC_DUMP, dcap, cu + 1);
     VNM_LAUNCH(ctx, k_l_claim, lgrid(ctx, nseg), 256, 0, L, active, ci, round, prm->seed, best, claim);
