@@ -99,6 +99,8 @@ __global__ void k_l_seg_hist(LMat L) {
 // in the offsets for each chunk, a round of the search took five launches
 // and 25 us more at 65536 rows.)
 constexpr int L_CHUNK = 256;
+constexpr int L_ROWS = L_CHUNK / 32;  // a lane's rows of a chunk, all in flight (one after the other,
+                                      // k_l_colh_rows took 195 us of eleven rounds and k_l_apply_rows 180, 152 and 142 now)
 
 // Counters of a call, on the device.
 enum { LC_ACTIVE, LC_ACC, LC_SWAP_ITEMS, LC_DUMP, LC_ERR, LC_COL_ITEMS, LC_N = 8 };
@@ -149,13 +151,15 @@ __global__ void k_l_colh_rows(LMat L, const int2* items, const int* nitems) {
     const int u = L.orig[it.x], s = it.x / L.M;
     const int beg = L.cptr[u] + it.y * L_CHUNK;
     const int end = min(beg + L_CHUNK, L.cptr[u + 1]);
-    int h[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int e = beg + lane; e < end; e += 32) {
-      const int r = L.crow[e];
-      const int k = __popc(L.G[(long long)r * L.nseg + s]);
+    int r[L_ROWS], k[L_ROWS], h[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-      for (int z = 0; z < 9; ++z) h[z] += (k == z);
-    }
+    for (int x = 0; x < L_ROWS; ++x) r[x] = beg + lane + 32 * x < end ? L.crow[beg + lane + 32 * x] : -1;
+#pragma unroll
+    for (int x = 0; x < L_ROWS; ++x) k[x] = r[x] >= 0 ? __popc(L.G[(long long)r[x] * L.nseg + s]) : -1;
+#pragma unroll
+    for (int x = 0; x < L_ROWS; ++x)
+#pragma unroll
+      for (int z = 0; z < 9; ++z) h[z] += (k[x] == z);
 #pragma unroll
     for (int z = 0; z < 9; ++z) {
       const int v = __reduce_add_sync(0xffffffffu, h[z]);
@@ -269,34 +273,39 @@ __device__ __forceinline__ int move_gain(int obj, int N, int from, int to) {  //
   return obj == 0 ? (from == N + 1) - (to == N) : (to < N) - (from <= N);
 }
 
+// The rows of both columns are one list, 8 a lane in flight, and the next
+// ones' numbers are fetched while the group bytes come: a hub column's rows
+// are a long chain of dependent loads on one warp.  (4 a lane, column after
+// column and without the fetch ahead, eleven rounds at 65536 rows: 618 us,
+// 447 now.)
 __device__ int exact_gain_warp(const LMat& L, int p, int i, int t, int j) {
-  constexpr int U = 4;  // rows per lane in flight: a hub column is a long chain of dependent loads
+  constexpr int U = 8;
   const int lane = threadIdx.x & 31;
   const int u = L.orig[p * L.M + i], w = L.orig[t * L.M + j];
   const unsigned bi = 1u << i, bj = 1u << j;
+  const int bu = L.cptr[u], du = L.cptr[u + 1] - bu, bw = L.cptr[w], n = du + L.cptr[w + 1] - bw;
+  auto row = [&](int e) { return e < du ? L.crow[bu + e] : e < n ? L.crow[bw + e - du] : -1; };
+  int r[U];
+#pragma unroll
+  for (int k = 0; k < U; ++k) r[k] = row(lane + 32 * k);
   int g = 0;
-  for (int side = 0; side < 2; ++side) {
-    const int col = side == 0 ? u : w;
-    const int end = L.cptr[col + 1];
-    for (int e0 = L.cptr[col] + lane; e0 < end; e0 += 32 * U) {
-      int r[U];
+  for (int e0 = lane; e0 - lane < n; e0 += 32 * U) {
+    unsigned gp[U], gt[U];
 #pragma unroll
-      for (int k = 0; k < U; ++k) r[k] = e0 + 32 * k < end ? L.crow[e0 + 32 * k] : -1;
-      unsigned gp[U], gt[U];
+    for (int k = 0; k < U; ++k) {
+      gp[k] = r[k] >= 0 ? L.G[(long long)r[k] * L.nseg + p] : 0u;
+      gt[k] = r[k] >= 0 ? L.G[(long long)r[k] * L.nseg + t] : 0u;
+    }
+    int next[U];
 #pragma unroll
-      for (int k = 0; k < U; ++k) {
-        gp[k] = r[k] >= 0 ? L.G[(long long)r[k] * L.nseg + p] : 0u;
-        gt[k] = r[k] >= 0 ? L.G[(long long)r[k] * L.nseg + t] : 0u;
-      }
+    for (int k = 0; k < U; ++k) next[k] = row(e0 + 32 * (U + k));
 #pragma unroll
-      for (int k = 0; k < U; ++k) {
-        if (r[k] < 0) continue;
-        if (side == 0) {
-          if (!(gt[k] & bj)) g += move_gain(L.obj, L.N, __popc(gp[k]), __popc(gt[k]));  // else w is here too
-        } else {
-          if (!(gp[k] & bi)) g += move_gain(L.obj, L.N, __popc(gt[k]), __popc(gp[k]));
-        }
-      }
+    for (int k = 0; k < U; ++k) {
+      const bool first = e0 + 32 * k < du;  // a row of column u, else of column w
+      const unsigned from = first ? gp[k] : gt[k], to = first ? gt[k] : gp[k];
+      if (r[k] >= 0 && !(to & (first ? bj : bi)))  // else both columns are here
+        g += move_gain(L.obj, L.N, __popc(from), __popc(to));
+      r[k] = next[k];
     }
   }
   return __reduce_add_sync(0xffffffffu, g);
@@ -775,10 +784,19 @@ __global__ void k_l_apply_rows(LMat L, const int4* acc, int* ci, const int2* uw,
     const int beg = L.cptr[col] + k * L_CHUNK, end = min(beg + L_CHUNK, L.cptr[col + 1]);
     int dp[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, dt[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     int dcp = 0, dct = 0;
-    for (int e = beg + lane; e < end; e += 32) {
-      const int r = L.crow[e];
-      const long long cp = (long long)r * L.nseg + p, ct = (long long)r * L.nseg + t;
-      const unsigned gp = L.G[cp], gt = L.G[ct];
+    int r[L_ROWS];
+    unsigned was_p[L_ROWS], was_t[L_ROWS];
+#pragma unroll
+    for (int x = 0; x < L_ROWS; ++x) r[x] = beg + lane + 32 * x < end ? L.crow[beg + lane + 32 * x] : -1;
+#pragma unroll
+    for (int x = 0; x < L_ROWS; ++x) {
+      was_p[x] = r[x] >= 0 ? L.G[(long long)r[x] * L.nseg + p] : 0u;
+      was_t[x] = r[x] >= 0 ? L.G[(long long)r[x] * L.nseg + t] : 0u;
+    }
+#pragma unroll
+    for (int x = 0; x < L_ROWS; ++x) {
+      const long long cp = (long long)r[x] * L.nseg + p, ct = (long long)r[x] * L.nseg + t;
+      const unsigned gp = was_p[x], gt = was_t[x];  // (no row: both 0, nothing moves)
       const bool inU = gp & bi, inW = gt & bj;
       if (inU == inW) continue;  // both columns or neither: nothing moves
       const unsigned np_ = inW ? (gp | bi) : (gp & ~bi);
