@@ -128,8 +128,6 @@ size_t radix_sort_scratch_bytes(int n);
 // the invalid / present row counts of each M-column segment.
 struct Pattern {
   int R = 0, nseg = 0, np = 0;
-  int* prow = nullptr;
-  int* pcol = nullptr;
   int* cptr = nullptr;
   int* crow = nullptr;    // rows of each column, grouped by row group (nm_reorder.cu row_group)
   int* csplit = nullptr;  // [16 R + 1] start of each (column, row group) in crow

@@ -58,10 +58,11 @@ struct LMat {  // one matrix's state
 // ---------------------------------------------------------------------------
 // State build and maintenance
 // ---------------------------------------------------------------------------
-__global__ void k_l_build_G(const int* prow, const int* pcol, int np, int M, int nseg, unsigned* Gw) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const long long cell = (long long)prow[i] * nseg + pcol[i] / M;
-    atomicOr(&Gw[cell >> 2], (1u << (pcol[i] % M)) << ((cell & 3) * 8));
+__global__ void k_l_build_G(const int* row, const int* col, const float* val, int nnz, int M, int nseg, unsigned* Gw) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
+    if (val[i] == 0.0f) continue;
+    const long long cell = (long long)row[i] * nseg + col[i] / M;
+    atomicOr(&Gw[cell >> 2], (1u << (col[i] % M)) << ((cell & 3) * 8));
   }
 }
 
@@ -1589,7 +1590,7 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   VNM_CUDA_TRY(cudaMemsetAsync(cu, 0, 8 * sizeof(unsigned long long) + LC_N * sizeof(int), st));
   if (R > 0) VNM_LAUNCH(ctx, k_l_iota2, lgrid(ctx, R), 256, 0, L.orig, L.pos, R);
   if (P.np > 0)
-    VNM_LAUNCH(ctx, k_l_build_G, lgrid(ctx, P.np), 256, 0, P.prow, P.pcol, P.np, M, nseg,
+    VNM_LAUNCH(ctx, k_l_build_G, lgrid(ctx, nnz), 256, 0, d_row, d_col, d_val, nnz, M, nseg,
                reinterpret_cast<unsigned*>(L.G));
   if (nseg > 0) {
     VNM_LAUNCH(ctx, k_l_all_columns, lgrid(ctx, R), 256, 0, L, col_items, ci + LC_COL_ITEMS);

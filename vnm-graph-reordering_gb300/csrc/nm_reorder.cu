@@ -129,7 +129,7 @@ struct NMJob {
   int trace_cap_rounds;
   int walk_wait_limit;  // polls before a wait of the walk gives up (WALK_WAIT_LIMIT)
   int hold_heaps;       // test only: the swap heaps publish no pop, so a walk that waits runs out
-  const int* err;       // the input check's flag (k_validate): nonzero, the job does nothing; null, no check
+  const int* err;       // the input check's flag (k_check_count): nonzero, the job does nothing; null, no check
   int timed;            // measure the round phases (the leader's thread 0 reads the global timer)
 };
 
@@ -137,91 +137,96 @@ struct NMJob {
 // Setup kernels
 // ---------------------------------------------------------------------------
 
-// Range and strict (row, col) order check of the caller's COO.
-__global__ void k_validate(const int* row, const int* col, int nnz, int R, int* err) {
+// Range and strict (row, col) order check of the caller's COO, the entries
+// with nonzero value (reorder/reorder.h:93: the bitmap bit is (val != 0)) in
+// all and per (column, row group).  err: [0] the flag (bit 1 unsorted, bit 2
+// out of range), [1] the count.  An entry out of range is counted nowhere;
+// every later kernel that takes indices as addresses does nothing when the
+// flag is set, so the host may read it once, at the end of the call.
+__global__ void k_check_count(const int* row, const int* col, const float* val, int nnz, int R, int* gdeg, int* err) {
+  int flag = 0, n = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
-    int r = row[i], c = col[i];
+    const int r = row[i], c = col[i];
     if (r < 0 || r >= R || c < 0 || c >= R) {
-      atomicOr(err, 2);
+      flag |= 2;
       continue;
     }
     if (i > 0) {
-      int rp = row[i - 1], cp = col[i - 1];
-      if (rp > r || (rp == r && cp >= c)) atomicOr(err, 1);
+      const int rp = row[i - 1], cp = col[i - 1];
+      if (rp > r || (rp == r && cp >= c)) flag |= 1;
     }
-  }
-}
-
-__global__ void k_nonzero_flags(const float* val, int nnz, int* flags) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x)
-    flags[i] = val[i] != 0.0f;  // reorder/reorder.h:93: the bitmap bit is (val != 0)
-}
-
-// Keep the entries with nonzero value, in order; count entries per
-// (column, row group).  This kernel and every later one that takes indices
-// as addresses do nothing when k_validate flagged the input (*err != 0): the
-// host reads the flag once, at the end of the call.
-__global__ void k_compact(const int* row, const int* col, const float* val, const int* pos, int nnz, int* prow,
-                          int* pcol, int* gdeg, const int* err) {
-  if (*err) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     if (val[i] != 0.0f) {
-      int p = pos[i];
-      prow[p] = row[i];
-      pcol[p] = col[i];
-      atomicAdd(&gdeg[(size_t)ROW_GROUPS * col[i] + row_group(row[i])], 1);
+      ++n;
+      atomicAdd(&gdeg[(size_t)ROW_GROUPS * c + row_group(r)], 1);
     }
   }
-}
-
-// cptr[c] = the start of column c's first group (c = 0 .. R)
-__global__ void k_cptr_from_split(const int* csplit, int R, int* cptr) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= R; c += gridDim.x * blockDim.x)
-    cptr[c] = csplit[(size_t)ROW_GROUPS * c];
-}
-
-// Column lists of the pattern, each grouped by row_group (the order inside
-// a group is whatever the atomics give; nothing depends on it).
-__global__ void k_csc_scatter(const int* prow, const int* pcol, const int* d_np, const int* csplit, int* cfill,
-                              int* crow, const int* err) {
-  if (*err) return;
-  const int np = *d_np;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const size_t g = (size_t)ROW_GROUPS * pcol[i] + row_group(prow[i]);
-    const int slot = atomicAdd(&cfill[g], 1);
-    crow[csplit[g] + slot] = prow[i];
+  flag = __reduce_or_sync(0xffffffffu, flag);
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0) {
+    if (flag) atomicOr(err, flag);
+    if (n) atomicAdd(err + 1, n);
   }
 }
 
-// Invalid and non-empty group counts per segment at the identity arrangement.
-// The pattern is sorted by (row, col), so a row's groups are runs of entries
-// with equal col / M; the last entry of each run does the counting.
+// From the group starts: the column starts; the pattern's column lists, each
+// grouped by row_group (the order inside a group is whatever the atomics give;
+// nothing depends on it); and, where wanted (inv not null), the invalid and
+// non-empty group counts of a segment at the identity arrangement.  The
+// entries are sorted by (row, col), so a row's groups are runs of at most M
+// entries with equal col / M, of which those of value 0 do not count; the last
+// other entry of a run does the counting.  (At 512 rows every operation on the
+// stream costs its launch: with the zeros taken out first, a kernel for each
+// part, five clears and three operations a job to set up, a search took 396 us
+// from call to return, 328 now.)
 template <int M>
-__global__ void k_locate(const int* prow, const int* pcol, const int* d_np, int N, int* inv, int* pres,
-                         const int* err) {
+__global__ void k_pattern(const int* row, const int* col, const float* val, int nnz, int R, int N, const int* csplit,
+                          int* cptr, int* cfill, int* crow, int* inv, int* pres, const int* err) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int c = i0; c <= R; c += step) cptr[c] = csplit[(size_t)ROW_GROUPS * c];
   if (*err) return;
-  const int np = *d_np;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const int r = prow[i], s = pcol[i] / M;
-    const bool last = (i + 1 == np) || prow[i + 1] != r || pcol[i + 1] / M != s;
+  for (int i = i0; i < nnz; i += step) {
+    if (val[i] == 0.0f) continue;
+    const int r = row[i], c = col[i], s = c / M;
+    const size_t g = (size_t)ROW_GROUPS * c + row_group(r);
+    crow[csplit[g] + atomicAdd(&cfill[g], 1)] = r;
+    if (!inv) continue;
+    bool last = true;
+#pragma unroll
+    for (int b = 1; b < M; ++b) {
+      const int k = i + b;
+      if (k < nnz && row[k] == r && col[k] / M == s && val[k] != 0.0f) last = false;
+    }
     if (!last) continue;
     int len = 1;
 #pragma unroll
     for (int b = 1; b < M; ++b) {
-      int k = i - b;
-      if (k >= 0 && prow[k] == r && pcol[k] / M == s) len++;
+      const int k = i - b;
+      if (k >= 0 && row[k] == r && col[k] / M == s && val[k] != 0.0f) len++;
     }
     atomicAdd(&pres[s], 1);
     if (len > N) atomicAdd(&inv[s], 1);
   }
 }
 
-__global__ void k_init_job(int* orig, int* cnt, int* zc, const int* inv0, const int* pres0, int R, int nseg) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
-    orig[i] = i;
-    if (i < nseg) {
-      cnt[i] = inv0[i];
-      zc[i] = R - pres0[i];
+// Up to four jobs on one pattern: the identity arrangement and its counts, and
+// clear scratch and results.  tail (if not null): the check's words, to be
+// read back next to the results.
+struct JobSet {
+  NMJob j[4];
+};
+__global__ void k_init_jobs(JobSet set, int njobs, const int* inv0, const int* pres0, const int* err, int* tail) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (tail && i0 < 2) tail[i0] = err[i0];
+  for (int q = 0; q < njobs; ++q) {
+    const NMJob& J = set.j[q];
+    if (i0 < JOB_RES) J.res[i0] = 0;
+    for (int i = i0; i < J.R; i += step) {
+      J.orig[i] = i;
+      J.rec[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < J.nseg) {
+        J.cnt[i] = inv0[i];
+        J.zc[i] = J.R - pres0[i];
+      }
     }
   }
 }
@@ -1928,18 +1933,17 @@ static inline int grid_for(const vnm_ctx* ctx, long long n, int nt = 256) {
   return g < 1 ? 1 : (int)g;
 }
 
+// ints before the arrays in a pattern's block of words that start at 0: the
+// check's flag and the entry count, padded
+constexpr size_t PATTERN_CLEAR = 64;
+
 size_t pattern_bytes(int R, int nnz) {
   size_t b = 0;
-  b += arena_bytes(2, sizeof(int));              // the input check's flag and the entry count
-  b += arena_bytes(nnz, sizeof(int));            // flags / positions
-  b += 2 * arena_bytes(nnz, sizeof(int));        // prow, pcol
   const size_t ng = (size_t)ROW_GROUPS * R + 1;
-  b += arena_bytes(R + 1, sizeof(int));          // cptr
-  b += 2 * arena_bytes(ng, sizeof(int));         // group counts -> csplit, cfill
-  b += arena_bytes(nnz, sizeof(int));            // crow
-  b += 2 * arena_bytes(R / 2 + 1, sizeof(int));  // inv0, pres0 (nseg <= R/2)
-  b += arena_bytes(1, sizeof(int)) * 2;          // totals
-  b += scan_scratch_bytes((size_t)nnz > ng ? nnz : (int)ng) * 2;
+  b += arena_bytes(PATTERN_CLEAR + 2 * ng + 2 * (size_t)(R / 2 + 1), sizeof(int));  // the cleared words
+  b += arena_bytes(R + 1, sizeof(int));                                            // cptr
+  b += arena_bytes(nnz, sizeof(int));                                              // crow
+  b += scan_scratch_bytes((int)ng);
   return b;
 }
 
@@ -1948,67 +1952,34 @@ static vnm_status build_pattern_t(vnm_ctx* ctx, int R, int nnz, const int* d_row
                                   const float* d_val, int N, Pattern& P, int* h_scratch, bool deferred, bool counts) {
   P.R = R;
   P.nseg = R / M;
-  int* err = arena_take<int>(ctx, 2);  // [0] the input check's flag, [1] the pattern's entry count
-  int* pos = arena_take<int>(ctx, nnz > 0 ? nnz : 1);
-  P.prow = arena_take<int>(ctx, nnz > 0 ? nnz : 1);
-  P.pcol = arena_take<int>(ctx, nnz > 0 ? nnz : 1);
-  const size_t ng = (size_t)ROW_GROUPS * R + 1;
+  const size_t ng = (size_t)ROW_GROUPS * R + 1, ns = (size_t)P.nseg + 1;
+  const size_t nclear = PATTERN_CLEAR + 2 * ng + 2 * ns;
+  int* clear = arena_take<int>(ctx, nclear);
   P.cptr = arena_take<int>(ctx, R + 1);
-  P.csplit = arena_take<int>(ctx, ng);
-  int* cfill = arena_take<int>(ctx, ng);
   P.crow = arena_take<int>(ctx, nnz > 0 ? nnz : 1);
-  P.inv0 = arena_take<int>(ctx, R / 2 + 1);
-  P.pres0 = arena_take<int>(ctx, R / 2 + 1);
-  int* d_tot = arena_take<int>(ctx, 1);
-  if (!err || !pos || !P.prow || !P.pcol || !P.cptr || !P.csplit || !cfill || !P.crow || !P.inv0 || !P.pres0 ||
-      !d_tot)
-    return VNM_ERR_NOMEM;
-  int* d_np = err + 1;
+  if (!clear || !P.cptr || !P.crow) return VNM_ERR_NOMEM;
+  int* err = clear;
+  P.csplit = clear + PATTERN_CLEAR;  // the groups' counts, then their starts
+  int* cfill = P.csplit + ng;
+  P.inv0 = cfill + ng;
+  P.pres0 = P.inv0 + ns;
   P.d_err = err;
-  VNM_CUDA_TRY(cudaMemsetAsync(err, 0, 2 * sizeof(int), ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(P.csplit, 0, sizeof(int) * ng, ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(cfill, 0, sizeof(int) * ng, ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(P.inv0, 0, sizeof(int) * (P.nseg + 1), ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(P.pres0, 0, sizeof(int) * (P.nseg + 1), ctx->stream));
-  if (nnz > 0) {
-    // indices are checked before any kernel uses them as addresses: here,
-    // or (deferred) by the kernels themselves, which skip their work when
-    // the flag is set
-    VNM_LAUNCH(ctx, k_validate, grid_for(ctx, nnz), 256, 0, d_row, d_col, nnz, R, err);
-    if (!deferred) {
-      VNM_CUDA_TRY(cudaMemcpyAsync(h_scratch, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-      VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-      if (h_scratch[0] & 2) return VNM_ERR_RANGE;
-      if (h_scratch[0] & 1) return VNM_ERR_UNSORTED;
-    }
-    VNM_LAUNCH(ctx, k_nonzero_flags, grid_for(ctx, nnz), 256, 0, d_val, nnz, pos);
-    VNM_TRY(exclusive_scan(ctx, pos, pos, nnz, d_np));
-    VNM_LAUNCH(ctx, k_compact, grid_for(ctx, nnz), 256, 0, d_row, d_col, d_val, pos, nnz, P.prow, P.pcol,
-               P.csplit, err);
+  VNM_CUDA_TRY(cudaMemsetAsync(clear, 0, sizeof(int) * nclear, ctx->stream));
+  // indices are checked before any kernel uses them as addresses: here, or
+  // (deferred) by the kernels themselves, which skip their work when the flag
+  // is set
+  if (nnz > 0) VNM_LAUNCH(ctx, k_check_count, grid_for(ctx, nnz), 256, 0, d_row, d_col, d_val, nnz, R, P.csplit, err);
+  P.np = -1;
+  if (!deferred) {
+    VNM_CUDA_TRY(cudaMemcpyAsync(h_scratch, err, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (h_scratch[0] & 2) return VNM_ERR_RANGE;
+    if (h_scratch[0] & 1) return VNM_ERR_UNSORTED;
+    P.np = h_scratch[1];
   }
-  VNM_TRY(exclusive_scan(ctx, P.csplit, P.csplit, (int)ng, d_tot));
-  VNM_LAUNCH(ctx, k_cptr_from_split, grid_for(ctx, (long long)R + 1), 256, 0, P.csplit, R, P.cptr);
-  if (deferred) {
-    // the entry count stays on the device (read back with the call's
-    // results); the grids cover every stored entry
-    P.np = -1;
-    if (nnz > 0) {
-      VNM_LAUNCH(ctx, k_csc_scatter, grid_for(ctx, nnz), 256, 0, P.prow, P.pcol, d_np, P.csplit, cfill, P.crow,
-                 err);
-      if (counts)
-        VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, nnz), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
-    }
-    return VNM_OK;
-  }
-  VNM_CUDA_TRY(cudaMemcpyAsync(h_scratch + 1, d_np, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  P.np = h_scratch[1];
-  if (P.np > 0) {
-    VNM_LAUNCH(ctx, k_csc_scatter, grid_for(ctx, P.np), 256, 0, P.prow, P.pcol, d_np, P.csplit, cfill, P.crow,
-               err);
-    if (counts)
-      VNM_LAUNCH(ctx, k_locate<M>, grid_for(ctx, P.np), 256, 0, P.prow, P.pcol, d_np, N, P.inv0, P.pres0, err);
-  }
+  VNM_TRY(exclusive_scan(ctx, P.csplit, P.csplit, (int)ng, nullptr));
+  VNM_LAUNCH(ctx, k_pattern<M>, grid_for(ctx, std::max((long long)nnz, (long long)R + 1)), 256, 0, d_row, d_col, d_val,
+             nnz, R, N, P.csplit, P.cptr, cfill, P.crow, counts ? P.inv0 : nullptr, P.pres0, err);
   return VNM_OK;
 }
 
@@ -2032,8 +2003,9 @@ size_t job_bytes(int R) {
          arena_bytes((size_t)R + 2 * ROW_GROUPS, sizeof(int)) + arena_bytes(JOB_RES, sizeof(int));
 }
 
-// Carve one job's state out of the arena and initialise it.
-static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J) {
+// Carve one job's state out of the arena (its results at `res`, if given);
+// init_jobs sets it up.
+static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J, int* res = nullptr) {
   J.R = P.R;
   J.row0 = 0;
   J.nseg = P.nseg;
@@ -2047,7 +2019,7 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   J.zc = arena_take<int>(ctx, P.nseg + 1);
   J.rec = arena_take<uint4>(ctx, P.R > 0 ? P.R : 1);
   J.touched = arena_take<int>(ctx, (size_t)P.R + 2 * ROW_GROUPS);
-  J.res = arena_take<int>(ctx, JOB_RES);
+  J.res = res ? res : arena_take<int>(ctx, JOB_RES);
   J.trace_pairs = nullptr;
   J.trace_rounds = nullptr;
   J.trace_cap_pairs = 0;
@@ -2066,10 +2038,13 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   }
   if (const char* e = getenv("VNM_NM_TEST_HOLD_HEAPS")) J.hold_heaps = atoi(e) == 1 ? 1 : 0;
   if (!J.orig || !J.cnt || !J.zc || !J.rec || !J.touched || !J.res) return VNM_ERR_NOMEM;
-  VNM_CUDA_TRY(cudaMemsetAsync(J.rec, 0, sizeof(uint4) * (P.R > 0 ? P.R : 1), ctx->stream));
-  VNM_CUDA_TRY(cudaMemsetAsync(J.res, 0, sizeof(int) * JOB_RES, ctx->stream));
-  if (P.R > 0)
-    VNM_LAUNCH(ctx, k_init_job, grid_for(ctx, P.R), 256, 0, J.orig, J.cnt, J.zc, P.inv0, P.pres0, P.R, P.nseg);
+  return VNM_OK;
+}
+
+static vnm_status init_jobs(vnm_ctx* ctx, const Pattern& P, const NMJob* jobs, int njobs, int* tail = nullptr) {
+  JobSet set{};
+  for (int q = 0; q < njobs; ++q) set.j[q] = jobs[q];
+  VNM_LAUNCH(ctx, k_init_jobs, grid_for(ctx, P.R > 0 ? P.R : 1), 256, 0, set, njobs, P.inv0, P.pres0, P.d_err, tail);
   return VNM_OK;
 }
 
@@ -2265,10 +2240,11 @@ __global__ void k_pick_invert(const NMJob* jobs, int njobs, int nnz, int job, in
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) newpos[orig[i]] = i;
 }
 
-// Pinned host words of run_matrix: the jobs' results, then the input
-// check's flag, the pattern's entry count and the device's pick, then the
-// job records on their way to the device.
-constexpr int PIN_FLAGS = 4 * JOB_RES, PIN_JOBS = 256;
+// Pinned host words of run_matrix: the jobs' results and after them, as on
+// the device, the input check's flag, the pattern's entry count and the
+// device's pick; then the job records on their way to the device.
+constexpr int PIN_JOBS = 256, RES_TAIL = 3;
+static_assert(4 * JOB_RES + RES_TAIL <= PIN_JOBS, "results before the job records");
 static_assert(4 * sizeof(NMJob) <= 256 * sizeof(int), "four job records fit the pinned words after PIN_JOBS");
 
 // Run `nsched` jobs on one matrix (schedules sched0 .. sched0+nsched-1).
@@ -2281,7 +2257,8 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   const int trace_pairs_cap = trace ? 2 * (M + 1) * M * 4096 : 0;
   const int trace_rounds_cap = trace ? 65536 : 0;
   size_t need = pattern_bytes(R, nnz) + (size_t)nsched * job_bytes(R) + arena_bytes(nsched, sizeof(NMJob)) +
-                arena_bytes(R, sizeof(int)) + 3 * arena_bytes(nnz, sizeof(int)) +
+                arena_bytes(nsched * JOB_RES + RES_TAIL, sizeof(int)) + arena_bytes(R, sizeof(int)) +
+                3 * arena_bytes(nnz, sizeof(int)) +
                 arena_bytes(trace_pairs_cap * 2, sizeof(int)) + arena_bytes(trace_rounds_cap, sizeof(int)) + 4096;
   VNM_TRY(arena_reserve(ctx, need));
   VNM_TRY(pinned_reserve(ctx, 512 + (size_t)trace_pairs_cap * 2 + trace_rounds_cap));
@@ -2298,10 +2275,14 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   Pattern P;
   VNM_TRY(build_pattern(ctx, R, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned, true));
   NMJob hj[4];
+  int* d_res = arena_take<int>(ctx, nsched * JOB_RES + RES_TAIL);  // read back in one copy
+  if (!d_res) return VNM_ERR_NOMEM;
+  int* d_tail = d_res + nsched * JOB_RES;
   for (int s = 0; s < nsched; ++s) {
-    VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s]));
+    VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s], d_res + s * JOB_RES));
     hj[s].err = P.d_err;
   }
+  VNM_TRY(init_jobs(ctx, P, hj, nsched, d_tail));
   int* d_tp = nullptr;
   int* d_tr = nullptr;
   if (trace) {
@@ -2327,23 +2308,20 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, nm_cluster_size(nnz)));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hp = ctx->h_pinned;
-  for (int s = 0; s < nsched; ++s)
-    VNM_CUDA_TRY(cudaMemcpyAsync(hp + JOB_RES * s, hj[s].res, sizeof(int) * JOB_RES, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-  VNM_CUDA_TRY(cudaMemcpyAsync(hp + PIN_FLAGS, P.d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   if (d_newpos) {
-    VNM_LAUNCH(ctx, k_pick_invert, grid_for(ctx, R), 256, 0, d_jobs, nsched, nnz, newpos_job, R, d_newpos,
-               P.d_err + 1);  // the entry count was read back above: its word now takes the pick
-    VNM_CUDA_TRY(cudaMemcpyAsync(hp + PIN_FLAGS + 2, P.d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    VNM_LAUNCH(ctx, k_pick_invert, grid_for(ctx, R), 256, 0, d_jobs, nsched, nnz, newpos_job, R, d_newpos, d_tail + 2);
     VNM_CUDA_TRY(cudaMemcpyAsync(newpos_out, d_newpos, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream));
   }
+  VNM_CUDA_TRY(cudaMemcpyAsync(hp, d_res, sizeof(int) * (nsched * JOB_RES + RES_TAIL), cudaMemcpyDeviceToHost,
+                               ctx->stream));
   VNM_TRY(end_call(ctx));
   VNM_CUDA_TRY(cudaEventElapsedTime(&ctx->main_ms, ctx->ev_main0, ctx->ev_main1));
-  const int flag = hp[PIN_FLAGS];
+  const int* tail = hp + nsched * JOB_RES;
+  const int flag = tail[0];
   if (flag & 2) return VNM_ERR_RANGE;
   if (flag & 1) return VNM_ERR_UNSORTED;
-  P.np = nnz > 0 ? hp[PIN_FLAGS + 1] : 0;
-  const int dev_pick = hp[PIN_FLAGS + 2];
+  P.np = tail[1];
+  const int dev_pick = tail[2];
   int hres_copy[4 * JOB_RES];
   memcpy(hres_copy, hp, sizeof(int) * JOB_RES * nsched);
   for (int q = 0; q < 28; ++q) ctx->stats[q] = 0;
@@ -2740,6 +2718,7 @@ vnm_status vnm_nm_pair_score(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   VNM_TRY(build_pattern(ctx, nrows, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned));
   NMJob J;
   VNM_TRY(make_job(ctx, P, 0, 10, J));
+  VNM_TRY(init_jobs(ctx, P, &J, 1));
   int* d_score = arena_take<int>(ctx, 2 * M * M);
   if (!d_score) return VNM_ERR_NOMEM;
   switch (M) {
@@ -2836,7 +2815,8 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   Pattern P;
   VNM_TRY(build_pattern(&c, nrows, nnz, row, col, val, N, M, P, hs));
   NMJob hj;
-  VNM_TRY(make_job(&c, P, sched, nm_maxiter, hj));  // clears the job's scratch
+  VNM_TRY(make_job(&c, P, sched, nm_maxiter, hj));
+  VNM_TRY(init_jobs(&c, P, &hj, 1));
   NMJob* d_job = arena_take<NMJob>(&c, 1);
   if (!d_job) return VNM_ERR_LIMIT;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_job, &hj, sizeof(NMJob), cudaMemcpyHostToDevice, c.stream));
