@@ -62,3 +62,16 @@ def test_batch_clusters_match_single_runs(ctx, nmat):
     for b, m in enumerate(mats):
         r1, p1 = ctx.nm_reorder(*m, 2, 8, 1)
         assert np.array_equal(res[b], r1) and np.array_equal(pos[b], p1), b
+
+
+# batches that run their largest jobs on wider clusters beside the others: few, the most (18), more
+@pytest.mark.parametrize("large", [1, 6, 18, 20])
+def test_batch_wide_jobs_match_single_runs(ctx, large):
+    rng = np.random.default_rng(large)
+    sizes = [(8 * int(rng.integers(200, 400)), 30000 + 500 * b) for b in range(large)]
+    sizes += [(8 * int(rng.integers(1, 60)), int(rng.integers(1, 3000))) for _ in range(160)]
+    mats = [_matrix(*sizes[b], 1000 * large + int(b)) for b in rng.permutation(len(sizes))]
+    res, pos = ctx.nm_reorder_batch(mats, 2, 8, 0)
+    for b, m in enumerate(mats):
+        r1, p1 = ctx.nm_reorder(*m, 2, 8, 0)
+        assert np.array_equal(res[b], r1) and np.array_equal(pos[b], p1), b

@@ -61,6 +61,8 @@ struct vnm_ctx {
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;                       // second stream of a batch's rounds (run_batch), made on first use
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // between the two
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   cudaEvent_t ev_main0 = nullptr, ev_main1 = nullptr;  // around the call's main kernel
   float last_ms = 0.f;

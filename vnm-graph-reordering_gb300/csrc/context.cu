@@ -247,6 +247,9 @@ vnm_status vnm_destroy(vnm_ctx* c) {
   if (c->ev_stop) cudaEventDestroy(c->ev_stop);
   if (c->ev_main0) cudaEventDestroy(c->ev_main0);
   if (c->ev_main1) cudaEventDestroy(c->ev_main1);
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+  if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->spare) {
     bool last;

@@ -41,6 +41,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <functional>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -2094,8 +2095,8 @@ static RoundShape round_shape(int max_nseg, int max_runs, int cs) {
 static std::mutex g_round_launch_mu;
 
 template <int M>
-static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int max_nseg, int max_runs,
-                                  int cs) {
+static vnm_status launch_rounds_t(vnm_ctx* ctx, cudaStream_t st, const NMJob* d_jobs, int njobs, int N, int max_nseg,
+                                  int max_runs, int cs) {
   std::lock_guard<std::mutex> launch_lock(g_round_launch_mu);
   ctx->last_clusters_fit = 0;
   const int in_smem = (size_t)max_nseg * sizeof(int) <= (64u << 10) ? 1 : 0;
@@ -2113,7 +2114,7 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
     // fits at all.
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(NM_THREADS);
-    cfg.stream = ctx->stream;
+    cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.y = 1;
@@ -2157,7 +2158,9 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, 
   // one block per job (asked for, or no cluster fits)
   const RoundShape f = round_shape<M>(max_nseg, max_runs, 1);
   VNM_CUDA_TRY(set_dyn(f));
-  VNM_LAUNCH(ctx, k_nm_rounds<M>, njobs, NM_THREADS, f.dyn, d_jobs, N, in_smem, f.ts, f.dslots, 1);
+  k_nm_rounds<M><<<njobs, NM_THREADS, f.dyn, st>>>(d_jobs, N, in_smem, f.ts, f.dslots, 1);
+  ctx->launches++;
+  VNM_CUDA_TRY(cudaGetLastError());
   ctx->last_cluster = 1;
   return VNM_OK;
 }
@@ -2179,15 +2182,15 @@ static int nm_cluster_size(long long np) {
 
 // max_runs: aligned runs of 16 rows a job's rows lie in, at most.
 static vnm_status launch_rounds(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int M, int max_nseg, int max_runs,
-                                int cs) {
+                                int cs, cudaStream_t st = nullptr) {
   switch (M) {
-    case 2: return launch_rounds_t<2>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 3: return launch_rounds_t<3>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 4: return launch_rounds_t<4>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 5: return launch_rounds_t<5>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 6: return launch_rounds_t<6>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 7: return launch_rounds_t<7>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 8: return launch_rounds_t<8>(ctx, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 2: return launch_rounds_t<2>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 3: return launch_rounds_t<3>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 4: return launch_rounds_t<4>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 5: return launch_rounds_t<5>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 6: return launch_rounds_t<6>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 7: return launch_rounds_t<7>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 8: return launch_rounds_t<8>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
   }
   return VNM_ERR_ARG;
 }
@@ -2431,6 +2434,51 @@ __global__ void k_batch_invert(const NMJob* jobs, const int* row_off, int* newpo
   for (int i = threadIdx.x; i < J.R; i += blockDim.x) out[J.orig[i]] = i;
 }
 
+// How many of a batch's jobs (entries in descending order) to run on clusters
+// of 4 blocks when the others run on 2.  A job's time goes with its entries
+// (0.135 us each on 2 blocks, R-MAT 2:8) and is about 0.74 of that on 4; the
+// others start in order wherever two SMs come free, and the number with the
+// earliest end is taken, within half of the SMs and where it gains at least 10
+// %.  (256 R-MAT matrices, 256-8192 rows: the largest job alone took all of
+// the batch's 25.2 ms.)
+static int wide_jobs(const std::vector<long long>& sizes, int num_sms) {
+  const int n = (int)sizes.size(), pairs = num_sms / 2;
+  if (n < 2 || pairs < 1) return 0;
+  int best = 0;
+  double best_end = 0;
+  std::vector<double> ends;  // when each pair of SMs comes free: a heap, earliest on top
+  for (int k = 0; k < n && 4 * k <= pairs; k += k < 4 ? 1 : 2) {
+    ends.assign(pairs, 0.0);
+    double end = 0;
+    for (int q = 0; q < k; ++q) {
+      const double t = 0.74 * (double)sizes[q];
+      ends[2 * q] = ends[2 * q + 1] = t;
+      end = std::max(end, t);
+    }
+    std::make_heap(ends.begin(), ends.end(), std::greater<double>());
+    for (int q = k; q < n; ++q) {
+      std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
+      ends.back() += (double)sizes[q];
+      end = std::max(end, ends.back());
+      std::push_heap(ends.begin(), ends.end(), std::greater<double>());
+    }
+    if (k == 0 || end < best_end * (best == 0 ? 0.9 : 1.0)) {
+      best = k;
+      best_end = end;
+    }
+  }
+  return best;
+}
+
+// The context's second stream, made on first use.
+static vnm_status side_stream(vnm_ctx* ctx) {
+  if (ctx->side) return VNM_OK;
+  if (!ctx->ev_fork) VNM_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+  if (!ctx->ev_join) VNM_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+  VNM_CUDA_TRY(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+  return VNM_OK;
+}
+
 static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int64_t* nnz_offset, const int* row,
                             const int* col, const float* val, int N, int M, int sched, int maxiter, int* res5,
                             int* newpos) {
@@ -2499,7 +2547,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   VNM_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(uint4) * (R > 0 ? R : 1), ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(res, 0, sizeof(int) * JOB_RES * nmat, ctx->stream));
   std::vector<NMJob> hj(nmat);
-  int max_nseg = 0, max_runs = 0;
+  int max_nseg = 0;
   for (int b = 0; b < nmat; ++b) {
     NMJob& J = hj[b];
     J.R = nrows[b];
@@ -2525,7 +2573,6 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     J.err = nullptr;
     J.timed = ctx->phase_timing ? 1 : 0;
     if (J.nseg > max_nseg) max_nseg = J.nseg;
-    if (J.R > 0) max_runs = std::max(max_runs, ((row_off[b] + J.R - 1) >> 4) - (row_off[b] >> 4) + 1);
   }
   // The rounds run in the order of the matrices' entries, most first: the
   // batch lasts as long as its largest jobs, which must not start late (256
@@ -2543,15 +2590,39 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   VNM_CUDA_TRY(cudaMemcpyAsync(d_sorted, sj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
   VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, d_soff);
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  // Clusters of 2 blocks per job: the batch's time is its largest matrices'
-  // jobs, and two SMs each shorten them more than the extra waves cost
-  // (88 ms with one block per job, 63 ms with 2, 69 ms with 4, measured on
-  // an earlier form of the kernel).  Clusters of 4 or 8 where all jobs may
-  // still run at once (launch_rounds halves them if they do not): 12 matrices
-  // of 2048-8192 rows 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms,
-  // 12 of 256-512 rows 2.25 ms either way.
+  // Clusters of 4 or 8 blocks per job where all jobs may still run at once
+  // (launch_rounds halves them if they do not): 12 matrices of 2048-8192 rows
+  // 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms, 12 of 256-512 rows
+  // 2.25 ms either way.  Else of 2 (88 ms with one block per job, 63 ms with
+  // 2, 69 ms with 4, measured on an earlier form of the kernel), but of 4 for
+  // the largest jobs if the batch would end with those alone.
+  std::vector<long long> sizes(nmat);
+  for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
   const int cs = nmat * 8 <= ctx->num_sms ? 8 : nmat * 4 <= ctx->num_sms ? 4 : 2;
-  VNM_TRY(launch_rounds(ctx, d_sorted, nmat, N, M, max_nseg, max_runs, cs));
+  const int wide = cs == 2 ? wide_jobs(sizes, ctx->num_sms) : 0;
+  auto rounds = [&](int from, int to, int c, cudaStream_t st) {
+    int nseg = 0, runs = 0;  // the largest of these jobs
+    for (int q = from; q < to; ++q) {
+      const NMJob& J = sj[q];
+      nseg = std::max(nseg, J.nseg);
+      if (J.R > 0) runs = std::max(runs, ((J.row0 + J.R - 1) >> 4) - (J.row0 >> 4) + 1);
+    }
+    return launch_rounds(ctx, d_sorted + from, to - from, N, M, nseg, runs, c, st);
+  };
+  if (wide > 0) {
+    // the wide jobs' launch first, the others' on a second stream beside it;
+    // the streams join again whatever comes of the launches
+    VNM_TRY(side_stream(ctx));
+    VNM_CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->stream));
+    vnm_status s0 = rounds(0, wide, 4, ctx->stream);
+    VNM_CUDA_TRY(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+    vnm_status s1 = s0 == VNM_OK ? rounds(wide, nmat, 2, ctx->side) : s0;
+    VNM_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->side));
+    VNM_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+    VNM_TRY(s1);
+  } else {
+    VNM_TRY(rounds(0, nmat, cs, ctx->stream));
+  }
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hres = ctx->h_pinned + 256;
   VNM_CUDA_TRY(cudaMemcpyAsync(hres, res, sizeof(int) * JOB_RES * nmat, cudaMemcpyDeviceToHost, ctx->stream));
