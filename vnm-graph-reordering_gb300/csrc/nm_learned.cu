@@ -68,7 +68,7 @@ __global__ void k_l_build_G(const int* row, const int* col, const float* val, in
 
 // hist / cnt of a segment from its columns' histograms: a group of k bits is
 // counted by each of its k columns.  (Counting runs of the sorted pattern with
-// atomics took 44 us at 65536 rows, 2 M entries; this takes 5.)
+// atomics took 44 us at 65536 rows, 2 M entries; this takes 7.)
 __global__ void k_l_seg_hist(LMat L) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < L.nseg; s += gridDim.x * blockDim.x) {
     int h[9], t = 0, c = 0;

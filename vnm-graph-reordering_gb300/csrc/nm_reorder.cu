@@ -107,6 +107,7 @@ struct NMJob {
   const int* cptr;    // [R+1] column pointers of the nonzero pattern (original ids)
   const int* crow;    // rows of each column, grouped by row_group
   const int* csplit;  // [16 R + 1] start of each (column, row group) in crow
+  int2* runs;         // [cs][R] scratch: each block's entries {start in crow, count} of the column at a position
   int* orig;          // [R] original node at each position (identity on entry)
   int* cnt;           // [nseg] invalid rows per segment
   int* zc;            // [nseg] all-zero rows per segment
@@ -292,6 +293,7 @@ struct RoundSmem {
   static constexpr int SCR_U4 = ((PROC_BYTES > HEAP_BYTES ? PROC_BYTES : HEAP_BYTES) + 15) / 16;
   uint8_t ord[MM][HSTR];       // pop order: ord[k][a * K + b] is the k-th pop of ordered pair (a, b)
   int colstart[K * M];
+  int onode[K * M];            // leader: the round's columns' nodes
   int colpre[K * M + 1];
   static constexpr int DEST_W = (K * M + 3) / 4;  // dest in 32-bit words
   union {
@@ -614,6 +616,21 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
 // the run of 16 rows that a range not starting at a multiple of 16 adds).
 constexpr int DIRECT_MAX = 4352;
 
+// The block's run of every column, by position, at the identity arrangement.
+// A round's swaps move runs that the block has at hand then (apply_recount),
+// so a round reads a column's run in one step where position -> node -> run
+// were two dependent L2 round trips (the gather of R-MAT 16384 2:4, schedule 0:
+// 3.1 -> 2.9 us; of 65536 2:8 9.5 -> 8.7; of 512 rows 3.1 -> 2.4).
+__device__ void fill_runs(const NMJob& J, Slice sl) {
+  const int g0 = sl.rank * (ROW_GROUPS / sl.cs), g1 = g0 + ROW_GROUPS / sl.cs;
+  int2* runs = J.runs + (size_t)sl.rank * J.R;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < J.R; c += NM_THREADS) {
+    const int b = J.csplit[(size_t)ROW_GROUPS * c + g0];
+    runs[c] = make_int2(b, J.csplit[(size_t)ROW_GROUPS * c + g1] - b);
+  }
+}
+
 // OR the bitmaps of the round's segments into the records of the rows this
 // block owns.  Every column's rows are stored grouped by row_group (csplit),
 // so the block's entries of a column are one contiguous run of it, and no
@@ -627,7 +644,7 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
   constexpr int K = M + 1;
   const int tid = threadIdx.x;
   const int KM = sm.K_ * M;
-  const int g0 = sl.rank * (ROW_GROUPS / sl.cs), g1 = g0 + ROW_GROUPS / sl.cs;
+  const int g0 = sl.rank * (ROW_GROUPS / sl.cs);
   if (tid < 32) {  // this block's run of each column of the round and their prefix sums, on one warp
     constexpr int CPL = (K * M + 31) / 32;  // columns per lane
     int len[CPL], tot = 0;
@@ -636,10 +653,9 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
       const int col = tid * CPL + q;
       len[q] = 0;
       if (col < KM) {
-        const int u = J.orig[sm.xseg[col / M] * M + col % M];
-        const int b = J.csplit[(size_t)ROW_GROUPS * u + g0];
-        sm.colstart[col] = b;
-        len[q] = J.csplit[(size_t)ROW_GROUPS * u + g1] - b;
+        const int2 run = J.runs[(size_t)sl.rank * J.R + sm.xseg[col / M] * M + col % M];
+        sm.colstart[col] = run.x;
+        len[q] = run.y;
       }
       tot += len[q];
     }
@@ -662,6 +678,9 @@ __device__ void gather_phase(RoundSmem<M>& sm, const NMJob& J, Slice sl = Slice{
       sm.use_table = sm.dslots > 0 || (sm.ts_max > 0 && incl <= (sm.ts_max >> 2) * 3);
     }
   }
+  // (the leader's nodes of the columns, for the swaps: on threads that would wait here)
+  if (sl.rank == 0 && tid >= 32 && tid < 32 + KM)
+    sm.onode[tid - 32] = J.orig[sm.xseg[(tid - 32) / M] * M + (tid - 32) % M];
   __syncthreads();
   const int E = sm.E;
   if (sm.dslots > 0) {
@@ -1469,20 +1488,12 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
   }
 }
 
-// Apply the swaps to orig[] (the leader block) and recount this block's
-// slice of the touched rows into newinv / newpres.
+// Apply the swaps to orig[] (the leader block) and the block's runs, and recount
+// this block's slice of the touched rows into newinv / newpres.
 template <int M>
 __device__ void apply_recount(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl) {
   constexpr int K = M + 1;
   const int tid = threadIdx.x;
-  // a round's swaps are disjoint transpositions (the walk never reuses a
-  // visited position), so each thread applies one of them
-  if (sl.rank == 0 && tid < sm.nswaps) {
-    const int v1 = sm.swaps[2 * tid], v2 = sm.swaps[2 * tid + 1];
-    const int o1 = J.orig[v1], o2 = J.orig[v2];
-    J.orig[v1] = o2;
-    J.orig[v2] = o1;
-  }
   // A swap moves whole columns of bits, so the rows' groups afterwards are
   // the same column masks in other places: a thread takes a segment and a
   // chunk, reads the masks of the columns it now holds, and counts the rows
@@ -1496,8 +1507,13 @@ __device__ void apply_recount(RoundSmem<M>& sm, const NMJob& J, int N, Slice sl)
   const int n = sm.use_table ? sm.tcount : sm.ntouched;
   const int nchunks = (n + 31) / 32;
   if (tid < Kn * M) {
-    const int d = sm.dest[tid / M][tid % M];
-    sm.from[(d >> 4) * M + (d & 15)] = (uint8_t)tid;
+    const int d = sm.dest[tid / M][tid % M], to = (d >> 4) * M + (d & 15);
+    sm.from[to] = (uint8_t)tid;
+    if (to != tid) {  // the column moves: its node and the block's run of it
+      const int pos = sm.xseg[d >> 4] * M + (d & 15);
+      if (sl.rank == 0) J.orig[pos] = sm.onode[tid];
+      J.runs[(size_t)sl.rank * J.R + pos] = make_int2(sm.colstart[tid], sm.colpre[tid + 1] - sm.colpre[tid]);
+    }
   }
   const bool tmain = threadIdx.x == 0 && sl.rank == 0 && J.timed;
   const unsigned long long t_in = tmain ? global_ns() : 0ull;
@@ -1710,6 +1726,7 @@ __global__ void __launch_bounds__(NM_THREADS, 1) k_nm_rounds(const NMJob* __rest
     sm.go = 0;
   }
   clear_round_smem<M>(sm);
+  fill_runs(J, sl);
   __syncthreads();
   if (lead) select_phase<M>(sm, J, cnt);
   const int init_size = sm.lsize, init_cnt = sm.ltotal;
@@ -1910,6 +1927,7 @@ __global__ void __launch_bounds__(NM_THREADS) k_pair_score(NMJob J, int N, int s
       sm.K_ = 2;
     }
   }
+  fill_runs(J, Slice{0, 1});
   __syncthreads();
   gather_phase<M>(sm, J);
   process_phase<M>(sm, J, N);
@@ -2000,13 +2018,14 @@ vnm_status build_pattern(vnm_ctx* ctx, int R, int nnz, const int* d_row, const i
 
 size_t job_bytes(int R) {
   const int nseg = R / 2 + 1;
-  return arena_bytes(R, sizeof(int)) + 2 * arena_bytes(nseg, sizeof(int)) + arena_bytes(R, sizeof(uint4)) +
+  return arena_bytes((size_t)ROW_GROUPS * R, sizeof(int2)) + arena_bytes(R, sizeof(int)) +
+         2 * arena_bytes(nseg, sizeof(int)) + arena_bytes(R, sizeof(uint4)) +
          arena_bytes((size_t)R + 2 * ROW_GROUPS, sizeof(int)) + arena_bytes(JOB_RES, sizeof(int));
 }
 
-// Carve one job's state out of the arena (its results at `res`, if given);
-// init_jobs sets it up.
-static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J, int* res = nullptr) {
+// Carve one job's state out of the arena, for clusters of up to cs blocks (its
+// results at `res`, if given); init_jobs sets it up.
+static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J, int cs, int* res = nullptr) {
   J.R = P.R;
   J.row0 = 0;
   J.nseg = P.nseg;
@@ -2015,6 +2034,7 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   J.cptr = P.cptr;
   J.crow = P.crow;
   J.csplit = P.csplit;
+  J.runs = arena_take<int2>(ctx, (size_t)cs * (P.R > 0 ? P.R : 1));
   J.orig = arena_take<int>(ctx, P.R > 0 ? P.R : 1);
   J.cnt = arena_take<int>(ctx, P.nseg + 1);
   J.zc = arena_take<int>(ctx, P.nseg + 1);
@@ -2038,7 +2058,7 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
     if (v > 0 && v < WALK_WAIT_LIMIT) J.walk_wait_limit = v;
   }
   if (const char* e = getenv("VNM_NM_TEST_HOLD_HEAPS")) J.hold_heaps = atoi(e) == 1 ? 1 : 0;
-  if (!J.orig || !J.cnt || !J.zc || !J.rec || !J.touched || !J.res) return VNM_ERR_NOMEM;
+  if (!J.runs || !J.orig || !J.cnt || !J.zc || !J.rec || !J.touched || !J.res) return VNM_ERR_NOMEM;
   return VNM_OK;
 }
 
@@ -2281,8 +2301,11 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   int* d_res = arena_take<int>(ctx, nsched * JOB_RES + RES_TAIL);  // read back in one copy
   if (!d_res) return VNM_ERR_NOMEM;
   int* d_tail = d_res + nsched * JOB_RES;
+  // the stored entries stand in for the pattern's (nonzero-valued) entries
+  // when sizing the clusters: their count is known without a readback
+  const int cs = nm_cluster_size(nnz);
   for (int s = 0; s < nsched; ++s) {
-    VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s], d_res + s * JOB_RES));
+    VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s], cs, d_res + s * JOB_RES));
     hj[s].err = P.d_err;
   }
   VNM_TRY(init_jobs(ctx, P, hj, nsched, d_tail));
@@ -2306,9 +2329,7 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   memcpy(pj, hj, sizeof(NMJob) * nsched);
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, pj, sizeof(NMJob) * nsched, cudaMemcpyHostToDevice, ctx->stream));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  // the stored entries stand in for the pattern's (nonzero-valued) entries
-  // when sizing the clusters: their count is known without a readback
-  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, nm_cluster_size(nnz)));
+  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, cs));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hp = ctx->h_pinned;
   if (d_newpos) {
@@ -2479,6 +2500,8 @@ static vnm_status side_stream(vnm_ctx* ctx) {
   return VNM_OK;
 }
 
+constexpr int BATCH_CS = 8;  // blocks of a batch job's cluster, at most
+
 static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int64_t* nnz_offset, const int* row,
                             const int* col, const float* val, int N, int M, int sched, int maxiter, int* res5,
                             int* newpos) {
@@ -2501,6 +2524,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   size_t need = pattern_bytes(R, n) + 5 * arena_bytes(n, sizeof(int)) + arena_bytes(nmat + 1, 8) +
                 3 * arena_bytes(nmat + 1, sizeof(int)) + 2 * arena_bytes(nmat, sizeof(NMJob)) +
                 arena_bytes(R, sizeof(int)) + arena_bytes((size_t)R + (size_t)2 * ROW_GROUPS * nmat, sizeof(int)) +
+                arena_bytes((size_t)BATCH_CS * R, sizeof(int2)) +
                 arena_bytes(R, sizeof(uint4)) + 2 * arena_bytes(R / M + nmat, sizeof(int)) +
                 arena_bytes((size_t)JOB_RES * nmat, sizeof(int)) + arena_bytes(R, sizeof(int)) + 8192;
   VNM_TRY(arena_reserve(ctx, need));
@@ -2536,6 +2560,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   Pattern P;
   VNM_TRY(build_pattern(ctx, R, n, grow, gcol, d_val, N, M, P, ctx->h_pinned));
   // per-job state, one allocation per field for the whole batch
+  int2* runs = arena_take<int2>(ctx, (size_t)BATCH_CS * (R > 0 ? R : 1));
   int* orig = arena_take<int>(ctx, R > 0 ? R : 1);
   int* touched = arena_take<int>(ctx, (size_t)R + (size_t)2 * ROW_GROUPS * nmat);  // 32 of slack per job
   uint4* rec = arena_take<uint4>(ctx, R > 0 ? R : 1);
@@ -2543,7 +2568,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   int* zc = arena_take<int>(ctx, R / M + nmat);
   int* res = arena_take<int>(ctx, (size_t)JOB_RES * nmat);
   NMJob* d_jobs = arena_take<NMJob>(ctx, nmat);
-  if (!orig || !touched || !rec || !cnt || !zc || !res || !d_jobs) return VNM_ERR_NOMEM;
+  if (!runs || !orig || !touched || !rec || !cnt || !zc || !res || !d_jobs) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(uint4) * (R > 0 ? R : 1), ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(res, 0, sizeof(int) * JOB_RES * nmat, ctx->stream));
   std::vector<NMJob> hj(nmat);
@@ -2558,6 +2583,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     J.cptr = P.cptr + row_off[b];
     J.crow = P.crow;
     J.csplit = P.csplit + (size_t)ROW_GROUPS * row_off[b];
+    J.runs = runs + (size_t)BATCH_CS * row_off[b];
     J.orig = orig + row_off[b];
     J.cnt = cnt + seg_off[b] + b;
     J.zc = zc + seg_off[b] + b;
@@ -2598,7 +2624,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   // the largest jobs if the batch would end with those alone.
   std::vector<long long> sizes(nmat);
   for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
-  const int cs = nmat * 8 <= ctx->num_sms ? 8 : nmat * 4 <= ctx->num_sms ? 4 : 2;
+  const int cs = nmat * BATCH_CS <= ctx->num_sms ? BATCH_CS : nmat * 4 <= ctx->num_sms ? 4 : 2;
   const int wide = cs == 2 ? wide_jobs(sizes, ctx->num_sms) : 0;
   auto rounds = [&](int from, int to, int c, cudaStream_t st) {
     int nseg = 0, runs = 0;  // the largest of these jobs
@@ -2788,7 +2814,7 @@ vnm_status vnm_nm_pair_score(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   Pattern P;
   VNM_TRY(build_pattern(ctx, nrows, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned));
   NMJob J;
-  VNM_TRY(make_job(ctx, P, 0, 10, J));
+  VNM_TRY(make_job(ctx, P, 0, 10, J, 1));
   VNM_TRY(init_jobs(ctx, P, &J, 1));
   int* d_score = arena_take<int>(ctx, 2 * M * M);
   if (!d_score) return VNM_ERR_NOMEM;
@@ -2886,14 +2912,15 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   Pattern P;
   VNM_TRY(build_pattern(&c, nrows, nnz, row, col, val, N, M, P, hs));
   NMJob hj;
-  VNM_TRY(make_job(&c, P, sched, nm_maxiter, hj));
+  const int cs = nm_cluster_size(P.np);
+  VNM_TRY(make_job(&c, P, sched, nm_maxiter, hj, cs));
   VNM_TRY(init_jobs(&c, P, &hj, 1));
   NMJob* d_job = arena_take<NMJob>(&c, 1);
   if (!d_job) return VNM_ERR_LIMIT;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_job, &hj, sizeof(NMJob), cudaMemcpyHostToDevice, c.stream));
   // the same launch shape as vnm_nm_reorder (a cluster of blocks per job);
   // the scratch it needs does not depend on the cluster size
-  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, nm_cluster_size(P.np)));
+  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, cs));
   VNM_CUDA_TRY(cudaMemcpyAsync(hs, hj.res, sizeof(int) * 16, cudaMemcpyDeviceToHost, c.stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(c.stream));
   if (hs[5] != 0) return VNM_ERR_INTERNAL;
