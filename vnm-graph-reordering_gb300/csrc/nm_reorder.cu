@@ -46,6 +46,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "common.cuh"
@@ -2836,7 +2837,11 @@ vnm_status vnm_nm_pair_score(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
 vnm_status vnm_nm_reorder_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int64_t* nnz_offset,
                                 const int* row, const int* col, const float* val, int N, int M, int sched,
                                 int nm_maxiter, int* res5, int* newpos) {
-  return run_batch(ctx, nmat, nrows, nnz_offset, row, col, val, N, M, sched, nm_maxiter, res5, newpos);
+  try {
+    return run_batch(ctx, nmat, nrows, nnz_offset, row, col, val, N, M, sched, nm_maxiter, res5, newpos);
+  } catch (const std::bad_alloc&) {  // of the host's lists, all made before the launches
+    return VNM_ERR_NOMEM;
+  }
 }
 
 }  // extern "C"
