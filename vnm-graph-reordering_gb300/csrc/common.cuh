@@ -53,6 +53,7 @@ struct vnm_spmm_spare {
   int device = 0;
   void* ptr = nullptr;
   size_t bytes = 0;
+  bool pending = false;  // asynchronous products of the freed operand may still use it
   int refs = 1;  // the context and its live operands
   bool ctx_alive = true;
 };

@@ -90,6 +90,7 @@ struct vnm_spmm_matrix {
   size_t part_floats = 0;
   bool part_own = false;       // an allocation of its own (the first PART_COLS columns' worth lies in `base`)
   int* err = nullptr;          // sticky failure flag of the tensor-core kernel
+  bool pending = false;        // products were enqueued on a caller's stream, which nothing here waits for
 };
 
 namespace vnm {
@@ -1212,11 +1213,13 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   const size_t need = b_pt + b_ts + b_cols + b_a + b_sc + b_rc + b_tk + b_mu + b_err + b_part;
   void* base = nullptr;
   size_t have = 0;
+  bool pending = false;
   if (ctx->spare) {  // a freed operand's storage, when large enough
     std::lock_guard<std::mutex> g(ctx->spare->m);
     if (ctx->spare->ptr && ctx->spare->bytes >= need) {
       base = ctx->spare->ptr;
       have = ctx->spare->bytes;
+      pending = ctx->spare->pending;
       ctx->spare->ptr = nullptr;
       ctx->spare->bytes = 0;
     }
@@ -1227,6 +1230,11 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   }
   out->base = base;
   out->bytes = have;
+  // The freed operand's asynchronous products run on its caller's streams,
+  // possibly from a captured graph, and read and write this storage: they end
+  // before anything is written to it.  (The wait is here and not in the free,
+  // which a training loop calls beside its running products.)
+  if (pending) VNM_CUDA_TRY(cudaDeviceSynchronize());
   char* pb = static_cast<char*>(base);
   size_t o = 0;
   out->part_list = reinterpret_cast<int4*>(pb + o);
@@ -1368,6 +1376,7 @@ vnm_status vnm_spmm_free(vnm_spmm_matrix* A) {
       if (A->spare->ptr) cudaFree(A->spare->ptr);
       A->spare->ptr = A->base;
       A->spare->bytes = A->bytes;
+      A->spare->pending = A->pending;
       A->base = nullptr;
     }
     last = --A->spare->refs == 0;
@@ -1521,6 +1530,7 @@ vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, i
   ctx->last_ms = ctx->main_ms = 0.f;
   cudaStream_t own = ctx->stream;
   ctx->stream = static_cast<cudaStream_t>(stream);
+  A->pending = true;
   const vnm_status st = spmm_enqueue(ctx, A, B, n, C, A->part, A->err, false);
   ctx->stream = own;
   return st;
