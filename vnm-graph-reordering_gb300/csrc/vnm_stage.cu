@@ -919,12 +919,23 @@ static vnm_status vnm_rows_analyse(vnm_ctx* ctx, VnmRows& W, const int* comp, in
   return VNM_OK;
 }
 
+static size_t vo_smem(int cap) { return sizeof(OrderSmem) + (size_t)2 * cap * sizeof(unsigned long long); }
+
 // Launch shape of k_vs_order for m rows: a block for each 1024 rows (1, 2, 4,
 // 8 or 16, then more rows a block), fewer blocks where the GPU cannot hold
 // the cluster; false when the rows do not fit any it can hold.
 static bool vnm_order_shape(vnm_ctx* ctx, int m, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int& cap) {
   int nct = 1;
   while (nct < VO_MAX_CTAS && nct * VO_THREADS < m) nct *= 2;
+  // The kernel's ceilings belong to the function, which every host thread
+  // shares: always the largest shape's, so that no call lowers another's
+  // between its launches.
+  if (cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vo_smem(VO_MAX_CAP)) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
   cfg = cudaLaunchConfig_t{};
   cfg.blockDim = dim3(VO_THREADS);
   cfg.stream = ctx->stream;
@@ -938,15 +949,10 @@ static bool vnm_order_shape(vnm_ctx* ctx, int m, cudaLaunchConfig_t& cfg, cudaLa
     while (nct * cap < m) cap *= 2;
     if (cap > VO_MAX_CAP) break;
     cfg.gridDim = dim3(nct);
-    cfg.dynamicSmemBytes = sizeof(OrderSmem) + (size_t)2 * cap * sizeof(unsigned long long);
+    cfg.dynamicSmemBytes = vo_smem(cap);
     attr[0].val.clusterDim.x = (unsigned)nct;
     int fit = 0;
-    if (cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
-            cudaSuccess &&
-        (nct <= 8 || cudaFuncSetAttribute(k_vs_order, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                         cudaSuccess) &&
-        cudaOccupancyMaxActiveClusters(&fit, k_vs_order, &cfg) == cudaSuccess && fit >= 1)
-      return true;
+    if (cudaOccupancyMaxActiveClusters(&fit, k_vs_order, &cfg) == cudaSuccess && fit >= 1) return true;
     (void)cudaGetLastError();
   }
   return false;
