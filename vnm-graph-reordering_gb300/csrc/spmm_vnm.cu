@@ -55,6 +55,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -692,15 +693,14 @@ __device__ __forceinline__ void res_step(unsigned long long (&acc)[4], const int
 }
 
 template <int LW, bool BF16>
-__global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS_PER_SM)
-    k_spmm_res(const int4* __restrict__ task, int ntask, const int2* __restrict__ rcv,
-               const unsigned char* __restrict__ B, unsigned ldb, float* __restrict__ C, int ldc,
-               float* __restrict__ P, int ldp) {
+__device__ __forceinline__ void res_tasks(const int4* __restrict__ task, int ntask, const int2* __restrict__ rcv,
+                                          const unsigned char* __restrict__ B, unsigned ldb, float* __restrict__ C,
+                                          int ldc, float* __restrict__ P, int ldp, int col0,
+                                          int2 (*recs)[2][32]) {
   constexpr int G = 32 / LW;
-  __shared__ __align__(16) int2 recs[RES_THREADS / 32][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / LW, lid = lane % LW;
   const int stride = gridDim.x * (RES_THREADS / 32);
-  const int cb = blockIdx.y * (8 * LW) + lid * 8;  // this lane's first column
+  const int cb = col0 + lid * 8;  // this lane's first column
   const unsigned char* bcol = B + (size_t)cb * 2;
   int t = blockIdx.x * (RES_THREADS / 32) + warp, par = 0;
   if (t >= ntask) return;
@@ -746,6 +746,28 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS_PER_SM)
     tkn = tk2;
     rc = rc1;
   }
+}
+
+// The column blocks of a product's C: 256 columns each, then one of 128 and one
+// of 64 where they are left.  All in one launch: the blocks of the next
+// width start where the ones before leave the SMs, and a small operand's
+// widths run beside one another.  (A launch a width put their times end to
+// end: 4096 rows, 64 K records, n = 192 / 320 / 448: 40 / 51 / 71 us, 25 / 34 / 35 now.)
+static inline int col_blocks(int n) { return n / 256 + (n % 256) / 128 + (n % 128) / 64; }
+
+template <bool BF16>
+__global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS_PER_SM)
+    k_spmm_res(const int4* __restrict__ task, int ntask, const int2* __restrict__ rcv,
+               const unsigned char* __restrict__ B, unsigned ldb, float* __restrict__ C, int ldc,
+               float* __restrict__ P, int ldp) {
+  __shared__ __align__(16) int2 recs[RES_THREADS / 32][2][32];
+  const int col0 = blockIdx.y * 256, left = ldc - col0;  // (ldc: the columns of C)
+  if (left >= 256)
+    res_tasks<32, BF16>(task, ntask, rcv, B, ldb, C, ldc, P, ldp, col0, recs);
+  else if (left >= 128)
+    res_tasks<16, BF16>(task, ntask, rcv, B, ldb, C, ldc, P, ldp, col0, recs);
+  else  // the last 64 columns
+    res_tasks<8, BF16>(task, ntask, rcv, B, ldb, C, ldc, P, ldp, ldc - 64, recs);
 }
 
 // C row of a split row = the sum of its partial rows in a fixed order: a
@@ -831,8 +853,8 @@ struct SpmmArgs {
   float* C;
   float* P;                // partial tiles of 128 rows, row stride ldc
   int R, n, ldc;
-  int col0;                // first column of the launch
-  uint32_t idesc;
+  int n256, n128;          // column blocks of 256 and of 128 columns; the others have 64
+  uint32_t idesc[3];       // of 64, 128 and 256 columns
   int* err;
   uint32_t wait_limit;  // polls of a pipeline wait (copies <-> MMAs) before it gives up
 };
@@ -868,11 +890,9 @@ struct SpmmSmem {
 // stay in uniform registers (on one lane of a divergent branch an MMA took 85
 // cycles to issue).
 template <int NT, int KS, int ST>
-__global__ void __launch_bounds__(SP_THREADS, 1)
-    k_spmm_vnm(SpmmArgs p) {
+__device__ __forceinline__ void spmm_item(const SpmmArgs& p, int n0, unsigned char* sp_raw) {
   static_assert(SP_THREADS == 32 * (SP_PW + 1), "the producer warps and the issuing warp");
   constexpr int WR = KS * 16 / SP_PW;  // a stage's B rows a producer warp
-  extern __shared__ unsigned char sp_raw[];
   using Smem = SpmmSmem<NT, KS, ST>;
   Smem& sm = *reinterpret_cast<Smem*>(
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sp_raw) + 1023) & ~uintptr_t(1023)));
@@ -880,7 +900,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   const int4 item = p.part[blockIdx.x];
   const int t = item.x >> 1;
   const bool add = item.x & 1;  // the residual kernel wrote these rows first
-  const int n0 = p.col0 + blockIdx.y * NT;
+  const uint32_t idesc = p.idesc[NT >> 7];  // (made here it cost 0.3 of 18 us: 4096 rows, V = 64, n = 128)
   const int s0 = item.y, nsteps = item.z - item.y;
   const int nst = (nsteps + KS - 1) / KS;  // stage fills
   ptx::grid_dependents_launch();
@@ -998,7 +1018,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
         for (int k = 0; k < KS; ++k)
           if (k < ks)
             ptx::mma_f16(tmem, adesc + (uint64_t)(k * (SP_KSTEP_BYTES >> 4)),
-                         bdesc + (uint64_t)(k * (Smem::B_BYTES >> 4)), p.idesc, (i | k) > 0 ? 1u : 0u);
+                         bdesc + (uint64_t)(k * (Smem::B_BYTES >> 4)), idesc, (i | k) > 0 ? 1u : 0u);
         ptx::mma_commit(&sm.empty[s]);
       }
     }
@@ -1065,6 +1085,21 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 0) ptx::tmem_dealloc(tmem, NT);
+}
+
+// Stages of each width: 192 KB of copies in flight.
+using SpmmSmem256 = SpmmSmem<256, 4, 4>;
+using SpmmSmem128 = SpmmSmem<128, 8, 3>;
+using SpmmSmem64 = SpmmSmem<64, 8, 4>;
+// W: the width of all column blocks, or 0 for several (a product of 2048 rows,
+// V:2:8, n = 64 takes 7.0 us, with the width chosen in the kernel 7.2).
+template <int W>
+__global__ void __launch_bounds__(SP_THREADS, 1) k_spmm_vnm(const __grid_constant__ SpmmArgs p) {
+  extern __shared__ unsigned char sp_raw[];
+  const int y = blockIdx.y, y128 = W == 256 ? -1 : W ? y : y - p.n256, y64 = W == 128 ? -1 : W ? y : y128 - p.n128;
+  if (y128 < 0) spmm_item<256, 4, 4>(p, 256 * y, sp_raw);
+  else if (y64 < 0) spmm_item<128, 8, 3>(p, W ? 128 * y : 256 * p.n256 + 128 * y128, sp_raw);
+  else spmm_item<64, 8, 4>(p, W ? 64 * y : 256 * p.n256 + 128 * p.n128 + 64 * y64, sp_raw);
 }
 
 // Rows of a split tile: the sum of its parts in order, scaled, added to what
@@ -1292,19 +1327,23 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   return VNM_OK;
 }
 
-template <int NT, int KS, int ST>
-static vnm_status launch_spmm(vnm_ctx* ctx, const vnm_spmm_matrix* A, SpmmArgs& p, int col0, int blocks) {
-  // enough shared memory that at most 512 / NT CTAs share an SM: their NT
-  // column accumulators then fit the SM's 512 tensor-memory columns, so an
-  // allocation never waits for another CTA (228 KB of shared memory per SM)
-  constexpr size_t floor_bytes = (228u << 10) / (512 / NT + 1) + 1024;
-  size_t smem = sizeof(SpmmSmem<NT, KS, ST>) + 1024;
-  if (smem < floor_bytes) smem = floor_bytes;
-  p.col0 = col0;
-  dim3 grid(A->npart, blocks);
-  VNM_CUDA_TRY(cudaFuncSetAttribute(k_spmm_vnm<NT, KS, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  p.idesc = ptx::idesc_f16(A->dtype == 1 ? 1u : 0u, 0u, 1u, SP_TM, NT);
-  VNM_LAUNCH(ctx, (k_spmm_vnm<NT, KS, ST>), grid, SP_THREADS, smem, p);
+// One launch for all column blocks (n256 of 256 columns, n128 of 128, n64 of
+// 64): for the same reason as the residual kernel's, and so that no width
+// waits for another's last tiles.
+static vnm_status launch_spmm(vnm_ctx* ctx, const vnm_spmm_matrix* A, SpmmArgs& p, int n256, int n128, int n64) {
+  constexpr size_t smem =
+      std::max({sizeof(SpmmSmem256), sizeof(SpmmSmem128), sizeof(SpmmSmem64)}) + 1024;
+  // one CTA an SM: its accumulator's tensor-memory columns are always free
+  static_assert(2 * smem > (228u << 10), "an allocation never waits for another CTA");
+  p.n256 = n256;
+  p.n128 = n128;
+  for (int k = 0; k < 3; ++k) p.idesc[k] = ptx::idesc_f16(A->dtype == 1 ? 1u : 0u, 0u, 1u, SP_TM, 64u << k);
+  const auto kernel = n128 + n64 == 0    ? k_spmm_vnm<256>
+                      : n256 + n64 == 0  ? k_spmm_vnm<128>
+                      : n256 + n128 == 0 ? k_spmm_vnm<64>
+                                         : k_spmm_vnm<0>;
+  VNM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  VNM_LAUNCH(ctx, kernel, dim3(A->npart, n256 + n128 + n64), SP_THREADS, smem, p);
   return VNM_OK;
 }
 
@@ -1405,41 +1444,27 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
   p.ldc = n;
   p.err = err;
   p.wait_limit = spmm_wait_limit();
-  // the CUDA-core part: 8 columns a lane, in blocks of 256 columns, then 128
-  // and 64 where they are left
+  // the CUDA-core part: 8 columns a lane
   auto launch_res = [&]() -> vnm_status {
     if (A->ntask > 0) {
       // one wave of resident blocks (the task list is walked with a stride)
       const int per_block = RES_THREADS / 32;
       int bx = (A->ntask + per_block - 1) / per_block;
       if (bx > ctx->num_sms * RES_BLOCKS_PER_SM) bx = ctx->num_sms * RES_BLOCKS_PER_SM;
-      int col = 0;
-#define VNM_RES(LWV, COUNT)                                                                                          \
-  do {                                                                                                               \
-    const int count_ = (COUNT);                                                                                      \
-    if (count_ > 0) {                                                                                                \
-      const dim3 grid((unsigned)bx, (unsigned)count_);                                                               \
-      if (A->dtype == 1)                                                                                             \
-        VNM_LAUNCH(ctx, (k_spmm_res<LWV, true>), grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B + 2 * col,     \
-                   (unsigned)p.ldb, dC + col, n, P + col, n);                                                        \
-      else                                                                                                           \
-        VNM_LAUNCH(ctx, (k_spmm_res<LWV, false>), grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B + 2 * col,    \
-                   (unsigned)p.ldb, dC + col, n, P + col, n);                                                        \
-      col += count_ * 8 * LWV;                                                                                       \
-    }                                                                                                                \
-  } while (0)
-      VNM_RES(32, n / 256);
-      VNM_RES(16, (n % 256) / 128);
-      VNM_RES(8, (n % 128) / 64);
-#undef VNM_RES
+      const dim3 grid((unsigned)bx, (unsigned)col_blocks(n));
+      if (A->dtype == 1)
+        VNM_LAUNCH(ctx, k_spmm_res<true>, grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B, (unsigned)p.ldb, dC, n,
+                   P, n);
+      else
+        VNM_LAUNCH(ctx, k_spmm_res<false>, grid, RES_THREADS, 0, A->task, A->ntask, A->rcv, p.B, (unsigned)p.ldb, dC, n,
+                   P, n);
     }
     if (A->nmulti > 0)
       VNM_LAUNCH(ctx, k_spmm_fin, dim3(A->nmulti, n / (4 * FIN_COLS)), FIN_THREADS, 0, A->multi, P, n, dC, n);
     return VNM_OK;
   };
-  // Column blocks of 256, then one of 128 and one of 64 where they are left:
-  // the operand is read once a block (n = 192 as 128 + 64 instead of three
-  // times 64).  VNM_SPMM_WIDTH (64, 128 or 256) in the environment fixes the
+  // The operand is read once a column block: n = 192 as 128 + 64 instead of
+  // three times 64.  VNM_SPMM_WIDTH (64, 128 or 256) in the environment fixes the
   // tensor kernel's width where it divides n.
   int fixed = 0;
   if (const char* e = getenv("VNM_SPMM_WIDTH")) {
@@ -1451,9 +1476,7 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
     const int n256 = fixed == 256 ? n / 256 : fixed ? 0 : n / 256;
     const int n128 = fixed == 128 ? n / 128 : fixed ? 0 : (n % 256) / 128;
     const int n64 = fixed == 64 ? n / 64 : fixed ? 0 : (n % 128) / 64;
-    if (n256) VNM_TRY((launch_spmm<256, 4, 4>(ctx, A, p, 0, n256)));
-    if (n128) VNM_TRY((launch_spmm<128, 8, 3>(ctx, A, p, n256 * 256, n128)));
-    if (n64) VNM_TRY((launch_spmm<64, 8, 4>(ctx, A, p, n256 * 256 + n128 * 128, n64)));
+    VNM_TRY(launch_spmm(ctx, A, p, n256, n128, n64));
     if (A->ntsplit == 0) return VNM_OK;
     cudaLaunchAttribute attr[1];  // set up while the parts are made
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
