@@ -1561,11 +1561,13 @@ vnm_status vnm_spmm_run_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* B, i
 
 vnm_status vnm_spmm_run_cast_async(vnm_ctx* ctx, vnm_spmm_matrix* A, const void* X, int xtype, long long ldx, int F,
                                    void* B, int n, float* C, void* stream) {
-  if (!ctx || !A || !X || !B || xtype < 0 || xtype > 2 || F <= 0 || ldx < F || n < F || (n % 64) != 0)
+  if (!ctx || !A || !X || !B || !C || xtype < 0 || xtype > 2 || F <= 0 || ldx < F || n < F || (n % 64) != 0)
     return VNM_ERR_ARG;
-  if (A->device != ctx->device || (reinterpret_cast<uintptr_t>(B) & 15) != 0) return VNM_ERR_ARG;
-  VNM_CUDA_TRY(cudaSetDevice(ctx->device));
   const size_t xsize = xtype == 2 ? 4 : 2;
+  if (A->device != ctx->device || reinterpret_cast<uintptr_t>(X) % xsize != 0 ||
+      (reinterpret_cast<uintptr_t>(B) & 15) != 0 || (reinterpret_cast<uintptr_t>(C) & 15) != 0)
+    return VNM_ERR_ARG;
+  VNM_CUDA_TRY(cudaSetDevice(ctx->device));
   const bool vec = (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (ldx * xsize) % 16 == 0;
   long long g = ((long long)A->R * (n / 8) + 255) / 256;
   if (g > (long long)ctx->num_sms * 32) g = (long long)ctx->num_sms * 32;

@@ -393,13 +393,18 @@ class SpmmMatrix:
         return C
 
     def run_cast_async(self, X):
-        """A X as FP32 (nrows x F) for a CUDA tensor X of FP32, FP16 or BF16
-        with contiguous rows, rounded to the operand's type, enqueued on
-        torch's current stream of X's device without waiting."""
+        """A X as FP32 (nrows x F) for a CUDA tensor X (nrows x F) of FP32, FP16
+        or BF16 with contiguous rows (stride(1) = 1, rows apart), rounded to
+        the operand's type, enqueued on torch's current stream of X's device
+        without waiting.  Raises ValueError for any other X."""
         import torch
+        xtype = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}.get(X.dtype)
+        if xtype is None or not X.is_cuda or X.dim() != 2 or X.shape[0] != self.nrows or X.shape[1] < 1:
+            raise ValueError("X must be a CUDA tensor of float32, float16 or bfloat16 with nrows rows")
         F, dev = X.shape[1], X.device
+        if X.stride(1) != 1 or X.stride(0) < F:
+            raise ValueError("the rows of X must be contiguous and not overlap")
         n = (F + 63) // 64 * 64
-        xtype = 2 if X.dtype == torch.float32 else 1 if X.dtype == torch.bfloat16 else 0
         B = torch.empty((self.nrows, n), dtype=torch.bfloat16 if self.dtype == "bf16" else torch.float16, device=dev)
         C = torch.empty((self.nrows, n), dtype=torch.float32, device=dev)
         st = lib().vnm_spmm_run_cast_async(self.ctx.h, self.h, X.data_ptr(), xtype, X.stride(0), F, B.data_ptr(), n,
