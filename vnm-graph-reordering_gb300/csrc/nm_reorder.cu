@@ -49,6 +49,7 @@
 #include <new>
 #include <vector>
 
+#include "batch_plan.h"
 #include "common.cuh"
 #include "swap_heap.h"
 
@@ -2443,9 +2444,9 @@ __global__ void k_batch_offset(const int* row, const int* col, const long long* 
   }
 }
 
-__global__ void k_batch_init(const NMJob* jobs, const int* inv0, const int* pres0, const int* seg_off) {
+__global__ void k_batch_init(const NMJob* jobs, const int* inv0, const int* pres0, int M) {
   const NMJob J = jobs[blockIdx.x];
-  const int so = seg_off[blockIdx.x];
+  const int so = J.row0 / M;  // the matrices' rows are multiples of M
   for (int i = threadIdx.x; i < J.R; i += blockDim.x) {
     J.orig[i] = i;
     if (i < J.nseg) {
@@ -2455,46 +2456,10 @@ __global__ void k_batch_init(const NMJob* jobs, const int* inv0, const int* pres
   }
 }
 
-__global__ void k_batch_invert(const NMJob* jobs, const int* row_off, int* newpos) {
+__global__ void k_batch_invert(const NMJob* jobs, int* newpos) {
   const NMJob J = jobs[blockIdx.x];
-  int* out = newpos + row_off[blockIdx.x];
+  int* out = newpos + J.row0;
   for (int i = threadIdx.x; i < J.R; i += blockDim.x) out[J.orig[i]] = i;
-}
-
-// How many of a batch's jobs (entries in descending order) to run on clusters
-// of 4 blocks when the others run on 2.  A job's time goes with its entries
-// (0.135 us each on 2 blocks, R-MAT 2:8) and is about 0.74 of that on 4; the
-// others start in order wherever two SMs come free, and the number with the
-// earliest end is taken, within half of the SMs and where it gains at least 10
-// %.  (256 R-MAT matrices, 256-8192 rows: the largest job alone took all of
-// the batch's 25.2 ms.)
-static int wide_jobs(const std::vector<long long>& sizes, int num_sms) {
-  const int n = (int)sizes.size(), pairs = num_sms / 2;
-  if (n < 2 || pairs < 1) return 0;
-  int best = 0;
-  double best_end = 0;
-  std::vector<double> ends;  // when each pair of SMs comes free: a heap, earliest on top
-  for (int k = 0; k < n && 4 * k <= pairs; k += k < 4 ? 1 : 2) {
-    ends.assign(pairs, 0.0);
-    double end = 0;
-    for (int q = 0; q < k; ++q) {
-      const double t = 0.74 * (double)sizes[q];
-      ends[2 * q] = ends[2 * q + 1] = t;
-      end = std::max(end, t);
-    }
-    std::make_heap(ends.begin(), ends.end(), std::greater<double>());
-    for (int q = k; q < n; ++q) {
-      std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
-      ends.back() += (double)sizes[q];
-      end = std::max(end, ends.back());
-      std::push_heap(ends.begin(), ends.end(), std::greater<double>());
-    }
-    if (k == 0 || end < best_end * (best == 0 ? 0.9 : 1.0)) {
-      best = k;
-      best_end = end;
-    }
-  }
-  return best;
 }
 
 // The context's second stream, made on first use.
@@ -2528,7 +2493,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   if (nnz > 0 && (!row || !col || !val)) return VNM_ERR_ARG;
   const int R = (int)totR, n = (int)nnz;
   size_t need = pattern_bytes(R, n) + 5 * arena_bytes(n, sizeof(int)) + arena_bytes(nmat + 1, 8) +
-                3 * arena_bytes(nmat + 1, sizeof(int)) + 2 * arena_bytes(nmat, sizeof(NMJob)) +
+                2 * arena_bytes(nmat + 1, sizeof(int)) + arena_bytes(nmat, sizeof(NMJob)) +
                 arena_bytes(R, sizeof(int)) + arena_bytes((size_t)R + (size_t)2 * ROW_GROUPS * nmat, sizeof(int)) +
                 arena_bytes((size_t)BATCH_CS * R, sizeof(int2)) +
                 arena_bytes(R, sizeof(uint4)) + 2 * arena_bytes(R / M + nmat, sizeof(int)) +
@@ -2543,23 +2508,40 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   VNM_TRY(stage_in(ctx, val, n, VNM_MEM_HOST, &d_val));
   long long* d_noff = arena_take<long long>(ctx, nmat + 1);
   int* d_roff = arena_take<int>(ctx, nmat + 1);
-  int* d_soff = arena_take<int>(ctx, nmat + 1);
   int* d_nrows = arena_take<int>(ctx, nmat + 1);
   int* grow = arena_take<int>(ctx, n > 0 ? n : 1);
   int* gcol = arena_take<int>(ctx, n > 0 ? n : 1);
   int* err = arena_take<int>(ctx, 1);
-  if (!d_noff || !d_roff || !d_soff || !d_nrows || !grow || !gcol || !err) return VNM_ERR_NOMEM;
+  if (!d_noff || !d_roff || !d_nrows || !grow || !gcol || !err) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_noff, nnz_offset, sizeof(long long) * (nmat + 1), cudaMemcpyHostToDevice,
                                ctx->stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(d_roff, row_off.data(), sizeof(int) * (nmat + 1), cudaMemcpyHostToDevice,
                                ctx->stream));
-  VNM_CUDA_TRY(cudaMemcpyAsync(d_soff, seg_off.data(), sizeof(int) * nmat, cudaMemcpyHostToDevice, ctx->stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(d_nrows, nrows, sizeof(int) * nmat, cudaMemcpyHostToDevice, ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
   if (n > 0)
     VNM_LAUNCH(ctx, k_batch_offset, grid_for(ctx, n), 256, 0, d_row, d_col, d_noff, d_roff, d_nrows, nmat,
                (long long)n, grow, gcol, err);
   VNM_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  // (on the host, while the GPU checks the entries)
+  // The rounds run in the order of the matrices' entries, most first: the
+  // batch lasts as long as its largest jobs, which must not start late (256
+  // R-MAT matrices 256-8192 rows at 2:8: 36.8 -> 27.1 ms).
+  std::vector<int> by_size(nmat);
+  for (int b = 0; b < nmat; ++b) by_size[b] = b;
+  std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int y) {
+    return nnz_offset[x + 1] - nnz_offset[x] > nnz_offset[y + 1] - nnz_offset[y];
+  });
+  // Clusters of 4 or 8 blocks per job where all jobs may still run at once
+  // (launch_rounds halves them if they do not): 12 matrices of 2048-8192 rows
+  // 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms, 12 of 256-512 rows
+  // 2.25 ms either way.  Else of 2 (88 ms with one block per job, 63 ms with
+  // 2, 69 ms with 4, measured on an earlier form of the kernel), but of 4 for
+  // the largest jobs if the batch would end with those alone.
+  std::vector<long long> sizes(nmat);
+  for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
+  const int cs = nmat * BATCH_CS <= ctx->num_sms ? BATCH_CS : nmat * 4 <= ctx->num_sms ? 4 : 2;
+  const int wide = cs == 2 ? wide_jobs(sizes, ctx->num_sms) : 0;
   VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (ctx->h_pinned[0] & 2) return VNM_ERR_RANGE;
   if (ctx->h_pinned[0] & 1) return VNM_ERR_UNSORTED;
@@ -2577,10 +2559,11 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   if (!runs || !orig || !touched || !rec || !cnt || !zc || !res || !d_jobs) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemsetAsync(rec, 0, sizeof(uint4) * (R > 0 ? R : 1), ctx->stream));
   VNM_CUDA_TRY(cudaMemsetAsync(res, 0, sizeof(int) * JOB_RES * nmat, ctx->stream));
-  std::vector<NMJob> hj(nmat);
+  std::vector<NMJob> hj(nmat);  // in the order of the launches
   int max_nseg = 0;
-  for (int b = 0; b < nmat; ++b) {
-    NMJob& J = hj[b];
+  for (int q = 0; q < nmat; ++q) {
+    NMJob& J = hj[q];
+    const int b = by_size[q];
     J.R = nrows[b];
     J.row0 = row_off[b];
     J.nseg = nrows[b] / M;
@@ -2604,42 +2587,19 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     J.hold_heaps = 0;
     J.err = nullptr;
     J.timed = ctx->phase_timing ? 1 : 0;
-    if (J.nseg > max_nseg) max_nseg = J.nseg;
+    max_nseg = std::max(max_nseg, J.nseg);
   }
-  // The rounds run in the order of the matrices' entries, most first: the
-  // batch lasts as long as its largest jobs, which must not start late (256
-  // R-MAT matrices 256-8192 rows at 2:8: 36.8 -> 27.1 ms).
-  std::vector<int> by_size(nmat);
-  for (int b = 0; b < nmat; ++b) by_size[b] = b;
-  std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int y) {
-    return nnz_offset[x + 1] - nnz_offset[x] > nnz_offset[y + 1] - nnz_offset[y];
-  });
-  std::vector<NMJob> sj(nmat);
-  for (int b = 0; b < nmat; ++b) sj[b] = hj[by_size[b]];
-  NMJob* d_sorted = arena_take<NMJob>(ctx, nmat);
-  if (!d_sorted) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, hj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
-  VNM_CUDA_TRY(cudaMemcpyAsync(d_sorted, sj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
-  VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, d_soff);
+  VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, M);
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  // Clusters of 4 or 8 blocks per job where all jobs may still run at once
-  // (launch_rounds halves them if they do not): 12 matrices of 2048-8192 rows
-  // 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms, 12 of 256-512 rows
-  // 2.25 ms either way.  Else of 2 (88 ms with one block per job, 63 ms with
-  // 2, 69 ms with 4, measured on an earlier form of the kernel), but of 4 for
-  // the largest jobs if the batch would end with those alone.
-  std::vector<long long> sizes(nmat);
-  for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
-  const int cs = nmat * BATCH_CS <= ctx->num_sms ? BATCH_CS : nmat * 4 <= ctx->num_sms ? 4 : 2;
-  const int wide = cs == 2 ? wide_jobs(sizes, ctx->num_sms) : 0;
   auto rounds = [&](int from, int to, int c, cudaStream_t st) {
     int nseg = 0, runs = 0;  // the largest of these jobs
     for (int q = from; q < to; ++q) {
-      const NMJob& J = sj[q];
+      const NMJob& J = hj[q];
       nseg = std::max(nseg, J.nseg);
       if (J.R > 0) runs = std::max(runs, ((J.row0 + J.R - 1) >> 4) - (J.row0 >> 4) + 1);
     }
-    return launch_rounds(ctx, d_sorted + from, to - from, N, M, nseg, runs, c, st);
+    return launch_rounds(ctx, d_jobs + from, to - from, N, M, nseg, runs, c, st);
   };
   if (wide > 0) {
     // the wide jobs' launch first, the others' on a second stream beside it;
@@ -2661,7 +2621,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   if (newpos && R > 0) {
     int* d_np = arena_take<int>(ctx, R);
     if (!d_np) return VNM_ERR_NOMEM;
-    VNM_LAUNCH(ctx, k_batch_invert, nmat, 256, 0, d_jobs, d_roff, d_np);
+    VNM_LAUNCH(ctx, k_batch_invert, nmat, 256, 0, d_jobs, d_np);
     VNM_CUDA_TRY(cudaMemcpyAsync(newpos, d_np, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream));
   }
   VNM_TRY(end_call(ctx));
