@@ -16,6 +16,10 @@
  *     is in after the reference's reader (mtx/readMtx.hpp:354-425).  The NM
  *     calls take nrows < 2^27 (a batch: the sum of its nrows), else
  *     VNM_ERR_LIMIT.
+ *     A reorder's scratch is at most 136 bytes a row for the pattern and 8 c +
+ *     28 a row and schedule (c blocks a job: 8, or 16 from 2^17 entries on; a
+ *     batch 92), and 4 an entry (16 for arrays on the host, a batch 24); a
+ *     context allocates a quarter more than a call needs.
  *   - `mem` says where the caller's arrays live: VNM_MEM_HOST (pageable or
  *     pinned host memory; the call copies them) or VNM_MEM_DEVICE (device
  *     memory of the context's GPU; nothing is copied).

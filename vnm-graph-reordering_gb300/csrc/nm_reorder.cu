@@ -2023,9 +2023,10 @@ vnm_status build_pattern(vnm_ctx* ctx, int R, int nnz, const int* d_row, const i
   return VNM_ERR_ARG;
 }
 
-size_t job_bytes(int R) {
+// A job's arena bytes on clusters of up to cs blocks: at most 8 cs + 28 a row.
+static size_t job_bytes(int R, int cs) {
   const int nseg = R / 2 + 1;
-  return arena_bytes((size_t)ROW_GROUPS * R, sizeof(int2)) + arena_bytes(R, sizeof(int)) +
+  return arena_bytes((size_t)cs * (R > 0 ? R : 1), sizeof(int2)) + arena_bytes(R, sizeof(int)) +
          2 * arena_bytes(nseg, sizeof(int)) + arena_bytes(R, sizeof(uint4)) +
          arena_bytes((size_t)R + 2 * ROW_GROUPS, sizeof(int)) + arena_bytes(JOB_RES, sizeof(int));
 }
@@ -2286,7 +2287,10 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   const int R = nrows;
   const int trace_pairs_cap = trace ? 2 * (M + 1) * M * 4096 : 0;
   const int trace_rounds_cap = trace ? 65536 : 0;
-  size_t need = pattern_bytes(R, nnz) + (size_t)nsched * job_bytes(R) + arena_bytes(nsched, sizeof(NMJob)) +
+  // the stored entries stand in for the pattern's (nonzero-valued) entries
+  // when sizing the clusters: their count is known without a readback
+  const int cs = nm_cluster_size(nnz);
+  size_t need = pattern_bytes(R, nnz) + (size_t)nsched * job_bytes(R, cs) + arena_bytes(nsched, sizeof(NMJob)) +
                 arena_bytes(nsched * JOB_RES + RES_TAIL, sizeof(int)) + arena_bytes(R, sizeof(int)) +
                 3 * arena_bytes(nnz, sizeof(int)) +
                 arena_bytes(trace_pairs_cap * 2, sizeof(int)) + arena_bytes(trace_rounds_cap, sizeof(int)) + 4096;
@@ -2308,9 +2312,6 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   int* d_res = arena_take<int>(ctx, nsched * JOB_RES + RES_TAIL);  // read back in one copy
   if (!d_res) return VNM_ERR_NOMEM;
   int* d_tail = d_res + nsched * JOB_RES;
-  // the stored entries stand in for the pattern's (nonzero-valued) entries
-  // when sizing the clusters: their count is known without a readback
-  const int cs = nm_cluster_size(nnz);
   for (int s = 0; s < nsched; ++s) {
     VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s], cs, d_res + s * JOB_RES));
     hj[s].err = P.d_err;
@@ -2768,7 +2769,7 @@ vnm_status vnm_nm_pair_score(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   VNM_TRY(check_nm_args(nrows, nnz, row, col, val, mem, N, M));
   const int nseg = nrows / M;
   if (seg1 < 0 || seg2 < 0 || seg1 >= nseg || seg2 >= nseg) return VNM_ERR_ARG;
-  VNM_TRY(arena_reserve(ctx, pattern_bytes(nrows, nnz) + job_bytes(nrows) + 3 * arena_bytes(nnz, sizeof(int)) +
+  VNM_TRY(arena_reserve(ctx, pattern_bytes(nrows, nnz) + job_bytes(nrows, 1) + 3 * arena_bytes(nnz, sizeof(int)) +
                                  arena_bytes(2 * M * M, sizeof(int)) + 4096));
   VNM_TRY(pinned_reserve(ctx, 64));
   VNM_TRY(begin_call(ctx));
@@ -2862,7 +2863,8 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   VNM_TRY(check_nm_args(nrows, nnz, row, col, val, VNM_MEM_DEVICE, N, M));
   if (sched < 0 || sched > 3 || !res5 || !newpos) return VNM_ERR_ARG;
   if (nrows > NOALLOC_MAX_ROWS || nnz > NOALLOC_MAX_NNZ) return VNM_ERR_LIMIT;
-  const size_t need = pattern_bytes(nrows, nnz) + job_bytes(nrows) + arena_bytes(1, sizeof(NMJob)) + 4096;
+  const size_t need =
+      pattern_bytes(nrows, nnz) + job_bytes(nrows, nm_cluster_size(nnz)) + arena_bytes(1, sizeof(NMJob)) + 4096;
   if (need > NOALLOC_BYTES) return VNM_ERR_LIMIT;
   int device = 0;
   VNM_CUDA_TRY(cudaGetDevice(&device));
@@ -2888,8 +2890,7 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   NMJob* d_job = arena_take<NMJob>(&c, 1);
   if (!d_job) return VNM_ERR_LIMIT;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_job, &hj, sizeof(NMJob), cudaMemcpyHostToDevice, c.stream));
-  // the same launch shape as vnm_nm_reorder (a cluster of blocks per job);
-  // the scratch it needs does not depend on the cluster size
+  // the same launch shape as vnm_nm_reorder (a cluster of blocks per job)
   VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, cs));
   VNM_CUDA_TRY(cudaMemcpyAsync(hs, hj.res, sizeof(int) * 16, cudaMemcpyDeviceToHost, c.stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(c.stream));
