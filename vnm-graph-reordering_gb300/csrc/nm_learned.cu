@@ -1470,16 +1470,10 @@ static int lgrid(const vnm_ctx* ctx, long long n, int nt = 256) {
   return g < 1 ? 1 : (int)g;
 }
 
+// The kernel's shared-memory ceiling, set for the call's device.
+template <bool kPlain>
 static vnm_status mlp_launch_prep(size_t smem) {
-  static bool done[2] = {false, false};
-  if (!done[0]) {
-    VNM_CUDA_TRY(cudaFuncSetAttribute(k_l_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    done[0] = true;
-  }
-  if (!done[1]) {
-    VNM_CUDA_TRY(cudaFuncSetAttribute(k_l_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    done[1] = true;
-  }
+  VNM_CUDA_TRY(cudaFuncSetAttribute(k_l_mlp<kPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return VNM_OK;
 }
 
@@ -1500,7 +1494,7 @@ vnm_status vnm_mlp_forward(vnm_ctx* ctx, const vnm_mlp* net, const float* X, int
   if (!dY || !err) return VNM_ERR_NOMEM;
   VNM_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
   const size_t smem = mlp_smem();
-  VNM_TRY(mlp_launch_prep(smem));
+  VNM_TRY(mlp_launch_prep<true>(smem));
   LMat L{};
   const int tiles = (n + 127) / 128;
   const int grid = tiles < ctx->num_sms ? tiles : ctx->num_sms;
@@ -1613,7 +1607,7 @@ vnm_status vnm_nm_learned(vnm_ctx* ctx, int nrows, int nnz, const int* row, cons
   out->init_invalid = out->final_invalid = (long long)hcu[2];
   out->init_retained = out->final_retained = (long long)hcu[3];
   const size_t smem = mlp_smem();
-  if (mode == VNM_LEARNED_MLP) VNM_TRY(mlp_launch_prep(smem));
+  if (mode == VNM_LEARNED_MLP) VNM_TRY(mlp_launch_prep<false>(smem));
   const MlpW W = net ? mlp_view(net) : MlpW{};
   const int pgrid = ctx->num_sms;  // the blocks beyond the active segments return at once
   const int egrid = ctx->num_sms * 8;
