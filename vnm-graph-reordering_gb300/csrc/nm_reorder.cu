@@ -106,7 +106,6 @@ struct NMJob {
   int nseg;           // R / M
   int sched;          // 0..3
   int maxiter;        // reorderUtil MAXITER before it is raised to init_size
-  const int* cptr;    // [R+1] column pointers of the nonzero pattern (original ids)
   const int* crow;    // rows of each column, grouped by row_group
   const int* csplit;  // [16 R + 1] start of each (column, row group) in crow
   int2* runs;         // [cs][R] scratch: each block's entries {start in crow, count} of the column at a position
@@ -2039,7 +2038,6 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   J.nseg = P.nseg;
   J.sched = sched;
   J.maxiter = maxiter;
-  J.cptr = P.cptr;
   J.crow = P.crow;
   J.csplit = P.csplit;
   J.runs = arena_take<int2>(ctx, (size_t)cs * (P.R > 0 ? P.R : 1));
@@ -2570,7 +2568,6 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     J.nseg = nrows[b] / M;
     J.sched = sched;
     J.maxiter = maxiter;
-    J.cptr = P.cptr + row_off[b];
     J.crow = P.crow;
     J.csplit = P.csplit + (size_t)ROW_GROUPS * row_off[b];
     J.runs = runs + (size_t)BATCH_CS * row_off[b];
