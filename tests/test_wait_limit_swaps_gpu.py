@@ -1,9 +1,9 @@
 """A wait of the walk that runs out between two swaps of a round: the job
-fails with VNM_ERR_INTERNAL, what the round had committed stays a permutation
-of its columns (the recount looks columns up by it), and the context keeps
-working.  The heaps publish nothing (a test hook), so the walk stops at the
-first pair whose best swap is tied; many invalid segments and few distinct
-gains make that happen after swaps of the same round."""
+fails with VNM_ERR_INTERNAL, the recount that still follows looks up columns
+of the round only (swaps after the failed one may move a column twice), and
+the context keeps working.  The heaps publish nothing (a test hook), so the
+walk fails at the first pair whose best swap is tied; many invalid segments
+and few distinct gains make that happen after swaps of the same round."""
 import os
 
 import numpy as np

@@ -302,7 +302,10 @@ struct RoundSmem {
     uint32_t dest_w[DEST_W];   // the same bytes as words, for copies to other blocks
   };
   int newinv[K], newpres[K];
-  uint8_t from[K * M];         // the column (xi * M + k) whose bits a column holds after the swaps
+  // The column (xi * M + k) whose bits a column holds after the swaps.  Always
+  // some column's: in a job that has failed, whose swaps may move one column
+  // twice, not every place is set anew.
+  uint8_t from[K * M];
   int swaps[2 * K * M];        // committed swaps (positions)
   unsigned long long wtop[2][NW][K];
   unsigned long long sel_top[15][2][K];  // leader: each helper's scan (top K both orders) ...
@@ -607,6 +610,7 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
     sm.newinv[threadIdx.x] = 0;
     sm.newpres[threadIdx.x] = 0;
   }
+  for (int i = threadIdx.x; i < K * M; i += NM_THREADS) sm.from[i] = 0;
   if (threadIdx.x == 0) {
     sm.ntouched = 0;
     sm.nswaps = 0;
@@ -1315,7 +1319,7 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
   volatile int* prog = sm.hprog;
   extern __shared__ uint4 smem_heap[];
   const unsigned* ent = reinterpret_cast<const unsigned*>(smem_heap) + MM * HS;  // [MM][HS], as rank_phase wrote
-  bool dead = false;  // the job has failed (a wait ran out): no further swap is read or committed
+  bool dead = false;  // a wait ran out: the job is failed, finish without reading ord
   // pops of pair column `col` published so far, once at least `need`; -1 at the limit
   unsigned long long waited = 0;  // ns spent waiting for pops (lane 0)
   auto wait_pops = [&](int col, int need) -> int {
@@ -1352,11 +1356,8 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
     // |L| == 1: best pair of (top, minseg) with no visited filter (:1837-1860)
     const int b = sm.mode == 2 ? 0 : 1;
     int pick = 0;
-    if (wait_pops(0 * K + b, 1) < 0) {
-      if (lane == 0) sm.status |= JOB_WAIT_LIMIT;
-    } else {
-      pick = ord0[0 * K + b];
-    }
+    if (wait_pops(0 * K + b, 1) < 0) dead = true;
+    else pick = ord0[0 * K + b];
     commit(0, b, pick);
   } else {
     const bool rev_list = sched >= 2;                  // inv_seg_list / updatePQ comparator
@@ -1379,7 +1380,7 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
       }
       return __ffs(at) - 1;
     };
-    while (__popc(Wm) >= 2 && !dead) {
+    while (__popc(Wm) >= 2) {
       // primary = top of the list
       const int pxi = top_lane(Wm, order_key_hi(cnt, rev_list), order_key_lo(seg, rev_list));
       int pc = __shfl_sync(FULL, cnt, pxi);
@@ -1438,12 +1439,11 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
           while (pick < 0 && !dead) {
             if (seen >= MM) {  // unreachable: a scored target always has an unvisited node
               if (lane == 0) sm.status |= JOB_EMPTY_HEAP;
-              dead = true;
+              pick = ord[(MM - 1) * HS];
               break;
             }
             const int avail = wait_pops(col, seen + 1);
             if (avail < 0) {
-              if (lane == 0) sm.status |= JOB_WAIT_LIMIT;
               dead = true;
               break;
             }
@@ -1456,9 +1456,7 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
             }
             seen = avail;
           }
-          // The job has failed: no further swap, so that the round's moves stay
-          // a permutation, on which the recount's column lookups rest.
-          if (dead) break;
+          if (dead) pick = 0;
           key = ent[pick * HS + col] >> 8;
         }
         int l, r;
@@ -1489,6 +1487,7 @@ __device__ void walk_phase(RoundSmem<M>& sm, int sched, int wait_limit) {
   }
   if (lane == 0) {
     sm.nswaps = nsw;
+    if (dead) sm.status |= JOB_WAIT_LIMIT;
     *(volatile int*)&sm.hstop = 1;
     s_tin[1] += waited;
   }
