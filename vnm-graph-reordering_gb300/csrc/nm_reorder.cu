@@ -102,6 +102,7 @@ __host__ __device__ __forceinline__ int row_group(int row) {
 
 struct NMJob {
   int R;              // padded rows = columns
+  int fill;           // rows whose runs the job's own blocks fill: R or 0 (RUNS_OWN)
   int row0;           // first row id in crow (a batch's matrices share one id range)
   int nseg;           // R / M
   int sched;          // 0..3
@@ -211,18 +212,39 @@ __global__ void k_pattern(const int* row, const int* col, const float* val, int 
   }
 }
 
+// Block r's run of the column at position c, at the identity arrangement, for
+// clusters of cs blocks.  A round's swaps move runs that the block has at hand
+// then (apply_recount), so a round reads a column's run in one step where
+// position -> node -> run were two dependent L2 round trips (the gather of R-MAT
+// 16384 2:4, schedule 0: 3.1 -> 2.9 us; of 65536 2:8 9.5 -> 8.7; of 512 rows 3.1
+// -> 2.4).
+// A job's blocks fill their own up to RUNS_OWN rows: 0.5 ns a row, and the L1
+// keeps some (filled by the set-up kernels, R-MAT 16384 2:4 took 1.3 % longer,
+// 65536 2:8 0.3 %).  Above, the set-up kernels do, on all SMs (524288 rows 2:8
+// 24.3 -> 24.1 ms; 2^20 rows without a round 1.07 -> 0.48 ms a call).
+constexpr int RUNS_OWN = 65536;
+__device__ __forceinline__ void fill_run(const NMJob& J, int cs, int r, int c) {
+  const int* g = J.csplit + (size_t)ROW_GROUPS * c + r * (ROW_GROUPS / cs);
+  const int b = g[0];
+  J.runs[(size_t)r * J.R + c] = make_int2(b, g[ROW_GROUPS / cs] - b);
+}
+
 // Up to four jobs on one pattern: the identity arrangement and its counts, and
-// clear scratch and results.  tail (if not null): the check's words, to be
+// clear scratch and results; cs: the blocks of a job's cluster, y of the grid
+// where they are told apart.  tail (if not null): the check's words, to be
 // read back next to the results.
 struct JobSet {
   NMJob j[4];
 };
-__global__ void k_init_jobs(JobSet set, int njobs, const int* inv0, const int* pres0, const int* err, int* tail) {
-  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-  if (tail && i0 < 2) tail[i0] = err[i0];
+__global__ void k_init_jobs(JobSet set, int njobs, int cs, const int* inv0, const int* pres0, const int* err, int* tail) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x, r = blockIdx.y;
+  if (tail && r == 0 && i0 < 2) tail[i0] = err[i0];
   for (int q = 0; q < njobs; ++q) {
     const NMJob& J = set.j[q];
-    if (i0 < JOB_RES) J.res[i0] = 0;
+    if (r == 0 && i0 < JOB_RES) J.res[i0] = 0;
+    if (J.R > RUNS_OWN)
+      for (int i = i0; i < J.R; i += step) fill_run(J, cs, r, i);
+    if (r > 0) continue;
     for (int i = i0; i < J.R; i += step) {
       J.orig[i] = i;
       J.rec[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -621,16 +643,12 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
 // the run of 16 rows that a range not starting at a multiple of 16 adds).
 constexpr int DIRECT_MAX = 4352;
 
-// The block's run of every column, by position, at the identity arrangement.
-// A round's swaps move runs that the block has at hand then (apply_recount),
-// so a round reads a column's run in one step where position -> node -> run
-// were two dependent L2 round trips (the gather of R-MAT 16384 2:4, schedule 0:
-// 3.1 -> 2.9 us; of 65536 2:8 9.5 -> 8.7; of 512 rows 3.1 -> 2.4).
+// The block's own runs (up to RUNS_OWN rows).
 __device__ void fill_runs(const NMJob& J, Slice sl) {
   const int g0 = sl.rank * (ROW_GROUPS / sl.cs), g1 = g0 + ROW_GROUPS / sl.cs;
   int2* runs = J.runs + (size_t)sl.rank * J.R;
 #pragma unroll 4
-  for (int c = threadIdx.x; c < J.R; c += NM_THREADS) {
+  for (int c = threadIdx.x; c < J.fill; c += NM_THREADS) {
     const int b = J.csplit[(size_t)ROW_GROUPS * c + g0];
     runs[c] = make_int2(b, J.csplit[(size_t)ROW_GROUPS * c + g1] - b);
   }
@@ -2033,6 +2051,7 @@ static size_t job_bytes(int R, int cs) {
 // results at `res`, if given); init_jobs sets it up.
 static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxiter, NMJob& J, int cs, int* res = nullptr) {
   J.R = P.R;
+  J.fill = P.R <= RUNS_OWN ? P.R : 0;
   J.row0 = 0;
   J.nseg = P.nseg;
   J.sched = sched;
@@ -2067,10 +2086,12 @@ static vnm_status make_job(vnm_ctx* ctx, const Pattern& P, int sched, int maxite
   return VNM_OK;
 }
 
-static vnm_status init_jobs(vnm_ctx* ctx, const Pattern& P, const NMJob* jobs, int njobs, int* tail = nullptr) {
+// cs: the blocks of a job's cluster as it will be launched.
+static vnm_status init_jobs(vnm_ctx* ctx, const Pattern& P, const NMJob* jobs, int njobs, int cs, int* tail = nullptr) {
   JobSet set{};
   for (int q = 0; q < njobs; ++q) set.j[q] = jobs[q];
-  VNM_LAUNCH(ctx, k_init_jobs, grid_for(ctx, P.R > 0 ? P.R : 1), 256, 0, set, njobs, P.inv0, P.pres0, P.d_err, tail);
+  VNM_LAUNCH(ctx, k_init_jobs, dim3(grid_for(ctx, P.R > 0 ? P.R : 1), P.R > RUNS_OWN ? cs : 1), 256, 0, set, njobs, cs,
+             P.inv0, P.pres0, P.d_err, tail);
   return VNM_OK;
 }
 
@@ -2119,74 +2140,78 @@ static RoundShape round_shape(int max_nseg, int max_runs, int cs) {
 // call on another thread cannot lower it in between.
 static std::mutex g_round_launch_mu;
 
+// static + dynamic shared memory may pass the 48 KB a launch gets without
+// opting in (RoundSmem<8> alone is ~30 KB)
+template <int M>
+static cudaError_t set_round_smem(const RoundShape& f) {
+  return cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.dyn);
+}
+
+// cs: how many blocks a job may have; then how many it gets.  How many clusters
+// of a size the GPU can hold at once depends on the SMs of each of its GPCs;
+// the largest size (halving from cs) at which every job of the call runs
+// concurrently, else the largest that fits at all, else one block.
+template <int M>
+static vnm_status pick_cluster_t(vnm_ctx* ctx, int njobs, int max_nseg, int max_runs, int& cs) {
+  std::lock_guard<std::mutex> launch_lock(g_round_launch_mu);
+  ctx->last_clusters_fit = 0;
+  if (cs > 8)
+    VNM_CUDA_TRY(cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(NM_THREADS);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int fallback = 1;
+  for (; cs > 1; cs >>= 1) {
+    const RoundShape f = round_shape<M>(max_nseg, max_runs, cs);
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    cfg.gridDim = dim3((unsigned)(njobs * cs));
+    cfg.dynamicSmemBytes = f.dyn;
+    int nclusters = 0;
+    if (set_round_smem<M>(f) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&nclusters, k_nm_rounds<M>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      continue;
+    }
+    if (nclusters >= 1 && fallback == 1) {
+      fallback = cs;
+      ctx->last_clusters_fit = nclusters;
+    }
+    if (nclusters >= njobs) {
+      ctx->last_clusters_fit = nclusters;
+      return VNM_OK;
+    }
+  }
+  cs = fallback;
+  return VNM_OK;
+}
+
 template <int M>
 static vnm_status launch_rounds_t(vnm_ctx* ctx, cudaStream_t st, const NMJob* d_jobs, int njobs, int N, int max_nseg,
                                   int max_runs, int cs) {
   std::lock_guard<std::mutex> launch_lock(g_round_launch_mu);
-  ctx->last_clusters_fit = 0;
   const int in_smem = (size_t)max_nseg * sizeof(int) <= (64u << 10) ? 1 : 0;
-  if (cs > 8)
-    VNM_CUDA_TRY(cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  // static + dynamic shared memory may pass the 48 KB a launch gets without
-  // opting in (RoundSmem<8> alone is ~30 KB)
-  auto set_dyn = [&](const RoundShape& f) {
-    return cudaFuncSetAttribute(k_nm_rounds<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.dyn);
-  };
-  if (cs > 1) {
-    // How many clusters of a size the GPU can hold at once depends on the
-    // SMs of each of its GPCs; take the largest size (halving from cs) at
-    // which every job of the call runs concurrently, else the largest that
-    // fits at all.
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(NM_THREADS);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int pick = 1, fallback = 1;
-    for (int c = cs; c > 1; c >>= 1) {
-      const RoundShape f = round_shape<M>(max_nseg, max_runs, c);
-      attr[0].val.clusterDim.x = (unsigned)c;
-      cfg.gridDim = dim3((unsigned)(njobs * c));
-      cfg.dynamicSmemBytes = f.dyn;
-      int nclusters = 0;
-      if (set_dyn(f) != cudaSuccess || cudaOccupancyMaxActiveClusters(&nclusters, k_nm_rounds<M>, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        continue;
-      }
-      if (nclusters >= 1 && fallback == 1) {
-        fallback = c;
-        ctx->last_clusters_fit = nclusters;
-      }
-      if (nclusters >= njobs) {
-        pick = c;
-        ctx->last_clusters_fit = nclusters;
-        break;
-      }
-    }
-    if (pick == 1) pick = fallback;
-    if (pick > 1) {
-      const RoundShape f = round_shape<M>(max_nseg, max_runs, pick);
-      VNM_CUDA_TRY(set_dyn(f));
-      attr[0].val.clusterDim.x = (unsigned)pick;
-      cfg.gridDim = dim3((unsigned)(njobs * pick));
-      cfg.dynamicSmemBytes = f.dyn;
-      VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_nm_rounds<M>, d_jobs, N, in_smem, f.ts, f.dslots, pick));
-      ctx->launches++;
-      ctx->last_cluster = pick;
-      return VNM_OK;
-    }
-  }
-  // one block per job (asked for, or no cluster fits)
-  const RoundShape f = round_shape<M>(max_nseg, max_runs, 1);
-  VNM_CUDA_TRY(set_dyn(f));
-  k_nm_rounds<M><<<njobs, NM_THREADS, f.dyn, st>>>(d_jobs, N, in_smem, f.ts, f.dslots, 1);
+  const RoundShape f = round_shape<M>(max_nseg, max_runs, cs);
+  VNM_CUDA_TRY(set_round_smem<M>(f));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(njobs * cs));
+  cfg.blockDim = dim3(NM_THREADS);
+  cfg.dynamicSmemBytes = f.dyn;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cs > 1 ? 1 : 0;
+  VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_nm_rounds<M>, d_jobs, N, in_smem, f.ts, f.dslots, cs));
   ctx->launches++;
-  VNM_CUDA_TRY(cudaGetLastError());
-  ctx->last_cluster = 1;
+  ctx->last_cluster = cs;
   return VNM_OK;
 }
 
@@ -2206,16 +2231,30 @@ static int nm_cluster_size(long long np) {
 }
 
 // max_runs: aligned runs of 16 rows a job's rows lie in, at most.
-static vnm_status launch_rounds(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int M, int max_nseg, int max_runs,
-                                int cs, cudaStream_t st = nullptr) {
+static vnm_status pick_cluster(vnm_ctx* ctx, int njobs, int M, int max_nseg, int max_runs, int& cs) {
   switch (M) {
-    case 2: return launch_rounds_t<2>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 3: return launch_rounds_t<3>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 4: return launch_rounds_t<4>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 5: return launch_rounds_t<5>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 6: return launch_rounds_t<6>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 7: return launch_rounds_t<7>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
-    case 8: return launch_rounds_t<8>(ctx, st ? st : ctx->stream, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 2: return pick_cluster_t<2>(ctx, njobs, max_nseg, max_runs, cs);
+    case 3: return pick_cluster_t<3>(ctx, njobs, max_nseg, max_runs, cs);
+    case 4: return pick_cluster_t<4>(ctx, njobs, max_nseg, max_runs, cs);
+    case 5: return pick_cluster_t<5>(ctx, njobs, max_nseg, max_runs, cs);
+    case 6: return pick_cluster_t<6>(ctx, njobs, max_nseg, max_runs, cs);
+    case 7: return pick_cluster_t<7>(ctx, njobs, max_nseg, max_runs, cs);
+    case 8: return pick_cluster_t<8>(ctx, njobs, max_nseg, max_runs, cs);
+  }
+  return VNM_ERR_ARG;
+}
+
+// cs: as picked, and as the jobs' runs were filled for.
+static vnm_status launch_rounds(vnm_ctx* ctx, const NMJob* d_jobs, int njobs, int N, int M, int max_nseg, int max_runs,
+                                int cs, cudaStream_t st) {
+  switch (M) {
+    case 2: return launch_rounds_t<2>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 3: return launch_rounds_t<3>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 4: return launch_rounds_t<4>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 5: return launch_rounds_t<5>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 6: return launch_rounds_t<6>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 7: return launch_rounds_t<7>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
+    case 8: return launch_rounds_t<8>(ctx, st, d_jobs, njobs, N, max_nseg, max_runs, cs);
   }
   return VNM_ERR_ARG;
 }
@@ -2286,7 +2325,7 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   const int trace_rounds_cap = trace ? 65536 : 0;
   // the stored entries stand in for the pattern's (nonzero-valued) entries
   // when sizing the clusters: their count is known without a readback
-  const int cs = nm_cluster_size(nnz);
+  int cs = nm_cluster_size(nnz);
   size_t need = pattern_bytes(R, nnz) + (size_t)nsched * job_bytes(R, cs) + arena_bytes(nsched, sizeof(NMJob)) +
                 arena_bytes(nsched * JOB_RES + RES_TAIL, sizeof(int)) + arena_bytes(R, sizeof(int)) +
                 3 * arena_bytes(nnz, sizeof(int)) +
@@ -2309,11 +2348,12 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   int* d_res = arena_take<int>(ctx, nsched * JOB_RES + RES_TAIL);  // read back in one copy
   if (!d_res) return VNM_ERR_NOMEM;
   int* d_tail = d_res + nsched * JOB_RES;
+  VNM_TRY(pick_cluster(ctx, nsched, M, P.nseg, (R + 15) / 16, cs));
   for (int s = 0; s < nsched; ++s) {
     VNM_TRY(make_job(ctx, P, sched0 + s, maxiter, hj[s], cs, d_res + s * JOB_RES));
     hj[s].err = P.d_err;
   }
-  VNM_TRY(init_jobs(ctx, P, hj, nsched, d_tail));
+  VNM_TRY(init_jobs(ctx, P, hj, nsched, cs, d_tail));
   int* d_tp = nullptr;
   int* d_tr = nullptr;
   if (trace) {
@@ -2334,7 +2374,7 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   memcpy(pj, hj, sizeof(NMJob) * nsched);
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, pj, sizeof(NMJob) * nsched, cudaMemcpyHostToDevice, ctx->stream));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, cs));
+  VNM_TRY(launch_rounds(ctx, d_jobs, nsched, N, M, P.nseg, (R + 15) / 16, cs, ctx->stream));
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hp = ctx->h_pinned;
   if (d_newpos) {
@@ -2442,10 +2482,14 @@ __global__ void k_batch_offset(const int* row, const int* col, const long long* 
   }
 }
 
-__global__ void k_batch_init(const NMJob* jobs, const int* inv0, const int* pres0, int M) {
+// The first `wide` jobs run on cs_wide blocks, the others on cs.
+__global__ void k_batch_init(const NMJob* jobs, const int* inv0, const int* pres0, int M, int wide, int cs_wide, int cs) {
   const NMJob J = jobs[blockIdx.x];
   const int so = J.row0 / M;  // the matrices' rows are multiples of M
-  for (int i = threadIdx.x; i < J.R; i += blockDim.x) {
+  const int c = (int)blockIdx.x < wide ? cs_wide : cs;
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < J.R; i += gridDim.y * blockDim.x) {
+    if (J.R > RUNS_OWN)
+      for (int r = 0; r < c; ++r) fill_run(J, c, r, i);
     J.orig[i] = i;
     if (i < J.nseg) {
       J.cnt[i] = inv0[so + i];
@@ -2531,7 +2575,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     return nnz_offset[x + 1] - nnz_offset[x] > nnz_offset[y + 1] - nnz_offset[y];
   });
   // Clusters of 4 or 8 blocks per job where all jobs may still run at once
-  // (launch_rounds halves them if they do not): 12 matrices of 2048-8192 rows
+  // (pick_cluster halves them if they do not): 12 matrices of 2048-8192 rows
   // 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms, 12 of 256-512 rows
   // 2.25 ms either way.  Else of 2 (88 ms with one block per job, 63 ms with
   // 2, 69 ms with 4, measured on an earlier form of the kernel), but of 4 for
@@ -2563,6 +2607,7 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     NMJob& J = hj[q];
     const int b = by_size[q];
     J.R = nrows[b];
+    J.fill = J.R <= RUNS_OWN ? J.R : 0;
     J.row0 = row_off[b];
     J.nseg = nrows[b] / M;
     J.sched = sched;
@@ -2587,30 +2632,40 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     max_nseg = std::max(max_nseg, J.nseg);
   }
   VNM_CUDA_TRY(cudaMemcpyAsync(d_jobs, hj.data(), sizeof(NMJob) * nmat, cudaMemcpyHostToDevice, ctx->stream));
-  VNM_LAUNCH(ctx, k_batch_init, nmat, 256, 0, d_jobs, P.inv0, P.pres0, M);
-  VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
-  auto rounds = [&](int from, int to, int c, cudaStream_t st) {
-    int nseg = 0, runs = 0;  // the largest of these jobs
-    for (int q = from; q < to; ++q) {
+  struct Part {  // of the jobs: a launch of its own
+    int from, to, cs;
+    int nseg = 0, runs = 0;  // the largest of its jobs
+  };
+  Part first{0, wide > 0 ? wide : nmat, wide > 0 ? 4 : cs}, others{first.to, nmat, cs};
+  for (Part* p : {&others, &first}) {
+    if (p->from == p->to) continue;
+    for (int q = p->from; q < p->to; ++q) {
       const NMJob& J = hj[q];
-      nseg = std::max(nseg, J.nseg);
-      if (J.R > 0) runs = std::max(runs, ((J.row0 + J.R - 1) >> 4) - (J.row0 >> 4) + 1);
+      p->nseg = std::max(p->nseg, J.nseg);
+      if (J.R > 0) p->runs = std::max(p->runs, ((J.row0 + J.R - 1) >> 4) - (J.row0 >> 4) + 1);
     }
-    return launch_rounds(ctx, d_jobs + from, to - from, N, M, nseg, runs, c, st);
+    VNM_TRY(pick_cluster(ctx, p->to - p->from, M, p->nseg, p->runs, p->cs));
+  }
+  // (a block a matrix, or more where few matrices leave SMs idle)
+  const int by = std::min(1 + max_nseg * M / 4096, std::max(1, 4 * ctx->num_sms / nmat));
+  VNM_LAUNCH(ctx, k_batch_init, dim3(nmat, by), 256, 0, d_jobs, P.inv0, P.pres0, M, first.to, first.cs, others.cs);
+  VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main0, ctx->stream));
+  auto rounds = [&](const Part& p, cudaStream_t st) {
+    return launch_rounds(ctx, d_jobs + p.from, p.to - p.from, N, M, p.nseg, p.runs, p.cs, st);
   };
   if (wide > 0) {
     // the wide jobs' launch first, the others' on a second stream beside it;
     // the streams join again whatever comes of the launches
     VNM_TRY(side_stream(ctx));
     VNM_CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->stream));
-    vnm_status s0 = rounds(0, wide, 4, ctx->stream);
+    vnm_status s0 = rounds(first, ctx->stream);
     VNM_CUDA_TRY(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    vnm_status s1 = s0 == VNM_OK ? rounds(wide, nmat, 2, ctx->side) : s0;
+    vnm_status s1 = s0 == VNM_OK ? rounds(others, ctx->side) : s0;
     VNM_CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->side));
     VNM_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
     VNM_TRY(s1);
   } else {
-    VNM_TRY(rounds(0, nmat, cs, ctx->stream));
+    VNM_TRY(rounds(first, ctx->stream));
   }
   VNM_CUDA_TRY(cudaEventRecord(ctx->ev_main1, ctx->stream));
   int* hres = ctx->h_pinned + 256;
@@ -2778,7 +2833,7 @@ vnm_status vnm_nm_pair_score(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
   VNM_TRY(build_pattern(ctx, nrows, nnz, d_row, d_col, d_val, N, M, P, ctx->h_pinned));
   NMJob J;
   VNM_TRY(make_job(ctx, P, 0, 10, J, 1));
-  VNM_TRY(init_jobs(ctx, P, &J, 1));
+  VNM_TRY(init_jobs(ctx, P, &J, 1, 1));
   int* d_score = arena_take<int>(ctx, 2 * M * M);
   if (!d_score) return VNM_ERR_NOMEM;
   switch (M) {
@@ -2880,14 +2935,15 @@ extern "C" vnm_status vnm_nm_reorder_noalloc(int nrows, int nnz, const int* row,
   Pattern P;
   VNM_TRY(build_pattern(&c, nrows, nnz, row, col, val, N, M, P, hs));
   NMJob hj;
-  const int cs = nm_cluster_size(P.np);
+  int cs = nm_cluster_size(P.np);
+  VNM_TRY(pick_cluster(&c, 1, M, P.nseg, (nrows + 15) / 16, cs));
   VNM_TRY(make_job(&c, P, sched, nm_maxiter, hj, cs));
-  VNM_TRY(init_jobs(&c, P, &hj, 1));
+  VNM_TRY(init_jobs(&c, P, &hj, 1, cs));
   NMJob* d_job = arena_take<NMJob>(&c, 1);
   if (!d_job) return VNM_ERR_LIMIT;
   VNM_CUDA_TRY(cudaMemcpyAsync(d_job, &hj, sizeof(NMJob), cudaMemcpyHostToDevice, c.stream));
   // the same launch shape as vnm_nm_reorder (a cluster of blocks per job)
-  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, cs));
+  VNM_TRY(launch_rounds(&c, d_job, 1, N, M, P.nseg, (nrows + 15) / 16, cs, c.stream));
   VNM_CUDA_TRY(cudaMemcpyAsync(hs, hj.res, sizeof(int) * 16, cudaMemcpyDeviceToHost, c.stream));
   VNM_CUDA_TRY(cudaStreamSynchronize(c.stream));
   if (hs[5] != 0) return VNM_ERR_INTERNAL;
