@@ -8,11 +8,12 @@ namespace vnm {
 
 // How many of a batch's jobs (entries in descending order) to run on clusters
 // of 4 blocks when the others run on 2.  A job's time goes with its entries
-// (0.135 us each on 2 blocks, R-MAT 2:8) and is about 0.74 of that on 4; the
-// others start in order wherever two SMs come free, and the number with the
+// (0.135 us each on 2 blocks) and is about 0.74 of that on 4, measured on R-MAT
+// at 2:8 and taken for every M; the others start in order wherever two SMs come free, and the number with the
 // earliest end is taken, within half of the SMs and where it gains at least 10
-// %.  (256 R-MAT matrices, 256-8192 rows: the largest job alone took all of
-// the batch's 25.2 ms.)
+// %.  (256 R-MAT matrices, 256-8192 rows: the largest job alone took all of the
+// 24.8 ms that the batch takes with 2 blocks for all; 19.2 ms so, at 2:4 11.9
+// and 8.8.)
 // The GPU waits for the answer, so it takes a small part of the time of sorting
 // the jobs: the starts are simulated for the jobs above a 16th of an even share
 // of the work (what is left fills the SMs evenly), and not at all where the

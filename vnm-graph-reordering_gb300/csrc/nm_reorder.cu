@@ -639,8 +639,12 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
   }
 }
 
-// Slots of the direct table, at most: 65536 rows on 16 blocks, 8192 on 2 (and
-// the run of 16 rows that a range not starting at a multiple of 16 adds).
+// Slots of the direct table, at most: 78 KB, with which clusters of 16 still fit
+// beside the largest segment counts at every M; 69632 rows on 16 blocks, 8704
+// on 2.  Rows with a slot of their own, and hashed: R-MAT 65536 2:8 95.9 and
+// 123.1 ms, 2:4 19.3 and 21.1.  6144 slots would take 70000 rows from 129 to
+// 101 ms at 2:8, but no cluster of 16 holds 98304 rows at 2:8 with them (138
+// instead of 92 ms).
 constexpr int DIRECT_MAX = 4352;
 
 // The block's own runs (up to RUNS_OWN rows).
@@ -2217,11 +2221,12 @@ static vnm_status launch_rounds_t(vnm_ctx* ctx, cudaStream_t st, const NMJob* d_
 
 // Blocks per job for calls with few jobs (one matrix, or its four
 // schedules); batches have their own rule (run_batch).  Measured on GB300 (find_best,
-// four jobs) with 4 / 8 / 16 blocks: R-MAT 2048 2:8 (26 K entries) 6.7 /
-// 6.8 / 7.3 ms, R-MAT 16384 2:4 (228 K entries) 17.1 / 12.9 / 12.4 ms,
-// R-MAT 65536 2:8 (1.8 M entries) 472 / 295 / 209 ms; so 16 (a non-portable
-// cluster size) from 128 K pattern entries on, 8 below.  VNM_NM_CLUSTER
-// (1..16) in the environment overrides the choice.
+// four jobs) with 4 / 8 / 16 blocks: R-MAT 2048 2:8 (21 K entries) 3.96 /
+// 4.00 / 4.15 ms, 8192 2:4 (111 K) 4.76 / 4.21 / 4.05, 8192 2:8 (159 K) 16.3 /
+// 14.2 / 14.6, 16384 2:4 (229 K) 9.9 / 7.2 / 6.5, 65536 2:8 (1.8 M) 306 / 185 /
+// 96 ms; so 16 (a non-portable cluster size) from 128 K pattern entries on,
+// where the two cross, 8 below.  VNM_NM_CLUSTER (1..16) in the environment
+// overrides the choice.
 static int nm_cluster_size(long long np) {
   if (const char* e = getenv("VNM_NM_CLUSTER")) {  // rounded down to a power of two (rows are dealt in 16 groups)
     const int v = atoi(e);
@@ -2454,7 +2459,8 @@ static vnm_status run_matrix(vnm_ctx* ctx, int nrows, int nnz, const int* row, c
 // shifted by its row offset, so one pattern build covers the whole batch;
 // job b sees the columns of its own diagonal block and the rows it reaches
 // are its own (global ids), so the jobs share the row-record array without
-// overlapping.  All jobs run as the blocks of one persistent launch.
+// overlapping.  All jobs run as the blocks of one persistent launch, or of two
+// beside one another (run_batch).
 // ---------------------------------------------------------------------------
 __global__ void k_batch_offset(const int* row, const int* col, const long long* nnz_off, const int* row_off,
                                const int* nrows, int nmat, long long nnz, int* grow, int* gcol, int* err) {
@@ -2575,11 +2581,12 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     return nnz_offset[x + 1] - nnz_offset[x] > nnz_offset[y + 1] - nnz_offset[y];
   });
   // Clusters of 4 or 8 blocks per job where all jobs may still run at once
-  // (pick_cluster halves them if they do not): 12 matrices of 2048-8192 rows
-  // 25.7 -> 16.5 ms, 30 of 1024-8192 rows 26.9 -> 20.6 ms, 12 of 256-512 rows
-  // 2.25 ms either way.  Else of 2 (88 ms with one block per job, 63 ms with
-  // 2, 69 ms with 4, measured on an earlier form of the kernel), but of 4 for
-  // the largest jobs if the batch would end with those alone.
+  // (pick_cluster halves them if they do not): 12 matrices of 2048-8192 rows at
+  // 2:8 11.5 ms, on clusters of 2 17.1; 30 of 1024-8192 rows 16.4 and 22.0.
+  // Else of 2 (256 matrices of 256-8192 rows on 1 / 2 / 4 blocks 54.4 / 24.8 /
+  // 30.1 ms, 100 of 2048 rows 8.2 / 6.7 / 11.9), but of 4 for the largest jobs
+  // if the batch would end with those alone (the 256: 19.2 ms at 2:8, 8.8 at
+  // 2:4 where 2 blocks for all take 11.9).
   std::vector<long long> sizes(nmat);
   for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
   const int cs = nmat * BATCH_CS <= ctx->num_sms ? BATCH_CS : nmat * 4 <= ctx->num_sms ? 4 : 2;

@@ -302,7 +302,7 @@ class Context:
 
     def nm_reorder_batch(self, mats, N, M, sched, nm_maxiter=10, want_newpos=True):
         """Reorder many matrices [(nrows, row, col, val), ...] (or the arrays
-        of pack_batch) in one launch.  Returns (res5 [nmat, 5], list of
+        of pack_batch) in one call, each a job of its own on the GPU.  Returns (res5 [nmat, 5], list of
         newpos arrays or None)."""
         nrows, off, row, col, val = mats if isinstance(mats, tuple) else self.pack_batch(mats)
         nmat = len(nrows)
