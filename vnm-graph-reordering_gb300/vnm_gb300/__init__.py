@@ -398,13 +398,19 @@ class SpmmMatrix:
         the operand's type, enqueued on torch's current stream of X's device
         without waiting.  Raises ValueError for any other X."""
         import torch
-        xtype = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}.get(X.dtype)
-        if xtype is None or not X.is_cuda or X.dim() != 2 or X.shape[0] != self.nrows or X.shape[1] < 1:
+        if X.dtype not in (torch.float32, torch.float16, torch.bfloat16) or not X.is_cuda or X.dim() != 2 \
+                or X.shape[0] != self.nrows or X.shape[1] < 1:
             raise ValueError("X must be a CUDA tensor of float32, float16 or bfloat16 with nrows rows")
-        F, dev = X.shape[1], X.device
-        if X.stride(1) != 1 or X.stride(0) < F:
+        if X.stride(1) != 1 or X.stride(0) < X.shape[1]:
             raise ValueError("the rows of X must be contiguous and not overlap")
+        return self._cast_async(X)
+
+    def _cast_async(self, X):
+        """run_cast_async for an X that the caller has checked."""
+        import torch
+        F, dev = X.shape[1], X.device
         n = (F + 63) // 64 * 64
+        xtype = 2 if X.dtype == torch.float32 else 1 if X.dtype == torch.bfloat16 else 0
         B = torch.empty((self.nrows, n), dtype=torch.bfloat16 if self.dtype == "bf16" else torch.float16, device=dev)
         C = torch.empty((self.nrows, n), dtype=torch.float32, device=dev)
         st = lib().vnm_spmm_run_cast_async(self.ctx.h, self.h, X.data_ptr(), xtype, X.stride(0), F, B.data_ptr(), n,

@@ -76,7 +76,7 @@ class VnmAdjacency:
         ready = X.dtype == self.torch_dtype and X.shape[1] % 64 == 0
         if not ready and X.stride(1) == 1 and X.stride(0) >= X.shape[1] > 0 and X.dtype in (
                 torch.float32, torch.float16, torch.bfloat16):
-            return op.run_cast_async(X)
+            return op._cast_async(X)
         Xp, F = _pad_cols(X.detach().to(self.torch_dtype))
         Y = op.run_async(Xp, stream=torch.cuda.current_stream(X.device))
         return Y[:, :F] if Y.shape[1] != F else Y
