@@ -786,11 +786,12 @@ __device__ __forceinline__ void add4(float4& s, const float4 x) {
 __global__ void __launch_bounds__(FIN_THREADS)
     k_spmm_fin(const int4* __restrict__ multi, const float* __restrict__ P, int ldp, float* C, int ldc) {
   __shared__ float4 red[FIN_THREADS];
-  const int nb = ldc / (4 * FIN_COLS);  // blocks a row (n is a multiple of 64); in x, as y ends at 65535
-  const int4 m = multi[blockIdx.x / nb];
+  const int cb = blockIdx.z * gridDim.y + blockIdx.y;  // column block (n is a multiple of 64: whole blocks)
+  if (cb >= ldc / (4 * FIN_COLS)) return;
+  const int4 m = multi[blockIdx.x];
   constexpr int ng = FIN_THREADS / FIN_COLS;
   const int g = threadIdx.x / FIN_COLS, qi = threadIdx.x % FIN_COLS;
-  const int q = blockIdx.x % nb * FIN_COLS + qi;
+  const int q = cb * FIN_COLS + qi;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4* src = reinterpret_cast<const float4*>(P + (size_t)m.y * ldp) + q;
   const size_t row = ldp / 4, step = (size_t)ng * row;
@@ -1107,14 +1108,14 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_spmm_vnm(const __grid_constan
 // the residual kernel wrote.  Bound by L2 (the parts were just written): one
 // float4 of C a thread, the parts' loads eight in flight.
 __global__ void __launch_bounds__(256)
-    k_spmm_tfin(const int4* __restrict__ split, const float* __restrict__ P, const float* __restrict__ rscale, int R,
-                int n, float* __restrict__ C) {
+    k_spmm_tfin(const int4* __restrict__ split, const float* __restrict__ P, const float* __restrict__ rscale, int R, int n,
+                float* __restrict__ C) {
   ptx::grid_dependency_wait();
-  const int nq = n / 4, nb = SP_TM * nq / 256;  // blocks a tile; in x, as y ends at 65535
-  const int4 m = split[blockIdx.x / nb];
-  const int t = m.x >> 1;
-  const int e = blockIdx.x % nb * blockDim.x + threadIdx.x, rt = e / nq, q = e % nq, row = t * SP_TM + rt;
-  if (row >= R) return;
+  const int4 m = split[blockIdx.x];
+  const int t = m.x >> 1, nq = n / 4;
+  const int e = (blockIdx.z * gridDim.y + blockIdx.y) * blockDim.x + threadIdx.x, rt = e / nq, q = e % nq;
+  const int row = t * SP_TM + rt;
+  if (rt >= SP_TM || row >= R) return;
   {
     const float4* src = reinterpret_cast<const float4*>(P + ((size_t)m.y * SP_TM + rt) * n) + q;
     const size_t step = (size_t)SP_TM * nq;
@@ -1329,6 +1330,12 @@ static vnm_status compress_t(vnm_ctx* ctx, int R, int nnz, const int* d_row, con
   return VNM_OK;
 }
 
+// x by `blocks` blocks, in y and, past what y holds, z (blocks may be a few more).
+static dim3 grid_yz(int x, int blocks) {
+  const int z = (blocks + 65534) / 65535;
+  return dim3((unsigned)x, (unsigned)((blocks + z - 1) / z), (unsigned)z);
+}
+
 // One launch for all column blocks (n256 of 256 columns, n128 of 128, n64 of
 // 64): for the same reason as the residual kernel's, and so that no width
 // waits for another's last tiles.
@@ -1462,7 +1469,7 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
                    P, n);
     }
     if (A->nmulti > 0)
-      VNM_LAUNCH(ctx, k_spmm_fin, (unsigned)A->nmulti * (n / (4 * FIN_COLS)), FIN_THREADS, 0, A->multi, P, n, dC, n);
+      VNM_LAUNCH(ctx, k_spmm_fin, grid_yz(A->nmulti, n / (4 * FIN_COLS)), FIN_THREADS, 0, A->multi, P, n, dC, n);
     return VNM_OK;
   };
   // The operand is read once a column block: n = 192 as 128 + 64 instead of
@@ -1487,7 +1494,7 @@ static vnm_status spmm_enqueue(vnm_ctx* ctx, const vnm_spmm_matrix* A, const voi
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3((unsigned)A->ntsplit * (SP_TM * (n / 4) / 256));
+    cfg.gridDim = grid_yz(A->ntsplit, SP_TM * (n / 4) / 256);
     cfg.blockDim = dim3(256);
     VNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmm_tfin, (const int4*)A->tsplit, (const float*)p.P,
                                     (const float*)A->rscale, A->R, n, dC));
