@@ -1106,9 +1106,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_spmm_vnm(const __grid_constan
 
 // Rows of a split tile: the sum of its parts in order, scaled, added to what
 // the residual kernel wrote.  Bound by L2 (the parts were just written): one
-// float4 of C a thread, the parts' loads eight in flight.
+// float4 of C a thread, the parts' loads eight in flight.  (P is written while
+// this kernel is set up already, so it is not __restrict__: loads of memory that
+// is constant for a kernel's life may be made before the wait.)
 __global__ void __launch_bounds__(256)
-    k_spmm_tfin(const int4* __restrict__ split, const float* __restrict__ P, const float* __restrict__ rscale, int R, int n,
+    k_spmm_tfin(const int4* __restrict__ split, const float* P, const float* __restrict__ rscale, int R, int n,
                 float* __restrict__ C) {
   ptx::grid_dependency_wait();
   const int4 m = split[blockIdx.x];
