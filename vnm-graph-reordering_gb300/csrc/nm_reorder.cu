@@ -640,8 +640,8 @@ __device__ void clear_round_smem(RoundSmem<M>& sm) {
 }
 
 // Slots of the direct table, at most: 78 KB, with which clusters of 16 still fit
-// beside the largest segment counts at every M; 69632 rows on 16 blocks, 8704
-// on 2.  Rows with a slot of their own, and hashed: R-MAT 65536 2:8 95.9 and
+// beside the segment counts of as many rows, at every M (69632 rows on 16
+// blocks, 8704 on 2).  Rows with a slot of their own, and hashed: R-MAT 65536 2:8 95.9 and
 // 123.1 ms, 2:4 19.3 and 21.1.  6144 slots would take 70000 rows from 129 to
 // 101 ms at 2:8, but no cluster of 16 holds 98304 rows at 2:8 with them (138
 // instead of 92 ms).
