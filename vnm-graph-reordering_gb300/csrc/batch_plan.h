@@ -16,7 +16,8 @@ namespace vnm {
 // and 8.8.)
 // The GPU waits for the answer, so it takes a small part of the time of sorting
 // the jobs: the starts are simulated for the jobs above a 16th of an even share
-// of the work (what is left fills the SMs evenly), and not at all where the
+// of the work (what is left fills the SMs evenly), for the numbers that the
+// work itself and the largest jobs leave a chance, and not at all where the
 // largest is below a ninth, as the plain order then ends within 10 % of what
 // any order could (all jobs simulated for each number: 2.9 ms of 76 at 50000
 // matrices of 64 rows).
@@ -25,13 +26,19 @@ inline int wide_jobs(const std::vector<long long>& sizes, int num_sms) {
   if (n < 2 || pairs < 1) return 0;
   double rest = 0;
   for (const long long s : sizes) rest += (double)s;
-  const double share = rest / pairs;
+  double work = rest;  // of the SM pairs, with the jobs so far wide
+  const double share = work / pairs;
   int heads = 0;
   for (; heads < n && 16.0 * (double)sizes[heads] > share; ++heads) rest -= (double)sizes[heads];
   int best = 0;
   double best_end = 0;
   std::vector<double> ends;  // when each pair of SMs comes free: a heap, earliest on top
   for (int k = 0; k < n && 4 * k <= pairs && 9.0 * (double)sizes[k > 0 ? k - 1 : 0] > share; ++k) {
+    const double limit = best_end * (best == 0 ? 0.9 : 1.0);
+    if (k > 0) {
+      work += (2 * 0.74 - 1) * (double)sizes[k - 1];
+      if (std::max(work / pairs, (double)sizes[k]) >= limit) continue;  // no end is earlier
+    }
     ends.assign(pairs, 0.0);
     double end = 0, busy = rest;
     for (int q = 0; q < k; ++q) {
@@ -49,7 +56,7 @@ inline int wide_jobs(const std::vector<long long>& sizes, int num_sms) {
       std::push_heap(ends.begin(), ends.end(), std::greater<double>());
     }
     end = std::max(end, busy / pairs);
-    if (k == 0 || end < best_end * (best == 0 ? 0.9 : 1.0)) {
+    if (k == 0 || end < limit) {
       best = k;
       best_end = end;
     }

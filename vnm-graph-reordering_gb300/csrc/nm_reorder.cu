@@ -2571,7 +2571,12 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
     VNM_LAUNCH(ctx, k_batch_offset, grid_for(ctx, n), 256, 0, d_row, d_col, d_noff, d_roff, d_nrows, nmat,
                (long long)n, grow, gcol, err);
   VNM_CUDA_TRY(cudaMemcpyAsync(ctx->h_pinned, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  // (on the host, while the GPU checks the entries)
+  VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (ctx->h_pinned[0] & 2) return VNM_ERR_RANGE;
+  if (ctx->h_pinned[0] & 1) return VNM_ERR_UNSORTED;
+  Pattern P;
+  VNM_TRY(build_pattern(ctx, R, n, grow, gcol, d_val, N, M, P, ctx->h_pinned));
+  // (on the host, while the GPU builds the pattern)
   // The rounds run in the order of the matrices' entries, most first: the
   // batch lasts as long as its largest jobs, which must not start late (256
   // R-MAT matrices 256-8192 rows at 2:8: 36.8 -> 27.1 ms).
@@ -2591,11 +2596,6 @@ static vnm_status run_batch(vnm_ctx* ctx, int nmat, const int* nrows, const int6
   for (int q = 0; q < nmat; ++q) sizes[q] = nnz_offset[by_size[q] + 1] - nnz_offset[by_size[q]];
   const int cs = nmat * BATCH_CS <= ctx->num_sms ? BATCH_CS : nmat * 4 <= ctx->num_sms ? 4 : 2;
   const int wide = cs == 2 ? wide_jobs(sizes, ctx->num_sms) : 0;
-  VNM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  if (ctx->h_pinned[0] & 2) return VNM_ERR_RANGE;
-  if (ctx->h_pinned[0] & 1) return VNM_ERR_UNSORTED;
-  Pattern P;
-  VNM_TRY(build_pattern(ctx, R, n, grow, gcol, d_val, N, M, P, ctx->h_pinned));
   // per-job state, one allocation per field for the whole batch
   int2* runs = arena_take<int2>(ctx, (size_t)BATCH_CS * (R > 0 ? R : 1));
   int* orig = arena_take<int>(ctx, R > 0 ? R : 1);
